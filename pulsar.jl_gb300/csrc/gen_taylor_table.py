@@ -8,7 +8,7 @@ scaling-and-squaring drivers pick, per slice, the degree m and squarings s
 with ||A||_1 / 2^s <= theta_m that minimise the matrix products: degrees
 {4,8,12,16,20} (3 + m/4 - 1 products, + s) in FP64 and FP32, and every degree
 m = q L with block size q in {2, 3, 4} in df (costed by the products it
-executes).  This is the standard
+executes), and the even degrees 4..20 (q = 2) in block fixed point.  This is the standard
 forward-error bound of a truncated exponential series; the constants below are
 computed here, not taken from any library.
 
@@ -16,6 +16,7 @@ Run:  python gen_taylor_table.py > taylor_table.h
 """
 import math
 import sys
+from fractions import Fraction
 
 DEGREES = (4, 8, 12, 16, 20)
 
@@ -55,6 +56,20 @@ def main(out=sys.stdout):
     # block size q in {2, 3, 4} (degrees m = q L)
     vals = ", ".join(f"{theta_for(m, udf):.17g}" for m in range(1, max(DEGREES) + 1))
     print(f"#define PGX_THETADF_ALL_INIT {{{vals}}}  /* index m - 1 */", file=out)
+    # block fixed point: log2 of the FP64 thresholds of the degrees 4, 6, ..., 20,
+    # and 1/k! = mant 2^(exp - 61)
+    logs = [math.log2(theta_for(m, u64)) for m in range(4, max(DEGREES) + 1, 2)]
+    print(f"#define PGX_N_FXDEGREES {len(logs)}", file=out)
+    print(f"#define PGX_LOG2_THETA64_EVEN_INIT {{{', '.join(f'{x:.9g}f' for x in logs)}}}", file=out)
+    coefs = []
+    for k in range(max(DEGREES) + 1):
+        e = 1 - (math.factorial(k) - 1).bit_length() if k > 1 else 1
+        if Fraction(2) ** (61 - e) / math.factorial(k) >= 2 ** 61:
+            e += 1
+        mant = round(Fraction(2) ** (61 - e) / math.factorial(k))
+        assert 2 ** 60 <= mant < 2 ** 61
+        coefs.append(f"{{{mant}ull, {e}}}")
+    print(f"#define PGX_INVFACT_FX_INIT {{{', '.join(coefs)}}}", file=out)
     inv = ", ".join(f"{1.0 / math.factorial(k):.17g}" for k in range(max(DEGREES) + 1))
     print(f"#define PGX_N_INVFACT {max(DEGREES) + 1}", file=out)
     print(f"#define PGX_INVFACT_INIT {{{inv}}}", file=out)

@@ -730,6 +730,7 @@ static cudaError_t do_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo&
   return cudaGetLastError();
 }
 cudaError_t launch_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  if (fx_expm_applies(p)) return launch_fx_expm(p, w, li);
   PGX_DISPATCH(p.Dp, return do_expm<D_>(p, w, li));
   return cudaSuccess;
 }
