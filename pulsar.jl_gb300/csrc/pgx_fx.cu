@@ -16,70 +16,64 @@ constexpr int kNever = 1 << 20;     // an exponent no finite entry reaches
 
 // The constant matrices of the generator, A_mk = c sum_j alpha_j K_j with
 // alpha = dt_k {1, scale u_1k, ..., tau_k} and K = {drift_m + off_m O, C_1,
-// ..., R_m}, as 64-bit integers K = (b1 2^32 + b0) 2^(E - 58), b0 balanced, in
+// ..., R_m}, as 64-bit integers K = (b1 2^32 + b0) 2^(E - 60), b0 balanced, in
 // the lanes' own order: 3 integer multiply-adds per real value and term in
 // place of one FP64 FMA, which is 18 times slower.
-template <int D> struct Terms {
-  int4* k;        // [n][NV / 2][32] (b0, b1, b0', b1')
+template <int D, int W> struct Terms {
+  using G = Geo<D, W>;
+  int4* k;        // [n][W][NV / 2][32] (b0, b1, b0', b1')
   int* e;         // [n] exponents; kNever: not finite
   int n;
-  __device__ __forceinline__ static size_t bytes(int n) { return (size_t)n * Geo<D>::INTS + (kMaxTerms + 8) * sizeof(int); }
+  __host__ __device__ __forceinline__ static size_t bytes(int n) { return (size_t)n * G::INTS + (kMaxTerms + 8) * sizeof(int); }
+  __device__ __forceinline__ int4* at(const Tm<D, W>& tm, int j) const {
+    return k + ((size_t)j * W + tm.w) * (G::NV / 2) * 32 + tm.lane;
+  }
 };
 
-// One warp converts a matrix (doubles in the lanes' order) into term j.
-template <int D>
-__device__ __forceinline__ void put_term(const Terms<D>& T, int j, int lane, const double (&x)[Geo<D>::NV]) {
-  constexpr int NV = Geo<D>::NV;
-  const int EX = max_exponent<NV>(x);
-  int4* dst = T.k + (size_t)j * (NV / 2) * 32;
+// A team converts a matrix (doubles in the lanes' order) into term j.
+template <int D, int W>
+__device__ __forceinline__ void put_term(const Terms<D, W>& T, int j, const Tm<D, W>& tm, const double (&x)[Geo<D, W>::NV]) {
+  constexpr int NV = Geo<D, W>::NV;
+  const int EX = max_exponent<D, W>(tm, x);
+  int4* dst = T.at(tm, j);
 #pragma unroll
   for (int v = 0; v < NV; v += 2) {
-    const long long a = from_double(x[v], EX, 4), b = from_double(x[v + 1], EX, 4);
-    dst[(v / 2) * 32 + lane] = make_int4((int)a, (int)((a + 0x80000000ll) >> 32), (int)b, (int)((b + 0x80000000ll) >> 32));
+    const long long a = from_double(x[v], EX, 6), b = from_double(x[v + 1], EX, 6);
+    dst[(v / 2) * 32] = make_int4((int)a, (int)((a + 0x80000000ll) >> 32), (int)b, (int)((b + 0x80000000ll) >> 32));
   }
-  if (lane == 0) T.e[j] = EX == 0x7ff ? kNever : EX - 1021;
-}
-
-template <int D>
-__device__ __forceinline__ void load_mat(const double2* A, int lane, double (&x)[Geo<D>::NV]) {
-  using G = Geo<D>;
-#pragma unroll
-  for (int q = 0; q < G::NQ; ++q)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const double2 a = A[G::row(lane, q) + D * G::col(lane, q, h)];
-      x[2 * q + h] = a.x;
-      x[G::NV / 2 + 2 * q + h] = a.y;
-    }
+  if (tm.lane == 0 && tm.w == 0) T.e[j] = EX == 0x7ff ? kNever : EX - 1021;
+  tm.sync();
 }
 
 // Member m's own terms: drift + offset, and its ramp operator.
-template <int D>
-__device__ __forceinline__ void put_member_terms(const Terms<D>& T, const ProbDev& p, int m, int lane) {
-  constexpr int NV = Geo<D>::NV;
+template <int D, int W>
+__device__ __forceinline__ void put_member_terms(const Terms<D, W>& T, const ProbDev& p, int m, const Tm<D, W>& tm) {
+  constexpr int NV = Geo<D, W>::NV;
   double x[NV], o[NV];
-  load_mat<D>(p.drifts + (size_t)p.m_drift[m] * D * D, lane, x);
-  load_mat<D>(p.offset_op, lane, o);
+  load_mat<D, W>(tm, p.drifts + (size_t)p.m_drift[m] * D * D, x);
+  load_mat<D, W>(tm, p.offset_op, o);
   const double off = p.m_offset[m];
 #pragma unroll
   for (int v = 0; v < NV; ++v) x[v] = fma(off, o[v], x[v]);
-  put_term<D>(T, 0, lane, x);
+  put_term<D, W>(T, 0, tm, x);
   if (p.n_ramp) {
     const int ro = p.m_ramp[m];
-    if (ro >= 0) load_mat<D>(p.ramp_ops + (size_t)ro * D * D, lane, x);
+    if (ro >= 0) load_mat<D, W>(tm, p.ramp_ops + (size_t)ro * D * D, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v)
       if (ro < 0) x[v] = 0.0;
-    put_term<D>(T, p.n_c + 1, lane, x);
+    put_term<D, W>(T, p.n_c + 1, tm, x);
   }
 }
 
-// A = c sum_j alpha_j K_j, 60 fractional bits in the frame returned; a frame
-// above kNever / 2 means a term is not finite.
-template <int D>
-__device__ __forceinline__ int assemble(const Terms<D>& T, const ProbDev& p, const double* u, int m, int k, int lane,
-                                        long long (&A)[Geo<D>::NV]) {
-  constexpr int NV = Geo<D>::NV;
+// A = c sum_j alpha_j K_j, 58 fractional bits in the frame returned; a frame
+// above kNever / 2 means a term is not finite.  |b1| <= 2^27, |a0| <= 2^31 and
+// sum |a1| <= 2^30 keep 24 terms' mixed products inside 63 bits.
+template <int D, int W>
+__device__ __forceinline__ int assemble(const Terms<D, W>& T, const ProbDev& p, const double* u, int m, int k,
+                                        const Tm<D, W>& tm, long long (&A)[Geo<D, W>::NV]) {
+  constexpr int NV = Geo<D, W>::NV;
+  const int lane = tm.lane;
   double al = 0.0;
   if (lane < T.n) {
     const double dt = p.dt[k];
@@ -91,20 +85,20 @@ __device__ __forceinline__ int assemble(const Terms<D>& T, const ProbDev& p, con
   if (ex == 0x7ff) te = kNever;
   else if (ex > 0) te = ex - 1022 + T.e[lane];  // ex > 0 only below T.n
   const int EA = __reduce_max_sync(0xffffffffu, te) + (32 - __clz(T.n - 1));
-  // |alpha_j| 2^(E_j - EA) <= 1 / n in 61 fractional bits
-  const int s = te == -kNever ? -64 : te - EA + 8;
+  // |alpha_j| 2^(E_j - EA) <= 1 / n in 62 fractional bits
+  const int s = te == -kNever ? -64 : te - EA + 9;
   unsigned long long am = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | (uint32_t)__double2loint(al);
-  am = s >= 0 ? am << min(s, 8) : shr64(am, min(-s, 64));
+  am = s >= 0 ? am << min(s, 9) : shr64(am, min(-s, 64));
   const long long sg = (long long)(int)hi >> 31;
   const long long a = ((long long)am ^ sg) - sg;
   const int my0 = (int)a, my1 = (int)((a + 0x80000000ll) >> 32);
   long long main[NV], mid[NV];
 #pragma unroll
   for (int v = 0; v < NV; ++v) main[v] = mid[v] = 0;
-  const int4* kp = T.k + lane;
 #pragma unroll 1
   for (int j = 0; j < T.n; ++j) {
     const int a0 = __shfl_sync(0xffffffffu, my0, j), a1 = __shfl_sync(0xffffffffu, my1, j);
+    const int4* kp = T.at(tm, j);
 #pragma unroll
     for (int v = 0; v < NV; v += 2) {
       const int4 b = kp[(v / 2) * 32];
@@ -115,11 +109,10 @@ __device__ __forceinline__ int assemble(const Terms<D>& T, const ProbDev& p, con
       mid[v + 1] += (long long)b.w * a0;
       mid[v + 1] += (long long)b.z * a1;
     }
-    kp += (NV / 2) * 32;
   }
   // times c: -i for a Hermitian generator, 1 for a Liouvillian
 #pragma unroll
-  for (int v = 0; v < NV; ++v) main[v] = (main[v] << 5) + (mid[v] >> 27);
+  for (int v = 0; v < NV; ++v) main[v] += (long long)(int)(mid[v] >> 32);
 #pragma unroll
   for (int v = 0; v < NV / 2; ++v) {
     A[v] = p.gen == GEN_HERM ? main[NV / 2 + v] : main[v];
@@ -128,27 +121,28 @@ __device__ __forceinline__ int assemble(const Terms<D>& T, const ProbDev& p, con
   return EA;
 }
 
-// log2 of a bound of ||A||_1 (60 fractional bits in frame EA).
-template <int D> __device__ __forceinline__ float log2_norm1(const long long (&A)[Geo<D>::NV], int EA) {
-  constexpr int NQ = Geo<D>::NQ, NV = Geo<D>::NV;
+// log2 of a bound of ||A||_1 (58 fractional bits in frame EA), D <= 16.
+template <int D, int W> __device__ __forceinline__ float log2_norm1(const Tm<D, W>& tm, const long long (&A)[Geo<D, W>::NV], int EA) {
+  using G = Geo<D, W>;
+  static_assert(G::RT == 1, "a column's rows belong to one warp");
   float best = 0.f;
 #pragma unroll
-  for (int cb = 0; cb < (NQ + 1) / 2; ++cb)
+  for (int nt = 0; nt < G::NTW; ++nt)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       float s = 0.f;
 #pragma unroll
-      for (int rb = 0; rb < (NQ + 1) / 2; ++rb) {
-        const int v = 2 * (2 * cb + rb) + h;
-        const float x = (float)(int)(A[v] >> 32), y = (float)(int)(A[NV / 2 + v] >> 32);
+      for (int i = 0; i < G::NI; ++i) {
+        const int b = 2 * (nt * G::NI + i) + h;
+        const float x = (float)(int)(A[b] >> 32), y = (float)(int)(A[G::NV / 2 + b] >> 32);
         s += __fsqrt_rn(fmaf(x, x, y * y));
       }
 #pragma unroll
       for (int o = 4; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       best = fmaxf(best, s);
     }
-  best = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(best)));
-  return __log2f(fmaf(best, 1.00001f, 2.f * D)) + (float)(EA - 28) + 1e-5f;
+  best = __uint_as_float(tm.max(__float_as_uint(best), 1));
+  return __log2f(fmaf(best, 1.00001f, 2.f * D)) + (float)(EA - 26) + 1e-5f;
 }
 
 // Degree 2 L and squarings s with ||A||_1 / 2^s <= theta_2L that minimise the
@@ -165,36 +159,40 @@ __device__ __forceinline__ void choose_degree2(float l2, int lane, int& L, int& 
 }
 
 template <int D> struct ExpmCfg {
-  static constexpr int WARP_BYTES = 2 * Geo<D>::PLANES + Geo<D>::INTS;  // planes of X, of Y; B
-  static constexpr int MAX_WARPS = D >= 16 ? 10 : 12;
+  static constexpr int W = D >= 16 ? 2 : 1;             // warps of a slice
+  static constexpr int TEAMS = D >= 16 ? 10 : 12;       // slices in flight per CTA, at most
+  static constexpr int TEAM_BYTES = 2 * Geo<D, W>::PLANES + Geo<D, W>::INTS + 64;  // planes of X, of Y; B; maxima
 };
 
-// U_mk = exp(A_mk), one warp per slice: T_2L(A / 2^s) in the q = 2
+// U_mk = exp(A_mk), one team per slice: T_2L(A / 2^s) in the q = 2
 // Paterson-Stockmeyer form (X = B^2, Horner in X), then s squarings.  A CTA
 // walks runs of `run` slices of one member.
 //
-// Bound: the tensor pipe (about 64 digit pairs of 16 SM cycles at D = 16) and,
-// as much again, the integer work around it: digits of each factor, joining
-// the levels, rescaling.  A unit's planes and integers take 18 KB of shared
-// memory, so an SM holds ten warps; the FP64 form kept the FP64 pipe busy for
-// 41,000 cycles a slice.
+// Bound: instruction issue (digits of each factor, joining the levels,
+// rescaling), then the tensor pipe (about 64 digit pairs of 16 SM cycles at
+// D = 16).  A slice's planes and integers take 18 KB of shared memory, so an SM
+// holds ten; two warps share one, each with half the columns.
 template <int D>
-__global__ void __launch_bounds__(32 * ExpmCfg<D>::MAX_WARPS) k_fx_expm(ProbDev p, WorkDev w, int run) {
-  using G = Geo<D>;
+__global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_expm(ProbDev p, WorkDev w, int run) {
+  using C = ExpmCfg<D>;
+  constexpr int W = C::W;
+  using G = Geo<D, W>;
   constexpr int NV = G::NV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  Terms<D> T;
+  const int team = threadIdx.x / (32 * W), nt = blockDim.x / (32 * W);
+  Terms<D, W> T;
   T.n = p.n_c + 1 + (p.n_ramp ? 1 : 0);
   T.k = reinterpret_cast<int4*>(smem_raw);
   T.e = reinterpret_cast<int*>(smem_raw + (size_t)T.n * G::INTS);
-  unsigned char* mine = smem_raw + Terms<D>::bytes(T.n) + (size_t)wid * ExpmCfg<D>::WARP_BYTES;
+  unsigned char* mine = smem_raw + Terms<D, W>::bytes(T.n) + (size_t)team * C::TEAM_BYTES;
   const uint32_t px = smem_u32(mine), py = px + G::PLANES;
-  longlong2* Bs = reinterpret_cast<longlong2*>(mine + 2 * G::PLANES);
-  for (int j = wid; j < p.n_c; j += nw) {
+  const Tm<D, W> tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
+                    reinterpret_cast<uint32_t*>(mine + 2 * G::PLANES + G::INTS)};
+  longlong2* Bs = tm.mine(reinterpret_cast<longlong2*>(mine + 2 * G::PLANES));
+  for (int j = team; j < p.n_c; j += nt) {
     double x[NV];
-    load_mat<D>(p.ctrls + (size_t)j * D * D, lane, x);
-    put_term<D>(T, j + 1, lane, x);
+    load_mat<D, W>(tm, p.ctrls + (size_t)j * D * D, x);
+    put_term<D, W>(T, j + 1, tm, x);
   }
   const int runs = (p.n_t + run - 1) / run;
   int cur = -1;
@@ -202,76 +200,81 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::MAX_WARPS) k_fx_expm(ProbDev 
     const int m = (int)(c / runs), k0 = (int)(c % runs) * run;
     if (m != cur) {
       __syncthreads();
-      if (wid == 0) put_member_terms<D>(T, p, m, lane);
+      if (team == 0) put_member_terms<D, W>(T, p, m, tm);
       __syncthreads();
       cur = m;
     }
     const int k1 = min(p.n_t, k0 + run);
 #pragma unroll 1
-    for (int k = k0 + wid; k < k1; k += nw) {
+    for (int k = k0 + team; k < k1; k += nt) {
       long long r[NV];
-      const int EA = assemble<D>(T, p, w.u, m, k, lane, r);
-      const float l2 = log2_norm1<D>(r, EA);
+      const int EA = assemble<D, W>(T, p, w.u, m, k, tm, r);
+      const float l2 = log2_norm1<D, W>(tm, r, EA);
       int L, s;
-      choose_degree2(l2, lane, L, s);
+      choose_degree2(l2, tm.lane, L, s);
       double2* out = w.U + ((size_t)m * p.n_t + k) * D * D;
       int ex;  // U = r 2^ex
       if (EA > kNever / 2 || s > 60) {
-#pragma unroll
-        for (int q = 0; q < G::NQ; ++q)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const double nan = __longlong_as_double(0x7ff8000000000000ll);
-            out[G::row(lane, q) + D * G::col(lane, q, h)] = make_double2(nan, nan);
-          }
+        store_nan<D, W>(tm, out);
+        tm.sync();  // the maxima are read
         continue;
       }
-      const int lx = min(0, 2 * (int)ceilf(l2 - (float)s));  // log2 of a bound of ||X||
-      const int EB = normalize<NV>(r, EA - 4 - s);
-      __syncwarp();
-      put_ints<NV>(Bs, lane, r);
-      store_planes<D>(lane, py, r, kSlices);
-      __syncwarp();
-      mul<D>(lane, py, py, levels(kBits2, 2 * EB), r);
-      const int EX = normalize<NV>(r, 2 * EB);
-      store_planes<D>(lane, px, r, kSlices);
-      // Y = c_2L X + c_{2L-1} B + c_{2L-2} I
-      int fr = max(max(EX + c_coef[2 * L].exp, EB + c_coef[2 * L - 1].exp), c_coef[2 * L - 2].exp) + 1;
-      const Scaled sx(c_coef[2 * L], EX, fr);
-#pragma unroll
-      for (int v = 0; v < NV; ++v) r[v] = sx(r[v]);
-      add_scaled<NV>(r, Bs, lane, EB, c_coef[2 * L - 1], fr);
-      add_diag<D>(r, lane, c_coef[2 * L - 2], fr);
-      int EY = normalize<NV>(r, fr - 4);
+      // bounds: |X| <= nu^2 (nu = the scaled norm), and |Y_i| <= c_2i e^nu, so
+      // Y_i keeps the fixed frame c_2i.exp + g
+      const float nu2 = l2 - (float)s;
+      const int lx = min(0, 2 * (int)ceilf(nu2));
+      const int g = nu2 <= -1.33f ? 1 : 3;  // e^nu <= 0.75 2^g, nu <= 0.397 or 1.51
+      const int EB = normalize<D, W>(tm, r, EA - 2 - s);
+      int EX = 0, EY = EB, n = kSlices, F = 60;
+      uint32_t pa = py;
+      // step 0: X = B B; L - 1 Horner steps Y <- X Y + c_{2i+1} B + c_2i I,
+      // whose error later meets X^i; s squarings.  One product in the loop
+      // body keeps the kernel inside the instruction cache.
 #pragma unroll 1
-      for (int i = L - 2; i >= 0; --i) {  // Y <- X Y + c_{2i+1} B + c_2i I, whose error later meets X^i
-        const int n = levels(kBits2, EX + EY + i * lx);
-        __syncwarp();
-        store_planes<D>(lane, py, r, n);
-        __syncwarp();
-        mul<D>(lane, px, py, n, r);
-        fr = max(max(EX + EY + 5, EB + c_coef[2 * i + 1].exp), c_coef[2 * i].exp) + 1;
-        to_frame<NV>(r, EX + EY, fr);
-        add_scaled<NV>(r, Bs, lane, EB, c_coef[2 * i + 1], fr);
-        add_diag<D>(r, lane, c_coef[2 * i], fr);
-        if (i > 0 || s > 0) EY = normalize<NV>(r, fr - 4);
-      }
-      ex = fr - 60;
-#pragma unroll 1
-      for (int q = 0; q < s; ++q) {
-        __syncwarp();
-        store_planes<D>(lane, py, r, kSlices);
-        __syncwarp();
-        mul<D>(lane, py, py, levels(kBits2, 2 * EY), r);
-        ex = 2 * EY - kFrac;
-        if (q + 1 < s) EY = normalize<NV>(r, 2 * EY);
-      }
+      for (int st = 0; st < L + s; ++st) {
+        const int i = L - 1 - st;
+        if (st == 0) n = levels(kBits2, 2 * EB);
+        else if (st < L) n = levels(kBits2, EX + EY + i * lx);
+        else n = levels(kBits2, 2 * EY);
+        tm.sync();
+        if (st == 0) {
+          long long x6[NV];
 #pragma unroll
-      for (int q = 0; q < G::NQ; ++q)
+          for (int v = 0; v < NV; ++v) x6[v] = r[v] << 6;
+          put_ints<NV>(Bs, x6);
+        }
+        store_planes<D, W>(tm, py, r, n);
+        tm.sync();
+        mul<D, W>(tm, pa, py, n, r);
+        if (st < L) {
+          const int fr = c_coef[2 * i].exp + g;
+          if (st == 0) {
+            // Y = c_2L X + c_{2L-1} B + c_{2L-2} I
+            EX = normalize<D, W>(tm, r, 2 * EB);
+            store_planes<D, W>(tm, px, r, kSlices);
+            pa = px;
+            F = kFrac;
+            const Scaled sx(c_coef[2 * L], EX, fr, F);
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-          out[G::row(lane, q) + D * G::col(lane, q, h)] =
-              make_double2(to_double(r[2 * q + h], ex), to_double(r[NV / 2 + 2 * q + h], ex));
+            for (int v = 0; v < NV; ++v) r[v] = sx(r[v] << 6, 0);
+          } else {
+            F = i > 0 ? kFrac : 60;
+            to_frame<NV>(r, EX + EY, fr, F);
+          }
+          add_scaled<NV>(r, Bs, Scaled(c_coef[2 * i + 1], EB, fr, F));
+          add_diag<D, W>(tm, r, c_coef[2 * i], fr, F);
+          EY = fr;
+          if (i == 0) {
+            ex = fr - 60;
+            if (s > 0) EY = normalize<D, W>(tm, r, fr - 4);
+            pa = py;
+          }
+        } else {
+          ex = 2 * EY - kFrac;
+          if (st + 1 < L + s) EY = normalize<D, W>(tm, r, 2 * EY);
+        }
+      }
+      store_mat<D, W>(tm, out, r, ex);
     }
   }
 }
@@ -279,25 +282,26 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::MAX_WARPS) k_fx_expm(ProbDev 
 constexpr size_t kSmemMax = 232448;  // dynamic shared memory of a CTA
 
 template <int D> static cudaError_t do_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  using C = ExpmCfg<D>;
   const int n = p.n_c + 1 + (p.n_ramp ? 1 : 0);
-  const size_t consts = (size_t)n * Geo<D>::INTS + (kMaxTerms + 8) * sizeof(int);
-  const int fit = (int)((kSmemMax - consts) / ExpmCfg<D>::WARP_BYTES);
-  const int nw = fit < ExpmCfg<D>::MAX_WARPS ? fit : ExpmCfg<D>::MAX_WARPS;
-  const size_t smem = consts + (size_t)nw * ExpmCfg<D>::WARP_BYTES;
+  const size_t consts = Terms<D, C::W>::bytes(n);
+  const int fit = (int)((kSmemMax - consts) / C::TEAM_BYTES);
+  const int nt = fit < C::TEAMS ? fit : C::TEAMS, threads = 32 * C::W * nt;
+  const size_t smem = consts + (size_t)nt * C::TEAM_BYTES;
   set_smem_once((const void*)k_fx_expm<D>, smem);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fx_expm<D>, 32 * nw, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fx_expm<D>, threads, smem);
   if (per_sm < 1) per_sm = 1;
   // Runs long enough to amortise the member's own terms, short enough that
   // every CTA gets several.
   const long items = (long)p.n_members * p.n_t, ctas = (long)li.num_sms * per_sm;
-  long rounds = items / (ctas * nw * 4);
+  long rounds = items / (ctas * nt * 4);
   if (rounds < 1) rounds = 1;
   if (rounds > 8) rounds = 8;
-  const int run = (int)rounds * nw;
+  const int run = (int)rounds * nt;
   long grid = (long)p.n_members * ((p.n_t + run - 1) / run);
   if (grid > ctas) grid = ctas;
-  k_fx_expm<D><<<(int)grid, 32 * nw, smem, li.stream>>>(p, w, run);
+  k_fx_expm<D><<<(int)grid, threads, smem, li.stream>>>(p, w, run);
   ++*li.launches;
   return cudaGetLastError();
 }

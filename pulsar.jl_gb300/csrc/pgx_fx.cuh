@@ -34,36 +34,73 @@ constexpr int kFrac = 56;      // fractional bits of a normalised matrix
 constexpr int kSlices = 7;     // 8-bit digits of a factor
 constexpr int kMaxLevels = 8;  // levels 0..7 of digit pairs
 
-// One warp owns one D x D matrix.  Lane (g, t) = (lane / 4, lane % 4) holds,
-// of each real plane, the 8 x 8 blocks q: row g + 8 (q & 1), columns
-// 2 t + {0, 1} + 8 (q >> 1) -- the accumulator and left-factor fragments of
-// m16n8k16.  Value index v = part * NV / 2 + 2 q + h.
-template <int D> struct Geo {
-  static constexpr int NQ = D >= 16 ? 4 : 1;         // 8 x 8 blocks per plane
-  static constexpr int NV = 4 * NQ;                  // real values of a lane
-  static constexpr int PLANE = NQ * 128;             // bytes of one digit plane
-  static constexpr int PLANES = kSlices * 2 * PLANE; // digit planes of a matrix
-  static constexpr int INTS = NV * 32 * 8;           // 64-bit values of a matrix
-  __device__ __forceinline__ static int row(int lane, int q) { return (lane >> 2) + 8 * (q & 1); }
-  __device__ __forceinline__ static int col(int lane, int q, int h) { return 2 * (lane & 3) + h + 8 * (q >> 1); }
+// A team of W warps owns one D x D matrix; a warp owns RT-th rows x NTW 8-column
+// tiles.  Lane (g, t) = (lane / 4, lane % 4) holds, of each real plane, the
+// accumulator fragments of m16n8k16: rows 16 rt + g + 8 i, columns 8 (nt of the
+// warp) + 2 t + {0, 1}.  Value index v = part NV / 2 + 4 nt + 2 i + h.  D = 8
+// (W = 1) is one MMA with the real and imaginary part stacked in its 16 rows.
+//
+// A digit plane is 8 x 8 blocks of FP16, block (rb, cb) at (cb D / 8 + rb) 128
+// bytes, rows of 16 bytes: every ldmatrix reads, and every lane-private store
+// writes, whole conflict-free 128-byte lines.
+template <int D, int W> struct Geo {
+  static constexpr int RT = D >= 16 ? D / 16 : 1;      // 16-row tiles
+  static constexpr int CG = W / RT;                    // column groups
+  static constexpr int NTW = D / 8 / CG;               // 8-column tiles of a warp
+  static constexpr int NI = D >= 16 ? 2 : 1;           // 8-row blocks of a warp's tile
+  static constexpr int NV = 4 * NTW * NI;              // real values of a lane
+  static constexpr int KT = RT;                        // 16-deep steps of a product
+  static constexpr int PLANE = D * D * 2;              // bytes of one digit plane
+  static constexpr int PLANES = kSlices * 2 * PLANE;   // digit planes of a matrix
+  static constexpr int INTS = 2 * D * D * 8;           // 64-bit values of a matrix
+  static_assert(NV * 32 * W == 2 * D * D, "a team covers the matrix");
+};
+
+template <int D, int W> struct Tm {
+  using G = Geo<D, W>;
+  int lane, w, bar;     // bar: the team's hardware barrier (W > 1)
+  uint32_t* red;        // 3 W words of shared memory (W > 1)
+  __device__ __forceinline__ int rt() const { return W == 1 ? 0 : w % G::RT; }
+  __device__ __forceinline__ int nt0() const { return W == 1 ? 0 : w / G::RT * G::NTW; }
+  // coordinates of the lane's values (nt, i, h)
+  __device__ __forceinline__ int row(int i) const { return 16 * rt() + (lane >> 2) + 8 * i; }
+  __device__ __forceinline__ int col(int nt, int h) const { return 8 * (nt0() + nt) + 2 * (lane & 3) + h; }
+  __device__ __forceinline__ void sync() const {
+    if constexpr (W == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(32 * W) : "memory");
+  }
+  // largest x of the team's lanes; between two calls with one slot the team
+  // has to sync
+  __device__ __forceinline__ uint32_t max(uint32_t x, int slot) const {
+    x = __reduce_max_sync(0xffffffffu, x);
+    if constexpr (W > 1) {
+      volatile uint32_t* r = red + slot * W;
+      if (lane == 0) r[w] = x;
+      sync();
+#pragma unroll
+      for (int i = 0; i < W; ++i) x = ::max(x, r[i]);
+    }
+    return x;
+  }
+  __device__ __forceinline__ longlong2* mine(longlong2* s) const { return s + (size_t)w * (G::NV / 2) * 32 + lane; }
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
+__device__ __forceinline__ void ldsm4(uint32_t* r, uint32_t a) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t a) {
+__device__ __forceinline__ void ldsm4t(uint32_t* r, uint32_t a) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void ldsm2(uint32_t& r0, uint32_t& r1, uint32_t a) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(a) : "memory");
+__device__ __forceinline__ void ldsm2(uint32_t* r, uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void ldsm2t(uint32_t& r0, uint32_t& r1, uint32_t a) {
+__device__ __forceinline__ void ldsm2t(uint32_t* r, uint32_t a) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
-               : "=r"(r0), "=r"(r1) : "r"(a) : "memory");
+               : "=r"(r[0]), "=r"(r[1]) : "r"(a) : "memory");
 }
 __device__ __forceinline__ void mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                     uint32_t b1) {
@@ -72,91 +109,154 @@ __device__ __forceinline__ void mma(float* c, uint32_t a0, uint32_t a1, uint32_t
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// One digit (re, im) of a factor: the left or the right operand's fragments.
-template <int D> struct Frag {
-  uint32_t re[Geo<D>::NQ], im[Geo<D>::NQ];
-  __device__ __forceinline__ void left(uint32_t base, int s, int lane) {
+// One digit of the left factor: the warp's rows, columns 16 kt ..
+template <int D, int W> struct Left {
+  using G = Geo<D, W>;
+  uint32_t f[D >= 16 ? 8 : 2];  // re, im
+  // the lane's row address of digit 0, step 0
+  __device__ __forceinline__ static uint32_t at(const Tm<D, W>& tm, uint32_t planes) {
+    const int l = tm.lane;
+    if constexpr (D >= 16)
+      return planes + ((l >> 4) * (D / 8) + 2 * tm.rt() + ((l >> 3) & 1)) * 128 + (l & 7) * 16;
+    else
+      return planes + ((l >> 3) & 1) * G::PLANE + (l & 7) * 16;
+  }
+  __device__ __forceinline__ void load(uint32_t a) {
     if constexpr (D >= 16) {
-      ldsm4(re, base + (2 * s) * Geo<D>::PLANE + lane * 16);
-      ldsm4(im, base + (2 * s + 1) * Geo<D>::PLANE + lane * 16);
+      ldsm4(f, a);
+      ldsm4(f + 4, a + G::PLANE);
     } else {
-      ldsm2(re[0], im[0], base + 2 * s * Geo<D>::PLANE + (lane & 15) * 16);
+      ldsm2(f, a);
     }
   }
-  __device__ __forceinline__ void right(uint32_t base, int s, int lane) {
+};
+// One digit of the right factor: rows 16 kt .., the warp's columns.
+template <int D, int W> struct Right {
+  using G = Geo<D, W>;
+  uint32_t f[D >= 16 ? 4 * G::NTW : 2];    // per 8-column tile: re (2), im (2)
+  uint32_t neg[D >= 16 ? 2 * G::NTW : 1];  // -im
+  __device__ __forceinline__ static uint32_t at(const Tm<D, W>& tm, uint32_t planes) {
+    const int l = tm.lane;
+    if constexpr (D >= 16)
+      return planes + (l >> 4) * G::PLANE + (tm.nt0() * (D / 8) + ((l >> 3) & 1)) * 128 + (l & 7) * 16;
+    else
+      return planes + ((l >> 3) & 1) * G::PLANE + (l & 7) * 16;
+  }
+  __device__ __forceinline__ void load(uint32_t a) {
     if constexpr (D >= 16) {
-      ldsm4t(re, base + (2 * s) * Geo<D>::PLANE + lane * 16);
-      ldsm4t(im, base + (2 * s + 1) * Geo<D>::PLANE + lane * 16);
+#pragma unroll
+      for (int j = 0; j < G::NTW; ++j) {
+        ldsm4t(f + 4 * j, a + j * (D / 8) * 128);
+        neg[2 * j] = f[4 * j + 2] ^ 0x80008000u;
+        neg[2 * j + 1] = f[4 * j + 3] ^ 0x80008000u;
+      }
     } else {
-      ldsm2t(re[0], im[0], base + 2 * s * Geo<D>::PLANE + (lane & 15) * 16);
+      ldsm2t(f, a);
     }
   }
 };
 
-// acc += a b (complex), one digit pair.
-template <int D> __device__ __forceinline__ void mma_pair(float (&acc)[Geo<D>::NV], const Frag<D>& a, const Frag<D>& b) {
+// acc += a b (complex), one digit pair, one 16-deep step.
+template <int D, int W>
+__device__ __forceinline__ void mma_pair(float (&acc)[Geo<D, W>::NV], const Left<D, W>& a, const Right<D, W>& b) {
   if constexpr (D >= 16) {
-    uint32_t n[4];
+    constexpr int NTW = Geo<D, W>::NTW;
+    const uint32_t* x = a.f;
+    const uint32_t* y = a.f + 4;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) n[i] = a.im[i] ^ 0x80008000u;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      mma(acc + 4 * j, a.re[0], a.re[1], a.re[2], a.re[3], b.re[2 * j], b.re[2 * j + 1]);
-      mma(acc + 8 + 4 * j, a.re[0], a.re[1], a.re[2], a.re[3], b.im[2 * j], b.im[2 * j + 1]);
+    for (int j = 0; j < NTW; ++j) {
+      mma(acc + 4 * j, x[0], x[1], x[2], x[3], b.f[4 * j], b.f[4 * j + 1]);
+      mma(acc + 4 * (NTW + j), x[0], x[1], x[2], x[3], b.f[4 * j + 2], b.f[4 * j + 3]);
     }
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      mma(acc + 4 * j, n[0], n[1], n[2], n[3], b.im[2 * j], b.im[2 * j + 1]);
-      mma(acc + 8 + 4 * j, a.im[0], a.im[1], a.im[2], a.im[3], b.re[2 * j], b.re[2 * j + 1]);
+    for (int j = 0; j < NTW; ++j) {
+      mma(acc + 4 * j, y[0], y[1], y[2], y[3], b.neg[2 * j], b.neg[2 * j + 1]);
+      mma(acc + 4 * (NTW + j), y[0], y[1], y[2], y[3], b.f[4 * j], b.f[4 * j + 1]);
     }
   } else {  // [Re; Im] = [Ar -Ai; Ai Ar] [Br; Bi] in one MMA
-    mma(acc, a.re[0], a.im[0], a.im[0] ^ 0x80008000u, a.re[0], b.re[0], b.im[0]);
+    mma(acc, a.f[0], a.f[1], a.f[1] ^ 0x80008000u, a.f[0], b.f[0], b.f[1]);
   }
 }
 
 constexpr float kMagic = 12582912.0f;  // 1.5 2^23
 constexpr uint32_t kPairBias = (0x4B400000u << 8) + 0x4B400000u;  // two magic starts joined (mod 2^32)
 
-// r += the two levels (2 P, 2 P + 1) held in a0, a1: 56 fractional bits.
-template <int D>
-__device__ __forceinline__ void join_levels(long long (&r)[Geo<D>::NV], const float (&a0)[Geo<D>::NV],
-                                            const float (&a1)[Geo<D>::NV], int P) {
-  const uint32_t bias = P == 3 ? 0x8000u - kPairBias : 0u - kPairBias;  // P = 3 rounds its 16 lost bits
-#pragma unroll
-  for (int v = 0; v < Geo<D>::NV; ++v) {
-    const uint32_t t = (__float_as_uint(a0[v]) << 8) + __float_as_uint(a1[v]) + bias;
-    r[v] += (long long)((unsigned long long)t << 32) >> (16 * P);
-  }
-}
-
 // r = A B with `nlev` levels, as value 2^(EA + EB - 56): pa, pb address the
-// factors' digit planes.  The two levels of a pass share every left digit;
-// the right digit of level 2 P + 1 is the one level 2 P used before.
-template <int D>
-__device__ __forceinline__ void mul(int lane, uint32_t pa, uint32_t pb, int nlev, long long (&r)[Geo<D>::NV]) {
-  constexpr int NV = Geo<D>::NV;
+// factors' digit planes.  Two levels a pass, the lowest two first: r <- r 2^-16
+// + (level L) 2^40 + (level L + 1) 2^32 needs no carries, because the new
+// levels only touch the high word, and keeps 32 bits below the last one.  The
+// two levels share every left digit, and the right digit of level L + 1 is the
+// one level L uses next.
+template <int D, int W>
+__device__ __forceinline__ void mul(const Tm<D, W>& tm, uint32_t pa, uint32_t pb, int nlev,
+                                    long long (&r)[Geo<D, W>::NV]) {
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV;
+  constexpr uint32_t kDigit = 2 * G::PLANE;
+  const uint32_t la = Left<D, W>::at(tm, pa), rb = Right<D, W>::at(tm, pb);
 #pragma unroll
   for (int v = 0; v < NV; ++v) r[v] = 0;
 #pragma unroll 1
-  for (int P = 0; 2 * P < nlev; ++P) {
-    const int L = 2 * P;
-    const bool two = L + 1 < nlev;
-    float a0[NV], a1[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) a0[v] = a1[v] = kMagic;
-    const int last = two ? min(L + 1, kSlices - 1) : L;
-    Frag<D> bc, bn;
-    if (two && L + 1 < kSlices) bc.right(pb, L + 1, lane);
+  for (int L = (nlev - 1) & ~1; L >= 0; L -= 2) {
+    uint32_t t[NV];
 #pragma unroll 1
-    for (int i = 0; i <= last; ++i) {
-      Frag<D> a;
-      a.left(pa, i, lane);
-      if (i <= L) bn.right(pb, L - i, lane);
-      if (two && L + 1 - i < kSlices) mma_pair<D>(a1, a, bc);
-      if (i <= L) mma_pair<D>(a0, a, bn);
-      bc = bn;
+    for (int kt = 0; kt < G::KT; ++kt) {
+      float a0[NV], a1[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) a0[v] = a1[v] = kMagic;
+      Left<D, W> a;
+      Right<D, W> b0, b1;
+      uint32_t pl = la + kt * 2 * (D / 8) * 128, pr = rb + kt * 2 * 128 + L * kDigit;  // A_0, B_L
+      a.load(pl);
+      b0.load(pr);
+      mma_pair<D, W>(a0, a, b0);
+      if (L + 1 < nlev) {
+        if (L + 1 < kSlices) {
+          b1.load(pr + kDigit);
+          mma_pair<D, W>(a1, a, b1);
+        }
+#pragma unroll 1
+        for (int i = 0; i < L; i += 2) {
+          a.load(pl + kDigit);
+          b1.load(pr - kDigit);
+          mma_pair<D, W>(a1, a, b0);
+          mma_pair<D, W>(a0, a, b1);
+          pl += 2 * kDigit;
+          pr -= 2 * kDigit;
+          a.load(pl);
+          b0.load(pr);
+          mma_pair<D, W>(a1, a, b1);
+          mma_pair<D, W>(a0, a, b0);
+        }
+        if (L + 1 < kSlices) {
+          a.load(pl + kDigit);
+          mma_pair<D, W>(a1, a, b0);
+        }
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < L; i += 2) {
+          a.load(pl + kDigit);
+          b1.load(pr - kDigit);
+          mma_pair<D, W>(a0, a, b1);
+          pl += 2 * kDigit;
+          pr -= 2 * kDigit;
+          a.load(pl);
+          b0.load(pr);
+          mma_pair<D, W>(a0, a, b0);
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const uint32_t x = (__float_as_uint(a0[v]) << 8) + __float_as_uint(a1[v]) - kPairBias;
+        t[v] = kt == 0 ? x : t[v] + x;
+      }
     }
-    join_levels<D>(r, a0, a1, P);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int hi = (int)(r[v] >> 32);
+      const uint32_t lo = __funnelshift_r((uint32_t)r[v], (uint32_t)hi, 16);
+      r[v] = (long long)((unsigned long long)(t[v] + (uint32_t)(hi >> 16)) << 32 | lo);
+    }
   }
 }
 
@@ -172,12 +272,12 @@ __device__ __forceinline__ long long shift_round(long long v, int right) {  // v
 }
 
 // r 2^(e - 56) -> x 2^(E - 56) with 0.37 2^56 < max |x| < 0.75 2^56; returns E.
-template <int NV> __device__ __forceinline__ int normalize(long long (&r)[NV], int e) {
+template <int D, int W> __device__ __forceinline__ int normalize(const Tm<D, W>& tm, long long (&r)[Geo<D, W>::NV], int e) {
+  constexpr int NV = Geo<D, W>::NV;
   uint32_t M = 0;
 #pragma unroll
   for (int v = 0; v < NV; ++v) M = max(M, (uint32_t)abs((int)(r[v] >> 32)));
-  M = __reduce_max_sync(0xffffffffu, M);
-  const int sh = norm_shift(M);
+  const int sh = norm_shift(tm.max(M, 0));
   if (sh >= 0) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) r[v] <<= sh;
@@ -189,49 +289,53 @@ template <int NV> __device__ __forceinline__ int normalize(long long (&r)[NV], i
 }
 
 // The leading `ns` digit planes of a normalised matrix into shared memory.
-template <int D>
-__device__ __forceinline__ void store_planes(int lane, uint32_t base, const long long (&x)[Geo<D>::NV], int ns) {
-  constexpr int NQ = Geo<D>::NQ;
+template <int D, int W>
+__device__ __forceinline__ void store_planes(const Tm<D, W>& tm, uint32_t base, const long long (&x)[Geo<D, W>::NV],
+                                             int ns) {
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV;
   // balanced digits: 128 in every byte below the top; the top digit (|.| <=
   // 192) is read as the 16 bits above bit 48, offset by 512 to stay positive
   constexpr unsigned long long kBias = 0x0080808080808080ull + (512ull << 48);
+  uint32_t lo[NV], hi[NV];
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
+  for (int v = 0; v < NV; ++v) {
+    const unsigned long long a = (unsigned long long)x[v] + kBias;
+    lo[v] = (uint32_t)a;
+    hi[v] = (uint32_t)(a >> 32);
+  }
+  const uint32_t at = base + (tm.nt0() * (D / 8) + 2 * tm.rt()) * 128 + tm.lane * 4;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      const unsigned long long a = (unsigned long long)x[p * 2 * NQ + 2 * q] + kBias;
-      const unsigned long long b = (unsigned long long)x[p * 2 * NQ + 2 * q + 1] + kBias;
-      const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
-      const uint32_t at = base + p * Geo<D>::PLANE + q * 128 + lane * 4;
+  for (int s = 0; s < kSlices; ++s) {
+    if (s >= ns) break;
+    const int byte = 6 - s;  // of the 64-bit value
 #pragma unroll
-      for (int s = 0; s < kSlices; ++s) {
-        uint32_t t, off;
-        if (s == 0) {
-          t = __byte_perm(ah, bh, 0x7632) | 0x64006400u;
-          off = 0x66806680u;  // 1024 + 512 + 128
-        } else {
-          const int byte = 6 - s;  // of the 64-bit value
-          const uint32_t wa = byte >= 4 ? ah : al, wb = byte >= 4 ? bh : bl;
-          const int k = byte & 3;
-          t = (__byte_perm(wa, wb, (unsigned)(k | (4 + k) << 8)) & 0x00ff00ffu) | 0x64006400u;
-          off = 0x64806480u;  // 1024 + 128
-        }
-        uint32_t d;
-        asm("sub.f16x2 %0, %1, %2;" : "=r"(d) : "r"(t), "r"(off));
-        if (s < ns) asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + s * 2 * Geo<D>::PLANE), "r"(d) : "memory");
+    for (int b = 0; b < NV / 2; ++b) {  // columns 2 t, 2 t + 1 of one 8 x 8 block
+      const int part = b / (NV / 4), nt = b % (NV / 4) / G::NI, i = b % G::NI;
+      uint32_t t, d;
+      if (s == 0) {
+        t = __byte_perm(hi[2 * b], hi[2 * b + 1], 0x7632) | 0x64006400u;  // FP16 1024 + byte
+      } else {
+        const uint32_t wa = byte >= 4 ? hi[2 * b] : lo[2 * b], wb = byte >= 4 ? hi[2 * b + 1] : lo[2 * b + 1];
+        t = (__byte_perm(wa, wb, (unsigned)((byte & 3) | (4 + (byte & 3)) << 8)) & 0x00ff00ffu) | 0x64006400u;
       }
+      // minus 1024 + 512 + 128, minus 1024 + 128
+      asm("sub.f16x2 %0, %1, %2;" : "=r"(d) : "r"(t), "r"(s == 0 ? 0x66806680u : 0x64806480u));
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + (2 * s + part) * G::PLANE + (nt * (D / 8) + i) * 128), "r"(d)
+                   : "memory");
     }
+  }
 }
 
-// 64-bit values of a matrix, lane-private in shared memory (16-byte accesses).
-template <int NV> __device__ __forceinline__ void put_ints(longlong2* s, int lane, const long long (&x)[NV]) {
+// 64-bit values of a matrix, lane-private (16-byte accesses; s = tm.mine()).
+template <int NV> __device__ __forceinline__ void put_ints(longlong2* s, const long long (&x)[NV]) {
 #pragma unroll
-  for (int v = 0; v < NV; v += 2) s[(v / 2) * 32 + lane] = make_longlong2(x[v], x[v + 1]);
+  for (int v = 0; v < NV; v += 2) s[(v / 2) * 32] = make_longlong2(x[v], x[v + 1]);
 }
-template <int NV> __device__ __forceinline__ void get_ints(const longlong2* s, int lane, long long (&x)[NV]) {
+template <int NV> __device__ __forceinline__ void get_ints(const longlong2* s, long long (&x)[NV]) {
 #pragma unroll
   for (int v = 0; v < NV; v += 2) {
-    const longlong2 a = s[(v / 2) * 32 + lane];
+    const longlong2 a = s[(v / 2) * 32];
     x[v] = a.x;
     x[v + 1] = a.y;
   }
@@ -249,12 +353,12 @@ __device__ __forceinline__ unsigned long long shr64(unsigned long long v, int s)
   return r;
 }
 
-// Largest biased exponent of the warp's doubles (0x7ff = not finite).
-template <int N> __device__ __forceinline__ int max_exponent(const double (&x)[N]) {
+// Largest biased exponent of the team's doubles (0x7ff = not finite).
+template <int D, int W> __device__ __forceinline__ int max_exponent(const Tm<D, W>& tm, const double (&x)[Geo<D, W>::NV]) {
   uint32_t M = 0;
 #pragma unroll
-  for (int v = 0; v < N; ++v) M = max(M, (uint32_t)__double2hiint(x[v]) & 0x7ff00000u);
-  return (int)(__reduce_max_sync(0xffffffffu, M) >> 20);
+  for (int v = 0; v < Geo<D, W>::NV; ++v) M = max(M, (uint32_t)__double2hiint(x[v]) & 0x7ff00000u);
+  return (int)(tm.max(M, 2) >> 20);
 }
 // Double -> integer d 2^(1075 + guard - EX), EX the matrix's largest biased
 // exponent: |result| < 2^(53 + guard).  guard = 2: the format above with
@@ -286,47 +390,79 @@ struct Coef {
   int exp;
 };
 
-// A coefficient aligned to a frame: c x (x 2^(E - 56)) with 60 fractional bits
-// in frame fr is x m 2^-57; the 64-bit product's low quarter is left out (its
-// part of the result is below 2^-64 of the frame).
+// A coefficient aligned to a frame: r += c x, x 2^(E - 62) the matrix kept by
+// put_ints and r an integer with F <= 60 fractional bits in frame fr (value
+// r 2^(fr - F), fr >= E + c.exp).  The product's high 64 bits without its low
+// quarter: one multiply-add into r and the high word of the two mixed terms.
 struct Scaled {
   int m1, m0;  // m = m1 2^32 + m0, m0 balanced
-  __device__ __forceinline__ Scaled(Coef c, int E, int fr) {
-    const unsigned long long m = shr64(c.mant, min(fr - E - c.exp, 63));
+  __device__ __forceinline__ Scaled(Coef c, int E, int fr, int F) {
+    const unsigned long long m = shr64(c.mant << 1, min(fr - E - c.exp + 60 - F, 63));
     m0 = (int)(uint32_t)m;
     m1 = (int)((m + 0x80000000ull) >> 32);
   }
-  __device__ __forceinline__ long long operator()(long long x) const {
+  __device__ __forceinline__ long long operator()(long long x, long long r) const {
     const int b1 = (int)(x >> 32);
     const long long mid = (long long)((unsigned long long)(uint32_t)x * (uint32_t)m1) + (long long)b1 * m0;
-    return ((long long)b1 * m1 << 7) + (mid >> 25);
+    return r + (long long)b1 * m1 + (long long)(int)(mid >> 32);
   }
 };
-// r (60 fractional bits in frame fr) += c x, x 2^(E - 56) normalised.
 template <int NV>
-__device__ __forceinline__ void add_scaled(long long (&r)[NV], const longlong2* xs, int lane, int E, Coef c, int fr) {
-  const Scaled sc(c, E, fr);
+__device__ __forceinline__ void add_scaled(long long (&r)[NV], const longlong2* xs, const Scaled& sc) {
 #pragma unroll
   for (int v = 0; v < NV; v += 2) {
-    const longlong2 a = xs[(v / 2) * 32 + lane];
-    r[v] += sc(a.x);
-    r[v + 1] += sc(a.y);
+    const longlong2 a = xs[(v / 2) * 32];
+    r[v] = sc(a.x, r[v]);
+    r[v + 1] = sc(a.y, r[v + 1]);
   }
 }
-// r (56 fractional bits at e) -> 60 fractional bits in frame fr >= e + 6.
-template <int NV> __device__ __forceinline__ void to_frame(long long (&r)[NV], int e, int fr) {
-  const int sh = min(fr - e - 4, 63);
+// r (56 fractional bits at e) -> F fractional bits in frame fr.
+template <int NV> __device__ __forceinline__ void to_frame(long long (&r)[NV], int e, int fr, int F) {
+  const int sh = fr - e + kFrac - F;
+  if (sh >= 0) {
 #pragma unroll
-  for (int v = 0; v < NV; ++v) r[v] = shift_round(r[v], sh);
+    for (int v = 0; v < NV; ++v) r[v] >>= min(sh, 63);
+  } else {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] <<= -sh;
+  }
 }
-// r += c I in frame fr.
-template <int D> __device__ __forceinline__ void add_diag(long long (&r)[Geo<D>::NV], int lane, Coef c, int fr) {
-  const long long d = (long long)shr64(c.mant >> 1, min(fr - c.exp, 63));
+// r += c I with F fractional bits in frame fr.
+template <int D, int W>
+__device__ __forceinline__ void add_diag(const Tm<D, W>& tm, long long (&r)[Geo<D, W>::NV], Coef c, int fr, int F) {
+  using G = Geo<D, W>;
+  const long long d = (long long)shr64(c.mant, min(fr - c.exp + 61 - F, 63));
 #pragma unroll
-  for (int q = 0; q < Geo<D>::NQ; ++q)
+  for (int b = 0; b < G::NV / 2; ++b)
+    if (tm.row(b / 2 % G::NI) == tm.col(b / 2 / G::NI, b % 2)) r[b] += d;
+}
+
+// A double matrix in the team's order, and back.
+template <int D, int W>
+__device__ __forceinline__ void load_mat(const Tm<D, W>& tm, const double2* A, double (&x)[Geo<D, W>::NV]) {
+  using G = Geo<D, W>;
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (Geo<D>::row(lane, q) == Geo<D>::col(lane, q, h)) r[2 * q + h] += d;
+  for (int b = 0; b < G::NV / 2; ++b) {
+    const double2 a = A[tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2)];
+    x[b] = a.x;
+    x[G::NV / 2 + b] = a.y;
+  }
+}
+// U = r 2^ex
+template <int D, int W>
+__device__ __forceinline__ void store_mat(const Tm<D, W>& tm, double2* U, const long long (&r)[Geo<D, W>::NV], int ex) {
+  using G = Geo<D, W>;
+#pragma unroll
+  for (int b = 0; b < G::NV / 2; ++b)
+    U[tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2)] =
+        make_double2(to_double(r[b], ex), to_double(r[G::NV / 2 + b], ex));
+}
+template <int D, int W> __device__ __forceinline__ void store_nan(const Tm<D, W>& tm, double2* U) {
+  using G = Geo<D, W>;
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+#pragma unroll
+  for (int b = 0; b < G::NV / 2; ++b)
+    U[tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2)] = make_double2(nan, nan);
 }
 
 }  // namespace fx
