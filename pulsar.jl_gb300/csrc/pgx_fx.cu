@@ -279,18 +279,274 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
   }
 }
 
+// M_k in the team's order: the gate chains' product, or sum_s psi_s[k]
+// lambda_s[k+1]' for state targets (pairing as k_grad's).
+template <int D, int W>
+__device__ __forceinline__ void load_M(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m, int k,
+                                       double (&x)[Geo<D, W>::NV]) {
+  using G = Geo<D, W>;
+  if (p.target == TGT_GATE) {
+    load_mat<D, W>(tm, w.P + ((size_t)m * p.n_t + k) * D * D, x);
+    return;
+  }
+  const int np = p.n_pairs;
+  const double2* psi = w.psi + ((size_t)m * (p.n_t + 1) + k) * np * D;
+  const double2* lam = w.lam + ((size_t)m * (p.n_t + 1) + k + 1) * np * D;
+#pragma unroll
+  for (int v = 0; v < G::NV; ++v) x[v] = 0.0;
+  for (int s = 0; s < np; ++s)
+#pragma unroll
+    for (int b = 0; b < G::NV / 2; ++b) {
+      const double2 y = psi[s * D + tm.row(b / 2 % G::NI)], l = lam[s * D + tm.col(b / 2 / G::NI, b % 2)];
+      const double2 acc = cmac(make_double2(x[b], x[G::NV / 2 + b]), y, make_double2(l.x, -l.y));
+      x[b] = acc.x;
+      x[G::NV / 2 + b] = acc.y;
+    }
+}
+
+// t = Tr(X K_j), its real (im = 0) or imaginary part, as an integer sum over
+// the team: the lanes' X (56 fractional bits) against the transposed term.
+// |x| < 2^56 and |K| < 2^59 keep the sum of all elements below 2^60 in units
+// of 2^-52; three further bits hold the lanes' rounding near 2^-54.
+template <int D, int W>
+__device__ __forceinline__ long long trace_term(const Terms<D, W>& T, const Tm<D, W>& tm, int j, int im,
+                                                const long long (&x)[Geo<D, W>::NV]) {
+  using G = Geo<D, W>;
+  const int2* kp = reinterpret_cast<const int2*>(T.k + (size_t)j * W * (G::NV / 2) * 32);
+  long long main = 0, mid = 0;
+#pragma unroll
+  for (int b = 0; b < G::NV / 2; ++b) {
+    // element (row', col') = (col, row) of the term in the team's layout
+    const int r = tm.col(b / 2 / G::NI, b % 2), c = tm.row(b / 2 % G::NI);
+    const int nt = c / 8 % G::NTW, wt = c / 8 / G::NTW;
+    const int v = 2 * (nt * G::NI + r / 8 % G::NI) + c % 2;
+    const int2* e = kp + ((size_t)(wt * (G::NV / 2) + v / 2) * 32 + (r % 8) * 4 + c % 8 / 2) * 2 + v % 2;
+    const int2 cr = e[0], ci = e[(G::NV / 4) * 64];
+    // re: xr cr - xi ci, im: xr ci + xi cr
+    const long long xr = x[b], xi = im ? x[G::NV / 2 + b] : -x[G::NV / 2 + b];
+    const int xr0 = (int)xr, xr1 = (int)((xr + 0x80000000ll) >> 32);
+    const int xi0 = (int)xi, xi1 = (int)((xi + 0x80000000ll) >> 32);
+    const int2 p = im ? ci : cr, q = im ? cr : ci;
+    main += (long long)xr1 * p.y;
+    main += (long long)xi1 * q.y;
+    mid += (long long)xr1 * p.x;
+    mid += (long long)xr0 * p.y;
+    mid += (long long)xi1 * q.x;
+    mid += (long long)xi0 * q.y;
+  }
+  long long t = ((main + (mid >> 32)) << 3) + (long long)((uint32_t)mid >> 29);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+constexpr int kGradBits2 = 2 * 56 + 1;
+
+template <int D> struct GradCfg {
+  static constexpr int W = D >= 16 ? 2 : 1;
+  static constexpr int TEAMS = D >= 16 ? 7 : 12;
+  // planes of X, dX, Y, dY; maxima; the warps' traces
+  static constexpr int TEAM_BYTES = 4 * Geo<D, W>::PLANES + 64 + (W > 1 ? kMaxTerms * 8 : 0);
+};
+
+// g_jk = Re(c dt scale Tr(L(A_k, M_k) C_j)), one team per slice: the Frechet
+// derivative of T_2L(A / 2^s)^(2^s) in the q = 2 form (three products a step),
+// carried in block fixed point like the propagator.  The derivative's matrices
+// keep an exponent of their own, so any magnitude of M_k does.
+//
+// Bound: instruction issue, then the tensor pipe.  Four matrices' planes (28 KB
+// at D = 16) limit an SM to seven slices; B and dB stay in registers.
+template <int D>
+__global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_grad(ProbDev p, WorkDev w, int run) {
+  using C = GradCfg<D>;
+  constexpr int W = C::W;
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int team = threadIdx.x / (32 * W), nt = blockDim.x / (32 * W);
+  Terms<D, W> T;
+  T.n = p.n_c + 1 + (p.n_ramp ? 1 : 0);
+  T.k = reinterpret_cast<int4*>(smem_raw);
+  T.e = reinterpret_cast<int*>(smem_raw + (size_t)T.n * G::INTS);
+  unsigned char* mine = smem_raw + Terms<D, W>::bytes(T.n) + (size_t)team * C::TEAM_BYTES;
+  const uint32_t px = smem_u32(mine), pdx = px + G::PLANES, py = px + 2 * G::PLANES, pdy = px + 3 * G::PLANES;
+  const Tm<D, W> tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
+                    reinterpret_cast<uint32_t*>(mine + 4 * G::PLANES)};
+  long long* traces = reinterpret_cast<long long*>(mine + 4 * G::PLANES + 64);  // W > 1
+  for (int j = team; j < p.n_c; j += nt) {
+    double x[NV];
+    load_mat<D, W>(tm, p.ctrls + (size_t)j * D * D, x);
+    put_term<D, W>(T, j + 1, tm, x);
+  }
+  const int runs = (p.n_t + run - 1) / run;
+  int cur = -1;
+  for (long c = blockIdx.x; c < (long)p.n_members * runs; c += gridDim.x) {
+    const int m = (int)(c / runs), k0 = (int)(c % runs) * run;
+    if (m != cur) {
+      __syncthreads();
+      if (team == 0) put_member_terms<D, W>(T, p, m, tm);
+      __syncthreads();
+      cur = m;
+    }
+    const int k1 = min(p.n_t, k0 + run);
+#pragma unroll 1
+    for (int k = k0 + team; k < k1; k += nt) {
+      long long b[NV], db[NV], r[NV], q[NV];
+      const int EA = assemble<D, W>(T, p, w.u, m, k, tm, b);
+      const float l2 = log2_norm1<D, W>(tm, b, EA);
+      int L, s;
+      choose_degree2(l2, tm.lane, L, s);
+      int EXd;
+      {
+        double x[NV];
+        load_M<D, W>(tm, p, w, m, k, x);
+        EXd = max_exponent<D, W>(tm, x);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) db[v] = from_double(x[v], EXd, 2);
+      }
+      const int ED = EXd - 1021 - s;  // dB = M / 2^s
+      if (EA > kNever / 2 || s > 60 || EXd == 0x7ff) {
+        if (tm.w == 0)
+          for (int j = tm.lane; j < p.n_c; j += 32)
+            w.Gm[((size_t)m * p.n_t + k) * p.n_c + j] = __longlong_as_double(0x7ff8000000000000ll);
+        tm.sync();
+        continue;
+      }
+      const float nu2 = l2 - (float)s;
+      const int lx = min(0, 2 * (int)ceilf(nu2));
+      const int g = nu2 <= -1.33f ? 1 : 3;
+      const int EB = normalize<D, W>(tm, b, EA - 2 - s);
+      tm.sync();
+      store_planes<D, W>(tm, py, b, kSlices);
+      store_planes<D, W>(tm, pdy, db, kSlices);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        b[v] <<= 6;
+        db[v] <<= 6;
+      }
+      int EX = EB, EdX = ED, EY = EB, EdY = ED;  // step 0: (X, dX) <- (B B, dB B + B dB)
+      uint32_t pl = py, pdl = pdy;
+#pragma unroll 1
+      for (int st = 0; st < L + s; ++st) {
+        const int i = L - 1 - st;
+        const bool last = st + 1 == L + s;
+        const int fq = max(EdX + EY, EX + EdY) + 6;
+        tm.sync();
+#pragma unroll 1
+        for (int h = 0; h < (last ? 2 : 3); ++h) {
+          const int ea = h == 0 ? EdX : EX, eb = h == 1 ? EdY : EY;
+          // relative to dB for the derivative, to I for Y; the error of step i
+          // meets X^i later, and Y only acts through dX Y
+          const int e = ea + eb + (st > 0 && st < L ? (h == 2 ? max(i - 1, 0) : i) * lx : 0) - (h == 2 ? 0 : ED);
+          mul<D, W>(tm, h == 0 ? pdl : pl, h == 1 ? pdy : py, levels(kGradBits2, e), r);
+          if (h < 2) {
+            to_frame<NV>(r, ea + eb, fq, 60);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) q[v] = h == 0 ? r[v] : q[v] + r[v];
+          }
+        }
+        // derivative
+        if (st < L) {
+          if (st == 0) {
+            EdX = normalize<D, W>(tm, q, fq - 4);
+            EX = normalize<D, W>(tm, r, 2 * EB, 1);
+            store_planes<D, W>(tm, pdx, q, kSlices);
+            store_planes<D, W>(tm, px, r, kSlices);
+            const int fr = c_coef[2 * i].exp + g, fd = max(EdX + c_coef[2 * L].exp, ED + c_coef[2 * i + 1].exp) + 1;
+            const Scaled sx(c_coef[2 * L], EX, fr, kFrac), sdx(c_coef[2 * L], EdX, fd, 60);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+              r[v] = sx(r[v] << 6, 0);
+              q[v] = sdx(q[v] << 6, 0);
+            }
+            const Scaled sb(c_coef[2 * i + 1], EB, fr, kFrac), sdb(c_coef[2 * i + 1], ED, fd, 60);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+              r[v] = sb(b[v], r[v]);
+              q[v] = sdb(db[v], q[v]);
+            }
+            add_diag<D, W>(tm, r, c_coef[2 * i], fr, kFrac);
+            EY = fr;
+            tm.sync();  // the maxima are read
+            EdY = normalize<D, W>(tm, q, fd - 4);
+            pl = px;
+            pdl = pdx;
+          } else {
+            const int fd = max(fq, ED + c_coef[2 * i + 1].exp + 1) + 1;
+            const Scaled sdb(c_coef[2 * i + 1], ED, fd, 60);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) q[v] = sdb(db[v], q[v] >> min(fd - fq, 63));
+            const int eq = normalize<D, W>(tm, q, fd - 4);
+            if (!last) {
+              const int fr = c_coef[2 * i].exp + g, F = i > 0 ? kFrac : 60;
+              to_frame<NV>(r, EX + EY, fr, F);
+              const Scaled sb(c_coef[2 * i + 1], EB, fr, F);
+#pragma unroll
+              for (int v = 0; v < NV; ++v) r[v] = sb(b[v], r[v]);
+              add_diag<D, W>(tm, r, c_coef[2 * i], fr, F);
+              EY = fr;
+              if (i == 0) {
+                tm.sync();
+                EY = normalize<D, W>(tm, r, fr - 4);
+              }
+            }
+            EdY = eq;
+          }
+        } else {
+          const int eq = normalize<D, W>(tm, q, fq - 4);
+          if (!last) {
+            tm.sync();
+            EY = normalize<D, W>(tm, r, 2 * EY);
+          }
+          EdY = eq;
+        }
+        if (!last) {
+          tm.sync();  // every product of this step has read its planes
+          store_planes<D, W>(tm, py, r, kSlices);
+          store_planes<D, W>(tm, pdy, q, kSlices);
+          if (i <= 0) {  // squarings: both factors are Y
+            pl = py;
+            pdl = pdy;
+            EX = EY;
+            EdX = EdY;
+          }
+        }
+      }
+      // traces, in integers; lane j keeps control j's
+      long long keep[(kMaxTerms + 31) / 32];
+      keep[0] = 0;
+      for (int j = 0; j < p.n_c; ++j) {
+        const long long t = trace_term<D, W>(T, tm, j + 1, p.gen == GEN_HERM ? 1 : 0, q);
+        if constexpr (W > 1) {
+          if (tm.lane == 0 && tm.w > 0) traces[j] = t;
+        }
+        if (tm.lane == j) keep[0] = t;
+      }
+      tm.sync();
+      if (tm.w == 0 && tm.lane < p.n_c) {
+        if constexpr (W > 1) keep[0] += traces[tm.lane];
+        w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] =
+            p.dt[k] * p.m_scale[m] * to_double(keep[0], EdY + T.e[tm.lane + 1] - 55);
+      }
+    }
+  }
+}
+
 constexpr size_t kSmemMax = 232448;  // dynamic shared memory of a CTA
 
-template <int D> static cudaError_t do_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  using C = ExpmCfg<D>;
+// Launches a slice-parallel kernel of configuration C (dimension D): as many
+// teams as the shared memory beside the generator's terms holds.
+template <class C, int D>
+static cudaError_t launch_slices(void (*kernel)(ProbDev, WorkDev, int), const ProbDev& p, const WorkDev& w,
+                                 const LaunchInfo& li) {
   const int n = p.n_c + 1 + (p.n_ramp ? 1 : 0);
   const size_t consts = Terms<D, C::W>::bytes(n);
   const int fit = (int)((kSmemMax - consts) / C::TEAM_BYTES);
   const int nt = fit < C::TEAMS ? fit : C::TEAMS, threads = 32 * C::W * nt;
   const size_t smem = consts + (size_t)nt * C::TEAM_BYTES;
-  set_smem_once((const void*)k_fx_expm<D>, smem);
+  set_smem_once((const void*)kernel, smem);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fx_expm<D>, threads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   if (per_sm < 1) per_sm = 1;
   // Runs long enough to amortise the member's own terms, short enough that
   // every CTA gets several.
@@ -301,18 +557,23 @@ template <int D> static cudaError_t do_expm(const ProbDev& p, const WorkDev& w, 
   const int run = (int)rounds * nt;
   long grid = (long)p.n_members * ((p.n_t + run - 1) / run);
   if (grid > ctas) grid = ctas;
-  k_fx_expm<D><<<(int)grid, threads, smem, li.stream>>>(p, w, run);
+  kernel<<<(int)grid, threads, smem, li.stream>>>(p, w, run);
   ++*li.launches;
   return cudaGetLastError();
 }
 
 }  // namespace fx
 
-bool fx_expm_applies(const ProbDev& p) {
+bool fx_applies(const ProbDev& p) {
   return (p.Dp == 8 || p.Dp == 16) && p.n_c + 1 + (p.n_ramp ? 1 : 0) <= fx::kMaxTerms;
 }
 cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  return p.Dp == 8 ? fx::do_expm<8>(p, w, li) : fx::do_expm<16>(p, w, li);
+  return p.Dp == 8 ? fx::launch_slices<fx::ExpmCfg<8>, 8>(fx::k_fx_expm<8>, p, w, li)
+                   : fx::launch_slices<fx::ExpmCfg<16>, 16>(fx::k_fx_expm<16>, p, w, li);
+}
+cudaError_t launch_fx_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  return p.Dp == 8 ? fx::launch_slices<fx::GradCfg<8>, 8>(fx::k_fx_grad<8>, p, w, li)
+                   : fx::launch_slices<fx::GradCfg<16>, 16>(fx::k_fx_grad<16>, p, w, li);
 }
 
 }  // namespace pgx

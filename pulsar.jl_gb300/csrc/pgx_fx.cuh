@@ -272,12 +272,13 @@ __device__ __forceinline__ long long shift_round(long long v, int right) {  // v
 }
 
 // r 2^(e - 56) -> x 2^(E - 56) with 0.37 2^56 < max |x| < 0.75 2^56; returns E.
-template <int D, int W> __device__ __forceinline__ int normalize(const Tm<D, W>& tm, long long (&r)[Geo<D, W>::NV], int e) {
+template <int D, int W> __device__ __forceinline__ int normalize(const Tm<D, W>& tm, long long (&r)[Geo<D, W>::NV], int e,
+                                                                        int slot = 0) {
   constexpr int NV = Geo<D, W>::NV;
   uint32_t M = 0;
 #pragma unroll
   for (int v = 0; v < NV; ++v) M = max(M, (uint32_t)abs((int)(r[v] >> 32)));
-  const int sh = norm_shift(tm.max(M, 0));
+  const int sh = norm_shift(tm.max(M, slot));
   if (sh >= 0) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) r[v] <<= sh;

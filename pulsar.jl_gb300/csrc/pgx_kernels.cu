@@ -730,7 +730,7 @@ static cudaError_t do_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo&
   return cudaGetLastError();
 }
 cudaError_t launch_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  if (fx_expm_applies(p)) return launch_fx_expm(p, w, li);
+  if (fx_applies(p)) return launch_fx_expm(p, w, li);
   PGX_DISPATCH(p.Dp, return do_expm<D_>(p, w, li));
   return cudaSuccess;
 }
@@ -793,6 +793,7 @@ static cudaError_t do_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo&
   return cudaGetLastError();
 }
 cudaError_t launch_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  if (p.grad_mode == GRAD_EXACT && fx_applies(p)) return launch_fx_grad(p, w, li);
   PGX_DISPATCH(p.Dp, return do_grad<D_>(p, w, li));
   return cudaSuccess;
 }

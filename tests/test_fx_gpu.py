@@ -50,3 +50,39 @@ def test_propagator_not_finite(pg):
     U = p.total_propagator(np.full((1, 1), 1e10))
     p.close()
     assert np.isnan(U).any()
+
+
+@pytest.mark.parametrize("target", ["gate", "states"])
+@pytest.mark.parametrize("gen", ["hermitian", "liouvillian"])
+@pytest.mark.parametrize("D,n_t,n_m", [(7, 1, 1), (8, 13, 3), (9, 2, 2), (16, 13, 3)])
+@pytest.mark.parametrize("nrm", [0.03, 0.4, 9.0])
+def test_exact_gradient(pg, target, gen, D, n_t, n_m, nrm):
+    """(F, G) of slices with few and many Horner steps and squarings, members of
+    different scale and offset, against the oracle.  FP64's own bars: |dF| <=
+    1e-10 and 1e-8 of the largest gradient entry; the sums of n_t D-term
+    products stay well inside both."""
+    from oracle import members as mb
+    rng = np.random.default_rng(D + n_t)
+    n_c = 3
+    H = rng.normal(size=(2, D, D)) + 1j * rng.normal(size=(2, D, D))
+    C = rng.normal(size=(n_c, D, D)) + 1j * rng.normal(size=(n_c, D, D))
+    O = rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D))
+    dag = lambda x: np.swapaxes(x.conj(), -1, -2)  # noqa: E731
+    if gen == "hermitian":
+        H, C, O = H + dag(H), C + dag(C), O + dag(O)
+    else:
+        H = H - dag(H) - 0.2 * np.eye(D) + 0.05 * np.triu(H, 1)
+        C, O = C - dag(C), O - dag(O)
+    u = rng.normal(size=(n_c, n_t))
+    dt = nrm / np.abs(H[0] + np.tensordot(u[:, 0], C, 1)).sum(0).max() * rng.uniform(0.5, 1.0, n_t)
+    Q, _ = np.linalg.qr(rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D)))
+    kw = dict(drifts=H, controls=C, dt=dt, generator=gen, offset_op=O, member_drift=np.arange(n_m) % 2,
+              member_scale=rng.uniform(0.9, 1.1, n_m), member_offset=rng.uniform(-0.1, 0.1, n_m), target=target,
+              fidelity="square")
+    kw.update(dict(target_op=Q) if target == "gate" else dict(states_init=Q[:2], states_target=Q[2:4]))
+    Fo, Go = mb.eval_problem(mb.Problem(n_members=n_m, **kw), u, "exact")
+    p = pg.Problem(grad_mode="exact", precision="fp64", **kw)
+    F, G = p.eval(u)
+    p.close()
+    assert abs(F - Fo) <= 1e-10
+    assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
