@@ -13,6 +13,11 @@ constexpr int kMaxTerms = 24;       // generator terms: drift, controls, ramp
 constexpr int kBits = 57;           // absolute error of a slice propagator: 2^-57 per product
 constexpr int kBits2 = 2 * kBits + 1;
 constexpr int kNever = 1 << 20;     // an exponent no finite entry reaches
+// Levels of a chain product: about 2^-55.5 of the factors' scale with 7, which
+// at D = 16 keeps a chain's error below that of an FP64 product's 64 roundings
+// (unitarity after 1000 slices 2.0e-14, FP64 products 3.0e-14); at D = 8 seven
+// levels fell behind (2.9e-14 against 1.1e-14 after 500), eight do not.
+template <int D> constexpr int kChainLevels = D >= 16 ? 7 : 8;
 
 // The constant matrices of the generator, A_mk = c sum_j alpha_j K_j with
 // alpha = dt_k {1, scale u_1k, ..., tau_k} and K = {drift_m + off_m O, C_1,
@@ -94,7 +99,10 @@ __device__ __forceinline__ int assemble(const Terms<D, W>& T, const ProbDev& p, 
   const int my0 = (int)a, my1 = (int)((a + 0x80000000ll) >> 32);
   long long main[NV], mid[NV];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) main[v] = mid[v] = 0;
+  for (int v = 0; v < NV; ++v) {
+    main[v] = 0;
+    mid[v] = 0x80000000ll;  // to nearest
+  }
 #pragma unroll 1
   for (int j = 0; j < T.n; ++j) {
     const int a0 = __shfl_sync(0xffffffffu, my0, j), a1 = __shfl_sync(0xffffffffu, my1, j);
@@ -213,9 +221,14 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
       int L, s;
       choose_degree2(l2, tm.lane, L, s);
       double2* out = w.U + ((size_t)m * p.n_t + k) * D * D;
+      const bool packed = p.target == TGT_GATE;  // the gate chains' own format
       int ex;  // U = r 2^ex
       if (EA > kNever / 2 || s > 60) {
-        store_nan<D, W>(tm, out);
+        if (packed) {
+          put_packed<D, W>(tm.mine((longlong2*)out), r, kNotFinite);
+        } else {
+          store_nan<D, W>(tm, out);
+        }
         tm.sync();  // the maxima are read
         continue;
       }
@@ -247,7 +260,8 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
         tm.sync();
         mul<D, W>(tm, pa, py, n, r);
         if (st < L) {
-          const int fr = c_coef[2 * i].exp + g;
+          const bool final = packed && i == 0 && s == 0;  // |U| <= e^nu <= 0.75 2^g
+          const int fr = final ? g : c_coef[2 * i].exp + g;
           if (st == 0) {
             // Y = c_2L X + c_{2L-1} B + c_{2L-2} I
             EX = normalize<D, W>(tm, r, 2 * EB);
@@ -271,24 +285,24 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
           }
         } else {
           ex = 2 * EY - kFrac;
-          if (st + 1 < L + s) EY = normalize<D, W>(tm, r, 2 * EY);
+          if (packed || st + 1 < L + s) EY = normalize<D, W>(tm, r, 2 * EY);
         }
       }
-      store_mat<D, W>(tm, out, r, ex);
+      if (packed && s == 0) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) r[v] = shift_round(r[v], 4);
+      }
+      if (packed) put_packed<D, W>(tm.mine((longlong2*)out), r, EY);
+      else store_mat<D, W>(tm, out, r, ex);
     }
   }
 }
 
-// M_k in the team's order: the gate chains' product, or sum_s psi_s[k]
-// lambda_s[k+1]' for state targets (pairing as k_grad's).
+// M_k of a state target in the team's order: sum_s psi_s[k] lambda_s[k+1]'.
 template <int D, int W>
 __device__ __forceinline__ void load_M(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m, int k,
                                        double (&x)[Geo<D, W>::NV]) {
   using G = Geo<D, W>;
-  if (p.target == TGT_GATE) {
-    load_mat<D, W>(tm, w.P + ((size_t)m * p.n_t + k) * D * D, x);
-    return;
-  }
   const int np = p.n_pairs;
   const double2* psi = w.psi + ((size_t)m * (p.n_t + 1) + k) * np * D;
   const double2* lam = w.lam + ((size_t)m * (p.n_t + 1) + k + 1) * np * D;
@@ -357,7 +371,7 @@ template <int D> struct GradCfg {
 // Bound: instruction issue, then the tensor pipe.  Four matrices' planes (28 KB
 // at D = 16) limit an SM to seven slices; B and dB stay in registers.
 template <int D>
-__global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_grad(ProbDev p, WorkDev w, int run) {
+__global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_grad(ProbDev p, WorkDev w, int run, int len) {
   using C = GradCfg<D>;
   constexpr int W = C::W;
   using G = Geo<D, W>;
@@ -392,26 +406,41 @@ __global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_g
 #pragma unroll 1
     for (int k = k0 + team; k < k1; k += nt) {
       long long b[NV], db[NV], r[NV], q[NV];
+      int EM;  // M_k = db 2^(EM - 56)
+      if (p.target == TGT_GATE) {
+        // M_k = R_k V_k of the chains (R = I at the start of a block)
+        get_ints<NV>(tm.mine((longlong2*)(w.U + ((size_t)m * p.n_t + k) * D * D)), db);
+        EM = unpack<D, W>(db);
+        if (k % len != 0) {
+          get_ints<NV>(tm.mine((longlong2*)(w.P + ((size_t)m * p.n_t + k) * D * D)), r);
+          const int ER = unpack<D, W>(r);
+          tm.sync();  // the last slice's products have read their planes
+          store_planes<D, W>(tm, py, db, kSlices);
+          store_planes<D, W>(tm, px, r, kSlices);
+          tm.sync();
+          if (max(EM, ER) == kNotFinite) EM = kNotFinite;
+          else {
+            mul<D, W>(tm, px, py, kChainLevels<D>, db);
+            EM = normalize<D, W>(tm, db, EM + ER);
+          }
+        }
+      } else {
+        double x[NV];
+        load_M<D, W>(tm, p, w, m, k, x);
+        const int EXd = max_exponent<D, W>(tm, x);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) db[v] = from_double(x[v], EXd, 2);
+        EM = EXd == 0x7ff ? kNotFinite : EXd - 1021;
+      }
+      int EdY = EM;
+      if (p.grad_mode == GRAD_EXACT) {
       const int EA = assemble<D, W>(T, p, w.u, m, k, tm, b);
       const float l2 = log2_norm1<D, W>(tm, b, EA);
       int L, s;
       choose_degree2(l2, tm.lane, L, s);
-      int EXd;
-      {
-        double x[NV];
-        load_M<D, W>(tm, p, w, m, k, x);
-        EXd = max_exponent<D, W>(tm, x);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) db[v] = from_double(x[v], EXd, 2);
-      }
-      const int ED = EXd - 1021 - s;  // dB = M / 2^s
-      if (EA > kNever / 2 || s > 60 || EXd == 0x7ff) {
-        if (tm.w == 0)
-          for (int j = tm.lane; j < p.n_c; j += 32)
-            w.Gm[((size_t)m * p.n_t + k) * p.n_c + j] = __longlong_as_double(0x7ff8000000000000ll);
-        tm.sync();
-        continue;
-      }
+      if (EA > kNever / 2 || s > 60) EM = kNotFinite;
+      if (EM != kNotFinite) {
+      const int ED = EM - s;  // dB = M / 2^s
       const float nu2 = l2 - (float)s;
       const int lx = min(0, 2 * (int)ceilf(nu2));
       const int g = nu2 <= -1.33f ? 1 : 3;
@@ -424,7 +453,8 @@ __global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_g
         b[v] <<= 6;
         db[v] <<= 6;
       }
-      int EX = EB, EdX = ED, EY = EB, EdY = ED;  // step 0: (X, dX) <- (B B, dB B + B dB)
+      int EX = EB, EdX = ED, EY = EB;  // step 0: (X, dX) <- (B B, dB B + B dB)
+      EdY = ED;
       uint32_t pl = py, pdl = pdy;
 #pragma unroll 1
       for (int st = 0; st < L + s; ++st) {
@@ -512,23 +542,254 @@ __global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_g
           }
         }
       }
+      }
+      } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) q[v] = db[v];
+        tm.sync();  // the last slice's traces are read
+      }
+      if (EM == kNotFinite) {
+        if (tm.w == 0 && tm.lane < p.n_c)
+          w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] = __longlong_as_double(0x7ff8000000000000ll);
+        tm.sync();
+        continue;
+      }
       // traces, in integers; lane j keeps control j's
-      long long keep[(kMaxTerms + 31) / 32];
-      keep[0] = 0;
+      long long keep = 0;
       for (int j = 0; j < p.n_c; ++j) {
         const long long t = trace_term<D, W>(T, tm, j + 1, p.gen == GEN_HERM ? 1 : 0, q);
         if constexpr (W > 1) {
           if (tm.lane == 0 && tm.w > 0) traces[j] = t;
         }
-        if (tm.lane == j) keep[0] = t;
+        if (tm.lane == j) keep = t;
       }
-      tm.sync();
+      tm.sync();  // traces are written, and the maxima read
       if (tm.w == 0 && tm.lane < p.n_c) {
-        if constexpr (W > 1) keep[0] += traces[tm.lane];
+        if constexpr (W > 1) keep += traces[tm.lane];
         w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] =
-            p.dt[k] * p.m_scale[m] * to_double(keep[0], EdY + T.e[tm.lane + 1] - 55);
+            p.dt[k] * p.m_scale[m] * to_double(keep, EdY + T.e[tm.lane + 1] - 55);
       }
     }
+  }
+}
+
+// Gate chains, parallel in time over blocks of `len` slices (identical launches
+// read them as one shape, chain_shape):
+//   k_fx_chain_fwd      per (member, block): R_k = U_{k-1} ... U_{k0} into the P
+//                       slots (R_{k0} = I is implied) and the block product
+//                       into the block's first P slot (F only: U slot)
+//   k_fx_chain_combine  per member: T_b = the product before block b, z, f,
+//                       kappa; Lambda_b = T' (product after block b); W_b =
+//                       kappa T_b Lambda_b into the block's first P slot
+//   k_fx_chain_bwd      per (member, block): V_k = W_b U_{k1-1} ... U_{k+1}
+//                       into the U slots, so M_k = P_k Lambda_k = R_k V_k
+// A block product is a chain of its own, so short pulses of few members fill
+// the chip too; the forward, backward and gradient products are one each.
+template <int D> struct ChainCfg {
+  static constexpr int W = D >= 16 ? 2 : 1;
+  static constexpr int TEAMS = D >= 16 ? 4 : 8;          // (member, block) chains of a CTA
+  static constexpr int TEAM_BYTES = 2 * Geo<D, W>::PLANES + 64;
+  static constexpr int MAX_BLOCKS = D >= 16 ? 20 : 96;   // T_b and Lambda_b of a member in shared memory
+};
+
+template <int D, int W> struct ChainTeam {
+  Tm<D, W> tm;
+  uint32_t pl, pr;  // planes of the left and the right factor
+  __device__ __forceinline__ ChainTeam(unsigned char* smem, int team)
+      : tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
+           reinterpret_cast<uint32_t*>(smem + 2 * Geo<D, W>::PLANES)},
+        pl(smem_u32(smem)), pr(pl + Geo<D, W>::PLANES) {}
+  // (r, E) <- left (r, E); an operand that is not finite stays so
+  template <bool R_IS_LEFT>
+  __device__ __forceinline__ void step(long long (&r)[Geo<D, W>::NV], int& E, const long long (&x)[Geo<D, W>::NV], int Ex) {
+    tm.sync();  // the last product has read its planes
+    store_planes<D, W>(tm, R_IS_LEFT ? pl : pr, r, kSlices);
+    store_planes<D, W>(tm, R_IS_LEFT ? pr : pl, x, kSlices);
+    tm.sync();
+    mul<D, W>(tm, pl, pr, kChainLevels<D>, r);
+    const int e = normalize<D, W>(tm, r, E + Ex);
+    E = max(E, Ex) == kNotFinite ? kNotFinite : e;
+  }
+};
+
+template <int D, int W> __device__ __forceinline__ longlong2* slot(const Tm<D, W>& tm, double2* stack, size_t i) {
+  return tm.mine(reinterpret_cast<longlong2*>(stack + i * D * D));
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS)
+k_fx_chain_fwd(ProbDev p, WorkDev w, int blocks, int len, int store) {
+  using C = ChainCfg<D>;
+  constexpr int W = C::W, NV = Geo<D, W>::NV;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int team = threadIdx.x / (32 * W);
+  ChainTeam<D, W> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
+  const long item = (long)blockIdx.x * C::TEAMS + team;
+  if (item >= (long)p.n_members * blocks) return;  // whole teams
+  const int m = (int)(item / blocks), k0 = (int)(item % blocks) * len, k1 = min(p.n_t, k0 + len);
+  const size_t base = (size_t)m * p.n_t;
+  long long r[NV], x[NV];
+  get_ints<NV>(slot(ct.tm, w.U, base + k0), r);
+  int E = unpack<D, W>(r);
+  if (k0 + 1 < k1) get_ints<NV>(slot(ct.tm, w.U, base + k0 + 1), x);
+#pragma unroll 1
+  for (int k = k0 + 1; k < k1; ++k) {
+    long long u[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) u[v] = x[v];
+    const int Eu = unpack<D, W>(u);
+    if (k + 1 < k1) get_ints<NV>(slot(ct.tm, w.U, base + k + 1), x);  // while this product runs
+    if (store) put_packed<D, W>(slot(ct.tm, w.P, base + k), r, E);
+    ct.template step<false>(r, E, u, Eu);
+  }
+  put_packed<D, W>(slot(ct.tm, store ? w.P : w.U, base + k0), r, E);
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS)
+k_fx_chain_bwd(ProbDev p, WorkDev w, int blocks, int len) {
+  using C = ChainCfg<D>;
+  constexpr int W = C::W, NV = Geo<D, W>::NV;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int team = threadIdx.x / (32 * W);
+  ChainTeam<D, W> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
+  const long item = (long)blockIdx.x * C::TEAMS + team;
+  if (item >= (long)p.n_members * blocks) return;
+  const int m = (int)(item / blocks), k0 = (int)(item % blocks) * len, k1 = min(p.n_t, k0 + len);
+  const size_t base = (size_t)m * p.n_t;
+  const bool grape = p.grad_mode == GRAD_REF_GRAPE;  // Gradients.jl: the costate includes the slice's own U_k
+  long long r[NV], x[NV];
+  get_ints<NV>(slot(ct.tm, w.P, base + k0), r);
+  int E = unpack<D, W>(r);
+  get_ints<NV>(slot(ct.tm, w.U, base + k1 - 1), x);
+#pragma unroll 1
+  for (int k = k1 - 1; k >= k0; --k) {
+    long long u[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) u[v] = x[v];
+    const int Eu = unpack<D, W>(u);
+    if (k > k0) get_ints<NV>(slot(ct.tm, w.U, base + k - 1), x);
+    if (!grape) put_packed<D, W>(slot(ct.tm, w.U, base + k), r, E);
+    if (k > k0 || grape) ct.template step<true>(r, E, u, Eu);
+    if (grape) put_packed<D, W>(slot(ct.tm, w.U, base + k), r, E);
+  }
+}
+
+// x -> kappa x: each part times a double, in a common frame; returns its
+// exponent (the result is not normalised: |x| < 0.75 2^56 holds).
+template <int D, int W>
+__device__ __forceinline__ int scale_complex(long long (&x)[Geo<D, W>::NV], int E, double2 kap) {
+  constexpr int H = Geo<D, W>::NV / 2;
+  const int ex = max((int)((uint32_t)__double2hiint(kap.x) >> 20 & 0x7ff), (int)((uint32_t)__double2hiint(kap.y) >> 20 & 0x7ff));
+  if (ex == 0x7ff) return kNotFinite;
+  // parts below 2^(ex - 1022) in 60 fractional bits
+  const long long a = from_double(kap.x, ex, 7), b = from_double(kap.y, ex, 7);
+  const int a0 = (int)a, a1 = (int)((a + 0x80000000ll) >> 32), b0 = (int)b, b1 = (int)((b + 0x80000000ll) >> 32);
+#pragma unroll
+  for (int v = 0; v < H; ++v) {
+    const long long re = x[v] << 3, im = x[H + v] << 3;
+    const int r0 = (int)re, r1 = (int)((re + 0x80000000ll) >> 32);
+    const int i0 = (int)im, i1 = (int)((im + 0x80000000ll) >> 32);
+    const long long mr = 0x80000000ll + (long long)r1 * a0 + (long long)r0 * a1 - (long long)i1 * b0 - (long long)i0 * b1;
+    const long long mi = 0x80000000ll + (long long)r1 * b0 + (long long)r0 * b1 + (long long)i1 * a0 + (long long)i0 * a1;
+    x[v] = (long long)r1 * a1 - (long long)i1 * b1 + (mr >> 32);
+    x[H + v] = (long long)r1 * b1 + (long long)i1 * a1 + (mi >> 32);
+  }
+  return E == kNotFinite ? kNotFinite : E + ex - 1022 + 1;
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS)
+k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
+  using C = ChainCfg<D>;
+  constexpr int W = C::W;
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV, TEAMS = C::TEAMS;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double2 s_red[32 * W];
+  __shared__ double2 s_kap;
+  const int team = threadIdx.x / (32 * W);
+  ChainTeam<D, W> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
+  const Tm<D, W>& tm = ct.tm;
+  longlong2* Ts = reinterpret_cast<longlong2*>(smem_raw + (size_t)TEAMS * C::TEAM_BYTES);
+  longlong2* Ls = Ts + (size_t)blocks * (G::INTS / 16);
+  const int m = blockIdx.x;
+  const size_t base = (size_t)m * p.n_t;
+  double2* tot = want_grad ? w.P : w.U;  // where k_fx_chain_fwd left the block products
+  long long r[NV], x[NV];
+  if (team == 0) {  // T_1 = Tot_0, T_{b+1} = Tot_b T_b
+    get_ints<NV>(slot(tm, tot, base), r);
+    int E = unpack<D, W>(r);
+#pragma unroll 1
+    for (int b = 1; b < blocks; ++b) {
+      if (want_grad) put_packed<D, W>(tm.mine(Ts + (size_t)b * (G::INTS / 16)), r, E);
+      get_ints<NV>(slot(tm, tot, base + (size_t)b * len), x);
+      const int Ex = unpack<D, W>(x);
+      ct.template step<false>(r, E, x, Ex);
+    }
+    double2* Ut = w.Utot + (size_t)m * D * D;
+    if (E == kNotFinite) store_nan<D, W>(tm, Ut);
+    else store_mat<D, W>(tm, Ut, r, E - kFrac);
+    double2 acc = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int b = 0; b < NV / 2; ++b) {
+      double2 v = make_double2(to_double(r[b], E - kFrac), to_double(r[NV / 2 + b], E - kFrac));
+      if (E == kNotFinite) v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
+      acc = cmac_cj(acc, p.target_op[tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2)], v);
+    }
+    s_red[threadIdx.x] = acc;
+    tm.sync();
+    for (int h = 16 * W; h > 0; h >>= 1) {
+      if ((int)threadIdx.x < h) s_red[threadIdx.x] = cadd(s_red[threadIdx.x], s_red[threadIdx.x + h]);
+      tm.sync();
+    }
+    if (threadIdx.x == 0) {
+      double2 z = s_red[0], kap;
+      z.x /= p.D;
+      z.y /= p.D;
+      double f;
+      fid_kappa(z, p.fid, p.grad_mode, f, kap);
+      const double sc = p.m_weight[m] / p.D;
+      kap = make_double2(kap.x * sc, kap.y * sc);
+      w.z[m] = z;
+      w.kap[m] = kap;
+      w.Fm[m] = f;
+      s_kap = kap;
+    }
+  } else if (team == 1 && want_grad) {  // Lambda_B = T', Lambda_{b-1} = Lambda_b Tot_b
+    double t[NV];
+#pragma unroll
+    for (int b = 0; b < NV / 2; ++b) {
+      const double2 v = p.target_op[tm.col(b / 2 / G::NI, b % 2) + D * tm.row(b / 2 % G::NI)];
+      t[b] = v.x;
+      t[NV / 2 + b] = -v.y;
+    }
+    const int EX = max_exponent<D, W>(tm, t);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] = from_double(t[v], EX, 2);
+    int E = EX - 1021;
+#pragma unroll 1
+    for (int b = blocks - 1;; --b) {
+      put_packed<D, W>(tm.mine(Ls + (size_t)b * (G::INTS / 16)), r, E);
+      if (b == 0) break;
+      get_ints<NV>(slot(tm, tot, base + (size_t)b * len), x);
+      const int Ex = unpack<D, W>(x);
+      ct.template step<true>(r, E, x, Ex);
+    }
+  }
+  if (!want_grad) return;
+  __syncthreads();
+  const double2 kap = s_kap;
+  for (int b = team; b < blocks; b += TEAMS) {  // W_b = kappa T_b Lambda_b
+    get_ints<NV>(tm.mine(Ls + (size_t)b * (G::INTS / 16)), r);
+    int E = unpack<D, W>(r);
+    if (b > 0) {
+      get_ints<NV>(tm.mine(Ts + (size_t)b * (G::INTS / 16)), x);
+      const int Ex = unpack<D, W>(x);
+      ct.template step<false>(r, E, x, Ex);
+    }
+    E = scale_complex<D, W>(r, E, kap);
+    put_packed<D, W>(slot(tm, w.P, base + (size_t)b * len), r, E);
   }
 }
 
@@ -536,9 +797,9 @@ constexpr size_t kSmemMax = 232448;  // dynamic shared memory of a CTA
 
 // Launches a slice-parallel kernel of configuration C (dimension D): as many
 // teams as the shared memory beside the generator's terms holds.
-template <class C, int D>
-static cudaError_t launch_slices(void (*kernel)(ProbDev, WorkDev, int), const ProbDev& p, const WorkDev& w,
-                                 const LaunchInfo& li) {
+template <class C, int D, class... A>
+static cudaError_t launch_slices(void (*kernel)(ProbDev, WorkDev, int, A...), const ProbDev& p, const WorkDev& w,
+                                 const LaunchInfo& li, A... more) {
   const int n = p.n_c + 1 + (p.n_ramp ? 1 : 0);
   const size_t consts = Terms<D, C::W>::bytes(n);
   const int fit = (int)((kSmemMax - consts) / C::TEAM_BYTES);
@@ -557,9 +818,58 @@ static cudaError_t launch_slices(void (*kernel)(ProbDev, WorkDev, int), const Pr
   const int run = (int)rounds * nt;
   long grid = (long)p.n_members * ((p.n_t + run - 1) / run);
   if (grid > ctas) grid = ctas;
-  kernel<<<(int)grid, threads, smem, li.stream>>>(p, w, run);
+  kernel<<<(int)grid, threads, smem, li.stream>>>(p, w, run, more...);
   ++*li.launches;
   return cudaGetLastError();
+}
+
+// Blocks of the gate chains.  Chains run in two dependent passes of `len`
+// products with one of `blocks` between: more blocks than sqrt(2 n_t) only
+// lengthen the sum, and more (member, block) chains than the SMs hold (about
+// 10 of 14 KB at D = 16, 24 of 4 KB at D = 8) run as a second wave.
+template <int D> static void chain_shape(const ProbDev& p, int num_sms, int* blocks, int* len) {
+  const long chains = (long)num_sms * (D >= 16 ? 10 : 24);
+  long b = chains / p.n_members;
+  long most = 1;
+  while (most < ChainCfg<D>::MAX_BLOCKS && (most + 1) * (most + 1) <= 2L * p.n_t) ++most;
+  if (b > most) b = most;
+  if (b < 1) b = 1;
+  *len = (int)((p.n_t + b - 1) / b);
+  *blocks = (p.n_t + *len - 1) / *len;
+}
+
+template <int D> static cudaError_t do_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  using C = ChainCfg<D>;
+  int blocks, len;
+  chain_shape<D>(p, li.num_sms, &blocks, &len);
+  const size_t smem = (size_t)C::TEAMS * C::TEAM_BYTES;
+  const int threads = 32 * C::W * C::TEAMS;
+  set_smem_once((const void*)k_fx_chain_fwd<D>, smem);
+  const long items = (long)p.n_members * blocks;
+  k_fx_chain_fwd<D><<<(int)((items + C::TEAMS - 1) / C::TEAMS), threads, smem, li.stream>>>(p, w, blocks, len, store ? 1 : 0);
+  const size_t smem2 = smem + (store ? (size_t)2 * blocks * Geo<D, C::W>::INTS : 0);
+  set_smem_once((const void*)k_fx_chain_combine<D>, smem2);
+  k_fx_chain_combine<D><<<p.n_members, threads, smem2, li.stream>>>(p, w, blocks, len, store ? 1 : 0);
+  *li.launches += 2;
+  return cudaGetLastError();
+}
+
+template <int D> static cudaError_t do_chain_bwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  using C = ChainCfg<D>;
+  int blocks, len;
+  chain_shape<D>(p, li.num_sms, &blocks, &len);
+  const size_t smem = (size_t)C::TEAMS * C::TEAM_BYTES;
+  set_smem_once((const void*)k_fx_chain_bwd<D>, smem);
+  const long items = (long)p.n_members * blocks;
+  k_fx_chain_bwd<D><<<(int)((items + C::TEAMS - 1) / C::TEAMS), 32 * C::W * C::TEAMS, smem, li.stream>>>(p, w, blocks, len);
+  ++*li.launches;
+  return cudaGetLastError();
+}
+
+template <int D> static cudaError_t do_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  int blocks, len;
+  chain_shape<D>(p, li.num_sms, &blocks, &len);
+  return launch_slices<GradCfg<D>, D>(k_fx_grad<D>, p, w, li, len);
 }
 
 }  // namespace fx
@@ -571,9 +881,14 @@ cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo&
   return p.Dp == 8 ? fx::launch_slices<fx::ExpmCfg<8>, 8>(fx::k_fx_expm<8>, p, w, li)
                    : fx::launch_slices<fx::ExpmCfg<16>, 16>(fx::k_fx_expm<16>, p, w, li);
 }
+cudaError_t launch_fx_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  return p.Dp == 8 ? fx::do_chain_fwd<8>(p, w, li, store) : fx::do_chain_fwd<16>(p, w, li, store);
+}
+cudaError_t launch_fx_chain_bwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  return p.Dp == 8 ? fx::do_chain_bwd<8>(p, w, li) : fx::do_chain_bwd<16>(p, w, li);
+}
 cudaError_t launch_fx_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  return p.Dp == 8 ? fx::launch_slices<fx::GradCfg<8>, 8>(fx::k_fx_grad<8>, p, w, li)
-                   : fx::launch_slices<fx::GradCfg<16>, 16>(fx::k_fx_grad<16>, p, w, li);
+  return p.Dp == 8 ? fx::do_grad<8>(p, w, li) : fx::do_grad<16>(p, w, li);
 }
 
 }  // namespace pgx

@@ -251,6 +251,10 @@ __device__ __forceinline__ void mul(const Tm<D, W>& tm, uint32_t pa, uint32_t pb
         t[v] = kt == 0 ? x : t[v] + x;
       }
     }
+    if (L == 0) {  // to nearest: a floor's bias adds up over a chain of products
+#pragma unroll
+      for (int v = 0; v < NV; ++v) r[v] += 0x8000;
+    }
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       const int hi = (int)(r[v] >> 32);
@@ -404,7 +408,7 @@ struct Scaled {
   }
   __device__ __forceinline__ long long operator()(long long x, long long r) const {
     const int b1 = (int)(x >> 32);
-    const long long mid = (long long)((unsigned long long)(uint32_t)x * (uint32_t)m1) + (long long)b1 * m0;
+    const long long mid = (long long)((unsigned long long)(uint32_t)x * (uint32_t)m1) + 0x80000000ll + (long long)b1 * m0;
     return r + (long long)b1 * m1 + (long long)(int)(mid >> 32);
   }
 };
@@ -420,9 +424,9 @@ __device__ __forceinline__ void add_scaled(long long (&r)[NV], const longlong2* 
 // r (56 fractional bits at e) -> F fractional bits in frame fr.
 template <int NV> __device__ __forceinline__ void to_frame(long long (&r)[NV], int e, int fr, int F) {
   const int sh = fr - e + kFrac - F;
-  if (sh >= 0) {
+  if (sh > 0) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v) r[v] >>= min(sh, 63);
+    for (int v = 0; v < NV; ++v) r[v] = shift_round(r[v], min(sh, 63));
   } else {
 #pragma unroll
     for (int v = 0; v < NV; ++v) r[v] <<= -sh;
@@ -449,6 +453,27 @@ __device__ __forceinline__ void load_mat(const Tm<D, W>& tm, const double2* A, d
     x[G::NV / 2 + b] = a.y;
   }
 }
+// A normalised matrix in global memory, lane-private: x << 7 with its exponent
+// in the low seven bits of each lane's first three values.
+constexpr int kExpBias = 1 << 20;
+constexpr int kNotFinite = kExpBias - 1;  // the exponent of a matrix with no finite value
+template <int D, int W>
+__device__ __forceinline__ void put_packed(longlong2* s, const long long (&x)[Geo<D, W>::NV], int E) {
+  constexpr int NV = Geo<D, W>::NV;
+  const int e = max(min(E, kNotFinite), -kExpBias) + kExpBias;
+  long long y[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) y[v] = (x[v] << 7) | (v < 3 ? (e >> (7 * v)) & 127 : 0);
+  put_ints<NV>(s, y);
+}
+template <int D, int W>
+__device__ __forceinline__ int unpack(long long (&x)[Geo<D, W>::NV]) {
+  const int e = (int)(x[0] & 127) | (int)(x[1] & 127) << 7 | (int)(x[2] & 127) << 14;
+#pragma unroll
+  for (int v = 0; v < Geo<D, W>::NV; ++v) x[v] >>= 7;
+  return e - kExpBias;
+}
+
 // U = r 2^ex
 template <int D, int W>
 __device__ __forceinline__ void store_mat(const Tm<D, W>& tm, double2* U, const long long (&r)[Geo<D, W>::NV], int ex) {

@@ -221,11 +221,15 @@ cudaError_t launch_residual(const ProbDev& p, const WorkDev& w, int kind, int N,
 // G[q] = sum_i coef[i] Gm[idx[i]][q] (len = n_c n_t), in the order of idx.
 cudaError_t launch_select_sum(const double* Gm, const int* idx, const double* coef, int n_sel, int len, double* G,
                               const LaunchInfo& li);
-// The FP64 path's slice propagators and exact gradient on block fixed-point
-// tensor-core products (pgx_fx.cu): Dp = 8 and 16 with at most 24 generator
-// terms (drift, controls, ramp).
+// The FP64 path on block fixed-point tensor-core products (pgx_fx.cu): Dp = 8
+// and 16 with at most 24 generator terms (drift, controls, ramp).  Slice
+// propagators for every target (gate targets: in the gate chains' own format),
+// the gate chains, and the gradient of gate targets (any mode) and of exact
+// state targets.
 bool fx_applies(const ProbDev& p);
 cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
+cudaError_t launch_fx_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
+cudaError_t launch_fx_chain_bwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 cudaError_t launch_fx_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 // Mixed-precision stages (pgx_mixed.cu), gate targets: df expm and forward
 // chain, FP32 backward chain and gradient.  U stack holds df (float4), the P

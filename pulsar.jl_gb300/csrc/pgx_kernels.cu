@@ -754,6 +754,7 @@ static cudaError_t do_chain_fwd(const ProbDev& p, const WorkDev& w, const Launch
   return cudaGetLastError();
 }
 cudaError_t launch_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  if (p.target == TGT_GATE && fx_applies(p)) return launch_fx_chain_fwd(p, w, li, store);
   PGX_DISPATCH(p.Dp, return do_chain_fwd<D_>(p, w, li, store));
   return cudaSuccess;
 }
@@ -777,6 +778,7 @@ static cudaError_t do_chain_bwd(const ProbDev& p, const WorkDev& w, const Launch
   return cudaGetLastError();
 }
 cudaError_t launch_chain_bwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  if (p.target == TGT_GATE && fx_applies(p)) return launch_fx_chain_bwd(p, w, li);
   PGX_DISPATCH(p.Dp, return do_chain_bwd<D_>(p, w, li));
   return cudaSuccess;
 }
@@ -793,7 +795,7 @@ static cudaError_t do_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo&
   return cudaGetLastError();
 }
 cudaError_t launch_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  if (p.grad_mode == GRAD_EXACT && fx_applies(p)) return launch_fx_grad(p, w, li);
+  if ((p.target == TGT_GATE || p.grad_mode == GRAD_EXACT) && fx_applies(p)) return launch_fx_grad(p, w, li);
   PGX_DISPATCH(p.Dp, return do_grad<D_>(p, w, li));
   return cudaSuccess;
 }

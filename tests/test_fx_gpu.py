@@ -86,3 +86,37 @@ def test_exact_gradient(pg, target, gen, D, n_t, n_m, nrm):
     p.close()
     assert abs(F - Fo) <= 1e-10
     assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
+
+
+@pytest.mark.parametrize("mode", ["exact", "ref_mr", "ref_grape"])
+@pytest.mark.parametrize("D,n_t,n_m", [(5, 1, 2), (8, 7, 1), (8, 301, 2), (11, 2, 1), (16, 67, 1), (16, 41, 200)])
+def test_gate_chain_blocks(pg, mode, D, n_t, n_m):
+    """Gate chains in one block, in blocks with a short last one, of one slice,
+    and of many members, in every gradient mode; F-only gives the same F.  Bars
+    as above."""
+    from oracle import members as mb
+    rng = np.random.default_rng(7 * D + n_t)
+    dag = lambda x: np.swapaxes(x.conj(), -1, -2)  # noqa: E731
+    X = rng.normal(size=(3, D, D)) + 1j * rng.normal(size=(3, D, D))
+    X = X + dag(X)
+    Q, _ = np.linalg.qr(rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D)))
+    u = rng.normal(size=(2, n_t))
+    kw = dict(drifts=X[:1], controls=X[1:], dt=np.full(n_t, 0.3 / (D + 4)), member_scale=rng.uniform(0.9, 1.1, n_m),
+              target="gate", fidelity="square", target_op=Q)
+    Fo, Go = mb.eval_problem(mb.Problem(n_members=n_m, **kw), u, mode) if n_t * n_m < 2000 else (None, None)
+    p = pg.Problem(grad_mode=mode, precision="fp64", **kw)
+    F, G = p.eval(u)
+    F1, _ = p.eval(u, want_grad=False)
+    Ut = p.total_propagator(u, member=n_m - 1)
+    F2, G2 = p.eval(u)
+    p.close()
+    assert F1 == F and F2 == F and np.array_equal(G, G2)
+    assert np.abs(dag(Ut) @ Ut - np.eye(D)).max() <= n_t * (D + 40) * 2.0 ** -53
+    if Fo is None:  # many members: mean over two of them against the oracle
+        kw["member_scale"] = kw["member_scale"][[0, n_m - 1]]
+        Fo, Go = mb.eval_problem(mb.Problem(n_members=2, **kw), u, mode)
+        p = pg.Problem(grad_mode=mode, precision="fp64", **kw)
+        F, G = p.eval(u)
+        p.close()
+    assert abs(F - Fo) <= 1e-10
+    assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
