@@ -10,6 +10,7 @@ static __constant__ float c_log2theta[PGX_N_FXDEGREES] = PGX_LOG2_THETA64_EVEN_I
 static __constant__ Coef c_coef[PGX_N_INVFACT] = PGX_INVFACT_FX_INIT;
 
 constexpr int kMaxTerms = 24;       // generator terms: drift, controls, ramp
+constexpr int kMaxTerms32 = 7;      // at D = 32: 16 KB of shared memory each beside two teams
 constexpr int kBits = 57;           // absolute error of a slice propagator: 2^-57 per product
 constexpr int kBits2 = 2 * kBits + 1;
 constexpr int kNever = 1 << 20;     // an exponent no finite entry reaches
@@ -129,10 +130,10 @@ __device__ __forceinline__ int assemble(const Terms<D, W>& T, const ProbDev& p, 
   return EA;
 }
 
-// log2 of a bound of ||A||_1 (58 fractional bits in frame EA), D <= 16.
+// log2 of a bound of ||A||_1 (58 fractional bits in frame EA): the largest
+// column sum, from D = 32 on over each warp's rows and then added up.
 template <int D, int W> __device__ __forceinline__ float log2_norm1(const Tm<D, W>& tm, const long long (&A)[Geo<D, W>::NV], int EA) {
   using G = Geo<D, W>;
-  static_assert(G::RT == 1, "a column's rows belong to one warp");
   float best = 0.f;
 #pragma unroll
   for (int nt = 0; nt < G::NTW; ++nt)
@@ -149,7 +150,22 @@ template <int D, int W> __device__ __forceinline__ float log2_norm1(const Tm<D, 
       for (int o = 4; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       best = fmaxf(best, s);
     }
-  best = __uint_as_float(tm.max(__float_as_uint(best), 1));
+  if constexpr (G::RT == 1) {
+    best = __uint_as_float(tm.max(__float_as_uint(best), 1));
+  } else {
+    best = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(best)));
+    volatile uint32_t* part = tm.red + W;  // slot 1
+    if (tm.lane == 0) part[tm.w] = __float_as_uint(best);
+    tm.sync();
+    best = 0.f;
+#pragma unroll
+    for (int c = 0; c < G::CG; ++c) {
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < G::RT; ++i) s += __uint_as_float(part[c * G::RT + i]);
+      best = fmaxf(best, s);
+    }
+  }
   return __log2f(fmaf(best, 1.00001f, 2.f * D)) + (float)(EA - 26) + 1e-5f;
 }
 
@@ -166,10 +182,16 @@ __device__ __forceinline__ void choose_degree2(float l2, int lane, int& L, int& 
   L = 2 + (int)(key & 0xff);
 }
 
+// Warps of a matrix: eight columns each (and, at D = 32, sixteen rows).
+template <int D> constexpr int kWarps = D >= 32 ? 8 : D >= 16 ? 2 : 1;
+constexpr int kRed = 128;  // bytes of a team's maxima
+
 template <int D> struct ExpmCfg {
-  static constexpr int W = D >= 16 ? 2 : 1;             // warps of a slice
-  static constexpr int TEAMS = D >= 16 ? 10 : 12;       // slices in flight per CTA, at most
-  static constexpr int TEAM_BYTES = 2 * Geo<D, W>::PLANES + Geo<D, W>::INTS + 64;  // planes of X, of Y; B; maxima
+  static constexpr int W = kWarps<D>;
+  static constexpr int TEAMS = D >= 32 ? 2 : D >= 16 ? 10 : 12;  // slices in flight per CTA, at most
+  static constexpr bool REG_B = D >= 32;                         // B stays in registers
+  // planes of X, of Y; B; maxima
+  static constexpr int TEAM_BYTES = 2 * Geo<D, W>::PLANES + (REG_B ? 0 : Geo<D, W>::INTS) + kRed;
 };
 
 // U_mk = exp(A_mk), one team per slice: T_2L(A / 2^s) in the q = 2
@@ -195,8 +217,9 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
   unsigned char* mine = smem_raw + Terms<D, W>::bytes(T.n) + (size_t)team * C::TEAM_BYTES;
   const uint32_t px = smem_u32(mine), py = px + G::PLANES;
   const Tm<D, W> tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
-                    reinterpret_cast<uint32_t*>(mine + 2 * G::PLANES + G::INTS)};
+                    reinterpret_cast<uint32_t*>(mine + C::TEAM_BYTES - kRed)};
   longlong2* Bs = tm.mine(reinterpret_cast<longlong2*>(mine + 2 * G::PLANES));
+  long long bx[C::REG_B ? NV : 1];
   for (int j = team; j < p.n_c; j += nt) {
     double x[NV];
     load_mat<D, W>(tm, p.ctrls + (size_t)j * D * D, x);
@@ -254,7 +277,12 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
           long long x6[NV];
 #pragma unroll
           for (int v = 0; v < NV; ++v) x6[v] = r[v] << 6;
-          put_ints<NV>(Bs, x6);
+          if constexpr (C::REG_B) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) bx[v] = x6[v];
+          } else {
+            put_ints<NV>(Bs, x6);
+          }
         }
         store_planes<D, W>(tm, py, r, n);
         tm.sync();
@@ -275,7 +303,13 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
             F = i > 0 ? kFrac : 60;
             to_frame<NV>(r, EX + EY, fr, F);
           }
-          add_scaled<NV>(r, Bs, Scaled(c_coef[2 * i + 1], EB, fr, F));
+          const Scaled sb(c_coef[2 * i + 1], EB, fr, F);
+          if constexpr (C::REG_B) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) r[v] = sb(bx[v], r[v]);
+          } else {
+            add_scaled<NV>(r, Bs, sb);
+          }
           add_diag<D, W>(tm, r, c_coef[2 * i], fr, F);
           EY = fr;
           if (i == 0) {
@@ -298,14 +332,15 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
   }
 }
 
-// M_k of a state target in the team's order: sum_s psi_s[k] lambda_s[k+1]'.
+// sum_s psi_s[k] lambda_s[kl]' of a state target in the team's order: M_k (kl =
+// k + 1) or N_k = M_k U_k (kl = k).
 template <int D, int W>
-__device__ __forceinline__ void load_M(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m, int k,
+__device__ __forceinline__ void load_M(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m, int k, int kl,
                                        double (&x)[Geo<D, W>::NV]) {
   using G = Geo<D, W>;
   const int np = p.n_pairs;
   const double2* psi = w.psi + ((size_t)m * (p.n_t + 1) + k) * np * D;
-  const double2* lam = w.lam + ((size_t)m * (p.n_t + 1) + k + 1) * np * D;
+  const double2* lam = w.lam + ((size_t)m * (p.n_t + 1) + kl) * np * D;
 #pragma unroll
   for (int v = 0; v < G::NV; ++v) x[v] = 0.0;
   for (int s = 0; s < np; ++s)
@@ -332,7 +367,7 @@ __device__ __forceinline__ long long trace_term(const Terms<D, W>& T, const Tm<D
   for (int b = 0; b < G::NV / 2; ++b) {
     // element (row', col') = (col, row) of the term in the team's layout
     const int r = tm.col(b / 2 / G::NI, b % 2), c = tm.row(b / 2 % G::NI);
-    const int nt = c / 8 % G::NTW, wt = c / 8 / G::NTW;
+    const int nt = c / 8 % G::NTW, wt = c / 8 / G::NTW * G::RT + (D >= 16 ? r / 16 : 0);
     const int v = 2 * (nt * G::NI + r / 8 % G::NI) + c % 2;
     const int2* e = kp + ((size_t)(wt * (G::NV / 2) + v / 2) * 32 + (r % 8) * 4 + c % 8 / 2) * 2 + v % 2;
     const int2 cr = e[0], ci = e[(G::NV / 4) * 64];
@@ -355,24 +390,88 @@ __device__ __forceinline__ long long trace_term(const Terms<D, W>& T, const Tm<D
 }
 
 constexpr int kGradBits2 = 2 * 56 + 1;
+constexpr unsigned long long kTodo = 0x7ff8dead00000001ull;  // a slice left to k_fx_grad_norm (a NaN no sum produces)
 
-template <int D> struct GradCfg {
-  static constexpr int W = D >= 16 ? 2 : 1;
-  static constexpr int TEAMS = D >= 16 ? 7 : 12;
-  // planes of X, dX, Y, dY; maxima; the warps' traces
-  static constexpr int TEAM_BYTES = 4 * Geo<D, W>::PLANES + 64 + (W > 1 ? kMaxTerms * 8 : 0);
+template <int D> constexpr int kTraces = D >= 32 ? kMaxTerms32 + 1 : kMaxTerms;
+template <int D, int PLANE_SETS, int MAX_TEAMS> struct GradCfg {
+  static constexpr int W = kWarps<D>;
+  static constexpr int TEAMS = MAX_TEAMS;
+  static constexpr int TRACES = W > 1 ? W * kTraces<D> * 8 : 0;  // the warps' traces
+  static constexpr int TEAM_BYTES = PLANE_SETS * Geo<D, W>::PLANES + kRed + TRACES;
 };
+template <int D> using SeriesCfg = GradCfg<D, 2, (D >= 32 ? 2 : D >= 16 ? 10 : 12)>;
+template <int D> using NormCfg = GradCfg<D, 4, (D >= 32 ? 1 : D >= 16 ? 7 : 12)>;
 
-// g_jk = Re(c dt scale Tr(L(A_k, M_k) C_j)), one team per slice: the Frechet
-// derivative of T_2L(A / 2^s)^(2^s) in the q = 2 form (three products a step),
-// carried in block fixed point like the propagator.  The derivative's matrices
-// keep an exponent of their own, so any magnitude of M_k does.
+// g_jk = cds {Re, Im} Tr(X C_j), X 2^(E - 56) the team's: integer traces, lane
+// j keeps control j's.  `traces` is free again after the team's next sync.
+template <int D, int W>
+__device__ __forceinline__ void put_traces(const Terms<D, W>& T, const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w,
+                                           int m, int k, const long long (&x)[Geo<D, W>::NV], int E, long long* traces) {
+  long long keep = 0;
+#pragma unroll 1
+  for (int j = 0; j < p.n_c; ++j) {
+    const long long t = trace_term<D, W>(T, tm, j + 1, p.gen == GEN_HERM ? 1 : 0, x);
+    if constexpr (W > 1) {
+      if (tm.lane == 0) traces[tm.w * kTraces<D> + j] = t;
+    }
+    if (tm.lane == j) keep = t;
+  }
+  if constexpr (W > 1) tm.sync();
+  if (tm.w == 0 && tm.lane < p.n_c) {
+    if constexpr (W > 1) {
+#pragma unroll
+      for (int i = 1; i < W; ++i) keep += traces[i * kTraces<D> + tm.lane];
+    }
+    w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] = p.dt[k] * p.m_scale[m] * to_double(keep, E + T.e[tm.lane + 1] - 55);
+  }
+}
+template <int D, int W>
+__device__ __forceinline__ void put_grad_value(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m, int k,
+                                               unsigned long long bits) {
+  if (tm.w == 0 && tm.lane < p.n_c)
+    w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] = __longlong_as_double((long long)bits);
+}
+
+template <int D, int W> __device__ __forceinline__ longlong2* slot(const Tm<D, W>& tm, double2* stack, size_t i) {
+  return tm.mine(reinterpret_cast<longlong2*>(stack + i * D * D));
+}
+
+// (x, E) <- R_k x, the product before slice k inside its block (the identity at
+// its start); x's digits go to pr, R_k's to pl.  The result is normalised.
+template <int D, int W>
+__device__ __forceinline__ void times_prefix(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m, int k, int len,
+                                             uint32_t pl, uint32_t pr, long long (&x)[Geo<D, W>::NV], int& E) {
+  if (k % len == 0) return;
+  long long r[Geo<D, W>::NV];
+  get_ints<Geo<D, W>::NV>(slot(tm, w.P, (size_t)m * p.n_t + k), r);
+  const int ER = unpack<D, W>(r);
+  tm.sync();  // the last slice's products have read their planes
+  store_planes<D, W>(tm, pr, x, kSlices);
+  store_planes<D, W>(tm, pl, r, kSlices);
+  tm.sync();
+  mul<D, W>(tm, pl, pr, kChainLevels<D>, x);
+  const int e = normalize<D, W>(tm, x, E + ER);
+  E = max(E, ER) == kNotFinite ? kNotFinite : e;
+}
+
+// The gradient of gate targets in any mode, and of exact state targets.  One
+// team per slice: g_jk = Re(c dt scale Tr(X C_j)).
 //
-// Bound: instruction issue, then the tensor pipe.  Four matrices' planes (28 KB
-// at D = 16) limit an SM to seven slices; B and dB stay in registers.
+// Exact: X = L_exp(A, M) = sum_n ad_A^n(N) / (n + 1)!, N = M e^A = P_k
+// Lambda_{k-1} (ad_A X = A X - X A commutes with the factor e^A).  Two products
+// and one matrix a term, each term in block fixed point with the levels its
+// size asks for, until it is below 2^-56 of N: about ten terms at ||A|| = 0.15.
+// The Paterson-Stockmeyer derivative takes as many digit products, but four
+// matrices' planes where this takes two, so half as many slices an SM.  Where
+// the terms grow (norms above 2 or so), cancellation would cost bits: such
+// slices are left to k_fx_grad_norm.
+// First order: X = M_k = R_k V_k, or with the costate that includes U_k.
+//
+// Bound: instruction issue, then the tensor pipe.
 template <int D>
-__global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_grad(ProbDev p, WorkDev w, int run, int len) {
-  using C = GradCfg<D>;
+__global__ void __launch_bounds__(32 * SeriesCfg<D>::TEAMS * SeriesCfg<D>::W)
+k_fx_grad(ProbDev p, WorkDev w, int run, int len) {
+  using C = SeriesCfg<D>;
   constexpr int W = C::W;
   using G = Geo<D, W>;
   constexpr int NV = G::NV;
@@ -383,10 +482,10 @@ __global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_g
   T.k = reinterpret_cast<int4*>(smem_raw);
   T.e = reinterpret_cast<int*>(smem_raw + (size_t)T.n * G::INTS);
   unsigned char* mine = smem_raw + Terms<D, W>::bytes(T.n) + (size_t)team * C::TEAM_BYTES;
-  const uint32_t px = smem_u32(mine), pdx = px + G::PLANES, py = px + 2 * G::PLANES, pdy = px + 3 * G::PLANES;
+  const uint32_t pa = smem_u32(mine), pd = pa + G::PLANES;
   const Tm<D, W> tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
-                    reinterpret_cast<uint32_t*>(mine + 4 * G::PLANES)};
-  long long* traces = reinterpret_cast<long long*>(mine + 4 * G::PLANES + 64);  // W > 1
+                    reinterpret_cast<uint32_t*>(mine + 2 * G::PLANES)};
+  long long* traces = reinterpret_cast<long long*>(mine + 2 * G::PLANES + kRed);
   for (int j = team; j < p.n_c; j += nt) {
     double x[NV];
     load_mat<D, W>(tm, p.ctrls + (size_t)j * D * D, x);
@@ -405,41 +504,155 @@ __global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_g
     const int k1 = min(p.n_t, k0 + run);
 #pragma unroll 1
     for (int k = k0 + team; k < k1; k += nt) {
+      long long x[NV];
+      int E;  // N (exact) or M = x 2^(E - 56)
+      if (p.target == TGT_GATE) {
+        // slot k holds V_k U_k = Lambda_{k-1} up to the block's prefix; V_k is
+        // the next slice's, or W_b at the end of the block
+        if (p.grad_mode != GRAD_REF_MR) get_ints<NV>(slot(tm, w.U, (size_t)m * p.n_t + k), x);
+        else if ((k + 1) % len != 0 && k + 1 < p.n_t) get_ints<NV>(slot(tm, w.U, (size_t)m * p.n_t + k + 1), x);
+        else get_ints<NV>(slot(tm, w.P, (size_t)m * p.n_t + k / len * len), x);
+        E = unpack<D, W>(x);
+        times_prefix<D, W>(tm, p, w, m, k, len, pa, pd, x, E);
+      } else {
+        double d[NV];
+        load_M<D, W>(tm, p, w, m, k, k, d);
+        const int EXd = max_exponent<D, W>(tm, d);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) x[v] = from_double(d[v], EXd, 2);
+        E = EXd == 0x7ff ? kNotFinite : EXd - 1021;
+      }
+      tm.sync();
+      if (p.grad_mode == GRAD_EXACT && E != kNotFinite) {
+        long long sum[NV], r[NV];
+        const int EA = assemble<D, W>(T, p, w.u, m, k, tm, r);
+        const float l2 = log2_norm1<D, W>(tm, r, EA);
+        bool todo = l2 > 1.3f;
+        if (EA > kNever / 2) E = kNotFinite;
+        else if (!todo) {
+          const int EB = normalize<D, W, true>(tm, r, EA - 2);
+          store_planes<D, W>(tm, pa, r, kSlices);
+          tm.sync();  // the maxima are read
+          const int EN = normalize<D, W, true>(tm, x, E), fr = EN + 3;
+#pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            r[v] = x[v];
+            sum[v] = x[v] << 1;  // 60 fractional bits in frame EN + 3
+          }
+          int Er = EN;
+          float size = 1.f;  // of the terms, in units of N: below 7 the sum stays inside its frame
+          todo = true;
+#pragma unroll 1
+          for (int n = 1; n < PGX_N_INVFACT - 1; ++n) {
+            const Coef cf = c_coef[n + 1];
+            const int lev = (kGradBits2 + 2 * (EB + Er + cf.exp - EN) + 15) >> 4;
+            if (lev <= 0) {
+              todo = false;
+              break;
+            }
+            tm.sync();
+            store_planes<D, W>(tm, pd, r, min(lev, kSlices));
+            tm.sync();
+            commutator<D, W>(tm, pa, pd, min(lev, kMaxLevels), r);
+            Er = normalize<D, W, true>(tm, r, EB + Er);
+            size += exp2f((float)(Er + cf.exp - EN));
+            if (size > 7.f) break;
+            const Scaled sc(cf, Er, fr, 60);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) sum[v] = sc(r[v] << 6, sum[v]);
+          }
+          tm.sync();
+          E = normalize<D, W>(tm, sum, fr - 4);
+#pragma unroll
+          for (int v = 0; v < NV; ++v) x[v] = sum[v];
+        }
+        if (todo && E != kNotFinite) {
+          put_grad_value<D, W>(tm, p, w, m, k, kTodo);
+          tm.sync();
+          continue;
+        }
+      }
+      if (E == kNotFinite) {
+        put_grad_value<D, W>(tm, p, w, m, k, 0x7ff8000000000000ull);
+        tm.sync();
+      } else {
+        put_traces<D, W>(T, tm, p, w, m, k, x, E, traces);
+        tm.sync();  // the maxima and the traces are read
+      }
+    }
+  }
+}
+
+// The slices k_fx_grad left (kTodo): large norms.  X = L_f(A_k, M_k), the
+// Frechet derivative of f = T_2L(A / 2^s)^(2^s) in the q = 2 form (three
+// products a step).  The derivative's matrices keep an exponent of their own,
+// so any magnitude of M_k does.  Runs with no such slice cost one pass over
+// their flags.
+template <int D>
+__global__ void __launch_bounds__(32 * NormCfg<D>::TEAMS * NormCfg<D>::W)
+k_fx_grad_norm(ProbDev p, WorkDev w, int run, int len) {
+  using C = NormCfg<D>;
+  constexpr int W = C::W;
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int team = threadIdx.x / (32 * W), nt = blockDim.x / (32 * W);
+  Terms<D, W> T;
+  T.n = p.n_c + 1 + (p.n_ramp ? 1 : 0);
+  T.k = reinterpret_cast<int4*>(smem_raw);
+  T.e = reinterpret_cast<int*>(smem_raw + (size_t)T.n * G::INTS);
+  unsigned char* mine = smem_raw + Terms<D, W>::bytes(T.n) + (size_t)team * C::TEAM_BYTES;
+  const uint32_t px = smem_u32(mine), pdx = px + G::PLANES, py = px + 2 * G::PLANES, pdy = px + 3 * G::PLANES;
+  const Tm<D, W> tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
+                    reinterpret_cast<uint32_t*>(mine + 4 * G::PLANES)};
+  long long* traces = reinterpret_cast<long long*>(mine + 4 * G::PLANES + kRed);
+  const int runs = (p.n_t + run - 1) / run;
+  int cur = -1;
+  for (long c = blockIdx.x; c < (long)p.n_members * runs; c += gridDim.x) {
+    const int m = (int)(c / runs), k0 = (int)(c % runs) * run, k1 = min(p.n_t, k0 + run);
+    bool any = false;
+    for (int k = k0 + (int)threadIdx.x; k < k1; k += blockDim.x)
+      any |= (unsigned long long)__double_as_longlong(w.Gm[((size_t)m * p.n_t + k) * p.n_c]) == kTodo;
+    if (!__syncthreads_or(any)) continue;
+    if (cur < 0)
+      for (int j = team; j < p.n_c; j += nt) {
+        double x[NV];
+        load_mat<D, W>(tm, p.ctrls + (size_t)j * D * D, x);
+        put_term<D, W>(T, j + 1, tm, x);
+      }
+    if (m != cur) {
+      if (team == 0) put_member_terms<D, W>(T, p, m, tm);
+      cur = m;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = k0 + team; k < k1; k += nt) {
+      if ((unsigned long long)__double_as_longlong(w.Gm[((size_t)m * p.n_t + k) * p.n_c]) != kTodo) continue;
       long long b[NV], db[NV], r[NV], q[NV];
       int EM;  // M_k = db 2^(EM - 56)
       if (p.target == TGT_GATE) {
-        // M_k = R_k V_k of the chains (R = I at the start of a block)
-        get_ints<NV>(tm.mine((longlong2*)(w.U + ((size_t)m * p.n_t + k) * D * D)), db);
+        if ((k + 1) % len != 0 && k + 1 < p.n_t) get_ints<NV>(slot(tm, w.U, (size_t)m * p.n_t + k + 1), db);
+        else get_ints<NV>(slot(tm, w.P, (size_t)m * p.n_t + k / len * len), db);
         EM = unpack<D, W>(db);
-        if (k % len != 0) {
-          get_ints<NV>(tm.mine((longlong2*)(w.P + ((size_t)m * p.n_t + k) * D * D)), r);
-          const int ER = unpack<D, W>(r);
-          tm.sync();  // the last slice's products have read their planes
-          store_planes<D, W>(tm, py, db, kSlices);
-          store_planes<D, W>(tm, px, r, kSlices);
-          tm.sync();
-          if (max(EM, ER) == kNotFinite) EM = kNotFinite;
-          else {
-            mul<D, W>(tm, px, py, kChainLevels<D>, db);
-            EM = normalize<D, W>(tm, db, EM + ER);
-          }
-        }
+        times_prefix<D, W>(tm, p, w, m, k, len, px, py, db, EM);
       } else {
         double x[NV];
-        load_M<D, W>(tm, p, w, m, k, x);
+        load_M<D, W>(tm, p, w, m, k, k + 1, x);
         const int EXd = max_exponent<D, W>(tm, x);
 #pragma unroll
         for (int v = 0; v < NV; ++v) db[v] = from_double(x[v], EXd, 2);
-        EM = EXd == 0x7ff ? kNotFinite : EXd - 1021;
+        EM = EXd - 1021;
       }
-      int EdY = EM;
-      if (p.grad_mode == GRAD_EXACT) {
+      tm.sync();  // every lane has read the flag
       const int EA = assemble<D, W>(T, p, w.u, m, k, tm, b);
       const float l2 = log2_norm1<D, W>(tm, b, EA);
       int L, s;
       choose_degree2(l2, tm.lane, L, s);
-      if (EA > kNever / 2 || s > 60) EM = kNotFinite;
-      if (EM != kNotFinite) {
+      if (s > 60) {
+        put_grad_value<D, W>(tm, p, w, m, k, 0x7ff8000000000000ull);
+        tm.sync();
+        continue;
+      }
       const int ED = EM - s;  // dB = M / 2^s
       const float nu2 = l2 - (float)s;
       const int lx = min(0, 2 * (int)ceilf(nu2));
@@ -453,8 +666,7 @@ __global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_g
         b[v] <<= 6;
         db[v] <<= 6;
       }
-      int EX = EB, EdX = ED, EY = EB;  // step 0: (X, dX) <- (B B, dB B + B dB)
-      EdY = ED;
+      int EX = EB, EdX = ED, EY = EB, EdY = ED;  // step 0: (X, dX) <- (B B, dB B + B dB)
       uint32_t pl = py, pdl = pdy;
 #pragma unroll 1
       for (int st = 0; st < L + s; ++st) {
@@ -542,33 +754,8 @@ __global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_g
           }
         }
       }
-      }
-      } else {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) q[v] = db[v];
-        tm.sync();  // the last slice's traces are read
-      }
-      if (EM == kNotFinite) {
-        if (tm.w == 0 && tm.lane < p.n_c)
-          w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] = __longlong_as_double(0x7ff8000000000000ll);
-        tm.sync();
-        continue;
-      }
-      // traces, in integers; lane j keeps control j's
-      long long keep = 0;
-      for (int j = 0; j < p.n_c; ++j) {
-        const long long t = trace_term<D, W>(T, tm, j + 1, p.gen == GEN_HERM ? 1 : 0, q);
-        if constexpr (W > 1) {
-          if (tm.lane == 0 && tm.w > 0) traces[j] = t;
-        }
-        if (tm.lane == j) keep = t;
-      }
-      tm.sync();  // traces are written, and the maxima read
-      if (tm.w == 0 && tm.lane < p.n_c) {
-        if constexpr (W > 1) keep += traces[tm.lane];
-        w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] =
-            p.dt[k] * p.m_scale[m] * to_double(keep, EdY + T.e[tm.lane + 1] - 55);
-      }
+      put_traces<D, W>(T, tm, p, w, m, k, q, EdY, traces);
+      tm.sync();  // the maxima and the traces are read
     }
   }
 }
@@ -581,15 +768,18 @@ __global__ void __launch_bounds__(32 * GradCfg<D>::TEAMS * GradCfg<D>::W) k_fx_g
 //   k_fx_chain_combine  per member: T_b = the product before block b, z, f,
 //                       kappa; Lambda_b = T' (product after block b); W_b =
 //                       kappa T_b Lambda_b into the block's first P slot
-//   k_fx_chain_bwd      per (member, block): V_k = W_b U_{k1-1} ... U_{k+1}
-//                       into the U slots, so M_k = P_k Lambda_k = R_k V_k
+//   k_fx_chain_bwd      per (member, block): V_k U_k = W_b U_{k1-1} ... U_k
+//                       into the U slots, so P_k Lambda_{k-1} = R_k V_k U_k and
+//                       M_k = P_k Lambda_k = R_k V_k with V_k = V_{k+1} U_{k+1}
 // A block product is a chain of its own, so short pulses of few members fill
 // the chip too; the forward, backward and gradient products are one each.
 template <int D> struct ChainCfg {
-  static constexpr int W = D >= 16 ? 2 : 1;
-  static constexpr int TEAMS = D >= 16 ? 4 : 8;          // (member, block) chains of a CTA
-  static constexpr int TEAM_BYTES = 2 * Geo<D, W>::PLANES + 64;
-  static constexpr int MAX_BLOCKS = D >= 16 ? 20 : 96;   // T_b and Lambda_b of a member in shared memory
+  static constexpr int W = kWarps<D>;
+  static constexpr int TEAMS = D >= 32 ? 1 : D >= 16 ? 4 : 8;  // (member, block) chains of a CTA
+  static constexpr int COMBINE = D >= 32 ? 2 : TEAMS;          // teams of a member's combine
+  static constexpr int TEAM_BYTES = 2 * Geo<D, W>::PLANES + kRed;
+  // T_b and Lambda_b of a member in shared memory
+  static constexpr int MAX_BLOCKS = D >= 32 ? 3 : D >= 16 ? 20 : 96;
 };
 
 template <int D, int W> struct ChainTeam {
@@ -611,10 +801,6 @@ template <int D, int W> struct ChainTeam {
     E = max(E, Ex) == kNotFinite ? kNotFinite : e;
   }
 };
-
-template <int D, int W> __device__ __forceinline__ longlong2* slot(const Tm<D, W>& tm, double2* stack, size_t i) {
-  return tm.mine(reinterpret_cast<longlong2*>(stack + i * D * D));
-}
 
 template <int D>
 __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS)
@@ -657,7 +843,6 @@ k_fx_chain_bwd(ProbDev p, WorkDev w, int blocks, int len) {
   if (item >= (long)p.n_members * blocks) return;
   const int m = (int)(item / blocks), k0 = (int)(item % blocks) * len, k1 = min(p.n_t, k0 + len);
   const size_t base = (size_t)m * p.n_t;
-  const bool grape = p.grad_mode == GRAD_REF_GRAPE;  // Gradients.jl: the costate includes the slice's own U_k
   long long r[NV], x[NV];
   get_ints<NV>(slot(ct.tm, w.P, base + k0), r);
   int E = unpack<D, W>(r);
@@ -669,14 +854,13 @@ k_fx_chain_bwd(ProbDev p, WorkDev w, int blocks, int len) {
     for (int v = 0; v < NV; ++v) u[v] = x[v];
     const int Eu = unpack<D, W>(u);
     if (k > k0) get_ints<NV>(slot(ct.tm, w.U, base + k - 1), x);
-    if (!grape) put_packed<D, W>(slot(ct.tm, w.U, base + k), r, E);
-    if (k > k0 || grape) ct.template step<true>(r, E, u, Eu);
-    if (grape) put_packed<D, W>(slot(ct.tm, w.U, base + k), r, E);
+    ct.template step<true>(r, E, u, Eu);
+    put_packed<D, W>(slot(ct.tm, w.U, base + k), r, E);
   }
 }
 
 // x -> kappa x: each part times a double, in a common frame; returns its
-// exponent (the result is not normalised: |x| < 0.75 2^56 holds).
+// exponent (the result is not normalised, but below 2^55).
 template <int D, int W>
 __device__ __forceinline__ int scale_complex(long long (&x)[Geo<D, W>::NV], int E, double2 kap) {
   constexpr int H = Geo<D, W>::NV / 2;
@@ -687,7 +871,7 @@ __device__ __forceinline__ int scale_complex(long long (&x)[Geo<D, W>::NV], int 
   const int a0 = (int)a, a1 = (int)((a + 0x80000000ll) >> 32), b0 = (int)b, b1 = (int)((b + 0x80000000ll) >> 32);
 #pragma unroll
   for (int v = 0; v < H; ++v) {
-    const long long re = x[v] << 3, im = x[H + v] << 3;
+    const long long re = x[v] << 2, im = x[H + v] << 2;
     const int r0 = (int)re, r1 = (int)((re + 0x80000000ll) >> 32);
     const int i0 = (int)im, i1 = (int)((im + 0x80000000ll) >> 32);
     const long long mr = 0x80000000ll + (long long)r1 * a0 + (long long)r0 * a1 - (long long)i1 * b0 - (long long)i0 * b1;
@@ -695,16 +879,16 @@ __device__ __forceinline__ int scale_complex(long long (&x)[Geo<D, W>::NV], int 
     x[v] = (long long)r1 * a1 - (long long)i1 * b1 + (mr >> 32);
     x[H + v] = (long long)r1 * b1 + (long long)i1 * a1 + (mi >> 32);
   }
-  return E == kNotFinite ? kNotFinite : E + ex - 1022 + 1;
+  return E == kNotFinite ? kNotFinite : E + ex - 1022 + 2;
 }
 
 template <int D>
-__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS)
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::COMBINE)
 k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
   using C = ChainCfg<D>;
   constexpr int W = C::W;
   using G = Geo<D, W>;
-  constexpr int NV = G::NV, TEAMS = C::TEAMS;
+  constexpr int NV = G::NV, TEAMS = C::COMBINE;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double2 s_red[32 * W];
   __shared__ double2 s_kap;
@@ -826,9 +1010,9 @@ static cudaError_t launch_slices(void (*kernel)(ProbDev, WorkDev, int, A...), co
 // Blocks of the gate chains.  Chains run in two dependent passes of `len`
 // products with one of `blocks` between: more blocks than sqrt(2 n_t) only
 // lengthen the sum, and more (member, block) chains than the SMs hold (about
-// 10 of 14 KB at D = 16, 24 of 4 KB at D = 8) run as a second wave.
+// 3 of 57 KB at D = 32, 10 of 14 KB at D = 16, 24 of 4 KB at D = 8) run as a second wave.
 template <int D> static void chain_shape(const ProbDev& p, int num_sms, int* blocks, int* len) {
-  const long chains = (long)num_sms * (D >= 16 ? 10 : 24);
+  const long chains = (long)num_sms * (D >= 32 ? 3 : D >= 16 ? 10 : 24);
   long b = chains / p.n_members;
   long most = 1;
   while (most < ChainCfg<D>::MAX_BLOCKS && (most + 1) * (most + 1) <= 2L * p.n_t) ++most;
@@ -847,9 +1031,9 @@ template <int D> static cudaError_t do_chain_fwd(const ProbDev& p, const WorkDev
   set_smem_once((const void*)k_fx_chain_fwd<D>, smem);
   const long items = (long)p.n_members * blocks;
   k_fx_chain_fwd<D><<<(int)((items + C::TEAMS - 1) / C::TEAMS), threads, smem, li.stream>>>(p, w, blocks, len, store ? 1 : 0);
-  const size_t smem2 = smem + (store ? (size_t)2 * blocks * Geo<D, C::W>::INTS : 0);
+  const size_t smem2 = (size_t)C::COMBINE * C::TEAM_BYTES + (store ? (size_t)2 * blocks * Geo<D, C::W>::INTS : 0);
   set_smem_once((const void*)k_fx_chain_combine<D>, smem2);
-  k_fx_chain_combine<D><<<p.n_members, threads, smem2, li.stream>>>(p, w, blocks, len, store ? 1 : 0);
+  k_fx_chain_combine<D><<<p.n_members, 32 * C::W * C::COMBINE, smem2, li.stream>>>(p, w, blocks, len, store ? 1 : 0);
   *li.launches += 2;
   return cudaGetLastError();
 }
@@ -869,26 +1053,37 @@ template <int D> static cudaError_t do_chain_bwd(const ProbDev& p, const WorkDev
 template <int D> static cudaError_t do_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
   int blocks, len;
   chain_shape<D>(p, li.num_sms, &blocks, &len);
-  return launch_slices<GradCfg<D>, D>(k_fx_grad<D>, p, w, li, len);
+  const cudaError_t e = launch_slices<SeriesCfg<D>, D>(k_fx_grad<D>, p, w, li, len);
+  if (e != cudaSuccess || p.grad_mode != GRAD_EXACT) return e;
+  return launch_slices<NormCfg<D>, D>(k_fx_grad_norm<D>, p, w, li, len);
 }
 
 }  // namespace fx
 
 bool fx_applies(const ProbDev& p) {
-  return (p.Dp == 8 || p.Dp == 16) && p.n_c + 1 + (p.n_ramp ? 1 : 0) <= fx::kMaxTerms;
+  const int n = p.n_c + 1 + (p.n_ramp ? 1 : 0);
+  return ((p.Dp == 8 || p.Dp == 16) && n <= fx::kMaxTerms) || (p.Dp == 32 && n <= fx::kMaxTerms32);
 }
+
+#define PGX_FX_DISPATCH(CALL)                          \
+  switch (p.Dp) {                                      \
+    case 8: { constexpr int D_ = 8; return CALL; }     \
+    case 16: { constexpr int D_ = 16; return CALL; }   \
+    case 32: { constexpr int D_ = 32; return CALL; }   \
+    default: return cudaErrorInvalidValue;             \
+  }
+
 cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  return p.Dp == 8 ? fx::launch_slices<fx::ExpmCfg<8>, 8>(fx::k_fx_expm<8>, p, w, li)
-                   : fx::launch_slices<fx::ExpmCfg<16>, 16>(fx::k_fx_expm<16>, p, w, li);
+  PGX_FX_DISPATCH((fx::launch_slices<fx::ExpmCfg<D_>, D_>(fx::k_fx_expm<D_>, p, w, li)));
 }
 cudaError_t launch_fx_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
-  return p.Dp == 8 ? fx::do_chain_fwd<8>(p, w, li, store) : fx::do_chain_fwd<16>(p, w, li, store);
+  PGX_FX_DISPATCH(fx::do_chain_fwd<D_>(p, w, li, store));
 }
 cudaError_t launch_fx_chain_bwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  return p.Dp == 8 ? fx::do_chain_bwd<8>(p, w, li) : fx::do_chain_bwd<16>(p, w, li);
+  PGX_FX_DISPATCH(fx::do_chain_bwd<D_>(p, w, li));
 }
 cudaError_t launch_fx_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  return p.Dp == 8 ? fx::do_grad<8>(p, w, li) : fx::do_grad<16>(p, w, li);
+  PGX_FX_DISPATCH(fx::do_grad<D_>(p, w, li));
 }
 
 }  // namespace pgx

@@ -181,108 +181,160 @@ __device__ __forceinline__ void mma_pair(float (&acc)[Geo<D, W>::NV], const Left
 constexpr float kMagic = 12582912.0f;  // 1.5 2^23
 constexpr uint32_t kPairBias = (0x4B400000u << 8) + 0x4B400000u;  // two magic starts joined (mod 2^32)
 
-// r = A B with `nlev` levels, as value 2^(EA + EB - 56): pa, pb address the
-// factors' digit planes.  Two levels a pass, the lowest two first: r <- r 2^-16
-// + (level L) 2^40 + (level L + 1) 2^32 needs no carries, because the new
-// levels only touch the high word, and keeps 32 bits below the last one.  The
-// two levels share every left digit, and the right digit of level L + 1 is the
-// one level L uses next.
+// Levels (L, L + 1) of A B, L even, level L + 1 only if `two`: (level L) 2^8 +
+// (level L + 1), summed over the 16-deep steps.  The two levels share every
+// left digit, and the right digit of level L + 1 is the one level L uses next.
 template <int D, int W>
-__device__ __forceinline__ void mul(const Tm<D, W>& tm, uint32_t pa, uint32_t pb, int nlev,
-                                    long long (&r)[Geo<D, W>::NV]) {
+__device__ __forceinline__ void level_pair(uint32_t la, uint32_t rb, int L, bool two, uint32_t (&t)[Geo<D, W>::NV]) {
   using G = Geo<D, W>;
   constexpr int NV = G::NV;
   constexpr uint32_t kDigit = 2 * G::PLANE;
+#pragma unroll 1
+  for (int kt = 0; kt < G::KT; ++kt) {
+    float a0[NV], a1[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) a0[v] = a1[v] = kMagic;
+    Left<D, W> a;
+    Right<D, W> b0, b1;
+    uint32_t pl = la + kt * 2 * (D / 8) * 128, pr = rb + kt * 2 * 128 + L * kDigit;  // A_0, B_L
+    a.load(pl);
+    b0.load(pr);
+    mma_pair<D, W>(a0, a, b0);
+    if (two) {
+      if (L + 1 < kSlices) {
+        b1.load(pr + kDigit);
+        mma_pair<D, W>(a1, a, b1);
+      }
+#pragma unroll 1
+      for (int i = 0; i < L; i += 2) {
+        a.load(pl + kDigit);
+        b1.load(pr - kDigit);
+        mma_pair<D, W>(a1, a, b0);
+        mma_pair<D, W>(a0, a, b1);
+        pl += 2 * kDigit;
+        pr -= 2 * kDigit;
+        a.load(pl);
+        b0.load(pr);
+        mma_pair<D, W>(a1, a, b1);
+        mma_pair<D, W>(a0, a, b0);
+      }
+      if (L + 1 < kSlices) {
+        a.load(pl + kDigit);
+        mma_pair<D, W>(a1, a, b0);
+      }
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < L; i += 2) {
+        a.load(pl + kDigit);
+        b1.load(pr - kDigit);
+        mma_pair<D, W>(a0, a, b1);
+        pl += 2 * kDigit;
+        pr -= 2 * kDigit;
+        a.load(pl);
+        b0.load(pr);
+        mma_pair<D, W>(a0, a, b0);
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const uint32_t x = (__float_as_uint(a0[v]) << 8) + __float_as_uint(a1[v]) - kPairBias;
+      t[v] = kt == 0 ? x : t[v] + x;
+    }
+  }
+}
+
+// r <- r 2^-16 + t 2^32: needs no carries, because a level pair only touches
+// the high word.
+template <int NV> __device__ __forceinline__ void join_pair(long long (&r)[NV], const uint32_t (&t)[NV], int L) {
+  if (L == 0) {  // to nearest: a floor's bias adds up over a chain of products
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] += 0x8000;
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int hi = (int)(r[v] >> 32);
+    const uint32_t lo = __funnelshift_r((uint32_t)r[v], (uint32_t)hi, 16);
+    r[v] = (long long)((unsigned long long)(t[v] + (uint32_t)(hi >> 16)) << 32 | lo);
+  }
+}
+
+// r = A B with `nlev` levels, as value 2^(EA + EB - 56): pa, pb address the
+// factors' digit planes.  The lowest two levels first, which keeps 32 bits
+// below the last one.
+template <int D, int W>
+__device__ __forceinline__ void mul(const Tm<D, W>& tm, uint32_t pa, uint32_t pb, int nlev,
+                                    long long (&r)[Geo<D, W>::NV]) {
+  constexpr int NV = Geo<D, W>::NV;
   const uint32_t la = Left<D, W>::at(tm, pa), rb = Right<D, W>::at(tm, pb);
 #pragma unroll
   for (int v = 0; v < NV; ++v) r[v] = 0;
 #pragma unroll 1
   for (int L = (nlev - 1) & ~1; L >= 0; L -= 2) {
     uint32_t t[NV];
+    level_pair<D, W>(la, rb, L, L + 1 < nlev, t);
+    join_pair<NV>(r, t, L);
+  }
+}
+
+// r = A B - B A.  Up to D = 16 the level pairs (at most 2^29.9 each with both
+// factors below 2^55) are subtracted before they join; at D = 32 their
+// difference could pass 2^31, so the products join first.
+template <int D, int W>
+__device__ __forceinline__ void commutator(const Tm<D, W>& tm, uint32_t pa, uint32_t pb, int nlev,
+                                           long long (&r)[Geo<D, W>::NV]) {
+  constexpr int NV = Geo<D, W>::NV;
+  if constexpr (Geo<D, W>::KT > 1) {
+    long long s[NV];
 #pragma unroll 1
-    for (int kt = 0; kt < G::KT; ++kt) {
-      float a0[NV], a1[NV];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) a0[v] = a1[v] = kMagic;
-      Left<D, W> a;
-      Right<D, W> b0, b1;
-      uint32_t pl = la + kt * 2 * (D / 8) * 128, pr = rb + kt * 2 * 128 + L * kDigit;  // A_0, B_L
-      a.load(pl);
-      b0.load(pr);
-      mma_pair<D, W>(a0, a, b0);
-      if (L + 1 < nlev) {
-        if (L + 1 < kSlices) {
-          b1.load(pr + kDigit);
-          mma_pair<D, W>(a1, a, b1);
-        }
-#pragma unroll 1
-        for (int i = 0; i < L; i += 2) {
-          a.load(pl + kDigit);
-          b1.load(pr - kDigit);
-          mma_pair<D, W>(a1, a, b0);
-          mma_pair<D, W>(a0, a, b1);
-          pl += 2 * kDigit;
-          pr -= 2 * kDigit;
-          a.load(pl);
-          b0.load(pr);
-          mma_pair<D, W>(a1, a, b1);
-          mma_pair<D, W>(a0, a, b0);
-        }
-        if (L + 1 < kSlices) {
-          a.load(pl + kDigit);
-          mma_pair<D, W>(a1, a, b0);
-        }
-      } else {
-#pragma unroll 1
-        for (int i = 0; i < L; i += 2) {
-          a.load(pl + kDigit);
-          b1.load(pr - kDigit);
-          mma_pair<D, W>(a0, a, b1);
-          pl += 2 * kDigit;
-          pr -= 2 * kDigit;
-          a.load(pl);
-          b0.load(pr);
-          mma_pair<D, W>(a0, a, b0);
-        }
-      }
+    for (int h = 0; h < 2; ++h) {
+      mul<D, W>(tm, h ? pa : pb, h ? pb : pa, nlev, r);
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        const uint32_t x = (__float_as_uint(a0[v]) << 8) + __float_as_uint(a1[v]) - kPairBias;
-        t[v] = kt == 0 ? x : t[v] + x;
+        if (h) r[v] -= s[v];
+        else s[v] = r[v];
       }
     }
-    if (L == 0) {  // to nearest: a floor's bias adds up over a chain of products
+  } else {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) r[v] += 0x8000;
-    }
+    for (int v = 0; v < NV; ++v) r[v] = 0;
+#pragma unroll 1
+    for (int L = (nlev - 1) & ~1; L >= 0; L -= 2) {
+      uint32_t t[NV], s[NV];
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        level_pair<D, W>(Left<D, W>::at(tm, h ? pa : pb), Right<D, W>::at(tm, h ? pb : pa), L, L + 1 < nlev, t);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const int hi = (int)(r[v] >> 32);
-      const uint32_t lo = __funnelshift_r((uint32_t)r[v], (uint32_t)hi, 16);
-      r[v] = (long long)((unsigned long long)(t[v] + (uint32_t)(hi >> 16)) << 32 | lo);
+        for (int v = 0; v < NV; ++v) {
+          if (h) t[v] -= s[v];
+          else s[v] = t[v];
+        }
+      }
+      join_pair<NV>(r, t, L);
     }
   }
 }
 
-// Shift that brings max |r| just below 0.75 2^56 (positive = left); M = the
-// largest |high word|, so max |r| < (M + 1) 2^32.
-__device__ __forceinline__ int norm_shift(uint32_t M) {
+// Shift that brings max |r| just below 0.75 2^56 (positive = left), or below
+// 2^55 with HALF; M = the largest |high word|, so max |r| < (M + 1) 2^32.  HALF
+// bounds every digit by 128: two level pairs then add up within 32 bits (the
+// 16-deep steps of D = 32, commutators).
+template <bool HALF> __device__ __forceinline__ int norm_shift(uint32_t M) {
   const uint32_t m = M + 1;
   const int lz = __clz(m);
-  return lz - 8 - ((m << lz) >= 0xBF000000u ? 1 : 0);
+  return lz - 8 - (HALF || (m << lz) >= 0xBF000000u ? 1 : 0);
 }
 __device__ __forceinline__ long long shift_round(long long v, int right) {  // v >> right, to nearest; right in [1, 63]
   return (v + (1ll << (right - 1))) >> right;
 }
 
-// r 2^(e - 56) -> x 2^(E - 56) with 0.37 2^56 < max |x| < 0.75 2^56; returns E.
-template <int D, int W> __device__ __forceinline__ int normalize(const Tm<D, W>& tm, long long (&r)[Geo<D, W>::NV], int e,
+// r 2^(e - 56) -> x 2^(E - 56), normalised; returns E.
+template <int D, int W, bool HALF = (Geo<D, W>::KT > 1)> __device__ __forceinline__ int normalize(const Tm<D, W>& tm, long long (&r)[Geo<D, W>::NV], int e,
                                                                         int slot = 0) {
   constexpr int NV = Geo<D, W>::NV;
   uint32_t M = 0;
 #pragma unroll
   for (int v = 0; v < NV; ++v) M = max(M, (uint32_t)abs((int)(r[v] >> 32)));
-  const int sh = norm_shift(tm.max(M, slot));
+  const int sh = norm_shift<HALF>(tm.max(M, slot));
   if (sh >= 0) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) r[v] <<= sh;

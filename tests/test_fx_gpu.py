@@ -29,8 +29,8 @@ def _problem(pg, D, nrm, gen, n_c, rng):
 
 
 @pytest.mark.parametrize("gen", ["hermitian", "liouvillian"])
-@pytest.mark.parametrize("D", [5, 8, 9, 16])
-@pytest.mark.parametrize("nrm,n_c", [(0.0, 1), (1e-9, 2), (0.0016, 2), (0.07, 3), (0.5, 23), (1.6, 22), (60.0, 3)])
+@pytest.mark.parametrize("D", [5, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("nrm,n_c", [(0.0, 1), (1e-9, 2), (0.0016, 2), (0.07, 3), (0.5, 23), (1.6, 22), (0.3, 7), (60.0, 6)])
 def test_propagator(pg, gen, D, nrm, n_c):
     """Every degree, squarings, padding, one term to the last that fits (and one
     more, which takes the general kernel)."""
@@ -54,8 +54,8 @@ def test_propagator_not_finite(pg):
 
 @pytest.mark.parametrize("target", ["gate", "states"])
 @pytest.mark.parametrize("gen", ["hermitian", "liouvillian"])
-@pytest.mark.parametrize("D,n_t,n_m", [(7, 1, 1), (8, 13, 3), (9, 2, 2), (16, 13, 3)])
-@pytest.mark.parametrize("nrm", [0.03, 0.4, 9.0])
+@pytest.mark.parametrize("D,n_t,n_m", [(7, 1, 1), (8, 13, 3), (9, 2, 2), (16, 13, 3), (19, 3, 1), (32, 5, 2)])
+@pytest.mark.parametrize("nrm", [0.03, 0.4, 3.0, 9.0])
 def test_exact_gradient(pg, target, gen, D, n_t, n_m, nrm):
     """(F, G) of slices with few and many Horner steps and squarings, members of
     different scale and offset, against the oracle.  FP64's own bars: |dF| <=
@@ -74,7 +74,7 @@ def test_exact_gradient(pg, target, gen, D, n_t, n_m, nrm):
         H = H - dag(H) - 0.2 * np.eye(D) + 0.05 * np.triu(H, 1)
         C, O = C - dag(C), O - dag(O)
     u = rng.normal(size=(n_c, n_t))
-    dt = nrm / np.abs(H[0] + np.tensordot(u[:, 0], C, 1)).sum(0).max() * rng.uniform(0.5, 1.0, n_t)
+    dt = nrm / np.abs(H[0] + np.tensordot(u[:, 0], C, 1)).sum(0).max() * rng.uniform(0.1, 1.0, n_t)
     Q, _ = np.linalg.qr(rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D)))
     kw = dict(drifts=H, controls=C, dt=dt, generator=gen, offset_op=O, member_drift=np.arange(n_m) % 2,
               member_scale=rng.uniform(0.9, 1.1, n_m), member_offset=rng.uniform(-0.1, 0.1, n_m), target=target,
@@ -89,7 +89,8 @@ def test_exact_gradient(pg, target, gen, D, n_t, n_m, nrm):
 
 
 @pytest.mark.parametrize("mode", ["exact", "ref_mr", "ref_grape"])
-@pytest.mark.parametrize("D,n_t,n_m", [(5, 1, 2), (8, 7, 1), (8, 301, 2), (11, 2, 1), (16, 67, 1), (16, 41, 200)])
+@pytest.mark.parametrize("D,n_t,n_m", [(5, 1, 2), (8, 7, 1), (8, 301, 2), (11, 2, 1), (16, 67, 1), (16, 41, 200),
+                                       (32, 2, 1), (25, 23, 2)])
 def test_gate_chain_blocks(pg, mode, D, n_t, n_m):
     """Gate chains in one block, in blocks with a short last one, of one slice,
     and of many members, in every gradient mode; F-only gives the same F.  Bars
