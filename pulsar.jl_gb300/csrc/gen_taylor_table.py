@@ -56,11 +56,13 @@ def main(out=sys.stdout):
     # block size q in {2, 3, 4} (degrees m = q L)
     vals = ", ".join(f"{theta_for(m, udf):.17g}" for m in range(1, max(DEGREES) + 1))
     print(f"#define PGX_THETADF_ALL_INIT {{{vals}}}  /* index m - 1 */", file=out)
-    # block fixed point: log2 of the FP64 thresholds of the degrees 4, 6, ..., 20,
+    # block fixed point: log2 of the FP64 and df thresholds of the degrees 4, 6, ..., 20,
     # and 1/k! = mant 2^(exp - 61)
-    logs = [math.log2(theta_for(m, u64)) for m in range(4, max(DEGREES) + 1, 2)]
-    print(f"#define PGX_N_FXDEGREES {len(logs)}", file=out)
-    print(f"#define PGX_LOG2_THETA64_EVEN_INIT {{{', '.join(f'{x:.9g}f' for x in logs)}}}", file=out)
+    even = range(4, max(DEGREES) + 1, 2)
+    print(f"#define PGX_N_FXDEGREES {len(even)}", file=out)
+    for name, u in (("PGX_LOG2_THETA64_EVEN_INIT", u64), ("PGX_LOG2_THETADF_EVEN_INIT", udf)):
+        vals = ", ".join(f"{math.log2(theta_for(m, u)):.9g}f" for m in even)
+        print(f"#define {name} {{{vals}}}", file=out)
     coefs = []
     for k in range(max(DEGREES) + 1):
         e = 1 - (math.factorial(k) - 1).bit_length() if k > 1 else 1

@@ -6,13 +6,15 @@
 namespace pgx {
 namespace fx {
 
-static __constant__ float c_log2theta[PGX_N_FXDEGREES] = PGX_LOG2_THETA64_EVEN_INIT;
+static __constant__ float c_log2theta[2][PGX_N_FXDEGREES] = {PGX_LOG2_THETA64_EVEN_INIT, PGX_LOG2_THETADF_EVEN_INIT};
 static __constant__ Coef c_coef[PGX_N_INVFACT] = PGX_INVFACT_FX_INIT;
 
 constexpr int kMaxTerms = 24;       // generator terms: drift, controls, ramp
 constexpr int kMaxTerms32 = 7;      // at D = 32: 16 KB of shared memory each beside two teams
-constexpr int kBits = 57;           // absolute error of a slice propagator: 2^-57 per product
-constexpr int kBits2 = 2 * kBits + 1;
+// Absolute error of a slice propagator's products: 2^-57 on the FP64 path;
+// 2^-51 on the mixed path, whose df pairs hold 2^-48 of an element (with 2^-48
+// U_total's defect over 1000 slices stayed 2.5 times larger).
+template <bool DF> constexpr int kBits2 = 2 * (DF ? 51 : 57) + 1;
 constexpr int kNever = 1 << 20;     // an exponent no finite entry reaches
 // Levels of a chain product: about 2^-55.5 of the factors' scale with 7, which
 // at D = 16 keeps a chain's error below that of an FP64 product's 64 roundings
@@ -171,10 +173,10 @@ template <int D, int W> __device__ __forceinline__ float log2_norm1(const Tm<D, 
 
 // Degree 2 L and squarings s with ||A||_1 / 2^s <= theta_2L that minimise the
 // products L + s (squarings last: they double the error).
-__device__ __forceinline__ void choose_degree2(float l2, int lane, int& L, int& s) {
+template <bool DF> __device__ __forceinline__ void choose_degree2(float l2, int lane, int& L, int& s) {
   uint32_t key = 0xffffffffu;
   if (lane < PGX_N_FXDEGREES) {
-    const int si = (int)fmaxf(ceilf(l2 - c_log2theta[lane]), 0.f);
+    const int si = (int)fmaxf(ceilf(l2 - c_log2theta[DF][lane]), 0.f);
     if (si < 64) key = (uint32_t)((2 + lane + si) << 16 | si << 8 | lane);
   }
   key = __reduce_min_sync(0xffffffffu, key);
@@ -185,6 +187,18 @@ __device__ __forceinline__ void choose_degree2(float l2, int lane, int& L, int& 
 // Warps of a matrix: eight columns each (and, at D = 32, sixteen rows).
 template <int D> constexpr int kWarps = D >= 32 ? 8 : D >= 16 ? 2 : 1;
 constexpr int kRed = 128;  // bytes of a team's maxima
+
+// U = r 2^ex in df pairs (float4), |r| < 2^60; ex = 0x7ff: not finite.
+template <int D, int W>
+__device__ __forceinline__ void store_df(const Tm<D, W>& tm, float4* U, const long long (&r)[Geo<D, W>::NV], int ex) {
+  using G = Geo<D, W>;
+  const float sc = ex == 0x7ff ? __int_as_float(0x7fc00000) : ldexpf(1.f, ex);
+#pragma unroll
+  for (int b = 0; b < G::NV / 2; ++b) {
+    const float2 x = to_df(r[b], sc), y = to_df(r[G::NV / 2 + b], sc);
+    U[tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2)] = make_float4(x.x, y.x, x.y, y.y);
+  }
+}
 
 template <int D> struct ExpmCfg {
   static constexpr int W = kWarps<D>;
@@ -202,7 +216,8 @@ template <int D> struct ExpmCfg {
 // rescaling), then the tensor pipe (about 64 digit pairs of 16 SM cycles at
 // D = 16).  A slice's planes and integers take 18 KB of shared memory, so an SM
 // holds ten; two warps share one, each with half the columns.
-template <int D>
+// DF: the mixed path's propagators, df pairs with 2^-48 products.
+template <int D, bool DF>
 __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_expm(ProbDev p, WorkDev w, int run) {
   using C = ExpmCfg<D>;
   constexpr int W = C::W;
@@ -242,12 +257,14 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
       const int EA = assemble<D, W>(T, p, w.u, m, k, tm, r);
       const float l2 = log2_norm1<D, W>(tm, r, EA);
       int L, s;
-      choose_degree2(l2, tm.lane, L, s);
+      choose_degree2<DF>(l2, tm.lane, L, s);
       double2* out = w.U + ((size_t)m * p.n_t + k) * D * D;
-      const bool packed = p.target == TGT_GATE;  // the gate chains' own format
+      const bool packed = !DF && p.target == TGT_GATE;  // the FP64 gate chains' own format
       int ex;  // U = r 2^ex
       if (EA > kNever / 2 || s > 60) {
-        if (packed) {
+        if constexpr (DF) {
+          store_df<D, W>(tm, (float4*)out, r, 0x7ff);
+        } else if (packed) {
           put_packed<D, W>(tm.mine((longlong2*)out), r, kNotFinite);
         } else {
           store_nan<D, W>(tm, out);
@@ -259,7 +276,7 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
       // Y_i keeps the fixed frame c_2i.exp + g
       const float nu2 = l2 - (float)s;
       const int lx = min(0, 2 * (int)ceilf(nu2));
-      const int g = nu2 <= -1.33f ? 1 : 3;  // e^nu <= 0.75 2^g, nu <= 0.397 or 1.51
+      const int g = nu2 <= -1.33f ? 1 : nu2 <= 0.8f ? 3 : 4;  // e^nu <= 0.75 2^g: nu <= 0.397, 1.74, 1.84
       const int EB = normalize<D, W>(tm, r, EA - 2 - s);
       int EX = 0, EY = EB, n = kSlices, F = 60;
       uint32_t pa = py;
@@ -269,9 +286,9 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
 #pragma unroll 1
       for (int st = 0; st < L + s; ++st) {
         const int i = L - 1 - st;
-        if (st == 0) n = levels(kBits2, 2 * EB);
-        else if (st < L) n = levels(kBits2, EX + EY + i * lx);
-        else n = levels(kBits2, 2 * EY);
+        if (st == 0) n = levels(kBits2<DF>, 2 * EB);
+        else if (st < L) n = levels(kBits2<DF>, EX + EY + i * lx);
+        else n = levels(kBits2<DF>, 2 * EY);
         tm.sync();
         if (st == 0) {
           long long x6[NV];
@@ -321,6 +338,10 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
           ex = 2 * EY - kFrac;
           if (packed || st + 1 < L + s) EY = normalize<D, W>(tm, r, 2 * EY);
         }
+      }
+      if constexpr (DF) {
+        store_df<D, W>(tm, (float4*)out, r, ex);
+        continue;
       }
       if (packed && s == 0) {
 #pragma unroll
@@ -647,7 +668,7 @@ k_fx_grad_norm(ProbDev p, WorkDev w, int run, int len) {
       const int EA = assemble<D, W>(T, p, w.u, m, k, tm, b);
       const float l2 = log2_norm1<D, W>(tm, b, EA);
       int L, s;
-      choose_degree2(l2, tm.lane, L, s);
+      choose_degree2<false>(l2, tm.lane, L, s);
       if (s > 60) {
         put_grad_value<D, W>(tm, p, w, m, k, 0x7ff8000000000000ull);
         tm.sync();
@@ -791,12 +812,13 @@ template <int D, int W> struct ChainTeam {
         pl(smem_u32(smem)), pr(pl + Geo<D, W>::PLANES) {}
   // (r, E) <- left (r, E); an operand that is not finite stays so
   template <bool R_IS_LEFT>
-  __device__ __forceinline__ void step(long long (&r)[Geo<D, W>::NV], int& E, const long long (&x)[Geo<D, W>::NV], int Ex) {
+  __device__ __forceinline__ void step(long long (&r)[Geo<D, W>::NV], int& E, const long long (&x)[Geo<D, W>::NV], int Ex,
+                                       int levels = kChainLevels<D>) {
     tm.sync();  // the last product has read its planes
-    store_planes<D, W>(tm, R_IS_LEFT ? pl : pr, r, kSlices);
-    store_planes<D, W>(tm, R_IS_LEFT ? pr : pl, x, kSlices);
+    store_planes<D, W>(tm, R_IS_LEFT ? pl : pr, r, levels);
+    store_planes<D, W>(tm, R_IS_LEFT ? pr : pl, x, levels);
     tm.sync();
-    mul<D, W>(tm, pl, pr, kChainLevels<D>, r);
+    mul<D, W>(tm, pl, pr, levels, r);
     const int e = normalize<D, W>(tm, r, E + Ex);
     E = max(E, Ex) == kNotFinite ? kNotFinite : e;
   }
@@ -857,6 +879,70 @@ k_fx_chain_bwd(ProbDev p, WorkDev w, int blocks, int len) {
     ct.template step<true>(r, E, u, Eu);
     put_packed<D, W>(slot(ct.tm, w.U, base + k), r, E);
   }
+}
+
+// The mixed path's in-block prefixes: U_k as df pairs, R_k rounded to float2
+// for the FP32 fix-up, block products as df pairs.  Seven levels: with six
+// (2^-47.5 of the factors' scale) the defect of U_total, 4.8e-12 after 1000
+// slices, passed that of the df products (9.6e-13); seven leave 1e-13.
+constexpr int kPrefixLevelsDf = 7;
+
+template <int D>
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS) k_fx_prefix_df(ProbDev p, WorkDev w, int store) {
+  using C = ChainCfg<D>;
+  constexpr int W = C::W, H = Geo<D, W>::NV / 2;
+  using G = Geo<D, W>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int team = threadIdx.x / (32 * W);
+  ChainTeam<D, W> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
+  const Tm<D, W>& tm = ct.tm;
+  const long item = (long)blockIdx.x * C::TEAMS + team;
+  if (item >= (long)p.n_members * w.pit_blocks) return;  // whole teams
+  const int m = (int)(item / w.pit_blocks), k0 = (int)(item % w.pit_blocks) * w.pit_len, k1 = min(p.n_t, k0 + w.pit_len);
+  const float4* Um = reinterpret_cast<const float4*>(w.U) + (size_t)m * p.n_t * D * D;
+  float2* Pm = reinterpret_cast<float2*>(w.P) + (size_t)m * p.n_t * D * D;
+  int at[H];
+#pragma unroll
+  for (int b = 0; b < H; ++b) at[b] = tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2);
+  long long r[2 * H];
+  int E = 0;
+  float4 f[H];
+#pragma unroll
+  for (int b = 0; b < H; ++b) {
+    f[b] = Um[(size_t)k0 * D * D + at[b]];
+    if (store) Pm[(size_t)k0 * D * D + at[b]] = make_float2(at[b] % D == at[b] / D ? 1.f : 0.f, 0.f);
+  }
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    uint32_t M = 0;
+#pragma unroll
+    for (int b = 0; b < H; ++b) M = max(M, max(__float_as_uint(f[b].x) & 0x7f800000u, __float_as_uint(f[b].y) & 0x7f800000u));
+    const int EX = (int)(tm.max(M, 2) >> 23), Eu = EX == 0xff ? kNotFinite : EX - 125;
+    long long u[2 * H];
+#pragma unroll
+    for (int b = 0; b < H; ++b) {
+      u[b] = from_float(f[b].x, EX) + from_float(f[b].z, EX);
+      u[H + b] = from_float(f[b].y, EX) + from_float(f[b].w, EX);
+    }
+    if (k + 1 < k1) {
+#pragma unroll
+      for (int b = 0; b < H; ++b) f[b] = Um[(size_t)(k + 1) * D * D + at[b]];  // while this product runs
+    }
+    if (k == k0) {
+#pragma unroll
+      for (int v = 0; v < 2 * H; ++v) r[v] = u[v];
+      E = Eu;
+    } else {
+      ct.template step<false>(r, E, u, Eu, kPrefixLevelsDf);
+    }
+    if (store && k + 1 < k1) {
+      const float sc = E == kNotFinite ? __int_as_float(0x7fc00000) : ldexpf(1.f, E - kFrac);
+#pragma unroll
+      for (int b = 0; b < H; ++b)
+        Pm[(size_t)(k + 1) * D * D + at[b]] = make_float2(to_df(r[b], sc).x, to_df(r[H + b], sc).x);
+    }
+  }
+  store_df<D, W>(tm, w.pit_tot + (size_t)item * D * D, r, E == kNotFinite ? 0x7ff : E - kFrac);
 }
 
 // x -> kappa x: each part times a double, in a common frame; returns its
@@ -1058,6 +1144,25 @@ template <int D> static cudaError_t do_grad(const ProbDev& p, const WorkDev& w, 
   return launch_slices<NormCfg<D>, D>(k_fx_grad_norm<D>, p, w, li, len);
 }
 
+template <int D> static cudaError_t do_prefix_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  using C = ChainCfg<D>;
+  const size_t smem = (size_t)C::TEAMS * C::TEAM_BYTES;
+  set_smem_once((const void*)k_fx_prefix_df<D>, smem);
+  const long items = (long)p.n_members * w.pit_blocks;
+  k_fx_prefix_df<D><<<(int)((items + C::TEAMS - 1) / C::TEAMS), 32 * C::W * C::TEAMS, smem, li.stream>>>(p, w, store ? 1 : 0);
+  ++*li.launches;
+  return cudaGetLastError();
+}
+
+template <int D> static long prefix_capacity() {
+  using C = ChainCfg<D>;
+  const size_t smem = (size_t)C::TEAMS * C::TEAM_BYTES;
+  set_smem_once((const void*)k_fx_prefix_df<D>, smem);
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fx_prefix_df<D>, 32 * C::W * C::TEAMS, smem);
+  return (long)per_sm * C::TEAMS;
+}
+
 }  // namespace fx
 
 bool fx_applies(const ProbDev& p) {
@@ -1074,7 +1179,21 @@ bool fx_applies(const ProbDev& p) {
   }
 
 cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  PGX_FX_DISPATCH((fx::launch_slices<fx::ExpmCfg<D_>, D_>(fx::k_fx_expm<D_>, p, w, li)));
+  PGX_FX_DISPATCH((fx::launch_slices<fx::ExpmCfg<D_>, D_>(fx::k_fx_expm<D_, false>, p, w, li)));
+}
+cudaError_t launch_fx_expm_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  PGX_FX_DISPATCH((fx::launch_slices<fx::ExpmCfg<D_>, D_>(fx::k_fx_expm<D_, true>, p, w, li)));
+}
+cudaError_t launch_fx_prefix_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  PGX_FX_DISPATCH(fx::do_prefix_df<D_>(p, w, li, store));
+}
+long fx_prefix_capacity(int Dp) {
+  switch (Dp) {
+    case 8: return fx::prefix_capacity<8>();
+    case 16: return fx::prefix_capacity<16>();
+    case 32: return fx::prefix_capacity<32>();
+    default: return 0;
+  }
 }
 cudaError_t launch_fx_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
   PGX_FX_DISPATCH(fx::do_chain_fwd<D_>(p, w, li, store));

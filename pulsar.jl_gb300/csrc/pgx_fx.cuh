@@ -505,6 +505,25 @@ __device__ __forceinline__ void load_mat(const Tm<D, W>& tm, const double2* A, d
     x[G::NV / 2 + b] = a.y;
   }
 }
+// r 2^k -> df pair, |r| < 2^60: three exact float pieces (24, 24 and 12 bits)
+// joined by a fast two-sum.
+__device__ __forceinline__ float2 to_df(long long r, float scale) {
+  const float a = (float)(int)(r >> 36), b = (float)((uint32_t)(r >> 12) & 0xffffffu), c = (float)((uint32_t)r & 0xfffu);
+  const float x = a * 68719476736.f, y = b * 4096.f;  // 2^36, 2^12
+  const float hi = x + y;
+  return make_float2(hi * scale, ((y - (hi - x)) + c) * scale);
+}
+// Float of a matrix whose largest biased exponent is EX -> integer below 2^55,
+// value x 2^(E - 56) with E = EX - 125.
+__device__ __forceinline__ long long from_float(float f, int EX) {
+  const uint32_t u = __float_as_uint(f);
+  const int ex = (int)((u >> 23) & 0xff);
+  unsigned long long m = (unsigned long long)((u & 0x7fffffu) | 0x800000u) << 31;
+  m = ex == 0 ? 0 : shr64(m, EX - ex);
+  const long long s = (long long)((int)u >> 31);
+  return ((long long)m ^ s) - s;
+}
+
 // A normalised matrix in global memory, lane-private: x << 7 with its exponent
 // in the low seven bits of each lane's first three values.
 constexpr int kExpBias = 1 << 20;

@@ -173,7 +173,7 @@ cudaError_t launch_norm(const double* v, int n, double* out, cudaStream_t stream
 void set_smem_once(const void* fn, size_t bytes);
 
 // Team sizes the mixed slice-parallel kernel `kernel` (kTune*) admits at
-// padded dimension Dp (writes up to 4 values, returns the count), and the
+// padded dimension Dp (writes up to 5 values, returns the count), and the
 // default choice.
 // Team values of the tunable mixed kernels: candidates the autotuner times,
 // values pgx_problem_set_team admits, and the default.  kTeamTensor (1)
@@ -231,6 +231,11 @@ cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo&
 cudaError_t launch_fx_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
 cudaError_t launch_fx_chain_bwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 cudaError_t launch_fx_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
+// The mixed path's slice propagators and in-block prefixes on the same engine
+// (df pairs in and out), where fx_applies(p) at Dp = 16 and 32.
+cudaError_t launch_fx_expm_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
+cudaError_t launch_fx_prefix_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
+long fx_prefix_capacity(int Dp);  // prefix chains one SM holds
 // Mixed-precision stages (pgx_mixed.cu), gate targets: df expm and forward
 // chain, FP32 backward chain and gradient.  U stack holds df (float4), the P
 // stack float2.

@@ -15,6 +15,7 @@
 //              table) and traces; results accumulated as FP64.
 // F therefore carries df (~1e-13 per product) rounding; G carries FP32
 // (~1e-6 relative) rounding.
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 
@@ -1242,7 +1243,12 @@ static int grid_for(K kernel, int threads, size_t smem, long teams, int tpc, int
 bool grad_tc_eligible(const ProbDev& p) {
   return p.Dp == 64 && p.target == TGT_GATE && p.grad_mode == GRAD_EXACT;
 }
-static bool expm_tc_eligible(const ProbDev& p) { return p.Dp == 64; }
+// At D = 16 and 32 the tensor-core form is the block fixed-point expm and
+// prefix chain (pgx_fx.cuh), for every generator and target with as many
+// generator terms as its shared memory holds.
+static bool expm_tc_eligible(const ProbDev& p) {
+  return p.Dp == 64 || ((p.Dp == 16 || p.Dp == 32) && fx_applies(p));
+}
 static int variants_for(int Dp, int kernel, int* out) {
   int n = 0;
   if (Dp <= 8) out[n++] = 32;
@@ -1273,11 +1279,19 @@ int mixed_admitted(const ProbDev& p, int kernel, int* out) {
 // autotuner's usual choice on GB300 at each dimension.
 int mixed_default_team(const ProbDev& p, int kernel) {
   const int Dp = p.Dp;
+  if (tc_eligible(p, kernel)) return kTeamTensor;
   if (Dp <= 8) return 32;
   if (Dp == 16) return kernel == kTuneExpmMx ? 128 : 32;
   if (Dp == 32) return kernel == kTuneExpmMx ? 256 : 128;
-  if (tc_eligible(p, kernel)) return kTeamTensor;
   return kernel == kTuneExpmMx ? 256 : 512;
+}
+
+// The expm team of a launch.  A problem's choice of the tensor-core form falls
+// back to the CUDA-core default when a drift ramp set later adds the one
+// generator term that no longer fits.
+static int expm_team(const ProbDev& p, const LaunchInfo& li) {
+  const int t = li.team[kTuneExpmMx] ? li.team[kTuneExpmMx] : mixed_default_team(p, kTuneExpmMx);
+  return t == kTeamTensor && !expm_tc_eligible(p) ? (p.Dp == 16 ? 128 : 256) : t;
 }
 
 #define PGX_DISPATCH_MX_T(DP, TT, CALL)                                                        \
@@ -1379,11 +1393,8 @@ cudaError_t launch_expm_mx(const ProbDev& p, const WorkDev& w, const LaunchInfo&
     set.items = (long)p.n_members * p.n_t;
     return do_expm_small<2, false>(set, li);
   }
-  const int t = li.team[kTuneExpmMx] ? li.team[kTuneExpmMx] : mixed_default_team(p, kTuneExpmMx);
-  if (t == kTeamTensor) {
-    if (!expm_tc_eligible(p)) return cudaErrorInvalidValue;
-    return do_expm_oz64(p, w, li);
-  }
+  const int t = expm_team(p, li);
+  if (t == kTeamTensor) return p.Dp == 64 ? do_expm_oz64(p, w, li) : launch_fx_expm_df(p, w, li);
   PGX_DISPATCH_MX_T(p.Dp, t, return (do_expm_mx<D_, T_>(p, w, li)));
   return cudaSuccess;
 }
@@ -1413,8 +1424,12 @@ static cudaError_t do_chain_fwd_mx(const ProbDev& p, const WorkDev& w, const Lau
     ++*li.launches;
     return cudaGetLastError();
   }
-  const int expm_team = li.team[kTuneExpmMx] ? li.team[kTuneExpmMx] : mixed_default_team(p, kTuneExpmMx);
-  if (D == 64 && expm_team == kTeamTensor) {
+  const bool tensor = expm_team(p, li) == kTeamTensor;  // the prefixes follow the expm's engine
+  if ((D == 16 || D == 32) && tensor) {
+    const cudaError_t e = launch_fx_prefix_df(p, w, li, store);
+    if (e != cudaSuccess) return e;
+    --*li.launches;  // counted below
+  } else if (D == 64 && tensor) {
     // the in-block prefixes on the tensor-core expm's engine (pgx_expm_oz.cuh)
     ensure_smem_mx(k_chainf_local_oz64, oz::kExpmSmem);
     const long items = (long)p.n_members * w.pit_blocks;
@@ -1430,7 +1445,7 @@ static cudaError_t do_chain_fwd_mx(const ProbDev& p, const WorkDev& w, const Lau
     const int grid_l = grid_for(local, PC::THREADS, smem_l, (long)p.n_members * w.pit_blocks, PC::TPC, li.num_sms, 0);
     local<<<grid_l, PC::THREADS, smem_l, li.stream>>>(p, w, store);
   }
-  if (D == 64 && expm_team == kTeamTensor) {
+  if (D == 64 && tensor) {
     ensure_smem_mx(k_chainf_combine_oz64, oz::kExpmSmem);
     k_chainf_combine_oz64<<<p.n_members < li.num_sms ? p.n_members : li.num_sms, oz::kExpmThreads,
                             oz::kExpmSmem, li.stream>>>(p, w, store);
@@ -1490,8 +1505,8 @@ long chain_prefix_capacity(int Dp, int num_sms) {
     case 2: return prefix_teams_per_sm<2>() * num_sms;
     case 4: return prefix_teams_per_sm<4>() * num_sms;
     case 8: return prefix_teams_per_sm<8>() * num_sms;
-    case 16: return prefix_teams_per_sm<16>() * num_sms;
-    case 32: return prefix_teams_per_sm<32>() * num_sms;
+    case 16: return std::min(prefix_teams_per_sm<16>(), fx_prefix_capacity(16)) * num_sms;
+    case 32: return std::min(prefix_teams_per_sm<32>(), fx_prefix_capacity(32)) * num_sms;
     default: return 0;
   }
 }

@@ -915,7 +915,7 @@ extern "C" int pgx_autotune(pgx_problem* p, const double* u, int32_t reps, char*
 extern "C" int pgx_problem_set_team(pgx_problem* p, int32_t kernel, int32_t team) {
   if (!p || kernel < 0 || kernel >= pgx::kNumTunable) return PGX_ERR_INVALID;
   if (team != 0) {
-    int vs[4];
+    int vs[8];
     const int nv = pgx::mixed_admitted(p->pd, kernel, vs);
     if (std::find(vs, vs + nv, team) == vs + nv)
       return ctx_fail(p->ctx, PGX_ERR_INVALID, "team size not admitted at this dimension");
