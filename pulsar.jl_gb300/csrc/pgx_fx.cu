@@ -132,9 +132,10 @@ __device__ __forceinline__ int assemble(const Terms<D, W>& T, const ProbDev& p, 
   return EA;
 }
 
-// log2 of a bound of ||A||_1 (58 fractional bits in frame EA): the largest
+// log2 of a bound of ||A||_1 (F fractional bits in frame EA): the largest
 // column sum, from D = 32 on over each warp's rows and then added up.
-template <int D, int W> __device__ __forceinline__ float log2_norm1(const Tm<D, W>& tm, const long long (&A)[Geo<D, W>::NV], int EA) {
+template <int D, int W> __device__ __forceinline__ float log2_norm1(const Tm<D, W>& tm, const long long (&A)[Geo<D, W>::NV], int EA,
+                                                                                 int F = 58) {
   using G = Geo<D, W>;
   float best = 0.f;
 #pragma unroll
@@ -168,15 +169,20 @@ template <int D, int W> __device__ __forceinline__ float log2_norm1(const Tm<D, 
       best = fmaxf(best, s);
     }
   }
-  return __log2f(fmaf(best, 1.00001f, 2.f * D)) + (float)(EA - 26) + 1e-5f;
+  return __log2f(fmaf(best, 1.00001f, 2.f * D)) + (float)(EA + 32 - F) + 1e-5f;
 }
 
-// Degree 2 L and squarings s with ||A||_1 / 2^s <= theta_2L that minimise the
-// products L + s (squarings last: they double the error).
-template <bool DF> __device__ __forceinline__ void choose_degree2(float l2, int lane, int& L, int& s) {
+// Degree 2 L and squarings s that minimise the products L + s (squarings last:
+// they double the error), from l1 = log2 of a bound of ||A||_1 and lb = half of
+// log2 of a bound of ||A^2||_1 (l1 when A^2 is not known; lb <= l1).  The tail
+// of T_m is at most that of a scalar of norm 2^lb (2^(l1 - lb))^(1 / (m + 1)):
+// ||A^k|| <= ||A^2||^(k / 2), times ||A|| for odd k.  At d = 32 a random
+// generator's 2^lb is 0.4 of its 1-norm, which saves two products.
+template <bool DF> __device__ __forceinline__ void choose_degree2(float l1, float lb, int lane, int& L, int& s) {
   uint32_t key = 0xffffffffu;
   if (lane < PGX_N_FXDEGREES) {
-    const int si = (int)fmaxf(ceilf(l2 - c_log2theta[DF][lane]), 0.f);
+    const float x = lb + (l1 - lb) * (1.f / (2 * lane + 5)) - c_log2theta[DF][lane];
+    const int si = (int)fmaxf(ceilf(x), 0.f);
     if (si < 64) key = (uint32_t)((2 + lane + si) << 16 | si << 8 | lane);
   }
   key = __reduce_min_sync(0xffffffffu, key);
@@ -255,13 +261,11 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
     for (int k = k0 + team; k < k1; k += nt) {
       long long r[NV];
       const int EA = assemble<D, W>(T, p, w.u, m, k, tm, r);
-      const float l2 = log2_norm1<D, W>(tm, r, EA);
-      int L, s;
-      choose_degree2<DF>(l2, tm.lane, L, s);
+      const float l1 = log2_norm1<D, W>(tm, r, EA);
       double2* out = w.U + ((size_t)m * p.n_t + k) * D * D;
       const bool packed = !DF && p.target == TGT_GATE;  // the FP64 gate chains' own format
       int ex;  // U = r 2^ex
-      if (EA > kNever / 2 || s > 60) {
+      if (EA > kNever / 2 || l1 > 60.f) {
         if constexpr (DF) {
           store_df<D, W>(tm, (float4*)out, r, 0x7ff);
         } else if (packed) {
@@ -272,22 +276,18 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
         tm.sync();  // the maxima are read
         continue;
       }
-      // bounds: |X| <= nu^2 (nu = the scaled norm), and |Y_i| <= c_2i e^nu, so
-      // Y_i keeps the fixed frame c_2i.exp + g
-      const float nu2 = l2 - (float)s;
-      const int lx = min(0, 2 * (int)ceilf(nu2));
-      const int g = nu2 <= -1.33f ? 1 : nu2 <= 0.8f ? 3 : 4;  // e^nu <= 0.75 2^g: nu <= 0.397, 1.74, 1.84
-      const int EB = normalize<D, W>(tm, r, EA - 2 - s);
-      int EX = 0, EY = EB, n = kSlices, F = 60;
+      // B = A and X = B B before the degree is known: scaling by 2^-s only moves
+      // exponents
+      int EB = normalize<D, W>(tm, r, EA - 2), EX = 0, EY = EB, F = 60, L = 2, s = 0, g = 1, lx = 0;
       uint32_t pa = py;
       // step 0: X = B B; L - 1 Horner steps Y <- X Y + c_{2i+1} B + c_2i I,
       // whose error later meets X^i; s squarings.  One product in the loop
       // body keeps the kernel inside the instruction cache.
 #pragma unroll 1
       for (int st = 0; st < L + s; ++st) {
-        const int i = L - 1 - st;
-        if (st == 0) n = levels(kBits2<DF>, 2 * EB);
-        else if (st < L) n = levels(kBits2<DF>, EX + EY + i * lx);
+        int n;
+        if (st == 0) n = levels(kBits2<DF>, 2 * (EB - (int)fmaxf(l1, 0.f)));
+        else if (st < L) n = levels(kBits2<DF>, EX + EY + (L - 1 - st) * lx);
         else n = levels(kBits2<DF>, 2 * EY);
         tm.sync();
         if (st == 0) {
@@ -304,20 +304,33 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
         store_planes<D, W>(tm, py, r, n);
         tm.sync();
         mul<D, W>(tm, pa, py, n, r);
+        if (st == 0) {
+          EX = normalize<D, W>(tm, r, 2 * EB);
+          // below 2^-2.6 the 1-norm's own degree is within a product of the best
+          const float l2 = l1 > -2.6f ? log2_norm1<D, W>(tm, r, EX, kFrac) : 2.f * l1, lb = fminf(l1, 0.5f * l2);
+          choose_degree2<DF>(l1, lb, tm.lane, L, s);
+          EB -= s;
+          EX -= 2 * s;
+          // |X| <= 2^lx, and |Y_i| <= c_2i e^nu, nu = 2^(lb - s) -- for a matrix
+          // that is not normal, times ||B|| / nu -- so Y_i keeps the fixed
+          // frame c_2i.exp + g: e^nu <= 0.75 2^g
+          lx = min(0, (int)ceilf(l2 - 2.f * s));
+          const float nu = exp2f(lb - (float)s) * 1.4426951f + (p.gen == GEN_HERM ? 0.f : l1 - lb);
+          g = max(max(1, EB + 1), (int)ceilf(nu + 0.4151f));
+          store_planes<D, W>(tm, px, r, kSlices);
+          pa = px;
+        }
         if (st < L) {
+          const int i = L - 1 - st;
           const bool final = packed && i == 0 && s == 0;  // |U| <= e^nu <= 0.75 2^g
           const int fr = final ? g : c_coef[2 * i].exp + g;
+          F = st > 0 && i == 0 ? 60 : kFrac;
           if (st == 0) {
             // Y = c_2L X + c_{2L-1} B + c_{2L-2} I
-            EX = normalize<D, W>(tm, r, 2 * EB);
-            store_planes<D, W>(tm, px, r, kSlices);
-            pa = px;
-            F = kFrac;
             const Scaled sx(c_coef[2 * L], EX, fr, F);
 #pragma unroll
             for (int v = 0; v < NV; ++v) r[v] = sx(r[v] << 6, 0);
           } else {
-            F = i > 0 ? kFrac : 60;
             to_frame<NV>(r, EX + EY, fr, F);
           }
           const Scaled sb(c_coef[2 * i + 1], EB, fr, F);
@@ -367,7 +380,9 @@ __device__ __forceinline__ void load_M(const Tm<D, W>& tm, const ProbDev& p, con
   for (int s = 0; s < np; ++s)
 #pragma unroll
     for (int b = 0; b < G::NV / 2; ++b) {
-      const double2 y = psi[s * D + tm.row(b / 2 % G::NI)], l = lam[s * D + tm.col(b / 2 / G::NI, b % 2)];
+      double2 y = psi[s * D + tm.row(b / 2 % G::NI)];
+      const double2 l = lam[s * D + tm.col(b / 2 / G::NI, b % 2)];
+      if (lam_unscaled(p, D)) y = cmul(w.kap[(size_t)m * np + s], y);
       const double2 acc = cmac(make_double2(x[b], x[G::NV / 2 + b]), y, make_double2(l.x, -l.y));
       x[b] = acc.x;
       x[G::NV / 2 + b] = acc.y;
@@ -668,7 +683,7 @@ k_fx_grad_norm(ProbDev p, WorkDev w, int run, int len) {
       const int EA = assemble<D, W>(T, p, w.u, m, k, tm, b);
       const float l2 = log2_norm1<D, W>(tm, b, EA);
       int L, s;
-      choose_degree2<false>(l2, tm.lane, L, s);
+      choose_degree2<false>(l2, l2, tm.lane, L, s);
       if (s > 60) {
         put_grad_value<D, W>(tm, p, w, m, k, 0x7ff8000000000000ull);
         tm.sync();
@@ -1063,6 +1078,164 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
   }
 }
 
+// State chains, forward and backward together: one warp per (member, pair,
+// direction) applies the slices to its vector in 64-bit integers.
+//   forward   psi_{k+1} = U_k psi_k, z_s, f, kappa
+//   backward  lambda_k = U_k' lambda_{k+1} from lambda_n = t_s, stored without
+//             the factor conj(kappa_s) (the gradient applies it), so it does not
+//             wait for the forward chain
+// A warp's FP64 FMA takes 70 cycles of its scheduler's pipe, so the FP64 chain
+// spent 1,500 (D = 2) to 3,000 cycles a slice on one dot product and the exposed
+// load of U_k.  A complex multiply-add is 12 integer ones here; U streams into
+// shared memory with cp.async a few slices ahead.
+//
+// Vectors are x 2^(E - 57), |x| < 2^57, one exponent per vector; U_k's entries
+// u 2^(EX - 1081), |u| < 2^59.  A step keeps 57 bits of the products' scale.
+template <int D> struct StCfg {
+  static constexpr int QS = 32 / D < D ? 32 / D : D;  // lanes that share a row
+  static constexpr int QN = D / QS;                   // columns of a lane
+  static constexpr int ACTIVE = D * QS;               // the other lanes repeat their work
+  static constexpr int STAGE = D * D * 16;            // bytes of one slice
+  static constexpr int MAX_STAGES = 8;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+template <int D>
+__global__ void __launch_bounds__(512) k_fx_states(ProbDev p, WorkDev w, int store, int stages) {
+  using C = StCfg<D>;
+  constexpr int QN = C::QN, QS = C::QS;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double s_f[8];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, np = p.n_pairs, m = blockIdx.x;
+  const int s = wid % np;
+  const bool fwd = wid < np;
+  const int al = lane & (C::ACTIVE - 1), r = al % D, q0 = al / D * QN;
+  // per warp: the ring of U, then two copies of the vector
+  unsigned char* mine = smem_raw + (size_t)wid * ((size_t)stages * C::STAGE + 2 * D * 16);
+  const uint32_t ring = smem_u32(mine);
+  longlong2* vec = reinterpret_cast<longlong2*>(mine + (size_t)stages * C::STAGE);
+  const double2* Um = w.U + (size_t)m * p.n_t * D * D;
+  // element (i, c) of a slice at column c, row i ^ (c mod 8): rows and columns
+  // both read without bank conflicts
+  auto swz = [](int i, int c) { return c * D + (i ^ (c & (D < 8 ? D - 1 : 7))); };
+  auto fetch = [&](int step) {  // slice of chain step `step`
+    if (step < p.n_t) {
+      const double2* src = Um + (size_t)(fwd ? step : p.n_t - 1 - step) * D * D;
+      const uint32_t dst = ring + (uint32_t)(step % stages) * C::STAGE;
+      for (int e = lane; e < D * D; e += 32) cp_async16(dst + swz(e % D, e / D) * 16, src + e);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i + 1 < stages; ++i) fetch(i);
+
+  const size_t pan = (size_t)np * D;
+  double2* out = (fwd ? w.psi : w.lam) + (size_t)m * (p.n_t + 1) * pan + (size_t)s * D;
+  const double2 v0 = (fwd ? p.psi_init : p.psi_targ)[s * D + r];
+  int E = 0;
+  bool bad = false;
+  long long xr, xi;
+  {
+    double x[2] = {v0.x, v0.y};
+    uint32_t M = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) M = max(M, (uint32_t)__double2hiint(x[h]) & 0x7ff00000u);
+    const int EX = (int)(__reduce_max_sync(0xffffffffu, M) >> 20);
+    bad = EX == 0x7ff;
+    xr = from_double(x[0], EX, 4);
+    xi = from_double(x[1], EX, 4);
+    E = EX - 1022;
+  }
+  if (store && lane < D) out[(fwd ? (size_t)0 : (size_t)p.n_t * pan) + r] = v0;
+#pragma unroll 1
+  for (int step = 0; step < p.n_t; ++step) {
+    longlong2* v = vec + (step & 1) * D;
+    if (lane < D) v[r] = make_longlong2(xr, xi);
+    // stages - 1 groups stay in flight, one is needed now
+    if (stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else if (stages < 6) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 4;" ::: "memory");
+    __syncwarp();
+    const double2* U = reinterpret_cast<const double2*>(mine + (size_t)(step % stages) * C::STAGE);
+    double2 a[QN];
+    uint32_t M = 0;
+#pragma unroll
+    for (int i = 0; i < QN; ++i) {
+      a[i] = fwd ? U[swz(r, q0 + i)] : U[swz(q0 + i, r)];
+      M = max(M, max((uint32_t)__double2hiint(a[i].x) & 0x7ff00000u, (uint32_t)__double2hiint(a[i].y) & 0x7ff00000u));
+    }
+    const int EX = (int)(__reduce_max_sync(0xffffffffu, M) >> 20);
+    // re = sum ur xr -+ ui xi, im = sum ur xi +- ui xr (backward: conj(U))
+    long long pr = 0, pi = 0, nr = 0, ni = 0, mpr = 0, mpi = 0, mnr = 0, mni = 0;
+#pragma unroll
+    for (int i = 0; i < QN; ++i) {
+      const longlong2 x = v[q0 + i];
+      const long long ur = from_double(a[i].x, EX, 6), ui = from_double(a[i].y, EX, 6);
+      const int ur0 = (int)ur, ur1 = (int)((ur + 0x80000000ll) >> 32), ui0 = (int)ui, ui1 = (int)((ui + 0x80000000ll) >> 32);
+      const int xr0 = (int)x.x, xr1 = (int)((x.x + 0x80000000ll) >> 32), xi0 = (int)x.y, xi1 = (int)((x.y + 0x80000000ll) >> 32);
+      pr += (long long)ur1 * xr1;
+      mpr += (long long)ur1 * xr0 + (long long)ur0 * xr1;
+      nr += (long long)ui1 * xi1;
+      mnr += (long long)ui1 * xi0 + (long long)ui0 * xi1;
+      pi += (long long)ur1 * xi1;
+      mpi += (long long)ur1 * xi0 + (long long)ur0 * xi1;
+      ni += (long long)ui1 * xr1;
+      mni += (long long)ui1 * xr0 + (long long)ui0 * xr1;
+    }
+    const long long hr = fwd ? pr - nr : pr + nr, hi = fwd ? pi + ni : pi - ni;
+    const long long lr = fwd ? mpr - mnr : mpr + mnr, li = fwd ? mpi + mni : mpi - mni;
+    long long yr = (hr << 5) + shift_round(lr, 27), yi = (hi << 5) + shift_round(li, 27);
+#pragma unroll
+    for (int o = D; o < D * QS; o <<= 1) {
+      yr += __shfl_xor_sync(0xffffffffu, yr, o);
+      yi += __shfl_xor_sync(0xffffffffu, yi, o);
+    }
+    const uint32_t top = __reduce_max_sync(0xffffffffu, max((uint32_t)abs((int)(yr >> 32)), (uint32_t)abs((int)(yi >> 32))));
+    const int sh = __clz(top + 1) - 7;
+    xr = sh >= 0 ? yr << sh : shift_round(yr, -sh);
+    xi = sh >= 0 ? yi << sh : shift_round(yi, -sh);
+    bad |= EX == 0x7ff;
+    E = max(E + EX - 1022 - sh, -(1 << 20));
+    if (store && lane < D) {
+      const double nan = __longlong_as_double(0x7ff8000000000000ll);
+      double2 d = make_double2(to_double(xr, E - 57), to_double(xi, E - 57));
+      if (bad) d.x = d.y = nan;
+      out[(size_t)(fwd ? step + 1 : p.n_t - 1 - step) * pan + r] = d;
+    }
+    __syncwarp();  // the slot of this slice is free
+    fetch(step + stages - 1);
+  }
+  if (fwd) {
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    double2 d = make_double2(to_double(xr, E - 57), to_double(xi, E - 57));
+    if (bad) d.x = d.y = nan;
+    double2 z = make_double2(0.0, 0.0);
+    if (lane < D) z = cmac_cj(z, p.psi_targ[s * D + r], d);
+#pragma unroll
+    for (int o = D / 2; o > 0; o >>= 1) {
+      z.x += __shfl_xor_sync(0xffffffffu, z.x, o);
+      z.y += __shfl_xor_sync(0xffffffffu, z.y, o);
+    }
+    if (lane == 0) {
+      double f;
+      double2 kap;
+      fid_kappa(z, p.fid, p.grad_mode, f, kap);
+      const double wgt = p.m_weight[m];
+      w.z[(size_t)m * np + s] = z;
+      w.kap[(size_t)m * np + s] = make_double2(kap.x * wgt, kap.y * wgt);
+      s_f[s] = f;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double Fm = 0.0;
+    for (int i = 0; i < np; ++i) Fm += s_f[i];
+    w.Fm[m] = Fm;
+  }
+}
+
 constexpr size_t kSmemMax = 232448;  // dynamic shared memory of a CTA
 
 // Launches a slice-parallel kernel of configuration C (dimension D): as many
@@ -1163,6 +1336,18 @@ template <int D> static long prefix_capacity() {
   return (long)per_sm * C::TEAMS;
 }
 
+template <int D> static cudaError_t do_states(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  using C = StCfg<D>;
+  const int warps = p.n_pairs * (store ? 2 : 1);
+  int stages = (int)(196608 / ((size_t)warps * C::STAGE));
+  if (stages > C::MAX_STAGES) stages = C::MAX_STAGES;
+  const size_t smem = (size_t)warps * ((size_t)stages * C::STAGE + 2 * D * 16);
+  set_smem_once((const void*)k_fx_states<D>, smem);
+  k_fx_states<D><<<p.n_members, 32 * warps, smem, li.stream>>>(p, w, store ? 1 : 0, stages);
+  ++*li.launches;
+  return cudaGetLastError();
+}
+
 }  // namespace fx
 
 bool fx_applies(const ProbDev& p) {
@@ -1186,6 +1371,15 @@ cudaError_t launch_fx_expm_df(const ProbDev& p, const WorkDev& w, const LaunchIn
 }
 cudaError_t launch_fx_prefix_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
   PGX_FX_DISPATCH(fx::do_prefix_df<D_>(p, w, li, store));
+}
+cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  switch (p.Dp) {
+    case 2: return fx::do_states<2>(p, w, li, store);
+    case 4: return fx::do_states<4>(p, w, li, store);
+    case 8: return fx::do_states<8>(p, w, li, store);
+    case 16: return fx::do_states<16>(p, w, li, store);
+    default: return cudaErrorInvalidValue;
+  }
 }
 long fx_prefix_capacity(int Dp) {
   switch (Dp) {

@@ -156,6 +156,8 @@ template <int D, int W> struct Right {
   }
 };
 
+constexpr float kMagic = 12582912.0f;  // 1.5 2^23
+
 // acc += a b (complex), one digit pair, one 16-deep step.
 template <int D, int W>
 __device__ __forceinline__ void mma_pair(float (&acc)[Geo<D, W>::NV], const Left<D, W>& a, const Right<D, W>& b) {
@@ -178,7 +180,6 @@ __device__ __forceinline__ void mma_pair(float (&acc)[Geo<D, W>::NV], const Left
   }
 }
 
-constexpr float kMagic = 12582912.0f;  // 1.5 2^23
 constexpr uint32_t kPairBias = (0x4B400000u << 8) + 0x4B400000u;  // two magic starts joined (mod 2^32)
 
 // Levels (L, L + 1) of A B, L even, level L + 1 only if `two`: (level L) 2^8 +

@@ -510,16 +510,29 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_grad(ProbDev p, WorkDev w) 
       const int li = (p.grad_mode == GRAD_REF_GRAPE) ? k : k + 1;
       const double2* lam = w.lam + ((size_t)m * (p.n_t + 1) + li) * pan;
       if (!exact) {
-        // g_j = Re(c dt scale sum_s lambda_s' C_j psi_s)
+        // g_j = Re(c dt scale sum_s lambda_s' C_j psi_s): the outer product of
+        // an entry once, then every control
+        constexpr int NE = (D * D + T - 1) / T;
+        double2 lp[NE];
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+          const int e = tm.lane + i * T, r = e % D, c = e / D;
+          lp[i] = make_double2(0.0, 0.0);
+          if (e < D * D)
+            for (int s = 0; s < np; ++s) {
+              double2 y = psi[s * D + c];
+              if (lam_unscaled(p, D)) y = cmul(w.kap[(size_t)m * np + s], y);
+              lp[i] = cmac_cj(lp[i], lam[s * D + r], y);
+            }
+        }
         const double cds = p.dt[k] * p.m_scale[m];
         for (int j = 0; j < p.n_c; ++j) {
           const double2* Cj = p.ctrls + (size_t)j * D * D;
           double2 acc = make_double2(0.0, 0.0);
-          for (int e = tm.lane; e < D * D; e += T) {
-            const int r = e % D, c = e / D;
-            double2 lp = make_double2(0.0, 0.0);
-            for (int s = 0; s < np; ++s) lp = cmac_cj(lp, lam[s * D + r], psi[s * D + c]);
-            acc = cmac(acc, lp, Cj[e]);
+#pragma unroll
+          for (int i = 0; i < NE; ++i) {
+            const int e = tm.lane + i * T;
+            if (e < D * D) acc = cmac(acc, lp[i], Cj[e]);
           }
           const double2 t = team_sum<T>(tm, acc, red);
           if (tm.lane == 0) Gout[j] = cds * (p.gen == GEN_HERM ? t.y : t.x);
@@ -532,7 +545,9 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_grad(ProbDev p, WorkDev w) 
         double2 acc = make_double2(0.0, 0.0);
         for (int s = 0; s < np; ++s) {
           const double2 l = lam[s * D + c];
-          acc = cmac(acc, psi[s * D + r], make_double2(l.x, -l.y));
+          double2 y = psi[s * D + r];
+          if (lam_unscaled(p, D)) y = cmul(w.kap[(size_t)m * np + s], y);
+          acc = cmac(acc, y, make_double2(l.x, -l.y));
         }
         W.dB[e] = acc;
       }
@@ -746,7 +761,7 @@ static cudaError_t do_chain_fwd(const ProbDev& p, const WorkDev& w, const Launch
   } else if (p.n_ck > 0) {
     ensure_smem(k_track_fwd<D>, smem);
     k_track_fwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
-  } else {
+  } else if constexpr (D > 16) {  // launch_fx_states below
     ensure_smem(k_chain_states_fwd<D>, smem);
     k_chain_states_fwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w, store ? 1 : 0);
   }
@@ -755,6 +770,7 @@ static cudaError_t do_chain_fwd(const ProbDev& p, const WorkDev& w, const Launch
 }
 cudaError_t launch_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
   if (p.target == TGT_GATE && fx_applies(p)) return launch_fx_chain_fwd(p, w, li, store);
+  if (p.target == TGT_STATES && lam_unscaled(p, p.Dp)) return launch_fx_states(p, w, li, store);
   PGX_DISPATCH(p.Dp, return do_chain_fwd<D_>(p, w, li, store));
   return cudaSuccess;
 }
@@ -770,7 +786,7 @@ static cudaError_t do_chain_bwd(const ProbDev& p, const WorkDev& w, const Launch
   } else if (p.n_ck > 0) {
     ensure_smem(k_track_bwd<D>, smem);
     k_track_bwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
-  } else {
+  } else if constexpr (D > 16) {
     ensure_smem(k_chain_states_bwd<D>, smem);
     k_chain_states_bwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
   }
@@ -779,6 +795,7 @@ static cudaError_t do_chain_bwd(const ProbDev& p, const WorkDev& w, const Launch
 }
 cudaError_t launch_chain_bwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
   if (p.target == TGT_GATE && fx_applies(p)) return launch_fx_chain_bwd(p, w, li);
+  if (p.target == TGT_STATES && lam_unscaled(p, p.Dp)) return cudaSuccess;  // launch_fx_states ran both directions
   PGX_DISPATCH(p.Dp, return do_chain_bwd<D_>(p, w, li));
   return cudaSuccess;
 }

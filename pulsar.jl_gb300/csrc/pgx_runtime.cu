@@ -360,6 +360,11 @@ static void pit_shape(const pgx_problem_desc* d, int Dp, int num_sms, int* block
   const long cap = pgx::chain_prefix_capacity(Dp, num_sms);
   if (cap > 0) b = std::min<long>(b, std::max<long>(1, cap / d->n_members));
   b = std::min<long>(b, std::max(1, d->n_slices / 8));
+  // a member's block products and costates are combined one after another, in
+  // both directions: with few members, more than sqrt(2 n_t) blocks lengthen
+  // len + 2 blocks (one member, 2000 slices: 250 blocks of 8 took 221 us in
+  // the chains, 63 of 32 take a third)
+  while (b > 1 && b * b > 2L * d->n_slices) --b;
   if (b <= 1) return;
   const int L = (int)((d->n_slices + b - 1) / b);
   *len = L;

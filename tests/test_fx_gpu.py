@@ -121,3 +121,42 @@ def test_gate_chain_blocks(pg, mode, D, n_t, n_m):
         p.close()
     assert abs(F - Fo) <= 1e-10
     assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
+
+
+@pytest.mark.parametrize("mode", ["exact", "ref_mr", "ref_grape"])
+@pytest.mark.parametrize("D,n_t,n_m,n_p", [(2, 1, 1, 1), (2, 300, 2, 8), (3, 2, 3, 2), (4, 17, 1, 3), (7, 9, 2, 1),
+                                           (8, 40, 2, 8), (13, 3, 1, 5), (16, 21, 2, 8)])
+def test_state_chains(pg, mode, D, n_t, n_m, n_p):
+    """State chains of one slice to many, one to eight pairs (the fewest slices
+    in flight), pairs of very different norms, a dissipative generator.  FP64's
+    bars; a vector's own exponent keeps the small pair's overlap to the same
+    relative error."""
+    from oracle import members as mb
+    rng = np.random.default_rng(11 * D + n_t)
+    X = rng.normal(size=(3, D, D)) + 1j * rng.normal(size=(3, D, D))
+    X = X - np.swapaxes(X.conj(), -1, -2)
+    X[0] -= 0.05 * np.eye(D)
+    V = rng.normal(size=(2, n_p, D)) + 1j * rng.normal(size=(2, n_p, D))
+    V /= np.linalg.norm(V, axis=2, keepdims=True)
+    if n_p > 1:
+        V[:, -1] *= 1e-6
+    kw = dict(drifts=X[:1], controls=X[1:], dt=np.full(n_t, 0.2 / (D + 4)), generator="liouvillian",
+              member_scale=rng.uniform(0.9, 1.1, n_m), target="states", fidelity="square", states_init=V[0],
+              states_target=V[1])
+    u = rng.normal(size=(2, n_t))
+    Fo, Go = mb.eval_problem(mb.Problem(n_members=n_m, **kw), u, mode)
+    p = pg.Problem(grad_mode=mode, precision="fp64", **kw)
+    F, G = p.eval(u)
+    F1, _ = p.eval(u, want_grad=False)
+    p.close()
+    assert F1 == F
+    assert abs(F - Fo) <= 1e-10
+    assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
+    if n_p > 1:  # the small pair alone
+        kw.update(states_init=V[0, -1:], states_target=V[1, -1:])
+        Fo, Go = mb.eval_problem(mb.Problem(n_members=n_m, **kw), u, mode)
+        p = pg.Problem(grad_mode=mode, precision="fp64", **kw)
+        F, G = p.eval(u)
+        p.close()
+        assert abs(F - Fo) <= 1e-10 * abs(Fo)
+        assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
