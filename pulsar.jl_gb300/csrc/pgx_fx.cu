@@ -1084,133 +1084,236 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
 //   backward  lambda_k = U_k' lambda_{k+1} from lambda_n = t_s, stored without
 //             the factor conj(kappa_s) (the gradient applies it), so it does not
 //             wait for the forward chain
-// A warp's FP64 FMA takes 70 cycles of its scheduler's pipe, so the FP64 chain
-// spent 1,500 (D = 2) to 3,000 cycles a slice on one dot product and the exposed
-// load of U_k.  A complex multiply-add is 12 integer ones here; U streams into
-// shared memory with cp.async a few slices ahead.
 //
-// Vectors are x 2^(E - 57), |x| < 2^57, one exponent per vector; U_k's entries
-// u 2^(EX - 1081), |u| < 2^59.  A step keeps 57 bits of the products' scale.
+// Bound: the latency of one step, n_t times.  A warp's FP64 FMA takes 70 cycles
+// of its scheduler's pipe, so FP64 chains spent 1,500 (D = 2) to 3,000 cycles a
+// slice; a complex multiply-add is 12 integer ones here.  Only the multiply-
+// adds, their sum over the lanes of a row and the hand-over of the vector are
+// left on the chain: eight helper warps load and convert the next chunk of
+// slices and write the last chunk's vectors out meanwhile.  (With the
+// conversions in the chain's own warp a D = 2 step took 1,070 cycles.)
+//
+// Vectors are x 2^(E - 57) with one exponent, U_k's entries u 2^-G, both in two
+// balanced halves of 30 bits; y = x u 2^-G takes all four partial products, so
+// a step only rounds its result.  (Without the low one, overlaps of 1e-3 lost
+// five bits against FP64, which keeps small amplitudes to their own scale.)
+//   Hermitian generators keep the vector's norm, so its exponent never moves:
+//   |x| < 2^58 at the start, so ||x|| < 2^60.5, and G = 60 with ||u|| <= 2^60 in
+//   every row keep each sum inside 63 bits (Cauchy-Schwarz).
+//   Others: |x| < 2^57, renewed every step; |u| < 2^58 below U_k's largest
+//   entry, G = 58.
 template <int D> struct StCfg {
   static constexpr int QS = 32 / D < D ? 32 / D : D;  // lanes that share a row
   static constexpr int QN = D / QS;                   // columns of a lane
   static constexpr int ACTIVE = D * QS;               // the other lanes repeat their work
-  static constexpr int STAGE = D * D * 16;            // bytes of one slice
-  static constexpr int MAX_STAGES = 8;
+  static constexpr int CH = D >= 16 ? 2 : D >= 8 ? 8 : 128 / D;  // slices of a chunk
+  static constexpr int HELPERS = 8;
+  static constexpr int NPT = 2 * CH * D * D / (32 * HELPERS);  // entries of a helper lane and chunk, both directions
+  static constexpr int RING = 2 * CH * D * D;         // entries of one chunk
+  __host__ __device__ static constexpr size_t smem(int chains) {
+    return (size_t)16 * (2 * RING + 2 * chains * CH * D) + sizeof(int) * (2 * 2 * CH + 2 * chains * CH);
+  }
 };
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+__device__ __forceinline__ int4 split2(long long re, long long im) {  // x = hi 2^30 + lo, |lo| <= 2^29
+  const int r0 = (int)((uint32_t)re << 2) >> 2, i0 = (int)((uint32_t)im << 2) >> 2;
+  return make_int4(r0, (int)((re - r0) >> 30), i0, (int)((im - i0) >> 30));
 }
+__device__ __forceinline__ long long join2(int lo, int hi) { return ((long long)hi << 30) + lo; }
 
-template <int D>
-__global__ void __launch_bounds__(512) k_fx_states(ProbDev p, WorkDev w, int store, int stages) {
+template <int D, bool HERM>
+__global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(ProbDev p, WorkDev w, int store) {
   using C = StCfg<D>;
-  constexpr int QN = C::QN, QS = C::QS;
+  constexpr int QN = C::QN, QS = C::QS, CH = C::CH, NPT = C::NPT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_f[8];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, np = p.n_pairs, m = blockIdx.x;
-  const int s = wid % np;
-  const bool fwd = wid < np;
-  const int al = lane & (C::ACTIVE - 1), r = al % D, q0 = al / D * QN;
-  // per warp: the ring of U, then two copies of the vector
-  unsigned char* mine = smem_raw + (size_t)wid * ((size_t)stages * C::STAGE + 2 * D * 16);
-  const uint32_t ring = smem_u32(mine);
-  longlong2* vec = reinterpret_cast<longlong2*>(mine + (size_t)stages * C::STAGE);
+  __shared__ int s_bad;
+  const int np = p.n_pairs, chains = store ? 2 * np : np, m = blockIdx.x;
+  int4* ring = reinterpret_cast<int4*>(smem_raw);      // [2][direction][CH][D D]
+  int4* hist = ring + 2 * C::RING;                     // [2][chain][CH][D] the chunk's vectors
+  int* s_eu = reinterpret_cast<int*>(hist + 2 * chains * CH * D);  // [2][direction][CH] biased exponents
+  int* s_ev = s_eu + 2 * 2 * CH;                       // [2][chain][CH]
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double2* Um = w.U + (size_t)m * p.n_t * D * D;
-  // element (i, c) of a slice at column c, row i ^ (c mod 8): rows and columns
+  const size_t pan = (size_t)np * D;
+  const int chunks = (p.n_t + CH - 1) / CH;
+  // entry (i, c) of a slice at column c, row i ^ (c mod 8): rows and columns
   // both read without bank conflicts
   auto swz = [](int i, int c) { return c * D + (i ^ (c & (D < 8 ? D - 1 : 7))); };
-  auto fetch = [&](int step) {  // slice of chain step `step`
-    if (step < p.n_t) {
-      const double2* src = Um + (size_t)(fwd ? step : p.n_t - 1 - step) * D * D;
-      const uint32_t dst = ring + (uint32_t)(step % stages) * C::STAGE;
-      for (int e = lane; e < D * D; e += 32) cp_async16(dst + swz(e % D, e / D) * 16, src + e);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  for (int i = 0; i + 1 < stages; ++i) fetch(i);
+  if (threadIdx.x == 0) s_bad = 0;
+  if (!HERM)
+    for (int i = threadIdx.x; i < 2 * 2 * CH; i += blockDim.x) s_eu[i] = 0;
+  __syncthreads();
 
-  const size_t pan = (size_t)np * D;
-  double2* out = (fwd ? w.psi : w.lam) + (size_t)m * (p.n_t + 1) * pan + (size_t)s * D;
-  const double2 v0 = (fwd ? p.psi_init : p.psi_targ)[s * D + r];
-  int E = 0;
-  bool bad = false;
-  long long xr, xi;
-  {
-    double x[2] = {v0.x, v0.y};
-    uint32_t M = 0;
+  if (wid >= chains) {  // helpers
+    const int h = threadIdx.x - 32 * chains;
+    double2 raw[NPT];
+    auto where = [&](int c, int i, int& dir, int& sl, int& e) {  // entry i of chunk c: its slice, or -1
+      const int x = i * 32 * C::HELPERS + h;
+      dir = x / (CH * D * D);
+      sl = x / (D * D) % CH;
+      e = x % (D * D);
+      const int st = c * CH + sl;
+      return st < p.n_t && (dir == 0 || store) ? (dir == 0 ? st : p.n_t - 1 - st) : -1;
+    };
+    auto fetch = [&](int c) {
+      if (c >= chunks) return;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) M = max(M, (uint32_t)__double2hiint(x[h]) & 0x7ff00000u);
-    const int EX = (int)(__reduce_max_sync(0xffffffffu, M) >> 20);
-    bad = EX == 0x7ff;
-    xr = from_double(x[0], EX, 4);
-    xi = from_double(x[1], EX, 4);
-    E = EX - 1022;
-  }
-  if (store && lane < D) out[(fwd ? (size_t)0 : (size_t)p.n_t * pan) + r] = v0;
+      for (int i = 0; i < NPT; ++i) {
+        int dir, sl, e;
+        const int k = where(c, i, dir, sl, e);
+        raw[i] = k >= 0 ? Um[(size_t)k * D * D + e] : make_double2(0.0, 0.0);
+      }
+    };
+    auto convert = [&](int c) {
+      if (c >= chunks) return;
+      const int buf = c & 1;
+      int dir, sl, e;
+      bool bad = false;
+#pragma unroll
+      for (int i = 0; i < NPT; ++i) {
+        where(c, i, dir, sl, e);
+        const int ex = (int)(max((uint32_t)__double2hiint(raw[i].x) & 0x7ff00000u,
+                                 (uint32_t)__double2hiint(raw[i].y) & 0x7ff00000u) >> 20);
+        bad |= ex >= (HERM ? 1024 : 0x7ff);  // a unitary's entries stay below 2
+        if (!HERM) atomicMax(&s_eu[(buf * 2 + dir) * CH + sl], ex);
+      }
+      if (bad) s_bad = 1;
+      if (!HERM) asm volatile("bar.sync 1, %0;" ::"n"(32 * C::HELPERS) : "memory");
+#pragma unroll
+      for (int i = 0; i < NPT; ++i) {
+        where(c, i, dir, sl, e);
+        const int EX = HERM ? 1023 : s_eu[(buf * 2 + dir) * CH + sl];
+        ring[(size_t)(buf * 2 + dir) * CH * D * D + sl * D * D + swz(e % D, e / D)] =
+            split2(from_double(raw[i].x, EX, HERM ? 8 : 5), from_double(raw[i].y, EX, HERM ? 8 : 5));
+      }
+    };
+    auto put = [&](int c) {  // the vectors of chunk c
+      if (!store) return;
+      const int buf = c & 1;
+      for (int x = h; x < chains * CH * D; x += 32 * C::HELPERS) {
+        const int ch = x / (CH * D), sl = x / D % CH, r = x % D, st = c * CH + sl;
+        if (st >= p.n_t) continue;
+        const int4 v = hist[(size_t)(buf * chains + ch) * CH * D + sl * D + r];
+        const int E = s_ev[(buf * chains + ch) * CH + sl];
+        double2* out = (ch < np ? w.psi : w.lam) + ((size_t)m * (p.n_t + 1) + (ch < np ? st + 1 : p.n_t - 1 - st)) * pan;
+        double2 d = make_double2(to_double(join2(v.x, v.y), E - 57), to_double(join2(v.z, v.w), E - 57));
+        if (E == kNotFinite) d.x = d.y = __longlong_as_double(0x7ff8000000000000ll);
+        out[(size_t)(ch % np) * D + r] = d;
+      }
+    };
+    fetch(0);
+    convert(0);
+    fetch(1);
+    if (store)
+      for (int x = h; x < chains * D; x += 32 * C::HELPERS) {  // both ends
+        const int ch = x / D, r = x % D;
+        const size_t at = (size_t)(ch % np) * D + r;
+        if (ch < np) w.psi[(size_t)m * (p.n_t + 1) * pan + at] = p.psi_init[at];
+        else w.lam[((size_t)m * (p.n_t + 1) + p.n_t) * pan + at] = p.psi_targ[at];
+      }
+    __syncthreads();
 #pragma unroll 1
-  for (int step = 0; step < p.n_t; ++step) {
-    longlong2* v = vec + (step & 1) * D;
-    if (lane < D) v[r] = make_longlong2(xr, xi);
-    // stages - 1 groups stay in flight, one is needed now
-    if (stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
-    else if (stages < 6) asm volatile("cp.async.wait_group 1;" ::: "memory");
-    else asm volatile("cp.async.wait_group 4;" ::: "memory");
-    __syncwarp();
-    const double2* U = reinterpret_cast<const double2*>(mine + (size_t)(step % stages) * C::STAGE);
-    double2 a[QN];
-    uint32_t M = 0;
+    for (int c = 0; c < chunks; ++c) {
+      if (!HERM) {  // the exponents of the chunk before last are read
+        for (int i = h; i < 2 * CH; i += 32 * C::HELPERS) s_eu[((c + 1) & 1) * 2 * CH + i] = 0;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * C::HELPERS) : "memory");
+      }
+      convert(c + 1);
+      fetch(c + 2);
+      if (c > 0) put(c - 1);
+      __syncthreads();
+    }
+    put(chunks - 1);
+    __syncthreads();
+    return;
+  }
+
+  const bool fwd = wid < np;
+  const int s = wid % np, dir = fwd ? 0 : 1;
+  const int al = lane & (C::ACTIVE - 1), r = al % D, q0 = al / D * QN;
+  int E;
+  bool bad;
+  int4 first;  // the start vector, of row `r`
+  {
+    const double2 v0 = (fwd ? p.psi_init : p.psi_targ)[s * D + r];
+    const int EX = (int)(__reduce_max_sync(0xffffffffu, max((uint32_t)__double2hiint(v0.x) & 0x7ff00000u,
+                                                            (uint32_t)__double2hiint(v0.y) & 0x7ff00000u)) >> 20);
+    bad = EX == 0x7ff;
+    const int guard = HERM ? 5 : 4;
+    first = split2(from_double(v0.x, EX, guard), from_double(v0.y, EX, guard));
+    E = EX - 1018 - guard;  // x 2^(EX - 1075 - guard)
+  }
+  // the start vector goes where chunk -1 would have left its last one
+  int4* mine = hist + (size_t)wid * CH * D;
+  const size_t other = (size_t)chains * CH * D;
+  if (lane < D) mine[other + (CH - 1) * D + r] = first;
+  int4 last = first;
+  __syncthreads();
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    const int buf = c & 1, n = min(CH, p.n_t - c * CH);
+    const int4* U = ring + (size_t)(buf * 2 + dir) * CH * D * D;
+    const int4* prev = mine + (buf ? 0 : other) + (CH - 1) * D;
+    int4* cur = mine + (buf ? other : 0);
+    int4 u[QN];
 #pragma unroll
-    for (int i = 0; i < QN; ++i) {
-      a[i] = fwd ? U[swz(r, q0 + i)] : U[swz(q0 + i, r)];
-      M = max(M, max((uint32_t)__double2hiint(a[i].x) & 0x7ff00000u, (uint32_t)__double2hiint(a[i].y) & 0x7ff00000u));
-    }
-    const int EX = (int)(__reduce_max_sync(0xffffffffu, M) >> 20);
-    // re = sum ur xr -+ ui xi, im = sum ur xi +- ui xr (backward: conj(U))
-    long long pr = 0, pi = 0, nr = 0, ni = 0, mpr = 0, mpi = 0, mnr = 0, mni = 0;
+    for (int i = 0; i < QN; ++i) u[i] = fwd ? U[swz(r, q0 + i)] : U[swz(q0 + i, r)];
+#pragma unroll 1
+    for (int sl = 0; sl < n; ++sl) {
+      // re = sum ur xr -+ ui xi, im = sum ur xi +- ui xr (backward: conj(U))
+      // high, mixed and low partial products of the four sums
+      long long pr = 0, pi = 0, nr = 0, ni = 0, mpr = 0, mpi = 0, mnr = 0, mni = 0, lpr = 0, lpi = 0, lnr = 0, lni = 0;
 #pragma unroll
-    for (int i = 0; i < QN; ++i) {
-      const longlong2 x = v[q0 + i];
-      const long long ur = from_double(a[i].x, EX, 6), ui = from_double(a[i].y, EX, 6);
-      const int ur0 = (int)ur, ur1 = (int)((ur + 0x80000000ll) >> 32), ui0 = (int)ui, ui1 = (int)((ui + 0x80000000ll) >> 32);
-      const int xr0 = (int)x.x, xr1 = (int)((x.x + 0x80000000ll) >> 32), xi0 = (int)x.y, xi1 = (int)((x.y + 0x80000000ll) >> 32);
-      pr += (long long)ur1 * xr1;
-      mpr += (long long)ur1 * xr0 + (long long)ur0 * xr1;
-      nr += (long long)ui1 * xi1;
-      mnr += (long long)ui1 * xi0 + (long long)ui0 * xi1;
-      pi += (long long)ur1 * xi1;
-      mpi += (long long)ur1 * xi0 + (long long)ur0 * xi1;
-      ni += (long long)ui1 * xr1;
-      mni += (long long)ui1 * xr0 + (long long)ui0 * xr1;
-    }
-    const long long hr = fwd ? pr - nr : pr + nr, hi = fwd ? pi + ni : pi - ni;
-    const long long lr = fwd ? mpr - mnr : mpr + mnr, li = fwd ? mpi + mni : mpi - mni;
-    long long yr = (hr << 5) + shift_round(lr, 27), yi = (hi << 5) + shift_round(li, 27);
+      for (int i = 0; i < QN; ++i) {
+        const int4 x = prev[q0 + i];
+        pr += (long long)u[i].y * x.y;
+        mpr += (long long)u[i].y * x.x + (long long)u[i].x * x.y;
+        lpr += (long long)u[i].x * x.x;
+        nr += (long long)u[i].w * x.w;
+        mnr += (long long)u[i].w * x.z + (long long)u[i].z * x.w;
+        lnr += (long long)u[i].z * x.z;
+        pi += (long long)u[i].y * x.w;
+        mpi += (long long)u[i].y * x.z + (long long)u[i].x * x.w;
+        lpi += (long long)u[i].x * x.z;
+        ni += (long long)u[i].w * x.y;
+        mni += (long long)u[i].w * x.x + (long long)u[i].z * x.y;
+        lni += (long long)u[i].z * x.x;
+      }
+      const int EX = HERM ? 0 : s_eu[(buf * 2 + dir) * CH + sl];
+      if (sl + 1 < n) {
+        const int4* V = U + (sl + 1) * D * D;
 #pragma unroll
-    for (int o = D; o < D * QS; o <<= 1) {
-      yr += __shfl_xor_sync(0xffffffffu, yr, o);
-      yi += __shfl_xor_sync(0xffffffffu, yi, o);
+        for (int i = 0; i < QN; ++i) u[i] = fwd ? V[swz(r, q0 + i)] : V[swz(q0 + i, r)];
+      }
+      constexpr int SH = HERM ? 0 : 2;
+      const long long mr = (fwd ? mpr - mnr : mpr + mnr) + ((fwd ? lpr - lnr : lpr + lnr) >> 30);
+      const long long mi = (fwd ? mpi + mni : mpi - mni) + ((fwd ? lpi + lni : lpi - lni) >> 30);
+      long long yr = ((fwd ? pr - nr : pr + nr) << SH) + shift_round(mr, 30 - SH);
+      long long yi = ((fwd ? pi + ni : pi - ni) << SH) + shift_round(mi, 30 - SH);
+#pragma unroll
+      for (int o = D; o < D * QS; o <<= 1) {
+        yr += __shfl_xor_sync(0xffffffffu, yr, o);
+        yi += __shfl_xor_sync(0xffffffffu, yi, o);
+      }
+      if (!HERM) {
+        const uint32_t top = __reduce_max_sync(0xffffffffu, max((uint32_t)abs((int)(yr >> 32)), (uint32_t)abs((int)(yi >> 32))));
+        const int sh = __clz(top + 1) - 7;
+        yr = sh >= 0 ? yr << sh : shift_round(yr, -sh);
+        yi = sh >= 0 ? yi << sh : shift_round(yi, -sh);
+        E = max(E + EX - 1022 - sh, -(1 << 20));
+      }
+      last = split2(yr, yi);
+      if (lane < D) cur[sl * D + r] = last;
+      if (lane == 0) s_ev[(buf * chains + wid) * CH + sl] = bad ? kNotFinite : E;
+      __syncwarp();
+      prev = cur + sl * D;
     }
-    const uint32_t top = __reduce_max_sync(0xffffffffu, max((uint32_t)abs((int)(yr >> 32)), (uint32_t)abs((int)(yi >> 32))));
-    const int sh = __clz(top + 1) - 7;
-    xr = sh >= 0 ? yr << sh : shift_round(yr, -sh);
-    xi = sh >= 0 ? yi << sh : shift_round(yi, -sh);
-    bad |= EX == 0x7ff;
-    E = max(E + EX - 1022 - sh, -(1 << 20));
-    if (store && lane < D) {
-      const double nan = __longlong_as_double(0x7ff8000000000000ll);
-      double2 d = make_double2(to_double(xr, E - 57), to_double(xi, E - 57));
-      if (bad) d.x = d.y = nan;
-      out[(size_t)(fwd ? step + 1 : p.n_t - 1 - step) * pan + r] = d;
-    }
-    __syncwarp();  // the slot of this slice is free
-    fetch(step + stages - 1);
+    __syncthreads();
   }
   if (fwd) {
-    const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    double2 d = make_double2(to_double(xr, E - 57), to_double(xi, E - 57));
-    if (bad) d.x = d.y = nan;
+    double2 d = make_double2(to_double(join2(last.x, last.y), E - 57), to_double(join2(last.z, last.w), E - 57));
+    if (bad || s_bad) d.x = d.y = __longlong_as_double(0x7ff8000000000000ll);
     double2 z = make_double2(0.0, 0.0);
     if (lane < D) z = cmac_cj(z, p.psi_targ[s * D + r], d);
 #pragma unroll
@@ -1338,12 +1441,11 @@ template <int D> static long prefix_capacity() {
 
 template <int D> static cudaError_t do_states(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
   using C = StCfg<D>;
-  const int warps = p.n_pairs * (store ? 2 : 1);
-  int stages = (int)(196608 / ((size_t)warps * C::STAGE));
-  if (stages > C::MAX_STAGES) stages = C::MAX_STAGES;
-  const size_t smem = (size_t)warps * ((size_t)stages * C::STAGE + 2 * D * 16);
-  set_smem_once((const void*)k_fx_states<D>, smem);
-  k_fx_states<D><<<p.n_members, 32 * warps, smem, li.stream>>>(p, w, store ? 1 : 0, stages);
+  const int chains = p.n_pairs * (store ? 2 : 1);
+  const size_t smem = C::smem(chains);
+  auto kernel = p.gen == GEN_HERM ? k_fx_states<D, true> : k_fx_states<D, false>;
+  set_smem_once((const void*)kernel, smem);
+  kernel<<<p.n_members, 32 * (chains + C::HELPERS), smem, li.stream>>>(p, w, store ? 1 : 0);
   ++*li.launches;
   return cudaGetLastError();
 }

@@ -160,3 +160,27 @@ def test_state_chains(pg, mode, D, n_t, n_m, n_p):
         p.close()
         assert abs(F - Fo) <= 1e-10 * abs(Fo)
         assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
+
+
+@pytest.mark.parametrize("D,n_t,n_p", [(2, 64, 1), (2, 129, 2), (4, 33, 8), (8, 8, 3), (8, 9, 8), (16, 5, 8), (12, 2, 1)])
+def test_state_chains_hermitian(pg, D, n_t, n_p):
+    """Unitary state chains at the edges of a chunk of slices (one, exactly
+    full, one over), both gradient forms against the oracle."""
+    from oracle import members as mb
+    rng = np.random.default_rng(13 * D + n_t)
+    X = rng.normal(size=(3, D, D)) + 1j * rng.normal(size=(3, D, D))
+    X = X + np.swapaxes(X.conj(), -1, -2)
+    V = rng.normal(size=(2, n_p, D)) + 1j * rng.normal(size=(2, n_p, D))
+    V /= np.linalg.norm(V, axis=2, keepdims=True)
+    kw = dict(drifts=X[:1], controls=X[1:], dt=np.full(n_t, 0.3 / (D + 4)), member_scale=np.array([0.9, 1.0, 1.1]),
+              target="states", fidelity="square", states_init=V[0], states_target=V[1])
+    u = rng.normal(size=(2, n_t))
+    for mode in ("exact", "ref_grape"):
+        Fo, Go = mb.eval_problem(mb.Problem(n_members=3, **kw), u, mode)
+        p = pg.Problem(grad_mode=mode, precision="fp64", **kw)
+        F, G = p.eval(u)
+        F1, _ = p.eval(u, want_grad=False)
+        p.close()
+        assert F1 == F
+        assert abs(F - Fo) <= 1e-10
+        assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
