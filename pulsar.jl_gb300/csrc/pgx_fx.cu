@@ -485,7 +485,7 @@ __device__ __forceinline__ void times_prefix(const Tm<D, W>& tm, const ProbDev& 
   store_planes<D, W>(tm, pr, x, kSlices);
   store_planes<D, W>(tm, pl, r, kSlices);
   tm.sync();
-  mul<D, W>(tm, pl, pr, kChainLevels<D>, x);
+  mul_fixed<D, W, kChainLevels<D>>(tm, pl, pr, x);
   const int e = normalize<D, W>(tm, x, E + ER);
   E = max(E, ER) == kNotFinite ? kNotFinite : e;
 }
@@ -827,13 +827,12 @@ template <int D, int W> struct ChainTeam {
         pl(smem_u32(smem)), pr(pl + Geo<D, W>::PLANES) {}
   // (r, E) <- left (r, E); an operand that is not finite stays so
   template <bool R_IS_LEFT>
-  __device__ __forceinline__ void step(long long (&r)[Geo<D, W>::NV], int& E, const long long (&x)[Geo<D, W>::NV], int Ex,
-                                       int levels = kChainLevels<D>) {
+  __device__ __forceinline__ void step(long long (&r)[Geo<D, W>::NV], int& E, const long long (&x)[Geo<D, W>::NV], int Ex) {
     tm.sync();  // the last product has read its planes
-    store_planes<D, W>(tm, R_IS_LEFT ? pl : pr, r, levels);
-    store_planes<D, W>(tm, R_IS_LEFT ? pr : pl, x, levels);
+    store_planes<D, W>(tm, R_IS_LEFT ? pl : pr, r, kSlices);
+    store_planes<D, W>(tm, R_IS_LEFT ? pr : pl, x, kSlices);
     tm.sync();
-    mul<D, W>(tm, pl, pr, levels, r);
+    mul_fixed<D, W, kChainLevels<D>>(tm, pl, pr, r);
     const int e = normalize<D, W>(tm, r, E + Ex);
     E = max(E, Ex) == kNotFinite ? kNotFinite : e;
   }
@@ -900,10 +899,9 @@ k_fx_chain_bwd(ProbDev p, WorkDev w, int blocks, int len) {
 // for the FP32 fix-up, block products as df pairs.  Seven levels: with six
 // (2^-47.5 of the factors' scale) the defect of U_total, 4.8e-12 after 1000
 // slices, passed that of the df products (9.6e-13); seven leave 1e-13.
-constexpr int kPrefixLevelsDf = 7;
 
 template <int D>
-__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS) k_fx_prefix_df(ProbDev p, WorkDev w, int store) {
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS, 2) k_fx_prefix_df(ProbDev p, WorkDev w, int store) {
   using C = ChainCfg<D>;
   constexpr int W = C::W, H = Geo<D, W>::NV / 2;
   using G = Geo<D, W>;
@@ -948,7 +946,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS) k_fx
       for (int v = 0; v < 2 * H; ++v) r[v] = u[v];
       E = Eu;
     } else {
-      ct.template step<false>(r, E, u, Eu, kPrefixLevelsDf);
+      ct.template step<false>(r, E, u, Eu);
     }
     if (store && k + 1 < k1) {
       const float sc = E == kNotFinite ? __int_as_float(0x7fc00000) : ldexpf(1.f, E - kFrac);
@@ -1487,7 +1485,9 @@ long fx_prefix_capacity(int Dp) {
   switch (Dp) {
     case 8: return fx::prefix_capacity<8>();
     case 16: return fx::prefix_capacity<16>();
-    case 32: return fx::prefix_capacity<32>();
+    // two of 57 KB are resident, but the FP32 suffixes beside them gain from more
+    // blocks than the prefixes lose by queueing (64 x 500: 8.67 -> 8.41 ms with 4)
+    case 32: return 4;
     default: return 0;
   }
 }

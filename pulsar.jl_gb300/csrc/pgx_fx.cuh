@@ -182,11 +182,78 @@ __device__ __forceinline__ void mma_pair(float (&acc)[Geo<D, W>::NV], const Left
 
 constexpr uint32_t kPairBias = (0x4B400000u << 8) + 0x4B400000u;  // two magic starts joined (mod 2^32)
 
-// Levels (L, L + 1) of A B, L even, level L + 1 only if `two`: (level L) 2^8 +
+// Levels (L, L + 1) of A B, L even, level L + 1 only if TWO: (level L) 2^8 +
 // (level L + 1), summed over the 16-deep steps.  The two levels share every
 // left digit, and the right digit of level L + 1 is the one level L uses next.
+// All digit loops are unrolled: as rolled loops the products of the d = 8 and
+// d = 16 chains took 1.5 and 1.25 times as long.
+template <int D, int W, int L, bool TWO>
+__device__ __forceinline__ void level_pair(uint32_t la, uint32_t rb, uint32_t (&t)[Geo<D, W>::NV]) {
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV;
+  constexpr uint32_t kDigit = 2 * G::PLANE;
+#pragma unroll 1
+  for (int kt = 0; kt < G::KT; ++kt) {
+    float a0[NV], a1[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) a0[v] = a1[v] = kMagic;
+    const uint32_t pl = la + kt * 2 * (D / 8) * 128, pr = rb + kt * 2 * 128;
+    Right<D, W> b[2];
+    if (TWO && L + 1 < kSlices) b[1].load(pr + (L + 1) * kDigit);
+#pragma unroll
+    for (int i = 0; i < kSlices; ++i) {
+      if (i > L + (TWO ? 1 : 0)) break;
+      Left<D, W> a;
+      a.load(pl + i * kDigit);
+      if (i <= L) b[i & 1].load(pr + (L - i) * kDigit);  // b[(i + 1) & 1] holds B_{L + 1 - i}
+      if (TWO && L + 1 - i < kSlices) mma_pair<D, W>(a1, a, b[(i + 1) & 1]);
+      if (i <= L) mma_pair<D, W>(a0, a, b[i & 1]);
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const uint32_t x = (__float_as_uint(a0[v]) << 8) + __float_as_uint(a1[v]) - kPairBias;
+      t[v] = kt == 0 ? x : t[v] + x;
+    }
+  }
+}
+
+// r <- r 2^-16 + t 2^32: needs no carries, because a level pair only touches
+// the high word.
+template <int NV> __device__ __forceinline__ void join_pair(long long (&r)[NV], const uint32_t (&t)[NV], int L) {
+  if (L == 0) {  // to nearest: a floor's bias adds up over a chain of products
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] += 0x8000;
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int hi = (int)(r[v] >> 32);
+    const uint32_t lo = __funnelshift_r((uint32_t)r[v], (uint32_t)hi, 16);
+    r[v] = (long long)((unsigned long long)(t[v] + (uint32_t)(hi >> 16)) << 32 | lo);
+  }
+}
+
+// r = A B with N levels, as value 2^(EA + EB - 56): pa, pb address the factors'
+// digit planes.  The lowest two levels first, which keeps 32 bits below the
+// last one.
+template <int D, int W, int N, int L = (N - 1) & ~1>
+__device__ __forceinline__ void mul_levels(uint32_t la, uint32_t rb, long long (&r)[Geo<D, W>::NV]) {
+  uint32_t t[Geo<D, W>::NV];
+  level_pair<D, W, L, (L + 1 < N)>(la, rb, t);
+  join_pair<Geo<D, W>::NV>(r, t, L);
+  if constexpr (L > 0) mul_levels<D, W, N, L - 2>(la, rb, r);
+}
+template <int D, int W, int N>
+__device__ __forceinline__ void mul_fixed(const Tm<D, W>& tm, uint32_t pa, uint32_t pb, long long (&r)[Geo<D, W>::NV]) {
+#pragma unroll
+  for (int v = 0; v < Geo<D, W>::NV; ++v) r[v] = 0;
+  mul_levels<D, W, N>(Left<D, W>::at(tm, pa), Right<D, W>::at(tm, pb), r);
+}
+
+// Level pair (L, L + 1) with L and `two` chosen by the data: rolled digit loops
+// (eight unrolled forms behind a switch were as fast at D = 16 and a fifth
+// slower at D = 8).
 template <int D, int W>
-__device__ __forceinline__ void level_pair(uint32_t la, uint32_t rb, int L, bool two, uint32_t (&t)[Geo<D, W>::NV]) {
+__device__ __forceinline__ void any_level_pair(uint32_t la, uint32_t rb, int L, bool two, uint32_t (&t)[Geo<D, W>::NV]) {
   using G = Geo<D, W>;
   constexpr int NV = G::NV;
   constexpr uint32_t kDigit = 2 * G::PLANE;
@@ -244,36 +311,18 @@ __device__ __forceinline__ void level_pair(uint32_t la, uint32_t rb, int L, bool
   }
 }
 
-// r <- r 2^-16 + t 2^32: needs no carries, because a level pair only touches
-// the high word.
-template <int NV> __device__ __forceinline__ void join_pair(long long (&r)[NV], const uint32_t (&t)[NV], int L) {
-  if (L == 0) {  // to nearest: a floor's bias adds up over a chain of products
-#pragma unroll
-    for (int v = 0; v < NV; ++v) r[v] += 0x8000;
-  }
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    const int hi = (int)(r[v] >> 32);
-    const uint32_t lo = __funnelshift_r((uint32_t)r[v], (uint32_t)hi, 16);
-    r[v] = (long long)((unsigned long long)(t[v] + (uint32_t)(hi >> 16)) << 32 | lo);
-  }
-}
-
-// r = A B with `nlev` levels, as value 2^(EA + EB - 56): pa, pb address the
-// factors' digit planes.  The lowest two levels first, which keeps 32 bits
-// below the last one.
+// r = A B with `nlev` levels.
 template <int D, int W>
 __device__ __forceinline__ void mul(const Tm<D, W>& tm, uint32_t pa, uint32_t pb, int nlev,
                                     long long (&r)[Geo<D, W>::NV]) {
-  constexpr int NV = Geo<D, W>::NV;
   const uint32_t la = Left<D, W>::at(tm, pa), rb = Right<D, W>::at(tm, pb);
 #pragma unroll
-  for (int v = 0; v < NV; ++v) r[v] = 0;
+  for (int v = 0; v < Geo<D, W>::NV; ++v) r[v] = 0;
 #pragma unroll 1
   for (int L = (nlev - 1) & ~1; L >= 0; L -= 2) {
-    uint32_t t[NV];
-    level_pair<D, W>(la, rb, L, L + 1 < nlev, t);
-    join_pair<NV>(r, t, L);
+    uint32_t t[Geo<D, W>::NV];
+    any_level_pair<D, W>(la, rb, L, L + 1 < nlev, t);
+    join_pair<Geo<D, W>::NV>(r, t, L);
   }
 }
 
@@ -296,6 +345,8 @@ __device__ __forceinline__ void commutator(const Tm<D, W>& tm, uint32_t pa, uint
       }
     }
   } else {
+    const uint32_t la = Left<D, W>::at(tm, pa), rb = Right<D, W>::at(tm, pb);
+    const uint32_t lb = Left<D, W>::at(tm, pb), ra = Right<D, W>::at(tm, pa);
 #pragma unroll
     for (int v = 0; v < NV; ++v) r[v] = 0;
 #pragma unroll 1
@@ -303,7 +354,7 @@ __device__ __forceinline__ void commutator(const Tm<D, W>& tm, uint32_t pa, uint
       uint32_t t[NV], s[NV];
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
-        level_pair<D, W>(Left<D, W>::at(tm, h ? pa : pb), Right<D, W>::at(tm, h ? pb : pa), L, L + 1 < nlev, t);
+        any_level_pair<D, W>(h ? la : lb, h ? rb : ra, L, L + 1 < nlev, t);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
           if (h) t[v] -= s[v];
