@@ -268,6 +268,7 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
       if (EA > kNever / 2 || l1 > 60.f) {
         if constexpr (DF) {
           store_df<D, W>(tm, (float4*)out, r, 0x7ff);
+          if (tm.lane == 0 && tm.w == 0) *w.norm_flag = 1;
         } else if (packed) {
           put_packed<D, W>(tm.mine((longlong2*)out), r, kNotFinite);
         } else {
@@ -309,6 +310,7 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
           // below 2^-2.6 the 1-norm's own degree is within a product of the best
           const float l2 = l1 > -2.6f ? log2_norm1<D, W>(tm, r, EX, kFrac) : 2.f * l1, lb = fminf(l1, 0.5f * l2);
           choose_degree2<DF>(l1, lb, tm.lane, L, s);
+          if (DF && lb > 0.f && tm.lane == 0 && tm.w == 0) *w.norm_flag = 1;  // beyond the gradient's series
           EB -= s;
           EX -= 2 * s;
           // |X| <= 2^lx, and |Y_i| <= c_2i e^nu, nu = 2^(lb - s) -- for a matrix
@@ -1337,6 +1339,241 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
   }
 }
 
+// ---- the mixed path's exact gradient ---------------------------------------------
+// The commutator series of k_fx_grad in FP32 class: X = sum ad_A^n(N) / (n + 1)!
+// until a term is below 2^-27 of N, six or so at ||A|| = 0.15, each one
+// A D - D A in 3xFP16 (x = hi + lo in FP16, 22 bits; lo hi + hi lo + hi hi
+// accumulated in FP32).  N and every term are scaled by a power of two to a
+// largest entry in [1/2, 1), so FP16's range covers 2^-25 of it.
+//
+// The CUDA-core Frechet derivative (k_grad_gate_mx) executes 15 FP32 products
+// bound by shared-memory operand loads; here A's fragments stay in registers
+// and a term is 24 MMAs a warp and one pass of D through shared memory.
+//
+// The series needs ||A|| up to about 1: the propagator kernel raises
+// w.norm_flag for an evaluation that has larger slices, which then runs the
+// CUDA-core gradient (and its chains' pairing M_k instead of N_k).
+template <int D> struct TfCfg {
+  static constexpr int W = kWarps<D>;
+  static constexpr int TEAMS = D >= 32 ? 1 : 4;
+  static constexpr int MIN_CTAS = D >= 32 ? 2 : 3;
+  static constexpr int SPLIT = 4 * Geo<D, W>::PLANE;  // bytes of a hi, lo pair of matrices
+  static constexpr int TRACE = 32;                    // controls of one pass over the traces
+  static constexpr int TEAM_BYTES = 2 * SPLIT + W * TRACE * 4 + kRed;
+};
+
+// x -> hi, lo planes (FP16).
+template <int D, int W>
+__device__ __forceinline__ void store_split(const Tm<D, W>& tm, uint32_t base, const float (&x)[Geo<D, W>::NV]) {
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV;
+  const uint32_t at = base + (tm.nt0() * (D / 8) + 2 * tm.rt()) * 128 + tm.lane * 4;
+#pragma unroll
+  for (int b = 0; b < NV / 2; ++b) {
+    const int part = b / (NV / 4), nt = b % (NV / 4) / G::NI, i = b % G::NI;
+    const float u = x[2 * b], v = x[2 * b + 1];
+    uint32_t h, l;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(v), "f"(u));
+    float hu, hv;
+    asm("{.reg .f16 a, b; mov.b32 {a, b}, %2; cvt.f32.f16 %0, a; cvt.f32.f16 %1, b;}" : "=f"(hu), "=f"(hv) : "r"(h));
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(v - hv), "f"(u - hu));
+    const uint32_t to = at + part * G::PLANE + (nt * (D / 8) + i) * 128;
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(to), "r"(h) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(to + 2 * G::PLANE), "r"(l) : "memory");
+  }
+}
+
+// 2^-e with the team's largest |x| in [1/2, 1) after scaling by it (1 when all
+// are zero or not finite).
+template <int D, int W>
+__device__ __forceinline__ float unit_scale(const Tm<D, W>& tm, const float (&x)[Geo<D, W>::NV], int slot) {
+  uint32_t M = 0;
+#pragma unroll
+  for (int v = 0; v < Geo<D, W>::NV; ++v) M = max(M, __float_as_uint(x[v]) & 0x7fffffffu);
+  const int ex = (int)(tm.max(M, slot) >> 23);
+  return ex == 0 || ex >= 253 ? 1.f : __uint_as_float((uint32_t)(252 - ex + 1) << 23);  // 2^(126 - ex)
+}
+
+// A = c dt_k (drift + off O + tau_k R + scale sum_j u_jk C_j) in FP32.
+template <int D, int W>
+__device__ __forceinline__ void assemble32(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m, int k,
+                                           const int (&at)[Geo<D, W>::NV / 2], float (&A)[Geo<D, W>::NV]) {
+  constexpr int H = Geo<D, W>::NV / 2;
+  const float dt = p.dt_df[k].x, sc = p.m_scale_df[m].x, off = p.m_offset_df[m].x;
+  const float2* Gd = p.drifts_f32 + (size_t)p.m_drift[m] * D * D;
+  const float2* uk = w.u_df + (size_t)k * p.n_c;
+  const int ro = p.n_ramp ? p.m_ramp[m] : -1;
+  float2 v[H];
+#pragma unroll
+  for (int b = 0; b < H; ++b) {
+    const float2 g = Gd[at[b]], o = p.offset_f32[at[b]];
+    v[b] = make_float2(fmaf(off, o.x, g.x), fmaf(off, o.y, g.y));
+  }
+  if (ro >= 0) {
+    const float4* Rm = p.ramp_ops_df + (size_t)ro * D * D;
+    const float tk = p.tau_df[k].x;
+#pragma unroll
+    for (int b = 0; b < H; ++b) v[b] = make_float2(fmaf(tk, Rm[at[b]].x, v[b].x), fmaf(tk, Rm[at[b]].y, v[b].y));
+  }
+#pragma unroll 1
+  for (int j = 0; j < p.n_c; ++j) {
+    const float a = sc * uk[j].x;
+    const float2* Cj = p.ctrls_f32 + (size_t)j * D * D;
+#pragma unroll
+    for (int b = 0; b < H; ++b) {
+      const float2 c = Cj[at[b]];
+      v[b] = make_float2(fmaf(a, c.x, v[b].x), fmaf(a, c.y, v[b].y));
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < H; ++b) {
+    A[b] = dt * (p.gen == GEN_HERM ? v[b].y : v[b].x);
+    A[H + b] = dt * (p.gen == GEN_HERM ? -v[b].x : v[b].y);
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * TfCfg<D>::W * TfCfg<D>::TEAMS, TfCfg<D>::MIN_CTAS) k_tf_grad(ProbDev p, WorkDev w) {
+  using C = TfCfg<D>;
+  constexpr int W = C::W;
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV, H = NV / 2, KT = G::KT;
+  if (*w.norm_flag) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int team = threadIdx.x / (32 * W);
+  unsigned char* mine = smem_raw + (size_t)team * C::TEAM_BYTES;
+  const uint32_t pa = smem_u32(mine), pd = pa + C::SPLIT;
+  float* traces = reinterpret_cast<float*>(mine + 2 * C::SPLIT);  // [W][TRACE]
+  const Tm<D, W> tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
+                    reinterpret_cast<uint32_t*>(mine + C::TEAM_BYTES - kRed)};
+  int at[H], tr[H];  // the lane's entries, and their transposes
+#pragma unroll
+  for (int b = 0; b < H; ++b) {
+    const int r = tm.row(b / 2 % G::NI), c = tm.col(b / 2 / G::NI, b % 2);
+    at[b] = r + D * c;
+    tr[b] = c + D * r;
+  }
+  const uint32_t dl = Left<D, W>::at(tm, pd), dr = Right<D, W>::at(tm, pd);
+  const long items = (long)p.n_members * p.n_t;
+#pragma unroll 1
+  for (long it = (long)blockIdx.x * C::TEAMS + team; it < items; it += (long)gridDim.x * C::TEAMS) {
+    const int m = (int)(it / p.n_t), k = (int)(it % p.n_t);
+    float x[NV], sum[NV];
+    assemble32<D, W>(tm, p, w, m, k, at, x);
+    const float sa = unit_scale<D, W>(tm, x, 0);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) x[v] *= sa;
+    store_split<D, W>(tm, pa, x);
+    // N = P_k Lambda_{k-1}
+    if (p.target == TGT_GATE) {
+      const float2* N = reinterpret_cast<const float2*>(w.P) + (size_t)it * D * D;
+#pragma unroll
+      for (int b = 0; b < H; ++b) {
+        const float2 v = N[at[b]];
+        x[b] = v.x;
+        x[H + b] = v.y;
+      }
+    } else {
+      const int np = p.n_pairs, pan = np * D;
+      const float2* ps = reinterpret_cast<const float2*>(w.psi) + ((size_t)m * (p.n_t + 1) + k) * pan;
+      const float2* ls = reinterpret_cast<const float2*>(w.lam) + ((size_t)m * (p.n_t + 1) + k) * pan;
+#pragma unroll
+      for (int b = 0; b < H; ++b) {
+        float2 acc = make_float2(0.f, 0.f);
+        for (int s = 0; s < np; ++s) {
+          const float2 l = ls[s * D + at[b] / D];
+          acc = cmac(acc, ps[s * D + at[b] % D], make_float2(l.x, -l.y));
+        }
+        x[b] = acc.x;
+        x[H + b] = acc.y;
+      }
+    }
+    const float sn = unit_scale<D, W>(tm, x, 1);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      x[v] *= sn;
+      sum[v] = x[v];
+    }
+    store_split<D, W>(tm, pd, x);
+    tm.sync();
+    // A's fragments, those of the right operand negated
+    Left<D, W> al[2][KT];
+    Right<D, W> ar[2][KT];
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt) {
+        al[s][kt].load(Left<D, W>::at(tm, pa) + 2 * s * G::PLANE + kt * 2 * (D / 8) * 128);
+        ar[s][kt].load(Right<D, W>::at(tm, pa) + 2 * s * G::PLANE + kt * 2 * 128);
+#pragma unroll
+        for (int i = 0; i < 4 * G::NTW; ++i) ar[s][kt].f[i] ^= 0x80008000u;
+#pragma unroll
+        for (int i = 0; i < 2 * G::NTW; ++i) ar[s][kt].neg[i] ^= 0x80008000u;
+      }
+    float sig = 1.f;  // the term is sig x
+#pragma unroll 1
+    for (int n = 1; n < 40; ++n) {
+      float acc[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) acc[v] = 0.f;
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt) {
+        Left<D, W> l[2];
+        Right<D, W> r[2];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          l[s].load(dl + 2 * s * G::PLANE + kt * 2 * (D / 8) * 128);
+          r[s].load(dr + 2 * s * G::PLANE + kt * 2 * 128);
+        }
+        mma_pair<D, W>(acc, al[1][kt], r[0]);
+        mma_pair<D, W>(acc, l[1], ar[0][kt]);
+        mma_pair<D, W>(acc, al[0][kt], r[1]);
+        mma_pair<D, W>(acc, l[0], ar[1][kt]);
+        mma_pair<D, W>(acc, al[0][kt], r[0]);
+        mma_pair<D, W>(acc, l[0], ar[0][kt]);
+      }
+      sig *= __fdividef(1.f, sa * (float)(n + 1));  // sa is a power of two
+      const float su = unit_scale<D, W>(tm, acc, n & 1);  // (the sync inside: every product has read D)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) sum[v] = fmaf(sig, acc[v], sum[v]);
+      sig /= su;
+      if (!(sig >= 7.4505806e-9f)) break;  // 2^-27
+#pragma unroll
+      for (int v = 0; v < NV; ++v) x[v] = acc[v] * su;
+      if constexpr (W == 1) __syncwarp();
+      store_split<D, W>(tm, pd, x);
+      tm.sync();
+    }
+    // traces
+    const float inv = 1.f / sn;
+    for (int j0 = 0; j0 < p.n_c; j0 += C::TRACE) {
+      const int nj = min(C::TRACE, p.n_c - j0);
+      float keep = 0.f;
+#pragma unroll 1
+      for (int j = 0; j < nj; ++j) {
+        const float2* Cj = p.ctrls_f32 + (size_t)(j0 + j) * D * D;
+        float t = 0.f;
+#pragma unroll
+        for (int b = 0; b < H; ++b) {
+          const float2 c = Cj[tr[b]];
+          t = p.gen == GEN_HERM ? fmaf(sum[b], c.y, fmaf(sum[H + b], c.x, t)) : fmaf(sum[b], c.x, fmaf(-sum[H + b], c.y, t));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (W > 1 && tm.lane == 0) traces[tm.w * C::TRACE + j] = t;
+        if (tm.lane == j) keep = t;
+      }
+      tm.sync();
+      if (tm.w == 0 && tm.lane < nj) {
+#pragma unroll
+        for (int i = 1; i < W; ++i) keep += traces[i * C::TRACE + tm.lane];
+        w.Gm[(size_t)it * p.n_c + j0 + tm.lane] = p.dt[k] * p.m_scale[m] * (double)(keep * inv);
+      }
+      tm.sync();
+    }
+  }
+}
+
 constexpr size_t kSmemMax = 232448;  // dynamic shared memory of a CTA
 
 // Launches a slice-parallel kernel of configuration C (dimension D): as many
@@ -1448,6 +1685,19 @@ template <int D> static cudaError_t do_states(const ProbDev& p, const WorkDev& w
   return cudaGetLastError();
 }
 
+template <int D> static cudaError_t do_tf_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  using C = TfCfg<D>;
+  const size_t smem = (size_t)C::TEAMS * C::TEAM_BYTES;
+  const int threads = 32 * C::W * C::TEAMS;
+  set_smem_once((const void*)k_tf_grad<D>, smem);
+  int per_sm = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tf_grad<D>, threads, smem);
+  const long need = ((long)p.n_members * p.n_t + C::TEAMS - 1) / C::TEAMS, most = (long)li.num_sms * (per_sm < 1 ? 1 : per_sm);
+  k_tf_grad<D><<<(int)(need < most ? need : most), threads, smem, li.stream>>>(p, w);
+  ++*li.launches;
+  return cudaGetLastError();
+}
+
 }  // namespace fx
 
 bool fx_applies(const ProbDev& p) {
@@ -1471,6 +1721,9 @@ cudaError_t launch_fx_expm_df(const ProbDev& p, const WorkDev& w, const LaunchIn
 }
 cudaError_t launch_fx_prefix_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
   PGX_FX_DISPATCH(fx::do_prefix_df<D_>(p, w, li, store));
+}
+cudaError_t launch_tf_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+  return p.Dp == 16 ? fx::do_tf_grad<16>(p, w, li) : fx::do_tf_grad<32>(p, w, li);
 }
 cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
   switch (p.Dp) {

@@ -73,6 +73,7 @@ struct WorkDev {
   double* Gm;       // [n_members][n_t][n_c] per-member weighted gradient
   double2* slab;    // global Taylor workspace for Dp = 64: [slab_teams][10][Dp*Dp]
   int slab_teams;
+  int* norm_flag;   // mixed: raised by a slice of norm > 1 (k_fx_expm), cleared by k_prep_mx
   int* expm_plan;   // mixed, Dp = 64: [n_members][n_t] degree choice of each slice's expm
   const double* u;  // [n_t][n_c]  (column-major [n_c x n_t])
   double* G;        // [n_t][n_c]
@@ -239,6 +240,9 @@ cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInf
 // (df pairs in and out), where fx_applies(p) at Dp = 16 and 32.
 cudaError_t launch_fx_expm_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 cudaError_t launch_fx_prefix_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
+// The mixed path's exact gradient as a commutator series in 3xFP16 (Dp = 16 and
+// 32; a no-op when w.norm_flag is raised): P holds N_k = P_k Lambda_{k-1}.
+cudaError_t launch_tf_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 long fx_prefix_capacity(int Dp);  // prefix chains one SM holds
 // Mixed-precision stages (pgx_mixed.cu), gate targets: df expm and forward
 // chain, FP32 backward chain and gradient.  U stack holds df (float4), the P

@@ -74,8 +74,9 @@ __device__ __forceinline__ Team<T> team_of() {
 // kernels assemble A_k from df copies of the constants (expm: df arithmetic,
 // gradient: FP32) and take the 1-norm in FP32.
 
-__global__ void k_prep_mx(const double* u, float2* u_df, int n) {
+__global__ void k_prep_mx(const double* u, float2* u_df, int n, int* norm_flag) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *norm_flag = 0;
   if (i < n) {
     const double x = u[i];
     const float hi = (float)x;
@@ -630,8 +631,16 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_chain_gate_fwd_mx(ProbDev p
 }
 
 // ---- backward chain in FP32 -------------------------------------------------------
+// Which costate M_k takes: kPairM Lambda_{k+1}, kPairN Lambda_k (the first-order
+// GRAPE formula, and the commutator series of the tensor-core gradient, for
+// which kPairFlag: N unless the evaluation's norm flag is raised).
+enum { kPairM = 0, kPairN = 1, kPairFlag = 2 };
+__device__ __forceinline__ bool pair_n(const WorkDev& w, int pair) {
+  return pair == kPairN || (pair == kPairFlag && *w.norm_flag == 0);
+}
+
 template <int D>
-__global__ void __launch_bounds__(Cfg<D>::THREADS) k_chain_gate_bwd_mx(ProbDev p, WorkDev w) {
+__global__ void __launch_bounds__(Cfg<D>::THREADS) k_chain_gate_bwd_mx(ProbDev p, WorkDev w, int pair) {
   using G = Cfg<D>;
   constexpr int T = G::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -652,7 +661,7 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_chain_gate_bwd_mx(ProbDev p
   tm.sync();
   const float4* Um = reinterpret_cast<const float4*>(w.U) + (size_t)m * p.n_t * D * D;
   float2* Pm = reinterpret_cast<float2*>(w.P) + (size_t)m * p.n_t * D * D;
-  const bool grape = (p.grad_mode == GRAD_REF_GRAPE);
+  const bool grape = pair_n(w, pair);
   for (int k = p.n_t - 1; k >= 0; --k) {
     if (grape) {
       for (int e = tm.lane; e < D * D; e += T) {
@@ -758,7 +767,7 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_chainb_combine_mx(ProbDev p
 }
 
 template <int D>
-__global__ void __launch_bounds__(FixCfg<D>::THREADS) k_chainb_fix_mx(ProbDev p, WorkDev w) {
+__global__ void __launch_bounds__(FixCfg<D>::THREADS) k_chainb_fix_mx(ProbDev p, WorkDev w, int pair) {
   using F = FixCfg<D>;
   using L = Lay<D, 2>;
   constexpr int T = F::T;
@@ -768,7 +777,7 @@ __global__ void __launch_bounds__(FixCfg<D>::THREADS) k_chainb_fix_mx(ProbDev p,
   float2* Lam = reinterpret_cast<float2*>(smem_raw) + (size_t)team * 3 * L::SIZE;
   float2* R = Lam + L::SIZE;
   float2* Pm = R + L::SIZE;
-  const bool grape = (p.grad_mode == GRAD_REF_GRAPE);
+  const bool grape = pair_n(w, pair);
   const long items = (long)p.n_members * p.n_t;
   for (long it = (long)blockIdx.x * F::TPC + team; it < items; it += (long)gridDim.x * F::TPC) {
     const int m = (int)(it / p.n_t), k = (int)(it % p.n_t), b = k / w.pit_len;
@@ -1131,7 +1140,8 @@ __device__ __forceinline__ void trace_controls32(const Team<T>& tm, const ProbDe
 }
 
 template <int D, int T>
-__global__ void __launch_bounds__(CfgM<D, T>::THREADS) k_grad_gate_mx(ProbDev p, WorkDev w) {
+__global__ void __launch_bounds__(CfgM<D, T>::THREADS) k_grad_gate_mx(ProbDev p, WorkDev w, const int* only_if) {
+  if (only_if && *only_if == 0) return;  // the series kernel ran
   using G = CfgM<D, T>;
   using L = Lay<D, kSwzGrad>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1260,8 +1270,13 @@ static int variants_for(int Dp, int kernel, int* out) {
   }
   return n;
 }
+// At D = 16 and 32 the exact gradient's tensor-core form is the commutator
+// series (k_tf_grad), which relies on the tensor-core expm for its norm flag.
+static bool series_eligible(const ProbDev& p) {
+  return (p.Dp == 16 || p.Dp == 32) && p.grad_mode == GRAD_EXACT && expm_tc_eligible(p);
+}
 static bool tc_eligible(const ProbDev& p, int kernel) {
-  return kernel == kTuneGradMx ? grad_tc_eligible(p) : expm_tc_eligible(p);
+  return kernel == kTuneGradMx ? grad_tc_eligible(p) || series_eligible(p) : expm_tc_eligible(p);
 }
 int mixed_variants(const ProbDev& p, int kernel, int* out) {
   if (tc_eligible(p, kernel)) {
@@ -1277,13 +1292,14 @@ int mixed_admitted(const ProbDev& p, int kernel, int* out) {
 }
 // Defaults (problems that were never tuned: batches, served jobs) are the
 // autotuner's usual choice on GB300 at each dimension.
-int mixed_default_team(const ProbDev& p, int kernel) {
-  const int Dp = p.Dp;
-  if (tc_eligible(p, kernel)) return kTeamTensor;
+static int cuda_core_team(int Dp, int kernel) {
   if (Dp <= 8) return 32;
   if (Dp == 16) return kernel == kTuneExpmMx ? 128 : 32;
   if (Dp == 32) return kernel == kTuneExpmMx ? 256 : 128;
   return kernel == kTuneExpmMx ? 256 : 512;
+}
+int mixed_default_team(const ProbDev& p, int kernel) {
+  return tc_eligible(p, kernel) ? kTeamTensor : cuda_core_team(p.Dp, kernel);
 }
 
 // The expm team of a launch.  A problem's choice of the tensor-core form falls
@@ -1291,8 +1307,16 @@ int mixed_default_team(const ProbDev& p, int kernel) {
 // generator term that no longer fits.
 static int expm_team(const ProbDev& p, const LaunchInfo& li) {
   const int t = li.team[kTuneExpmMx] ? li.team[kTuneExpmMx] : mixed_default_team(p, kTuneExpmMx);
-  return t == kTeamTensor && !expm_tc_eligible(p) ? (p.Dp == 16 ? 128 : 256) : t;
+  return t == kTeamTensor && !expm_tc_eligible(p) ? cuda_core_team(p.Dp, kTuneExpmMx) : t;
 }
+// The gradient team of a launch; the series steps back where the expm does, or
+// where its team was set to a CUDA-core one.
+static int grad_team(const ProbDev& p, const LaunchInfo& li) {
+  const int t = li.team[kTuneGradMx] ? li.team[kTuneGradMx] : mixed_default_team(p, kTuneGradMx);
+  if (t != kTeamTensor || p.Dp == 64) return t;
+  return series_eligible(p) && expm_team(p, li) == kTeamTensor ? t : cuda_core_team(p.Dp, kTuneGradMx);
+}
+static bool grad_series(const ProbDev& p, const LaunchInfo& li) { return p.Dp < 64 && grad_team(p, li) == kTeamTensor; }
 
 #define PGX_DISPATCH_MX_T(DP, TT, CALL)                                                        \
   switch (DP) {                                                                                \
@@ -1537,10 +1561,11 @@ static cudaError_t do_chain_bwd_mx(const ProbDev& p, const WorkDev& w, const Lau
     ++*li.launches;
     return cudaGetLastError();
   }
+  const int pair = p.grad_mode == GRAD_REF_GRAPE ? kPairN : grad_series(p, li) ? kPairFlag : kPairM;
   if (w.pit_blocks <= 1) {
     const size_t smem = (size_t)G::TPC * 2 * D * D * sizeof(float2);
     ensure_smem_mx(k_chain_gate_bwd_mx<D>, smem);
-    k_chain_gate_bwd_mx<D><<<(p.n_members + G::TPC - 1) / G::TPC, G::THREADS, smem, li.stream>>>(p, w);
+    k_chain_gate_bwd_mx<D><<<(p.n_members + G::TPC - 1) / G::TPC, G::THREADS, smem, li.stream>>>(p, w, pair);
     ++*li.launches;
     return cudaGetLastError();
   }
@@ -1564,7 +1589,7 @@ static cudaError_t do_chain_bwd_mx(const ProbDev& p, const WorkDev& w, const Lau
   ensure_smem_mx(k_chainb_fix_mx<D>, smem_f);
   const int grid_f = grid_for(k_chainb_fix_mx<D>, F::THREADS, smem_f, (long)p.n_members * p.n_t, F::TPC,
                               li.num_sms, 0);
-  k_chainb_fix_mx<D><<<grid_f, F::THREADS, smem_f, li.stream>>>(p, w);
+  k_chainb_fix_mx<D><<<grid_f, F::THREADS, smem_f, li.stream>>>(p, w, pair);
   *li.launches += 2;
   return cudaGetLastError();
 }
@@ -1579,19 +1604,19 @@ cudaError_t launch_chain_bwd_local_mx(const ProbDev& p, const WorkDev& w, const 
 }
 
 template <int D, int T>
-static cudaError_t do_grad_mx(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
+static cudaError_t do_grad_mx(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, const int* only_if = nullptr) {
   using G = CfgM<D, T>;
   const size_t smem = G::SMEM_G;
   ensure_smem_mx(k_grad_gate_mx<D, T>, smem);
   const int grid = grid_for(k_grad_gate_mx<D, T>, G::THREADS, smem, (long)p.n_members * p.n_t, G::TPC,
                             li.num_sms, 0);
-  k_grad_gate_mx<D, T><<<grid, G::THREADS, smem, li.stream>>>(p, w);
+  k_grad_gate_mx<D, T><<<grid, G::THREADS, smem, li.stream>>>(p, w, only_if);
   ++*li.launches;
   return cudaGetLastError();
 }
 cudaError_t launch_prep_mx(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
   const int n = p.n_t * p.n_c;
-  k_prep_mx<<<(n + 255) / 256, 256, 0, li.stream>>>(w.u, w.u_df, n);
+  k_prep_mx<<<(n + 255) / 256, 256, 0, li.stream>>>(w.u, w.u_df, n, w.norm_flag);
   ++*li.launches;
   return cudaGetLastError();
 }
@@ -1642,8 +1667,14 @@ cudaError_t launch_refine_mx(const ProbDev& p, const WorkDev& w, const LaunchInf
 }
 
 cudaError_t launch_grad_mx(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  const int t = li.team[kTuneGradMx] ? li.team[kTuneGradMx] : mixed_default_team(p, kTuneGradMx);
+  const int t = grad_team(p, li);
   if (t == kTeamTensor) {
+    if (p.Dp != 64) {
+      const cudaError_t e = launch_tf_grad(p, w, li);
+      if (e != cudaSuccess) return e;
+      // evaluations with large norms: the CUDA-core gradient, a no-op otherwise
+      return p.Dp == 16 ? do_grad_mx<16, 32>(p, w, li, w.norm_flag) : do_grad_mx<32, 128>(p, w, li, w.norm_flag);
+    }
     if (!grad_tc_eligible(p)) return cudaErrorInvalidValue;
     return do_grad_tc64(p, w, li);
   }

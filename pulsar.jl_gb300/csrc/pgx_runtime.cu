@@ -391,7 +391,7 @@ static uint64_t footprint(const pgx_problem_desc* d, int num_sms) {
                                  sizeof(float2) * ((size_t)d->n_slices + 2 * (size_t)d->n_members) + s.u
                            : 0);
   return s.U + s.P + s.Utot + 2 * s.psi + 2 * s.z + s.Fm + s.Gm + s.slab + s.plan + s.u + s.G +
-         3 * sizeof(double) + consts + mixed;
+         4 * sizeof(double) + consts + mixed;
 }
 
 int validate_desc(pgx_ctx* c, const pgx_problem_desc* d) { return validate(c, d); }
@@ -645,7 +645,8 @@ extern "C" int pgx_problem_create(pgx_ctx* c, const pgx_problem_desc* d, pgx_pro
   w.expm_plan = (int*)A(s.plan);
   p->d_u = (double*)A(s.u);
   p->d_G = (double*)A(s.G);
-  p->d_F = (double*)A(3 * sizeof(double));  // objective, gradient-pass scratch, residual bits
+  p->d_F = (double*)A(4 * sizeof(double));  // objective, gradient-pass scratch, residual bits, norm flag
+  w.norm_flag = st ? nullptr : (int*)(p->d_F + 3);
   if (d->precision == PGX_PREC_MIXED) w.u_df = (float2*)A(s.u);
   p->d_pen = (pgx_penalty*)A(sizeof(pgx_penalty) * PGX_MAX_PENALTIES);
   pit_shape(d, Dp, c->num_sms, &w.pit_blocks, &w.pit_len);

@@ -184,3 +184,36 @@ def test_state_chains_hermitian(pg, D, n_t, n_p):
         assert F1 == F
         assert abs(F - Fo) <= 1e-10
         assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
+
+
+@pytest.mark.parametrize("target", ["gate", "states"])
+@pytest.mark.parametrize("gen", ["hermitian", "liouvillian"])
+@pytest.mark.parametrize("D,n_t,n_m,n_c", [(16, 1, 1, 1), (9, 30, 3, 23), (16, 37, 2, 3), (32, 3, 2, 6), (21, 26, 1, 2), (32, 9, 1, 7)])
+@pytest.mark.parametrize("nrm", [0.02, 0.7, 4.0])
+def test_mixed_series_gradient(pg, target, gen, D, n_t, n_m, n_c, nrm):
+    """The mixed path at D = 16 and 32: the series gradient, the CUDA-core one
+    that takes over for norms above 1 (nrm = 4), more controls than the
+    generator's shared memory holds; against the oracle with the mixed path's
+    bars (|dF| <= 1e-8, gradient 1e-4), and the CUDA-core team's own gradient
+    within FP32's rounding of it."""
+    from oracle import members as mb
+    rng = np.random.default_rng(D + n_t + n_c)
+    dag = lambda x: np.swapaxes(x.conj(), -1, -2)  # noqa: E731
+    X = rng.normal(size=(1 + n_c, D, D)) + 1j * rng.normal(size=(1 + n_c, D, D))
+    X = X + dag(X) if gen == "hermitian" else X - dag(X)
+    if gen == "liouvillian":
+        X[0] -= 0.1 * np.eye(D)
+    u = rng.normal(size=(n_c, n_t))
+    dt = nrm / np.abs(X[0] + np.tensordot(u[:, 0], X[1:], 1)).sum(0).max() * rng.uniform(0.1, 1.0, n_t)
+    Q, _ = np.linalg.qr(rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D)))
+    kw = dict(drifts=X[:1], controls=X[1:], dt=dt, generator=gen, member_scale=rng.uniform(0.9, 1.1, n_m), target=target)
+    kw.update(dict(target_op=Q) if target == "gate" else dict(states_init=Q[:2], states_target=Q[2:4]))
+    Fo, Go = mb.eval_problem(mb.Problem(n_members=n_m, **kw), u, "exact")
+    p = pg.Problem(grad_mode="exact", precision="mixed", **kw)
+    F, G = p.eval(u)
+    p.set_teams(grad=128)
+    F1, G1 = p.eval(u)
+    p.close()
+    scale = np.abs(Go).max()
+    assert F1 == F and abs(F - Fo) <= 1e-8
+    assert np.abs(G - Go).max() <= 1e-4 * scale and np.abs(G1 - Go).max() <= 1e-4 * scale
