@@ -515,13 +515,35 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_chainf_combine_mx(ProbDev p
   float4* Tb = Pc + D * D;
   double2* red = reinterpret_cast<double2*>(Tb + D * D);
   for (int e = tm.lane; e < D * D; e += T) Pc[e] = make_float4((e % D) == (e / D) ? 1.f : 0.f, 0.f, 0.f, 0.f);
+  constexpr int NE = (D * D + T - 1) / T;
+  constexpr bool AHEAD = NE <= 4;  // T_{b+1} loads while T_b P is formed
+  const float4* tots = w.pit_tot + (size_t)m * w.pit_blocks * D * D;
+  float4 pre[AHEAD ? NE : 1];
+  auto fetch = [&](int b) {
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int i = 0; i < NE; ++i) {
+        const int e = tm.lane + i * T;
+        if (e < D * D && b < w.pit_blocks) pre[i] = tots[(size_t)b * D * D + e];
+      }
+    }
+  };
+  fetch(0);
   for (int b = 0; b < w.pit_blocks; ++b) {
-    const float4* tot = w.pit_tot + ((size_t)m * w.pit_blocks + b) * D * D;
-    for (int e = tm.lane; e < D * D; e += T) Tb[e] = tot[e];
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int i = 0; i < NE; ++i) {
+        const int e = tm.lane + i * T;
+        if (e < D * D) Tb[e] = pre[i];
+      }
+      fetch(b + 1);
+    } else {
+      for (int e = tm.lane; e < D * D; e += T) Tb[e] = tots[(size_t)b * D * D + e];
+    }
     tm.sync();
     if (store) {
-      float2* pre = w.pit_pre + ((size_t)m * w.pit_blocks + b) * D * D;
-      for (int e = tm.lane; e < D * D; e += T) pre[e] = make_float2(Pc[e].x, Pc[e].y);
+      float2* pfx = w.pit_pre + ((size_t)m * w.pit_blocks + b) * D * D;
+      for (int e = tm.lane; e < D * D; e += T) pfx[e] = make_float2(Pc[e].x, Pc[e].y);
     }
     if constexpr (LSYM)
       mm_df_lsym<D, T, false, 0>(tm, Pc, Tb, Pc, DfEpiNone{});
@@ -687,8 +709,8 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_chain_gate_bwd_mx(ProbDev p
 
 // Backward chain in parallel in time (FP32), blocks as the forward chain's:
 //   local   per (m, b): in-block suffixes R_k = U_{k1-1} ... U_k;
-//   combine per m: Lambda_n = kappa T', Lambda_{k0} = Lambda_{k1} R_{k0} block
-//           by block from the end (Lambda_{k1} of each block saved);
+//   combine per m: Lambda_n = kappa T', Lambda_{k0} = Lambda_{k1} T_b block by
+//           block from the end (Lambda_{k1} of each block saved);
 //   fix     per (m, k): Lambda_{k+1} = Lambda_{k1} R_{k+1} (or Lambda_{k1} at
 //           the block end), M_k = P_k Lambda_{k+1}; the first-order GRAPE
 //           formula takes Lambda_k = Lambda_{k1} R_k instead.
@@ -749,7 +771,8 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_chainb_combine_mx(ProbDev p
   const Team<T> tm{(int)(threadIdx.x % T)};
   const int m = blockIdx.x * G::TPC + team;
   if (m >= p.n_members) return;
-  float2* Lam = smem + (size_t)team * D * D;
+  float2* Lam = smem + (size_t)team * 2 * D * D;
+  float2* Tb = Lam + D * D;
   const double2 kap = w.kap[m];
   for (int e = tm.lane; e < D * D; e += T) {
     const int r = e % D, c = e / D;
@@ -758,11 +781,34 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_chainb_combine_mx(ProbDev p
     Lam[e] = make_float2((float)v.x, (float)v.y);
   }
   tm.sync();
-  const float2* Rm = w.pit_r + (size_t)m * p.n_t * D * D;
+  // the block products are the forward chain's df ones: the FP32 suffixes'
+  // own (R_k0) carry the rounding of a whole block
+  constexpr int NE = (D * D + T - 1) / T;
+  const float4* tots = w.pit_tot + (size_t)m * w.pit_blocks * D * D;
+  float2 pre[NE];
+  auto fetch = [&](int b) {
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+      const int e = tm.lane + i * T;
+      if (e < D * D && b > 0) {
+        const float4 t = tots[(size_t)b * D * D + e];
+        pre[i] = make_float2(t.x, t.y);
+      }
+    }
+  };
+  fetch(w.pit_blocks - 1);
   for (int b = w.pit_blocks - 1; b >= 0; --b) {
     float2* lam_b = w.pit_lam + ((size_t)m * w.pit_blocks + b) * D * D;
     for (int e = tm.lane; e < D * D; e += T) lam_b[e] = Lam[e];
-    mm1<D, T>(tm, Lam, Lam, Rm + (size_t)(b * w.pit_len) * D * D);
+    if (b == 0) break;
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+      const int e = tm.lane + i * T;
+      if (e < D * D) Tb[e] = pre[i];
+    }
+    fetch(b - 1);
+    tm.sync();
+    mm1<D, T>(tm, Lam, Lam, Tb);
   }
 }
 
@@ -1573,7 +1619,7 @@ static cudaError_t do_chain_bwd_mx(const ProbDev& p, const WorkDev& w, const Lau
     const cudaError_t e = do_chain_bwd_local_mx<D>(p, w, li);
     if (e != cudaSuccess) return e;
   }
-  const size_t smem_c = (size_t)G::TPC * D * D * sizeof(float2);
+  const size_t smem_c = (size_t)G::TPC * 2 * D * D * sizeof(float2);
   ensure_smem_mx(k_chainb_combine_mx<D>, smem_c);
   k_chainb_combine_mx<D><<<(p.n_members + G::TPC - 1) / G::TPC, G::THREADS, smem_c, li.stream>>>(p, w);
   if constexpr (D == 64) {  // tensor cores (pgx_fix_tc.cuh)
