@@ -897,6 +897,22 @@ k_fx_chain_bwd(ProbDev p, WorkDev w, int blocks, int len) {
   }
 }
 
+// A df matrix (the lanes' entries) in block fixed point; returns its exponent.
+template <int D, int W>
+__device__ __forceinline__ int from_df(const Tm<D, W>& tm, const float4 (&f)[Geo<D, W>::NV / 2], long long (&u)[Geo<D, W>::NV]) {
+  constexpr int H = Geo<D, W>::NV / 2;
+  uint32_t M = 0;
+#pragma unroll
+  for (int b = 0; b < H; ++b) M = max(M, max(__float_as_uint(f[b].x) & 0x7f800000u, __float_as_uint(f[b].y) & 0x7f800000u));
+  const int EX = (int)(tm.max(M, 2) >> 23);
+#pragma unroll
+  for (int b = 0; b < H; ++b) {
+    u[b] = from_float(f[b].x, EX) + from_float(f[b].z, EX);
+    u[H + b] = from_float(f[b].y, EX) + from_float(f[b].w, EX);
+  }
+  return EX == 0xff ? kNotFinite : EX - 125;
+}
+
 // The mixed path's in-block prefixes: U_k as df pairs, R_k rounded to float2
 // for the FP32 fix-up, block products as df pairs.  Seven levels: with six
 // (2^-47.5 of the factors' scale) the defect of U_total, 4.8e-12 after 1000
@@ -929,16 +945,8 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS, 2) k
   }
 #pragma unroll 1
   for (int k = k0; k < k1; ++k) {
-    uint32_t M = 0;
-#pragma unroll
-    for (int b = 0; b < H; ++b) M = max(M, max(__float_as_uint(f[b].x) & 0x7f800000u, __float_as_uint(f[b].y) & 0x7f800000u));
-    const int EX = (int)(tm.max(M, 2) >> 23), Eu = EX == 0xff ? kNotFinite : EX - 125;
     long long u[2 * H];
-#pragma unroll
-    for (int b = 0; b < H; ++b) {
-      u[b] = from_float(f[b].x, EX) + from_float(f[b].z, EX);
-      u[H + b] = from_float(f[b].y, EX) + from_float(f[b].w, EX);
-    }
+    const int Eu = from_df<D, W>(tm, f, u);
     if (k + 1 < k1) {
 #pragma unroll
       for (int b = 0; b < H; ++b) f[b] = Um[(size_t)(k + 1) * D * D + at[b]];  // while this product runs
@@ -983,6 +991,121 @@ __device__ __forceinline__ int scale_complex(long long (&x)[Geo<D, W>::NV], int 
   return E == kNotFinite ? kNotFinite : E + ex - 1022 + 2;
 }
 
+template <int D, int W>
+__device__ __forceinline__ void put_total(const Tm<D, W>& tm, const WorkDev& w, int m, const long long (&r)[Geo<D, W>::NV], int E) {
+  double2* Ut = w.Utot + (size_t)m * D * D;
+  if (E == kNotFinite) store_nan<D, W>(tm, Ut);
+  else store_mat<D, W>(tm, Ut, r, E - kFrac);
+}
+// z = Tr(T' U) / D, f and the weighted kappa of a member from U, the team's
+// (r, E); the team is threads 0 .. 32 W - 1 of the block.
+template <int D, int W>
+__device__ __forceinline__ void finish_gate(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m,
+                                            const long long (&r)[Geo<D, W>::NV], int E, double2* s_red, double2* s_kap) {
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV;
+  double2 acc = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int b = 0; b < NV / 2; ++b) {
+    double2 v = make_double2(to_double(r[b], E - kFrac), to_double(r[NV / 2 + b], E - kFrac));
+    if (E == kNotFinite) v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
+    acc = cmac_cj(acc, p.target_op[tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2)], v);
+  }
+  s_red[threadIdx.x] = acc;
+  tm.sync();
+  for (int h = 16 * W; h > 0; h >>= 1) {
+    if ((int)threadIdx.x < h) s_red[threadIdx.x] = cadd(s_red[threadIdx.x], s_red[threadIdx.x + h]);
+    tm.sync();
+  }
+  if (threadIdx.x == 0) {
+    double2 z = s_red[0], kap;
+    z.x /= p.D;
+    z.y /= p.D;
+    double f;
+    fid_kappa(z, p.fid, p.grad_mode, f, kap);
+    const double sc = p.m_weight[m] / p.D;
+    kap = make_double2(kap.x * sc, kap.y * sc);
+    w.z[m] = z;
+    w.kap[m] = kap;
+    w.Fm[m] = f;
+    *s_kap = kap;
+  }
+}
+
+// Per member, the mixed path's block products in order (T_b in df pairs, the
+// prefixes before each block rounded to float2): a latency-bound chain of one
+// team, whose product takes about 1.5 us at D = 16 and 3 us at D = 32 where the
+// CUDA-core df product of the same chain took 2.2 and 10.
+template <int D>
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W) k_fx_combine_df(ProbDev p, WorkDev w, int store) {
+  using C = ChainCfg<D>;
+  constexpr int W = C::W, H = Geo<D, W>::NV / 2;
+  using G = Geo<D, W>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double2 s_red[32 * W];
+  __shared__ double2 s_kap;
+  ChainTeam<D, W> ct(smem_raw, 0);
+  const Tm<D, W>& tm = ct.tm;
+  const int m = blockIdx.x;
+  int at[H];
+#pragma unroll
+  for (int b = 0; b < H; ++b) at[b] = tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2);
+  long long r[2 * H];
+  int E = 0;
+  float4 f[H];
+#pragma unroll
+  for (int b = 0; b < H; ++b) f[b] = w.pit_tot[(size_t)m * w.pit_blocks * D * D + at[b]];
+#pragma unroll 1
+  for (int b = 0; b < w.pit_blocks; ++b) {
+    const size_t blk = ((size_t)m * w.pit_blocks + b) * D * D;
+    if (store) {
+      const float sc = E == kNotFinite ? __int_as_float(0x7fc00000) : ldexpf(1.f, E - kFrac);
+#pragma unroll
+      for (int i = 0; i < H; ++i)
+        w.pit_pre[blk + at[i]] = b == 0 ? make_float2(at[i] % D == at[i] / D ? 1.f : 0.f, 0.f)
+                                        : make_float2(to_df(r[i], sc).x, to_df(r[H + i], sc).x);
+    }
+    long long u[2 * H];
+    const int Eu = from_df<D, W>(tm, f, u);
+    if (b + 1 < w.pit_blocks) {
+#pragma unroll
+      for (int i = 0; i < H; ++i) f[i] = w.pit_tot[blk + D * D + at[i]];
+    }
+    if (b == 0) {
+#pragma unroll
+      for (int v = 0; v < 2 * H; ++v) r[v] = u[v];
+      E = Eu;
+      tm.sync();  // the maxima are read
+    } else {
+      ct.template step<false>(r, E, u, Eu);
+    }
+  }
+  put_total<D, W>(tm, w, m, r, E);
+  if constexpr (D >= 16) {
+    if (p.gen == GEN_HERM && E != kNotFinite) {
+      // one Newton-Schulz step of the polar decomposition, U (3I - U'U) / 2,
+      // before the overlap (k_refine_unitary_mx, which takes 10 us at D = 16
+      // and 76 us at D = 32 on the FP64 pipe)
+      tm.sync();
+      store_planes<D, W>(tm, ct.pl, r, kSlices);
+      tm.sync();
+      long long s[2 * H];
+      mul_fixed<D, W, kMaxLevels, LeftH<D, W>>(tm, ct.pl, ct.pl, s);
+      to_frame<2 * H>(s, 2 * E, 3, kFrac);
+#pragma unroll
+      for (int v = 0; v < 2 * H; ++v) s[v] = -s[v];
+#pragma unroll
+      for (int i = 0; i < H; ++i)
+        if (at[i] % D == at[i] / D) s[i] += 3ll << (kFrac - 3);
+      store_planes<D, W>(tm, ct.pr, s, kSlices);
+      tm.sync();
+      mul_fixed<D, W, kMaxLevels>(tm, ct.pl, ct.pr, r);
+      E += 2;  // frame 3, halved
+    }
+  }
+  finish_gate<D, W>(tm, p, w, m, r, E, s_red, &s_kap);
+}
+
 template <int D>
 __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::COMBINE)
 k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
@@ -1012,35 +1135,8 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
       const int Ex = unpack<D, W>(x);
       ct.template step<false>(r, E, x, Ex);
     }
-    double2* Ut = w.Utot + (size_t)m * D * D;
-    if (E == kNotFinite) store_nan<D, W>(tm, Ut);
-    else store_mat<D, W>(tm, Ut, r, E - kFrac);
-    double2 acc = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int b = 0; b < NV / 2; ++b) {
-      double2 v = make_double2(to_double(r[b], E - kFrac), to_double(r[NV / 2 + b], E - kFrac));
-      if (E == kNotFinite) v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
-      acc = cmac_cj(acc, p.target_op[tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2)], v);
-    }
-    s_red[threadIdx.x] = acc;
-    tm.sync();
-    for (int h = 16 * W; h > 0; h >>= 1) {
-      if ((int)threadIdx.x < h) s_red[threadIdx.x] = cadd(s_red[threadIdx.x], s_red[threadIdx.x + h]);
-      tm.sync();
-    }
-    if (threadIdx.x == 0) {
-      double2 z = s_red[0], kap;
-      z.x /= p.D;
-      z.y /= p.D;
-      double f;
-      fid_kappa(z, p.fid, p.grad_mode, f, kap);
-      const double sc = p.m_weight[m] / p.D;
-      kap = make_double2(kap.x * sc, kap.y * sc);
-      w.z[m] = z;
-      w.kap[m] = kap;
-      w.Fm[m] = f;
-      s_kap = kap;
-    }
+    put_total<D, W>(tm, w, m, r, E);
+    finish_gate<D, W>(tm, p, w, m, r, E, s_red, &s_kap);
   } else if (team == 1 && want_grad) {  // Lambda_B = T', Lambda_{b-1} = Lambda_b Tot_b
     double t[NV];
 #pragma unroll
@@ -1665,6 +1761,14 @@ template <int D> static cudaError_t do_prefix_df(const ProbDev& p, const WorkDev
   return cudaGetLastError();
 }
 
+template <int D> static cudaError_t do_combine_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  using C = ChainCfg<D>;
+  set_smem_once((const void*)k_fx_combine_df<D>, C::TEAM_BYTES);
+  k_fx_combine_df<D><<<p.n_members, 32 * C::W, C::TEAM_BYTES, li.stream>>>(p, w, store ? 1 : 0);
+  ++*li.launches;
+  return cudaGetLastError();
+}
+
 template <int D> static long prefix_capacity() {
   using C = ChainCfg<D>;
   const size_t smem = (size_t)C::TEAMS * C::TEAM_BYTES;
@@ -1733,6 +1837,9 @@ cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInf
     case 16: return fx::do_states<16>(p, w, li, store);
     default: return cudaErrorInvalidValue;
   }
+}
+cudaError_t launch_fx_combine_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
+  PGX_FX_DISPATCH(fx::do_combine_df<D_>(p, w, li, store));
 }
 long fx_prefix_capacity(int Dp) {
   switch (Dp) {

@@ -112,6 +112,7 @@ __device__ __forceinline__ void mma(float* c, uint32_t a0, uint32_t a1, uint32_t
 // One digit of the left factor: the warp's rows, columns 16 kt ..
 template <int D, int W> struct Left {
   using G = Geo<D, W>;
+  static constexpr uint32_t KSTEP = 2 * (D / 8) * 128;  // bytes of a 16-deep step
   uint32_t f[D >= 16 ? 8 : 2];  // re, im
   // the lane's row address of digit 0, step 0
   __device__ __forceinline__ static uint32_t at(const Tm<D, W>& tm, uint32_t planes) {
@@ -128,6 +129,22 @@ template <int D, int W> struct Left {
     } else {
       ldsm2(f, a);
     }
+  }
+};
+// The same of the conjugate transpose of the matrix in the planes (D >= 16).
+template <int D, int W> struct LeftH {
+  using G = Geo<D, W>;
+  static constexpr uint32_t KSTEP = 2 * 128;
+  uint32_t f[8];
+  __device__ __forceinline__ static uint32_t at(const Tm<D, W>& tm, uint32_t planes) {
+    const int l = tm.lane;
+    return planes + ((2 * tm.rt() + ((l >> 3) & 1)) * (D / 8) + (l >> 4)) * 128 + (l & 7) * 16;
+  }
+  __device__ __forceinline__ void load(uint32_t a) {
+    ldsm4t(f, a);
+    ldsm4t(f + 4, a + G::PLANE);
+#pragma unroll
+    for (int i = 4; i < 8; ++i) f[i] ^= 0x80008000u;
   }
 };
 // One digit of the right factor: rows 16 kt .., the warp's columns.
@@ -159,8 +176,8 @@ template <int D, int W> struct Right {
 constexpr float kMagic = 12582912.0f;  // 1.5 2^23
 
 // acc += a b (complex), one digit pair, one 16-deep step.
-template <int D, int W>
-__device__ __forceinline__ void mma_pair(float (&acc)[Geo<D, W>::NV], const Left<D, W>& a, const Right<D, W>& b) {
+template <int D, int W, class LeftT>
+__device__ __forceinline__ void mma_pair(float (&acc)[Geo<D, W>::NV], const LeftT& a, const Right<D, W>& b) {
   if constexpr (D >= 16) {
     constexpr int NTW = Geo<D, W>::NTW;
     const uint32_t* x = a.f;
@@ -187,7 +204,7 @@ constexpr uint32_t kPairBias = (0x4B400000u << 8) + 0x4B400000u;  // two magic s
 // left digit, and the right digit of level L + 1 is the one level L uses next.
 // All digit loops are unrolled: as rolled loops the products of the d = 8 and
 // d = 16 chains took 1.5 and 1.25 times as long.
-template <int D, int W, int L, bool TWO>
+template <int D, int W, int L, bool TWO, class LeftT = Left<D, W>>
 __device__ __forceinline__ void level_pair(uint32_t la, uint32_t rb, uint32_t (&t)[Geo<D, W>::NV]) {
   using G = Geo<D, W>;
   constexpr int NV = G::NV;
@@ -197,13 +214,13 @@ __device__ __forceinline__ void level_pair(uint32_t la, uint32_t rb, uint32_t (&
     float a0[NV], a1[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) a0[v] = a1[v] = kMagic;
-    const uint32_t pl = la + kt * 2 * (D / 8) * 128, pr = rb + kt * 2 * 128;
+    const uint32_t pl = la + kt * LeftT::KSTEP, pr = rb + kt * 2 * 128;
     Right<D, W> b[2];
     if (TWO && L + 1 < kSlices) b[1].load(pr + (L + 1) * kDigit);
 #pragma unroll
     for (int i = 0; i < kSlices; ++i) {
       if (i > L + (TWO ? 1 : 0)) break;
-      Left<D, W> a;
+      LeftT a;
       a.load(pl + i * kDigit);
       if (i <= L) b[i & 1].load(pr + (L - i) * kDigit);  // b[(i + 1) & 1] holds B_{L + 1 - i}
       if (TWO && L + 1 - i < kSlices) mma_pair<D, W>(a1, a, b[(i + 1) & 1]);
@@ -235,18 +252,18 @@ template <int NV> __device__ __forceinline__ void join_pair(long long (&r)[NV], 
 // r = A B with N levels, as value 2^(EA + EB - 56): pa, pb address the factors'
 // digit planes.  The lowest two levels first, which keeps 32 bits below the
 // last one.
-template <int D, int W, int N, int L = (N - 1) & ~1>
+template <int D, int W, int N, class LeftT, int L = (N - 1) & ~1>
 __device__ __forceinline__ void mul_levels(uint32_t la, uint32_t rb, long long (&r)[Geo<D, W>::NV]) {
   uint32_t t[Geo<D, W>::NV];
-  level_pair<D, W, L, (L + 1 < N)>(la, rb, t);
+  level_pair<D, W, L, (L + 1 < N), LeftT>(la, rb, t);
   join_pair<Geo<D, W>::NV>(r, t, L);
-  if constexpr (L > 0) mul_levels<D, W, N, L - 2>(la, rb, r);
+  if constexpr (L > 0) mul_levels<D, W, N, LeftT, L - 2>(la, rb, r);
 }
-template <int D, int W, int N>
+template <int D, int W, int N, class LeftT = Left<D, W>>
 __device__ __forceinline__ void mul_fixed(const Tm<D, W>& tm, uint32_t pa, uint32_t pb, long long (&r)[Geo<D, W>::NV]) {
 #pragma unroll
   for (int v = 0; v < Geo<D, W>::NV; ++v) r[v] = 0;
-  mul_levels<D, W, N>(Left<D, W>::at(tm, pa), Right<D, W>::at(tm, pb), r);
+  mul_levels<D, W, N, LeftT>(LeftT::at(tm, pa), Right<D, W>::at(tm, pb), r);
 }
 
 // Level pair (L, L + 1) with L and `two` chosen by the data: rolled digit loops

@@ -243,6 +243,7 @@ cudaError_t launch_fx_prefix_df(const ProbDev& p, const WorkDev& w, const Launch
 // The mixed path's exact gradient as a commutator series in 3xFP16 (Dp = 16 and
 // 32; a no-op when w.norm_flag is raised): P holds N_k = P_k Lambda_{k-1}.
 cudaError_t launch_tf_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
+cudaError_t launch_fx_combine_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
 long fx_prefix_capacity(int Dp);  // prefix chains one SM holds
 // Mixed-precision stages (pgx_mixed.cu), gate targets: df expm and forward
 // chain, FP32 backward chain and gradient.  U stack holds df (float4), the P

@@ -1496,9 +1496,9 @@ static cudaError_t do_chain_fwd_mx(const ProbDev& p, const WorkDev& w, const Lau
   }
   const bool tensor = expm_team(p, li) == kTeamTensor;  // the prefixes follow the expm's engine
   if ((D == 16 || D == 32) && tensor) {
-    const cudaError_t e = launch_fx_prefix_df(p, w, li, store);
+    cudaError_t e = launch_fx_prefix_df(p, w, li, store);
+    if (e == cudaSuccess) e = launch_fx_combine_df(p, w, li, store);
     if (e != cudaSuccess) return e;
-    --*li.launches;  // counted below
   } else if (D == 64 && tensor) {
     // the in-block prefixes on the tensor-core expm's engine (pgx_expm_oz.cuh)
     ensure_smem_mx(k_chainf_local_oz64, oz::kExpmSmem);
@@ -1515,7 +1515,9 @@ static cudaError_t do_chain_fwd_mx(const ProbDev& p, const WorkDev& w, const Lau
     const int grid_l = grid_for(local, PC::THREADS, smem_l, (long)p.n_members * w.pit_blocks, PC::TPC, li.num_sms, 0);
     local<<<grid_l, PC::THREADS, smem_l, li.stream>>>(p, w, store);
   }
-  if (D == 64 && tensor) {
+  if ((D == 16 || D == 32) && tensor) {
+    *li.launches -= 2;  // counted by the launchers above
+  } else if (D == 64 && tensor) {
     ensure_smem_mx(k_chainf_combine_oz64, oz::kExpmSmem);
     k_chainf_combine_oz64<<<p.n_members < li.num_sms ? p.n_members : li.num_sms, oz::kExpmThreads,
                             oz::kExpmSmem, li.stream>>>(p, w, store);
@@ -1708,6 +1710,8 @@ bool refine_applies(const ProbDev& p) { return p.gen == GEN_HERM && p.target == 
 bool tc_kernels_used(const ProbDev& p) { return p.Dp == 64; }
 cudaError_t launch_refine_mx(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
   if (!refine_applies(p)) return cudaSuccess;
+  // the tensor-core chain's combine has refined its own product
+  if ((p.Dp == 16 || p.Dp == 32) && w.pit_blocks > 1 && expm_team(p, li) == kTeamTensor) return cudaSuccess;
   PGX_DISPATCH_MX(p.Dp, return (do_refine_mx<D_>(p, w, li)));
   return cudaSuccess;
 }
