@@ -8,23 +8,34 @@
 // squarings.  Every product is a full one (no triangular or half-column
 // forms: the tensor-core product costs the same either way).
 //
-// One CTA per SM: 256 worker threads and one issuing warp.
-//   - Worker (TMEM lane L, column half) owns entries (L mod 64, c0 .. c0+31)
-//     of the real (L < 64) or imaginary part of every matrix: exactly the
-//     values it stages into both operands of a sliced product and the values
-//     it reads back from the accumulators.  So a product's result feeds the
-//     next product from registers.
-//   - The workers cut the left factor's six slices into two alternating
-//     buffers; after each slice one worker arrives on the buffer's "full"
-//     barrier with the slice index.  The issuing thread waits there, issues
-//     the slice's pairs and commits them to the buffer's "empty" barrier,
-//     which the workers wait on before they reuse the buffer.  The workers
-//     never wait for the issue itself, so the Horner block of a step is
-//     formed while its MMAs run.
+// What bounds it: the workers' instructions (slicing, level sums, Horner
+// blocks) and the latencies between a product's phases; the MMAs take about a
+// fifth of the time.  Measured on the three-qubit Lindblad gate (16,000
+// generators of 1-norm 0.13, four products each), prologue and kernel: 10.0 ms
+// with 256 workers, 26 slice pairs in every product, rintf slicing and one
+// thread issuing from a divergent branch; 6.9 ms now.
+//
+// One CTA per SM: 512 worker threads and one issuing warp.
+//   - Worker (TMEM lane L, column quarter) owns entries (L mod 64, c0 ..
+//     c0+15) of the real (L < 64) or imaginary part of every matrix: exactly
+//     the values it stages into both operands of a sliced product and the
+//     values it reads back from the accumulators.  So a product's result feeds
+//     the next product from registers.  (256 workers of 32 values leave two
+//     warps per SM sub-partition to hide each other's latencies: 9.6 against
+//     8.1 ms, all else equal.)
+//   - The workers cut the left factor's slices into two alternating buffers;
+//     after each slice every warp arrives on the buffer's "full" barrier.  The
+//     issuing warp waits there, issues the slice's pairs and commits them to
+//     the buffer's "empty" barrier, which the workers wait on before they
+//     reuse the buffer.  The workers never wait for the issue itself, so the
+//     Horner block of a step is formed, in registers, while its MMAs run.
+//   - A product takes as many levels (4 to 7, and as many slices, at most 6)
+//     as its entries' share of exp(A) needs: levels_of.
 //   - A prologue kernel assembles every unit's generator, takes its 1-norm
-//     and degree, and leaves B = A / 2^s in the unit's U slot.
+//     and degree, and leaves B = A / 2^s in the unit's U slot.  B arrives in
+//     shared memory by TMA bulk copies while the previous unit ends.
 //   - The slab (the per-CTA global workspace of the CUDA-core kernel) keeps
-//     B, B^2, B^3 as every worker's own values, thread-major, for the Horner
+//     B^2 and B^3 as every worker's own values, thread-major, for the Horner
 //     blocks C_i = sum_j c_{qi+j} B^j: each worker reads back only what it
 //     wrote.
 #pragma once
@@ -34,77 +45,91 @@ namespace pgx {
 namespace oz {
 
 constexpr int kExpmLevels = 7;
-constexpr int kWorkers = 256;
+constexpr int kExpmBits = 54;
+constexpr int kWorkers = 512;
+constexpr int kCols = 8192 / kWorkers;  // values of a matrix that one worker holds
 constexpr int kExpmThreads = kWorkers + 32;
-constexpr uint32_t kCiBytes = kWorkers * 32u * 8u;  // 32 df values per worker
+constexpr uint32_t kCiBytes = 8192u * 8u;  // kCols df values per worker
 constexpr size_t kExpmSmem = (size_t)kSlices * kBSlice + 2 * kASlice + kCiBytes + tc::kSmemAlign;
 
-// Barrier 1 of the 256 workers (the issuing warp never joins it).
-__device__ __forceinline__ void wsync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// A worker's place: TMEM lane (row of the stacked [re; im] matrix) and its
+// columns c0 .. c0 + kCols - 1.
+__device__ __forceinline__ Lane worker_lane() {
+  Lane l = tc::lane_of();
+  l.c0 = kCols * (int)(threadIdx.x >> 7);
+  return l;
+}
+
+// Barrier 1 of the workers (the issuing warp never joins it).
+__device__ __forceinline__ void wsync() { asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory"); }
 // The same, returning whether any worker's pred was true.
 __device__ __forceinline__ bool wsync_or(bool pred) {
   uint32_t r;
   asm volatile(
       "{\n\t.reg .pred pi, po;\n\tsetp.ne.u32 pi, %1, 0;\n\t"
-      "bar.red.or.pred po, 1, 256, pi;\n\tselp.u32 %0, 1, 0, po;\n\t}"
+      "bar.red.or.pred po, 1, %2, pi;\n\tselp.u32 %0, 1, 0, po;\n\t}"
       : "=r"(r)
-      : "r"((uint32_t)pred)
+      : "r"((uint32_t)pred), "n"(kWorkers)
       : "memory");
   return r != 0;
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
+__device__ __forceinline__ void mbar_init_n(uint32_t mbar, int n) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(n) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
 
 struct Engine {
   uint8_t* bsl;       // kSlices right-operand slices
   uint8_t* abuf;      // two left-operand slice buffers
-  float2* ci;         // [32][256] the next Horner block, every worker's values {hi, lo}
-  float* red;         // [2][8] block-maximum scratch, used alternately
-  volatile int* cmd;  // [2] the slice index behind each "full" arrival (-1: stop)
+  float2* ci;         // 64 KB: the expm's B (workers' own values), the chains' next left factor
+  float* red;         // [2][kWorkers / 32] block-maximum scratch, used alternately
+  volatile int* cmd;  // [2] the slice behind each "full" phase: index | levels << 8 (-1: stop)
   uint32_t tmem;
-  uint32_t full[2], empty[2];
-  uint32_t eph[2];  // parity of the next "empty" phase to wait for
-  int pend[2];      // slices committed on each buffer and not yet waited for
+  uint32_t bar;       // barriers at bar + 8 b: 0, 1 "full" of the two buffers, 2, 3 "empty"
+  uint32_t eph;       // bit b: parity of buffer b's next "empty" phase to wait for
+  uint32_t pend;      // byte b: slices committed on buffer b and not yet waited for
   int par;
   int seq;  // slices handed to the issuer so far (their buffer alternates)
   bool abort;
 };
 
 // Exponent of the scale of a matrix given by every worker's 32 leading parts.
-__device__ __forceinline__ int block_exp(Engine& g, const float (&h)[32]) {
+__device__ __forceinline__ int block_exp(Engine& g, const float (&h)[kCols]) {
   float mx = 0.f;
 #pragma unroll
-  for (int c = 0; c < 32; ++c) mx = fmaxf(mx, fabsf(h[c]));
+  for (int c = 0; c < kCols; ++c) mx = fmaxf(mx, fabsf(h[c]));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  float* r = g.red + 8 * g.par;  // alternate: a slow reader of the previous call is past a barrier
+  float* r = g.red + kWorkers / 32 * g.par;  // alternate: a slow reader of the previous call is past a barrier
   g.par ^= 1;
   if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = mx;
   wsync();
   mx = 0.f;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) mx = fmaxf(mx, r[w]);
+  for (int w = 0; w < kWorkers / 32; ++w) mx = fmaxf(mx, r[w]);
   return scale_exp(mx);
 }
 
 // Stages the six right-operand slices of the matrix whose values this worker
 // holds in (h, lo) (unchanged); returns its scale exponent.  No MMA may be
 // reading the slices (every product waits for its MMAs before it returns).
-__device__ __forceinline__ int stage_right(Engine& g, const Lane& l, const float (&h)[32], const float (&lo)[32]) {
+__device__ __forceinline__ int stage_right(Engine& g, const Lane& l, const float (&h)[kCols], const float (&lo)[kCols]) {
   const int e = block_exp(g, h);
   const float sc = ldexpf(1.f, -e);
-  float hh[32], ll[32];
+  float hh[kCols], ll[kCols];
 #pragma unroll
-  for (int c = 0; c < 32; ++c) {
+  for (int c = 0; c < kCols; ++c) {
     hh[c] = h[c] * sc;
     ll[c] = lo[c] * sc;
   }
 #pragma unroll 1
   for (int j = 0; j < kSlices; ++j) {
-    float s[32];
+    float s[kCols];
 #pragma unroll
-    for (int c = 0; c < 32; ++c) s[c] = next_slice(hh[c], ll[c], j);
+    for (int c = 0; c < kCols; ++c) s[c] = next_slice(hh[c], ll[c], j);
     stage_B(g.bsl + j * kBSlice, l, s);
   }
   return e;
@@ -112,139 +137,218 @@ __device__ __forceinline__ int stage_right(Engine& g, const Lane& l, const float
 
 // Waits for the MMAs still reading buffer b.  Returns false on timeout.
 __device__ __forceinline__ bool drain(Engine& g, int b) {
-  if (g.pend[b] == 0) return true;
-  if (!tc::mbar_wait(g.empty[b], g.eph[b])) return false;
-  g.eph[b] ^= 1;
-  --g.pend[b];
+  if (((g.pend >> (8 * b)) & 255u) == 0) return true;
+  if (!tc::mbar_wait(g.bar + 16u + 8u * (uint32_t)b, (g.eph >> b) & 1u)) return false;
+  g.eph ^= 1u << b;
+  g.pend -= 1u << (8 * b);
   return true;
 }
 
-// Hands a command (a staged slice index, or -1 to stop) to the issuing warp
-// on the next buffer.  Called by worker 0 after a workers' barrier.
+// Hands a command (a staged slice, or -1 to stop) to the issuing warp on the
+// next buffer: every worker calls it once its part of the slice is staged; the
+// "full" barrier counts one arrival per warp.
 __device__ __forceinline__ void hand_over(Engine& g, int cmd) {
   const int b = g.seq & 1;
-  g.cmd[b] = cmd;
-  mbar_arrive(g.full[b]);
+  if (threadIdx.x == 0) g.cmd[b] = cmd;  // its last reader has committed the buffer's previous slice
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(g.bar + 8u * (uint32_t)b);
+}
+
+// This worker's values of sum_l 2^(-8 l) L_l, scaled by sc, from the first
+// LEVELS level accumulators; with `add` plus the pairs in (h, lo).
+template <int LEVELS>
+__device__ __forceinline__ void read_levels(const Engine& g, const Lane& l, float (&h)[kCols], float (&lo)[kCols], float sc,
+                                            bool add) {
+#pragma unroll
+  for (int q = 0; q < kCols / 8; ++q) {
+    float Lv[LEVELS][8];
+    tmem_ld8xn<LEVELS>(g.tmem + l.lane_addr + (uint32_t)(l.c0 + 8 * q), Lv);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      float L[LEVELS];
+#pragma unroll
+      for (int lv = 0; lv < LEVELS; ++lv) L[lv] = Lv[lv][c];
+      float hi, lw;
+      combine_levels<LEVELS>(L, hi, lw);
+      df v{hi * sc, lw * sc};
+      if (add) {
+        v = df_add(v, df{h[8 * q + c], lo[8 * q + c]});
+      }
+      h[8 * q + c] = v.hi;
+      lo[8 * q + c] = v.lo;
+    }
+  }
+}
+
+// The levels of a product whose entries may be off by 2^-need: levels beyond
+// n leave about 2^(1 - 8 n) of the operands' scales 2^eX 2^eR (six or so slice
+// pairs of 128 products of two digits each, added with random signs).
+constexpr int kAllLevels = 1 << 16;  // need of a product with every level
+__device__ __forceinline__ int levels_of(int eX, int eR, int need) {
+  const int n = (eX + eR + need + 8) >> 3;
+  return n < 4 ? 4 : n > kExpmLevels ? kExpmLevels : n;
 }
 
 // (h, lo) <- this worker's values of X R in df: X given by this worker's
-// values (h, lo), R by the staged right-operand slices (exponent eR).
-// `during()` runs while the MMAs execute; with `add` the Horner block parked
-// in g.ci is added.  Returns false (g.abort set) when a wait gave up.
+// values (h, lo), R by the staged right-operand slices (exponent eR), entries
+// to about 2^-need.  `during(h, lo)` runs while the last slices' MMAs execute
+// (X is staged by then); with `add` the pairs it left in (h, lo) are added to
+// the product.  Returns false (g.abort set) when a wait gave up.
 template <class During>
-__device__ __forceinline__ bool product(Engine& g, const Lane& l, float (&h)[32], float (&lo)[32], int eR, bool add,
-                                        During during) {
+__device__ __forceinline__ bool product(Engine& g, const Lane& l, float (&h)[kCols], float (&lo)[kCols], int eR,
+                                        int need, bool add, During during) {
   const int eX = block_exp(g, h);
+  const int levels = levels_of(eX, eR, need);
+  const int n_slices = min(levels, kSlices);
   {
     const float sc = ldexpf(1.f, -eX);
 #pragma unroll
-    for (int c = 0; c < 32; ++c) {
+    for (int c = 0; c < kCols; ++c) {
       h[c] *= sc;
       lo[c] *= sc;
     }
   }
-  zero_level6(g.tmem, l);  // this worker read it in the previous product's combine
+  if (levels > kSlices) zero_level6<kCols>(g.tmem, l);  // this worker read it in the previous product's combine
+  bool ok = true;
 #pragma unroll 1
-  for (int i = 0; i < kSlices; ++i) {
+  for (int i = 0; i < n_slices; ++i) {
     const int b = g.seq & 1;
-    const bool ok = drain(g, b);  // the pairs of slice i - 2 have read buffer b
-    if (ok) {
-      float s[32];
+    ok &= drain(g, b);  // the pairs of slice i - 2 have read buffer b
+    float s[kCols];
 #pragma unroll
-      for (int c = 0; c < 32; ++c) s[c] = next_slice(h[c], lo[c], i);
-      stage_A(g.abuf + b * kASlice, l, s);
-      tc::fence_smem_to_async();
-      tc::fence_before_sync();
-    }
-    if (wsync_or(!ok)) {
-      g.abort = true;
-      return false;
-    }
-    if (threadIdx.x == 0) hand_over(g, i);
-    ++g.pend[b];
+    for (int c = 0; c < kCols; ++c) s[c] = next_slice(h[c], lo[c], i);
+    stage_A(g.abuf + b * kASlice, l, s);
+    tc::fence_smem_to_async();
+    tc::fence_before_sync();
+    hand_over(g, i | levels << 8);
+    g.pend += 1u << (8 * b);
     ++g.seq;
   }
-  during();
-  const bool ok = drain(g, 0) & drain(g, 1);
+  during(h, lo);
+  ok &= drain(g, 0) & drain(g, 1);
   if (wsync_or(!ok)) {
     g.abort = true;
     return false;
   }
   tc::fence_after_sync();
   const float sc = ldexpf(1.f, eX + eR - 16);
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    float Lv[kExpmLevels][8];
-    static_assert(kExpmLevels == 7, "one load batch per level set");
-    tmem_ld8x7(g.tmem + l.lane_addr + (uint32_t)(l.c0 + 8 * q), Lv);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      float L[kExpmLevels];
-#pragma unroll
-      for (int lv = 0; lv < kExpmLevels; ++lv) L[lv] = Lv[lv][c];
-      float hi, lw;
-      combine_levels<kExpmLevels>(L, hi, lw);
-      df v{hi * sc, lw * sc};
-      if (add) {
-        const float2 a = g.ci[(8 * q + c) * kWorkers + threadIdx.x];
-        v = df_add(v, df{a.x, a.y});
-      }
-      h[8 * q + c] = v.hi;
-      lo[8 * q + c] = v.lo;
-    }
+  switch (levels) {
+    case 4: read_levels<4>(g, l, h, lo, sc, add); break;
+    case 5: read_levels<5>(g, l, h, lo, sc, add); break;
+    case 6: read_levels<6>(g, l, h, lo, sc, add); break;
+    default: read_levels<7>(g, l, h, lo, sc, add); break;
   }
   tc::fence_before_sync();  // accumulators read before the next product's MMAs
   return true;
 }
 
-// The issuing thread: waits for each staged slice in turn, issues its pairs
-// and commits them to the buffer's "empty" barrier, until a stop command.
-// Every wait is bounded; a timeout stops it (the workers' own bounded waits
-// then fail too).
-__device__ __forceinline__ void issue_loop(Engine& g) {
-  uint32_t fph[2] = {0, 0};
-  for (int n = 0;; ++n) {
-    const int b = n & 1;
-    if (!tc::mbar_wait(g.full[b], fph[b])) return;
-    fph[b] ^= 1;
-    const int cmd = g.cmd[b];
+// The issuing warp: waits for each staged slice in turn, issues its pairs and
+// commits them to the buffer's "empty" barrier, until a stop command.  Every
+// wait is bounded; a timeout stops it (the workers' own bounded waits then
+// fail too).
+// What the issue needs is kept provably warp-uniform (votes and reductions
+// write uniform registers), so the descriptors are formed there.
+__device__ __forceinline__ void issue_loop(const Engine& g) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  const uint32_t bar = g.bar, abuf = tc::smem_u32(g.abuf), bsl = tc::smem_u32(g.bsl);
+  const uint32_t tmem = __reduce_or_sync(kAll, g.tmem);
+  const bool leader = (threadIdx.x & 31) == 0;
+  uint32_t fph = 0;
+#pragma unroll 1
+  for (uint32_t n = 0;; ++n) {
+    const uint32_t b = n & 1u;
+    if (__any_sync(kAll, !tc::mbar_wait(bar + 8u * b, (fph >> b) & 1u))) return;
+    fph ^= 1u << b;
+    const int cmd = (int)__reduce_or_sync(kAll, (unsigned)g.cmd[b]);
     if (cmd < 0) return;
     tc::fence_after_sync();
-    issue_slice<kExpmLevels>(g.tmem, tc::smem_u32(g.abuf + b * kASlice), tc::smem_u32(g.bsl), cmd);
-    tc::commit(g.empty[b]);
+    issue_slice(tmem, abuf + b * kASlice, bsl, cmd & 255, cmd >> 8);
+    if (leader) tc::commit(bar + 16u + 8u * b);
+    __syncwarp();
   }
 }
 
-// This worker's part of the Horner block C_i = sum_{j<q} c_{qi+j} B^j at two
-// of its entries (columns c0 + 2 cp, + 1; B^0 = I), from the own-value copies
-// of B, B^2, B^3 (float4 {hi, lo, hi, lo} per entry pair): v0, v1.
-__device__ __forceinline__ void block_pair(int i, int q, int row, int c0, bool real, const float4* own, int cp,
-                                           const df* coef, df& v0, df& v1) {
+// v <- a c and v <- v + a c as an unevaluated pair: the leading parts' sum
+// and product errors are kept exactly in .lo, which is not folded into .hi.
+__device__ __forceinline__ void df_scale(df a, df c, df& v) {
+  v.hi = a.hi * c.hi;
+  v.lo = fmaf(a.lo, c.hi, fmaf(a.hi, c.lo, fmaf(a.hi, c.hi, -v.hi)));
+}
+__device__ __forceinline__ void df_fma(df a, df c, df& v) {
+  df p;
+  df_scale(a, c, p);
+  float e;
+  two_sum(v.hi, p.hi, v.hi, e);
+  v.lo += p.lo + e;
+}
+
+// (h, lo) <- this worker's values of the Horner block C_i = sum_{j<q}
+// c_{qi+j} B^j (B^0 = I) as unevaluated pairs, with FROM_X plus c_{q(i+1)}
+// times the values (h, lo) came with, then folded.  B comes from shared memory
+// (g.ci), B^2 and B^3 from this worker's copies in the slab, whose loads are
+// issued together: one trip to L2 instead of one per entry pair.
+template <bool FROM_X>
+__device__ __forceinline__ void horner_block(const Engine& g, int i, int q, const Lane& l, const float4* own,
+                                             float (&h)[kCols], float (&lo)[kCols]) {
   const int o = q * i;
-  const float4 b1 = __ldcg(own + cp * kWorkers + threadIdx.x);
-  const float4 b2 = q >= 3 ? __ldcg(own + (16 + cp) * kWorkers + threadIdx.x) : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 b3 = q >= 4 ? __ldcg(own + (32 + cp) * kWorkers + threadIdx.x) : make_float4(0.f, 0.f, 0.f, 0.f);
-  v0 = df_mul(df{b1.x, b1.y}, coef[o + 1]);
-  v1 = df_mul(df{b1.z, b1.w}, coef[o + 1]);
-  if (q >= 3) {
-    v0 = df_add(v0, df_mul(df{b2.x, b2.y}, coef[o + 2]));
-    v1 = df_add(v1, df_mul(df{b2.z, b2.w}, coef[o + 2]));
+  const float4* B = reinterpret_cast<const float4*>(g.ci);
+  const auto add = [&](const float4& b, df c, int cp) {
+    df v0{h[2 * cp], lo[2 * cp]}, v1{h[2 * cp + 1], lo[2 * cp + 1]};
+    df_fma(df{b.x, b.y}, c, v0);
+    df_fma(df{b.z, b.w}, c, v1);
+    h[2 * cp] = v0.hi;
+    lo[2 * cp] = v0.lo;
+    h[2 * cp + 1] = v1.hi;
+    lo[2 * cp + 1] = v1.lo;
+  };
+  if constexpr (FROM_X) {
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) {
+      df v;
+      df_scale(df{h[c], lo[c]}, c_dfcoef[o + q], v);
+      h[c] = v.hi;
+      lo[c] = v.lo;
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) h[c] = lo[c] = 0.f;
   }
-  if (q >= 4) {
-    v0 = df_add(v0, df_mul(df{b3.x, b3.y}, coef[o + 3]));
-    v1 = df_add(v1, df_mul(df{b3.z, b3.w}, coef[o + 3]));
+#pragma unroll 1
+  for (int j = q - 1; j >= 2; --j) {
+    float4 b[kCols / 2];
+#pragma unroll
+    for (int cp = 0; cp < kCols / 2; ++cp) b[cp] = __ldcg(own + (kCols / 2 * (j - 2) + cp) * kWorkers + threadIdx.x);
+#pragma unroll
+    for (int cp = 0; cp < kCols / 2; ++cp) add(b[cp], c_dfcoef[o + j], cp);
   }
-  if (real && row == c0 + 2 * cp) v0 = df_add(v0, coef[o]);
-  if (real && row == c0 + 2 * cp + 1) v1 = df_add(v1, coef[o]);
+#pragma unroll
+  for (int cp = 0; cp < kCols / 2; ++cp) add(B[cp * kWorkers + threadIdx.x], c_dfcoef[o + 1], cp);
+#pragma unroll
+  for (int c = 0; c < kCols; ++c) {
+    if (l.im == 0 && l.i == l.c0 + c) {
+      const df v = df_add(df{h[c], lo[c]}, c_dfcoef[o]);
+      h[c] = v.hi;
+      lo[c] = v.lo;
+    }
+    if constexpr (FROM_X) fast_two_sum(h[c], lo[c], h[c], lo[c]);
+  }
 }
 
-// Writes this worker's values as matrix `mat` (0: B, 1: B^2, 2: B^3) of the
+// Writes this worker's values as matrix `mat` (0: B^2, 1: B^3) of the
 // own-value copies: thread-major float4 {hi, lo, hi, lo} per entry pair, so a
 // warp's loads are 512 contiguous bytes.
-__device__ __forceinline__ void store_own(float4* own, int mat, const float (&h)[32], const float (&lo)[32]) {
+__device__ __forceinline__ void store_own(float4* own, int mat, const float (&h)[kCols], const float (&lo)[kCols]) {
 #pragma unroll
-  for (int cp = 0; cp < 16; ++cp)
-    own[(16 * mat + cp) * kWorkers + threadIdx.x] = make_float4(h[2 * cp], lo[2 * cp], h[2 * cp + 1], lo[2 * cp + 1]);
+  for (int cp = 0; cp < kCols / 2; ++cp)
+    own[(kCols / 2 * mat + cp) * kWorkers + threadIdx.x] =
+        make_float4(h[2 * cp], lo[2 * cp], h[2 * cp + 1], lo[2 * cp + 1]);
+}
+
+// Index, in float4 {hi, lo, hi, lo} pairs, of row i, columns 2 cc and 2 cc + 1
+// of the real (im = 0) or imaginary part in a matrix stored as the workers'
+// own values.
+__device__ __forceinline__ int own_pair(int i, int cc, int im) {
+  return (cc % (kCols / 2)) * kWorkers + (cc / (kCols / 2)) * 128 + 64 * im + i;
 }
 
 // Shared-memory carve-up, TMEM, barriers and the engine state of a CTA of the
@@ -252,7 +356,7 @@ __device__ __forceinline__ void store_own(float4* own, int mat, const float (&h)
 struct CtaStatic {
   uint32_t tmem;
   uint64_t bar[5];  // full[2], empty[2], and the chain kernels' operand copies
-  float red[16];
+  float red[2 * kWorkers / 32];
   int cmd[2];
 };
 __device__ __forceinline__ void engine_setup(Engine& g, uint8_t* smem_raw, CtaStatic& st) {
@@ -265,15 +369,12 @@ __device__ __forceinline__ void engine_setup(Engine& g, uint8_t* smem_raw, CtaSt
   g.par = 0;
   g.seq = 0;
   g.abort = false;
-  g.eph[0] = g.eph[1] = 0;
-  g.pend[0] = g.pend[1] = 0;
-  for (int b = 0; b < 2; ++b) {
-    g.full[b] = tc::smem_u32(&st.bar[b]);
-    g.empty[b] = tc::smem_u32(&st.bar[2 + b]);
-  }
+  g.eph = 0;
+  g.pend = 0;
+  g.bar = tc::smem_u32(&st.bar[0]);
   if (threadIdx.x < 32) tc::tmem_alloc(&st.tmem, tc::kTmemCols);
   if (threadIdx.x == 0)
-    for (int b = 0; b < 5; ++b) tc::mbar_init(tc::smem_u32(&st.bar[b]));
+    for (int b = 0; b < 5; ++b) mbar_init_n(tc::smem_u32(&st.bar[b]), b < 2 ? kWorkers / 32 : 1);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -289,10 +390,10 @@ __device__ __forceinline__ void fetch_left(Engine& g, uint32_t mbar, const float
   tc::tma_bulk_copy(tc::smem_u32(g.ci) + 32768u, reinterpret_cast<const uint8_t*>(src) + 32768, 32768u, mbar);
 }
 // This worker's values of the fetched matrix (after waiting for the copy).
-__device__ __forceinline__ void read_left(const Engine& g, const Lane& l, float (&h)[32], float (&lo)[32]) {
+__device__ __forceinline__ void read_left(const Engine& g, const Lane& l, float (&h)[kCols], float (&lo)[kCols]) {
   const float4* M = reinterpret_cast<const float4*>(g.ci);
 #pragma unroll
-  for (int c = 0; c < 32; ++c) {
+  for (int c = 0; c < kCols; ++c) {
     const float4 v = M[l.i + 64 * (l.c0 + c)];
     h[c] = l.im ? v.y : v.x;
     lo[c] = l.im ? v.w : v.z;
@@ -300,8 +401,7 @@ __device__ __forceinline__ void read_left(const Engine& g, const Lane& l, float 
 }
 // Workers: stop the issuer, then (bounded) let the groups in flight finish.
 __device__ __forceinline__ void workers_finish(Engine& g) {
-  wsync();
-  if (threadIdx.x == 0) hand_over(g, -1);
+  hand_over(g, -1);
   drain(g, 0);
   drain(g, 1);
 }
@@ -369,20 +469,26 @@ __global__ void __launch_bounds__(256) k_expm_prep_oz64(ProbDev p, WorkDev w) {
     const float nrm = prep_norm1_64(A, red);
     const int pk = choose_expm_df<256>(tm, nrm, 64, false, reinterpret_cast<int*>(red));
     const float sc = ldexpf(1.f, -((pk >> 8) & 63));
-    float2* out = reinterpret_cast<float2*>(w.U) + (size_t)it * 8192;
-    for (int e = tm.lane; e < 4096; e += 256) {
-      const float4 v = A[L::idx(e % 64, e / 64)];
-      __stcs(out + e, make_float2(v.x * sc, v.z * sc));  // read once, by the expm
-      __stcs(out + 4096 + e, make_float2(v.y * sc, v.w * sc));
+    float4* out = reinterpret_cast<float4*>(w.U) + (size_t)it * 4096;
+    for (int e = tm.lane; e < 2048; e += 256) {
+      const int i = e % 64, cc = e / 64;
+      const float4 v0 = A[L::idx(i, 2 * cc)], v1 = A[L::idx(i, 2 * cc + 1)];
+      // read once, by the expm
+      __stcs(out + oz::own_pair(i, cc, 0), make_float4(v0.x * sc, v0.z * sc, v1.x * sc, v1.z * sc));
+      __stcs(out + oz::own_pair(i, cc, 1), make_float4(v0.y * sc, v0.w * sc, v1.y * sc, v1.w * sc));
     }
-    if (tm.lane == 0) w.expm_plan[it] = pk;
+    if (tm.lane == 0) {  // and the exponent of a bound of ||B||: ||B||_1 < 2^x, -31 <= x <= 31
+      int x;
+      frexpf(nrm * sc, &x);
+      w.expm_plan[it] = pk | (max(-31, min(31, x)) + 32) << 21;
+    }
     tm.sync();  // A is rebuilt by the next unit
   }
 }
 constexpr size_t kExpmPrepSmem = (size_t)Lay<64, kSwzExpm>::SIZE * sizeof(float4) + 256;
 
-// 288 threads: an SM sub-partition hosts three of the nine warps, so at most
-// 168 registers per thread.
+// 544 threads: an SM sub-partition hosts five of the 17 warps, so at most 96
+// registers per thread.
 __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_expm_oz64(ProbDev p, WorkDev w) {
   using namespace oz;
   extern __shared__ uint8_t smem_raw[];
@@ -390,36 +496,50 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_expm_oz64(ProbDev p, Wo
   Engine g;
   engine_setup(g, smem_raw, st);
   if (threadIdx.x >= kWorkers) {  // the issuing warp
-    if (threadIdx.x == kWorkers) issue_loop(g);
+    issue_loop(g);
     __syncwarp();
   } else {
-    const Lane l = tc::lane_of();
-    float4* own = reinterpret_cast<float4*>(w.slab) + (size_t)blockIdx.x * 3 * 16 * kWorkers;  // B, B^2, B^3
-    const auto nop = [] {};
+    const Lane l = worker_lane();
+    float4* own = reinterpret_cast<float4*>(w.slab) + (size_t)blockIdx.x * 3 * (kCols / 2) * kWorkers;  // B^2, B^3
+    const uint32_t tbar = tc::smem_u32(&st.bar[4]);
+    uint32_t tph = 0;
+    int tpend = 0;  // copies of B issued and not yet waited for
+    const auto fetch = [&](long unit) {  // B of `unit` into g.ci: every worker has read the last one
+      if (threadIdx.x == 0) fetch_left(g, tbar, reinterpret_cast<const float4*>(w.U) + (size_t)unit * 4096);
+      ++tpend;
+    };
     const long items = (long)p.n_members * p.n_t;
     long it = blockIdx.x;
+    if (it < items) fetch(it);
     for (; it < items; it += gridDim.x) {
       const int m = (int)(it / p.n_t), k = (int)(it % p.n_t);
       const int pk = w.expm_plan[it];
       const int deg = pk & 31, q = (pk >> 5) & 7, s = (pk >> 8) & 63, nL = deg / q;
-      // x: the values this worker holds of the matrix in hand, first B (the
-      // prologue's planar copy in the U slot)
-      float xh[32], xl[32];
+      const int nx = ((pk >> 21) & 63) - 32;  // ||B|| < 2^nx
+      // x: the values this worker holds of the matrix in hand, first B
+      float xh[kCols], xl[kCols];
       {
-        const float2* Bp = reinterpret_cast<const float2*>(w.U) + (size_t)it * 8192 + l.im * 4096 + l.i;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const float2 v = __ldcs(Bp + 64 * (l.c0 + c));
-          xh[c] = v.x;
-          xl[c] = v.y;
+        const bool got = tc::mbar_wait(tbar, tph);
+        if (wsync_or(!got)) {
+          g.abort = true;
+          break;
         }
-        store_own(own, 0, xh, xl);
+        tph ^= 1;
+        --tpend;
+        const float4* Bs = reinterpret_cast<const float4*>(g.ci);
+#pragma unroll
+        for (int cp = 0; cp < kCols / 2; ++cp) {
+          const float4 v = Bs[cp * kWorkers + threadIdx.x];
+          xh[2 * cp] = v.x;
+          xl[2 * cp] = v.y;
+          xh[2 * cp + 1] = v.z;
+          xl[2 * cp + 1] = v.w;
+        }
       }
       // The products of the unit, at one call site (one copy of the
       // product's code), in place on x:
       //   powers:  B^2 = B B (st 0), B^3 = B^2 B (st 1), B^4 = B^2 B^2 (st 2);
-      //   then x = B^q becomes the right factor and Y = C_{L-1} + c_m B^q
-      //   (C_{L-1} parked during the last power product);
+      //   then x = B^q becomes the right factor and Y = C_{L-1} + c_m B^q;
       //   Horner:  Y <- Y B^q + C_i, i = L-2 .. 0;
       //   squarings: Y <- Y Y.
       const int n_pow = q - 1, n_hor = nL - 1, n_steps = n_pow + n_hor + s;
@@ -427,12 +547,12 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_expm_oz64(ProbDev p, Wo
       bool ok = true;
 #pragma unroll 1
       for (int st = 0; st <= n_steps && ok; ++st) {
-        if (st == 1 && q >= 3) store_own(own, 1, xh, xl);
+        if (st == 1 && q >= 3) store_own(own, 0, xh, xl);
         if (st == 2 && q == 4) {  // B^4 = B^2 B^2
-          store_own(own, 2, xh, xl);
+          store_own(own, 1, xh, xl);
 #pragma unroll
-          for (int cp = 0; cp < 16; ++cp) {
-            const float4 v = own[(16 + cp) * kWorkers + threadIdx.x];
+          for (int cp = 0; cp < kCols / 2; ++cp) {
+            const float4 v = own[cp * kWorkers + threadIdx.x];
             xh[2 * cp] = v.x;
             xl[2 * cp] = v.y;
             xh[2 * cp + 1] = v.z;
@@ -441,42 +561,29 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_expm_oz64(ProbDev p, Wo
           eR = stage_right(g, l, xh, xl);
         }
         if (st == n_pow) {  // x = B^q
-          if (q == 2) store_own(own, 1, xh, xl);
-          if (q == 3) store_own(own, 2, xh, xl);
-          eR = stage_right(g, l, xh, xl);
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {  // C_{L-1} was parked during the last power product
-            const float2 a = g.ci[c * kWorkers + threadIdx.x];
-            const df v = df_add(df{a.x, a.y}, df_mul(df{xh[c], xl[c]}, c_dfcoef[deg]));
-            xh[c] = v.hi;
-            xl[c] = v.lo;
-          }
+          if (n_hor > 0) eR = stage_right(g, l, xh, xl);
+          horner_block<true>(g, nL - 1, q, l, own, xh, xl);
         }
         if (st == n_steps) break;
         if (st == 0 || st >= n_pow + n_hor) eR = stage_right(g, l, xh, xl);  // B; or a squaring's Y
-        // the last power product parks C_{L-1} (B^1 .. B^{q-1} are known), each
-        // Horner step the next block
-        if ((st >= n_pow && st < n_pow + n_hor) || st == n_pow - 1) {
-          const int i = st == n_pow - 1 ? nL - 1 : n_pow + n_hor - 1 - st;
-          const auto park = [&] {  // C_i into shared memory while the MMAs run
-#pragma unroll 4
-            for (int cp = 0; cp < 16; ++cp) {
-              df v0, v1;
-              block_pair(i, q, l.i, l.c0, l.im == 0, own, cp, c_dfcoef, v0, v1);
-              g.ci[(2 * cp) * kWorkers + threadIdx.x] = make_float2(v0.hi, v0.lo);
-              g.ci[(2 * cp + 1) * kWorkers + threadIdx.x] = make_float2(v1.hi, v1.lo);
-            }
-          };
-          ok = product(g, l, xh, xl, eR, st != n_pow - 1, park);
-        } else {
-          ok = product(g, l, xh, xl, eR, false, nop);
-        }
+        // The entries of exp(A) are wanted to 2^-kExpmBits: an error of Y after
+        // Horner step i reaches exp(B) times B^{q i}, an error of a power as it
+        // is (its coefficients are at most 1/2), and exp(B)'s grows by 2^s in
+        // the squarings.
+        const bool horner = st >= n_pow && st < n_pow + n_hor;
+        const int i = n_pow + n_hor - 1 - st;
+        const int need = st >= n_pow + n_hor ? kAllLevels : kExpmBits + s + (horner ? q * i * nx : 0);
+        ok = product(g, l, xh, xl, eR, need, horner, [&](float (&h)[kCols], float (&lo)[kCols]) {
+          if (horner) horner_block<false>(g, i, q, l, own, h, lo);
+        });
       }
       if (!ok) break;
+      wsync();  // every worker is done with B
+      if (it + gridDim.x < items) fetch(it + gridDim.x);
       // U: the stack streams out (gigabytes, read back from DRAM by the chains)
       float* out = reinterpret_cast<float*>(w.U) + ((size_t)m * p.n_t + k) * 64 * 64 * 4;
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
+      for (int c = 0; c < kCols; ++c) {
         const size_t e = (size_t)(l.i + 64 * (l.c0 + c)) * 4;
         __stcs(out + e + l.im, xh[c]);
         __stcs(out + e + 2 + l.im, xl[c]);
@@ -490,6 +597,7 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_expm_oz64(ProbDev p, Wo
         for (int e = threadIdx.x; e < 64 * 64 * 4; e += kWorkers) out[e] = nan;
       }
       if (threadIdx.x == 0) atomicOr(&g_expm_tc_timeout, 1);
+      if (tpend > 0) tc::mbar_wait(tbar, tph);  // bounded: the copy in flight lands before the CTA ends
     }
     workers_finish(g);
   }
@@ -512,10 +620,10 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_local_oz64(ProbD
   Engine g;
   engine_setup(g, smem_raw, st);  // g.ci receives U_{k+1}
   if (threadIdx.x >= kWorkers) {
-    if (threadIdx.x == kWorkers) issue_loop(g);
+    issue_loop(g);
     __syncwarp();
   } else {
-    const Lane l = tc::lane_of();
+    const Lane l = worker_lane();
     const long items = (long)p.n_members * w.pit_blocks;
     const uint32_t tbar = tc::smem_u32(&st.bar[4]);
     uint32_t tph = 0;
@@ -528,14 +636,14 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_local_oz64(ProbD
       const int k0 = b * w.pit_len, k1 = min(p.n_t, k0 + w.pit_len);
       const float4* Um = reinterpret_cast<const float4*>(w.U) + (size_t)m * p.n_t * 4096;
       float* Pst = reinterpret_cast<float*>(w.P) + (size_t)m * p.n_t * 4096 * 2;  // float2 {re, im} per entry
-      float xh[32], xl[32], uh[32], ul[32];
+      float xh[kCols], xl[kCols], uh[kCols], ul[kCols];
       if (store) {  // P_k0 = I
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
+        for (int c = 0; c < kCols; ++c)
           Pst[((size_t)k0 * 4096 + entry(c)) * 2 + l.im] = (l.im == 0 && l.i == l.c0 + c) ? 1.f : 0.f;
       }
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {  // x = P_{k0+1} = U_k0
+      for (int c = 0; c < kCols; ++c) {  // x = P_{k0+1} = U_k0
         const float4 v = Um[(size_t)k0 * 4096 + entry(c)];
         xh[c] = l.im ? v.y : v.x;
         xl[c] = l.im ? v.w : v.z;
@@ -549,7 +657,7 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_local_oz64(ProbD
       for (int k = k0 + 1; k <= k1 && ok; ++k) {  // x holds P_k
         if (store && k < k1)
 #pragma unroll
-          for (int c = 0; c < 32; ++c) Pst[((size_t)k * 4096 + entry(c)) * 2 + l.im] = xh[c];
+          for (int c = 0; c < kCols; ++c) Pst[((size_t)k * 4096 + entry(c)) * 2 + l.im] = xh[c];
         if (k == k1) break;
         const int eR = stage_right(g, l, xh, xl);  // P_k
         const bool got = tc::mbar_wait(tbar, tph);  // U_k in shared memory
@@ -561,15 +669,15 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_local_oz64(ProbD
         tph ^= 1;
         --tpend;
         read_left(g, l, uh, ul);
-        const auto prefetch = [&] {  // U_{k+1} while the MMAs run: every worker has read U_k
+        const auto prefetch = [&](float (&)[kCols], float (&)[kCols]) {  // U_{k+1} while the MMAs run: every worker has read U_k
           if (k + 1 < k1) {
             if (threadIdx.x == 0) fetch_left(g, tbar, Um + (size_t)(k + 1) * 4096);
             ++tpend;
           }
         };
-        ok = product(g, l, uh, ul, eR, false, prefetch);  // U_k P_k
+        ok = product(g, l, uh, ul, eR, kAllLevels, false, prefetch);  // U_k P_k
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
+        for (int c = 0; c < kCols; ++c) {
           xh[c] = uh[c];
           xl[c] = ul[c];
         }
@@ -577,7 +685,7 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_local_oz64(ProbD
       if (!ok) break;
       float* tot = reinterpret_cast<float*>(w.pit_tot + ((size_t)m * w.pit_blocks + b) * 4096);
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
+      for (int c = 0; c < kCols; ++c) {
         tot[entry(c) * 4 + l.im] = xh[c];
         tot[entry(c) * 4 + 2 + l.im] = xl[c];
       }
@@ -610,11 +718,11 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_combine_oz64(Pro
   Engine g;
   engine_setup(g, smem_raw, st);
   if (threadIdx.x >= kWorkers) {
-    if (threadIdx.x == kWorkers) issue_loop(g);
+    issue_loop(g);
     __syncwarp();
   } else {
-    const Lane l = tc::lane_of();
-    const Team<256> tm{(int)threadIdx.x, 1};           // the workers' barrier
+    const Lane l = worker_lane();
+    const Team<kWorkers> tm{(int)threadIdx.x, 1};           // the workers' barrier
     float4* Pc = reinterpret_cast<float4*>(g.ci);       // 64 KB: P for the epilogue
     double2* red = reinterpret_cast<double2*>(g.abuf);  // the epilogue's scratch (idle slice buffers)
     const auto entry = [&](int c) { return (size_t)(l.i + 64 * (l.c0 + c)); };
@@ -623,9 +731,9 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_combine_oz64(Pro
     int tpend = 0;  // operand copies issued and not yet waited for
     int m = blockIdx.x;
     for (; m < p.n_members; m += gridDim.x) {
-      float xh[32], xl[32], uh[32], ul[32];
+      float xh[kCols], xl[kCols], uh[kCols], ul[kCols];
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {  // P = I
+      for (int c = 0; c < kCols; ++c) {  // P = I
         xh[c] = (l.im == 0 && l.i == l.c0 + c) ? 1.f : 0.f;
         xl[c] = 0.f;
       }
@@ -634,10 +742,10 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_combine_oz64(Pro
       if (store) {  // pit_pre[0] = I
         float* pre = reinterpret_cast<float*>(w.pit_pre + (size_t)m * w.pit_blocks * 4096);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) pre[entry(c) * 2 + l.im] = xh[c];
+        for (int c = 0; c < kCols; ++c) pre[entry(c) * 2 + l.im] = xh[c];
       }
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {  // P = T_0 I = T_0
+      for (int c = 0; c < kCols; ++c) {  // P = T_0 I = T_0
         const float4 v = Tm[entry(c)];
         xh[c] = l.im ? v.y : v.x;
         xl[c] = l.im ? v.w : v.z;
@@ -651,7 +759,7 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_combine_oz64(Pro
         if (store) {
           float* pre = reinterpret_cast<float*>(w.pit_pre + ((size_t)m * w.pit_blocks + b) * 4096);
 #pragma unroll
-          for (int c = 0; c < 32; ++c) pre[entry(c) * 2 + l.im] = xh[c];
+          for (int c = 0; c < kCols; ++c) pre[entry(c) * 2 + l.im] = xh[c];
         }
         const int eR = stage_right(g, l, xh, xl);  // P
         const bool got = tc::mbar_wait(tbar, tph);  // T_b in shared memory
@@ -663,28 +771,28 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_chainf_combine_oz64(Pro
         tph ^= 1;
         --tpend;
         read_left(g, l, uh, ul);
-        const auto prefetch = [&] {  // T_{b+1} while the MMAs run: every worker has read T_b
+        const auto prefetch = [&](float (&)[kCols], float (&)[kCols]) {  // T_{b+1} while the MMAs run: every worker has read T_b
           if (b + 1 < w.pit_blocks) {
             if (threadIdx.x == 0) fetch_left(g, tbar, Tm + (size_t)(b + 1) * 4096);
             ++tpend;
           }
         };
-        ok = product(g, l, uh, ul, eR, false, prefetch);  // T_b P
+        ok = product(g, l, uh, ul, eR, kAllLevels, false, prefetch);  // T_b P
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
+        for (int c = 0; c < kCols; ++c) {
           xh[c] = uh[c];
           xl[c] = ul[c];
         }
       }
       if (!ok) break;
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
+      for (int c = 0; c < kCols; ++c) {
         float* f = reinterpret_cast<float*>(Pc + entry(c));
         f[l.im] = xh[c];
         f[2 + l.im] = xl[c];
       }
       wsync();
-      chain_epilogue_mx<64, 256>(tm, p, w, m, Pc, red);
+      chain_epilogue_mx<64, kWorkers>(tm, p, w, m, Pc, red);
       tc::fence_smem_to_async();  // these writes to g.ci before the next member's copies into it
       wsync();  // P and the scratch are read before the next member reuses them
     }

@@ -223,7 +223,7 @@ k_oz_cmm64(const float2* __restrict__ P, const float2* __restrict__ Q, float2* _
         lo[c] *= sc;
       }
     }
-    if (LEVELS > kSlices) zero_level6(tmem, l);  // the previous item's accumulators are read
+    if (LEVELS > kSlices) zero_level6<32>(tmem, l);  // the previous item's accumulators are read
 #pragma unroll 1
     for (int i = 0; i < kSlices; ++i) {
       const int b = i & 1;
@@ -246,10 +246,11 @@ k_oz_cmm64(const float2* __restrict__ P, const float2* __restrict__ Q, float2* _
       tc::fence_smem_to_async();
       tc::fence_before_sync();
       __syncthreads();
-      if (threadIdx.x == 0) {
+      if (warp == 0) {
         tc::fence_after_sync();
-        issue_slice<LEVELS>(tmem, tc::smem_u32(abuf + b * kASlice), tc::smem_u32(bsl), i);
-        tc::commit(bar[b]);
+        issue_slice(tmem, tc::smem_u32(abuf + b * kASlice), tc::smem_u32(bsl), i, LEVELS);
+        if (threadIdx.x == 0) tc::commit(bar[b]);
+        __syncwarp();
       }
       ++pend[b];
     }

@@ -13,7 +13,7 @@ import scipy.linalg as sla
 pytestmark = pytest.mark.gpu
 
 
-def _problem(pg, D, nrm, gen, n_c, rng):
+def _problem(pg, D, nrm, gen, n_c, rng, precision="fp64"):
     H = rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D))
     C = rng.normal(size=(n_c, D, D)) + 1j * rng.normal(size=(n_c, D, D))
     if gen == "hermitian":
@@ -24,7 +24,7 @@ def _problem(pg, D, nrm, gen, n_c, rng):
     u = rng.normal(size=(n_c, 1))
     A = H + np.tensordot(u[:, 0], C, 1)
     dt = nrm / np.abs(A).sum(0).max()
-    p = pg.Problem(H[None], C, np.array([dt]), generator=gen, target="gate", target_op=np.eye(D), precision="fp64")
+    p = pg.Problem(H[None], C, np.array([dt]), generator=gen, target="gate", target_op=np.eye(D), precision=precision)
     return p, u, (-1j if gen == "hermitian" else 1.0) * A * dt
 
 
@@ -40,6 +40,21 @@ def test_propagator(pg, gen, D, nrm, n_c):
     s = max(0, int(np.ceil(np.log2(max(nrm, 1e-300) / 1.5))))
     E = sla.expm(A)
     assert np.abs(U - E).max() <= 2.0 ** s * (D + 40) * 2.0 ** -53 * max(1.0, np.abs(E).max())
+
+
+@pytest.mark.parametrize("gen", ["hermitian", "liouvillian"])
+@pytest.mark.parametrize("D", [33, 64])
+@pytest.mark.parametrize("nrm", [0.0, 1e-9, 3e-5, 0.003, 0.03, 0.1, 0.17, 0.4, 0.8, 1.6, 7.0, 60.0])
+def test_mixed_propagator_64(pg, gen, D, nrm):
+    """The sliced tensor-core exponential with every block size and number of
+    levels.  Each product keeps its entries to about 2^-53 of 1 (2^-48 allows
+    for the double-float inputs and output), and squarings double the error."""
+    p, u, A = _problem(pg, D, nrm, gen, 3, np.random.default_rng(D), precision="mixed")
+    U = p.total_propagator(u)
+    p.close()
+    s = max(0, int(np.ceil(np.log2(max(nrm, 1e-300) / 0.1))))
+    E = sla.expm(A)
+    assert np.abs(U - E).max() <= 2.0 ** s * (D + 40) * 2.0 ** -48 * max(1.0, np.abs(E).max())
 
 
 def test_propagator_not_finite(pg):
