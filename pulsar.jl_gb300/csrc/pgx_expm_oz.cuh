@@ -13,7 +13,7 @@
 // fifth of the time.  Measured on the three-qubit Lindblad gate (16,000
 // generators of 1-norm 0.13, four products each), prologue and kernel: 10.0 ms
 // with 256 workers, 26 slice pairs in every product, rintf slicing and one
-// thread issuing from a divergent branch; 6.9 ms now.
+// thread issuing from a divergent branch; 6.5 ms now.
 //
 // One CTA per SM: 512 worker threads and one issuing warp.
 //   - Worker (TMEM lane L, column quarter) owns entries (L mod 64, c0 ..
@@ -422,26 +422,29 @@ __device__ __forceinline__ void engine_teardown(Engine& g) {
 __device__ int g_expm_tc_timeout;
 
 // Prologue of the tensor-core expm, per unit (member, slice): the generator
-// A_k in df (the CUDA-core kernel's assembly), its FP32 1-norm and the
-// degree, block size and squarings (the CUDA-core kernel's choice, without
-// the triangular costs), then B = A_k / 2^s as planar df {hi, lo} (real part,
-// then imaginary part, column-major) in the unit's U slot, which the expm
-// overwrites with exp(A_k) at the end.  Memory-bound work at full occupancy,
+// A_k in df, its FP32 1-norm and the degree, block size and squarings (the
+// CUDA-core kernel's choice, without the triangular costs).  A_k stays in the
+// unit's U slot as the expm workers' own values (the expm scales it by 2^-s
+// and overwrites the slot with exp(A_k) at the end).  Work for many warps,
 // kept out of the one-CTA-per-SM tensor-core kernel.
-// FP32 1-norm of the prologue's 64 x 64 df matrix by all 256 threads (x
-// 1.00001, as norm1f): thread t sums rows 16 (t % 4) .. + 15 of column t / 4,
-// the four partial sums of a column meet by two xor shuffles (every lane of
-// the four ends with the same sum), and the largest column comes from warp
-// and block maxima.  red: 8 floats.
-__device__ __forceinline__ float prep_norm1_64(const float4* A, float* red) {
-  using L = Lay<64, kSwzExpm>;
+//
+// A CTA assembles NS consecutive slices of one member, so the operators (64 KB
+// each) are read from L2 once for NS units, and thread t holds the pair
+// (i, 2 cc), (i, 2 cc + 1) of each.  At 500 slices of 32 members and six
+// controls 1.29 ms with one slice per CTA and renormalised sums; NS = 4 takes
+// 0.75 ms.  Fewer slices than that many CTAs fill the SMs with: NS = 1.
+
+// FP32 1-norm of a 64 x 64 matrix of moduli (column pitch kMagPitch) by all
+// 256 threads (x 1.00001, as norm1f): thread t sums rows 16 (t % 4) .. + 15 of
+// column t / 4, the four partial sums of a column meet by two xor shuffles
+// (every lane of the four ends with the same sum), and the largest column
+// comes from warp and block maxima.  red: 8 floats.
+constexpr int kMagPitch = 65;
+__device__ __forceinline__ float prep_norm1_64(const float* mag, float* red) {
   const int t = threadIdx.x, c = t >> 2, r0 = (t & 3) * 16;
   float s = 0.f;
 #pragma unroll 4
-  for (int r = r0; r < r0 + 16; ++r) {
-    const float4 a = A[L::idx(r, c)];
-    s += sqrtf(fmaf(a.x, a.x, a.y * a.y));
-  }
+  for (int r = r0; r < r0 + 16; ++r) s += mag[r + kMagPitch * c];
   s += __shfl_xor_sync(0xffffffffu, s, 1);
   s += __shfl_xor_sync(0xffffffffu, s, 2);
 #pragma unroll
@@ -455,37 +458,85 @@ __device__ __forceinline__ float prep_norm1_64(const float4* A, float* red) {
   return best * 1.00001f;
 }
 
+template <int NS>
 __global__ void __launch_bounds__(256) k_expm_prep_oz64(ProbDev p, WorkDev w) {
-  using L = Lay<64, kSwzExpm>;
+  using oz::df_fma;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float4* A = reinterpret_cast<float4*>(smem_raw);
-  float* red = reinterpret_cast<float*>(A + L::SIZE);
+  float* mag = reinterpret_cast<float*>(smem_raw);  // [NS][64 * kMagPitch] moduli
+  float* red = mag + NS * 64 * kMagPitch;
   const Team<256> tm{(int)threadIdx.x};
-  const long items = (long)p.n_members * p.n_t;
+  const int per = (p.n_t + NS - 1) / NS;
+  const long items = (long)p.n_members * per;
   for (long it = blockIdx.x; it < items; it += gridDim.x) {
-    const int m = (int)(it / p.n_t), k = (int)(it % p.n_t);
-    build_A_df<64, 256, kSwzExpm>(tm, p, w, m, k, A);
-    tm.sync();
-    const float nrm = prep_norm1_64(A, red);
-    const int pk = choose_expm_df<256>(tm, nrm, 64, false, reinterpret_cast<int*>(red));
-    const float sc = ldexpf(1.f, -((pk >> 8) & 63));
-    float4* out = reinterpret_cast<float4*>(w.U) + (size_t)it * 4096;
+    const int m = (int)(it / per), k0 = (int)(it % per) * NS, n = min(NS, p.n_t - k0);
+    const df sc = df_ld(p.m_scale_df[m]), off = df_ld(p.m_offset_df[m]);
+    const float4* Gd = p.drifts_df + (size_t)p.m_drift[m] * 4096;
+    const int ro = p.n_ramp ? p.m_ramp[m] : -1;
+    const size_t unit = (size_t)m * p.n_t + k0;
+#pragma unroll 1
     for (int e = tm.lane; e < 2048; e += 256) {
-      const int i = e % 64, cc = e / 64;
-      const float4 v0 = A[L::idx(i, 2 * cc)], v1 = A[L::idx(i, 2 * cc + 1)];
-      // read once, by the expm
-      __stcs(out + oz::own_pair(i, cc, 0), make_float4(v0.x * sc, v0.z * sc, v1.x * sc, v1.z * sc));
-      __stcs(out + oz::own_pair(i, cc, 1), make_float4(v0.y * sc, v0.w * sc, v1.y * sc, v1.w * sc));
+      const int i = e % 64, cc = e / 64, q0 = i + 128 * cc, q1 = q0 + 64;
+      dfc v[NS][2];
+      // v[s][.] += c[s] M, as pairs folded at the end
+      const auto add = [&](const float4* M, auto coef) {
+        const dfc a = dfc_load(M[q0]), b = dfc_load(M[q1]);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+          const df c = coef(min(k0 + s, p.n_t - 1));
+          df_fma(a.re, c, v[s][0].re);
+          df_fma(a.im, c, v[s][0].im);
+          df_fma(b.re, c, v[s][1].re);
+          df_fma(b.im, c, v[s][1].im);
+        }
+      };
+      {
+        const dfc a = dfc_load(Gd[q0]), b = dfc_load(Gd[q1]);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+          v[s][0] = a;
+          v[s][1] = b;
+        }
+      }
+      if (off.hi != 0.f) add(p.offset_df, [&](int) { return off; });
+      if (ro >= 0) add(p.ramp_ops_df + (size_t)ro * 4096, [&](int k) { return df_ld(p.tau_df[k]); });
+#pragma unroll 1
+      for (int j = 0; j < p.n_c; ++j)
+        add(p.ctrls_df + (size_t)j * 4096, [&](int k) { return df_mul(sc, df_ld(w.u_df[(size_t)k * p.n_c + j])); });
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const df dt = df_ld(p.dt_df[min(k0 + s, p.n_t - 1)]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          dfc& x = v[s][h];
+          fast_two_sum(x.re.hi, x.re.lo, x.re.hi, x.re.lo);
+          fast_two_sum(x.im.hi, x.im.lo, x.im.hi, x.im.lo);
+          x = dfc_scale(x, dt);
+          if (p.gen == GEN_HERM) x = {x.im, df_neg(x.re)};  // times -i
+          mag[s * 64 * kMagPitch + i + kMagPitch * (2 * cc + h)] = sqrtf(fmaf(x.re.hi, x.re.hi, x.im.hi * x.im.hi));
+        }
+        if (s < n) {
+          float4* out = reinterpret_cast<float4*>(w.U) + (unit + s) * 4096;
+          const dfc x = v[s][0], y = v[s][1];
+          // read once, by the expm
+          __stcs(out + oz::own_pair(i, cc, 0), make_float4(x.re.hi, x.re.lo, y.re.hi, y.re.lo));
+          __stcs(out + oz::own_pair(i, cc, 1), make_float4(x.im.hi, x.im.lo, y.im.hi, y.im.lo));
+        }
+      }
     }
-    if (tm.lane == 0) {  // and the exponent of a bound of ||B||: ||B||_1 < 2^x, -31 <= x <= 31
-      int x;
-      frexpf(nrm * sc, &x);
-      w.expm_plan[it] = pk | (max(-31, min(31, x)) + 32) << 21;
+    tm.sync();
+    for (int s = 0; s < n; ++s) {
+      const float nrm = prep_norm1_64(mag + s * 64 * kMagPitch, red);
+      const int pk = choose_expm_df<256>(tm, nrm, 64, false, reinterpret_cast<int*>(red));
+      if (tm.lane == 0) {  // and the exponent of a bound of ||B||: ||B||_1 < 2^x, -31 <= x <= 31
+        int x;
+        frexpf(ldexpf(nrm, -((pk >> 8) & 63)), &x);
+        w.expm_plan[unit + s] = pk | (max(-31, min(31, x)) + 32) << 21;
+      }
     }
-    tm.sync();  // A is rebuilt by the next unit
+    tm.sync();  // mag is rewritten by the next units
   }
 }
-constexpr size_t kExpmPrepSmem = (size_t)Lay<64, kSwzExpm>::SIZE * sizeof(float4) + 256;
+constexpr size_t expm_prep_smem(int ns) { return (size_t)(ns * 64 * kMagPitch + 64) * sizeof(float); }
 
 // 544 threads: an SM sub-partition hosts five of the 17 warps, so at most 96
 // registers per thread.
@@ -526,10 +577,13 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_expm_oz64(ProbDev p, Wo
         }
         tph ^= 1;
         --tpend;
-        const float4* Bs = reinterpret_cast<const float4*>(g.ci);
+        float4* Bs = reinterpret_cast<float4*>(g.ci);
+        const float sc = ldexpf(1.f, -s);
 #pragma unroll
         for (int cp = 0; cp < kCols / 2; ++cp) {
-          const float4 v = Bs[cp * kWorkers + threadIdx.x];
+          float4 v = Bs[cp * kWorkers + threadIdx.x];
+          v = make_float4(v.x * sc, v.y * sc, v.z * sc, v.w * sc);
+          if (s > 0) Bs[cp * kWorkers + threadIdx.x] = v;
           xh[2 * cp] = v.x;
           xl[2 * cp] = v.y;
           xh[2 * cp + 1] = v.z;
@@ -578,6 +632,7 @@ __global__ void __launch_bounds__(oz::kExpmThreads, 1) k_expm_oz64(ProbDev p, Wo
         });
       }
       if (!ok) break;
+      if (s > 0) tc::fence_smem_to_async();  // this worker's scaled B, before the next copy into its place
       wsync();  // every worker is done with B
       if (it + gridDim.x < items) fetch(it + gridDim.x);
       // U: the stack streams out (gigabytes, read back from DRAM by the chains)

@@ -1405,9 +1405,14 @@ static cudaError_t do_expm_mx(const ProbDev& p, const WorkDev& w, const LaunchIn
 static cudaError_t do_expm_oz64(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
   if (!w.expm_plan) return cudaErrorInvalidValue;
   const long items = (long)p.n_members * p.n_t;
-  ensure_smem_mx(k_expm_prep_oz64, kExpmPrepSmem);
-  const int pgrid = grid_for(k_expm_prep_oz64, 256, kExpmPrepSmem, items, 1, li.num_sms, 0);
-  k_expm_prep_oz64<<<pgrid, 256, kExpmPrepSmem, li.stream>>>(p, w);
+  constexpr int kSlicesPer = 4;
+  const long groups = (long)p.n_members * ((p.n_t + kSlicesPer - 1) / kSlicesPer);
+  const bool wide = groups >= 2 * li.num_sms;  // enough to fill the SMs
+  const auto prep = wide ? k_expm_prep_oz64<kSlicesPer> : k_expm_prep_oz64<1>;
+  const size_t psmem = expm_prep_smem(wide ? kSlicesPer : 1);
+  ensure_smem_mx(prep, psmem);
+  const int pgrid = grid_for(prep, 256, psmem, wide ? groups : items, 1, li.num_sms, 0);
+  prep<<<pgrid, 256, psmem, li.stream>>>(p, w);
   ++*li.launches;
   if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
   ensure_smem_mx(k_expm_oz64, oz::kExpmSmem);

@@ -24,8 +24,8 @@
 //
 // Measured on GB300: an M = 128 MMA of K = 16 takes 46-48 cycles at N = 64 and
 // 64 at N = 128; pairs that share a left slice go up to four at a time, so the
-// 26 pairs of levels 0..6 (4 MMA groups of N = 256, 4 of N = 128, 2 of N = 64,
-// K = 128 each) take ~7,000 cycles of one SM's tensor pipe, against ~48,000
+// 26 pairs of levels 0..6 (MMA groups of K = 128: four of N = 256, one of 192,
+// three of 128, one of 64) take ~7,000 cycles of one SM's tensor pipe, against ~48,000
 // FP32-pipe cycles for the same product in df arithmetic (~23 FP32
 // instructions per complex multiply-add).
 //

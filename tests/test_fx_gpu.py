@@ -57,6 +57,32 @@ def test_mixed_propagator_64(pg, gen, D, nrm):
     assert np.abs(U - E).max() <= 2.0 ** s * (D + 40) * 2.0 ** -48 * max(1.0, np.abs(E).max())
 
 
+@pytest.mark.parametrize("n_t", [1, 4, 6])
+def test_mixed_generators_64_by_groups(pg, n_t):
+    """Members enough for the prologue that assembles four slices at a time
+    (with a short last group) against each member alone (one at a time); bar
+    as above, per slice."""
+    rng = np.random.default_rng(n_t)
+    n_m, D = 320, 36
+    X = rng.normal(size=(4, D, D)) + 1j * rng.normal(size=(4, D, D))
+    X = X + X.conj().transpose(0, 2, 1)
+    u = rng.normal(size=(2, n_t))
+    sc, of = rng.uniform(0.9, 1.1, n_m), rng.uniform(-0.1, 0.1, n_m)
+    kw = dict(dt=rng.uniform(0.5, 1.0, n_t) * 0.02, target="gate", target_op=np.eye(D), precision="mixed")
+    p = pg.Problem(X[:1], X[1:3], offset_op=X[3], member_scale=sc, member_offset=of, **kw)
+    U = [p.total_propagator(u, member=m) for m in (0, n_m - 1)]
+    p.close()
+    for m, V in zip((0, n_m - 1), U):
+        p = pg.Problem(X[:1], X[1:3], offset_op=X[3], member_scale=sc[m:m + 1], member_offset=of[m:m + 1], **kw)
+        W = p.total_propagator(u)
+        p.close()
+        E = np.eye(D)
+        for k in range(n_t):
+            E = sla.expm(-1j * kw["dt"][k] * (X[0] + of[m] * X[3] + sc[m] * np.tensordot(u[:, k], X[1:3], 1))) @ E
+        for A in (V, W):
+            assert np.abs(A - E).max() <= n_t * 8 * (D + 40) * 2.0 ** -48
+
+
 def test_propagator_not_finite(pg):
     """A generator that overflows gives NaN, not a finite matrix."""
     D = 16
