@@ -25,6 +25,7 @@
 #include <utility>
 
 #include "pgx.h"
+#include "pgx_chain_small.cuh"
 #include "pgx_stages.cuh"
 
 namespace pgx {
@@ -756,8 +757,11 @@ static cudaError_t do_chain_fwd(const ProbDev& p, const WorkDev& w, const Launch
   const size_t smem = chain_smem_bytes<D>(p.n_pairs);
   const int grid = (p.n_members + G::TPC - 1) / G::TPC;
   if (p.target == TGT_GATE) {
-    ensure_smem(k_chain_gate_fwd<D>, smem);
-    k_chain_gate_fwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w, store ? 1 : 0);
+    if constexpr (D <= 4) return small::launch_fwd<D>(p, w, li, store);
+    else {
+      ensure_smem(k_chain_gate_fwd<D>, smem);
+      k_chain_gate_fwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w, store ? 1 : 0);
+    }
   } else if (p.n_ck > 0) {
     ensure_smem(k_track_fwd<D>, smem);
     k_track_fwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
@@ -781,8 +785,11 @@ static cudaError_t do_chain_bwd(const ProbDev& p, const WorkDev& w, const Launch
   const size_t smem = chain_smem_bytes<D>(p.n_pairs);
   const int grid = (p.n_members + G::TPC - 1) / G::TPC;
   if (p.target == TGT_GATE) {
-    ensure_smem(k_chain_gate_bwd<D>, smem);
-    k_chain_gate_bwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
+    if constexpr (D <= 4) return small::launch_bwd<D>(p, w, li);
+    else {
+      ensure_smem(k_chain_gate_bwd<D>, smem);
+      k_chain_gate_bwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
+    }
   } else if (p.n_ck > 0) {
     ensure_smem(k_track_bwd<D>, smem);
     k_track_bwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);

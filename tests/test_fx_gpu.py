@@ -130,7 +130,8 @@ def test_exact_gradient(pg, target, gen, D, n_t, n_m, nrm):
 
 
 @pytest.mark.parametrize("mode", ["exact", "ref_mr", "ref_grape"])
-@pytest.mark.parametrize("D,n_t,n_m", [(5, 1, 2), (8, 7, 1), (8, 301, 2), (11, 2, 1), (16, 67, 1), (16, 41, 200),
+@pytest.mark.parametrize("D,n_t,n_m", [(2, 1, 1), (2, 67, 1), (3, 2, 2), (3, 8, 3), (4, 301, 2), (4, 41, 200), (2, 5, 5000),
+                                       (5, 1, 2), (8, 7, 1), (8, 301, 2), (11, 2, 1), (16, 67, 1), (16, 41, 200),
                                        (32, 2, 1), (25, 23, 2)])
 def test_gate_chain_blocks(pg, mode, D, n_t, n_m):
     """Gate chains in one block, in blocks with a short last one, of one slice,
