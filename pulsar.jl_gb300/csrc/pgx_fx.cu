@@ -16,11 +16,13 @@ constexpr int kMaxTerms32 = 7;      // at D = 32: 16 KB of shared memory each be
 // U_total's defect over 1000 slices stayed 2.5 times larger).
 template <bool DF> constexpr int kBits2 = 2 * (DF ? 51 : 57) + 1;
 constexpr int kNever = 1 << 20;     // an exponent no finite entry reaches
-// Levels of a chain product: about 2^-55.5 of the factors' scale with 7, which
-// at D = 16 keeps a chain's error below that of an FP64 product's 64 roundings
-// (unitarity after 1000 slices 2.0e-14, FP64 products 3.0e-14); at D = 8 seven
-// levels fell behind (2.9e-14 against 1.1e-14 after 500), eight do not.
-template <int D> constexpr int kChainLevels = D >= 16 ? 7 : 8;
+// Levels of a chain product.  Seven leave about 2^-55.5 of the factors' scale,
+// which for matrices near the identity (scale 2 to 4) put U_total after 20
+// slices 2.3 times further off than FP64 products; eight cost 3 % of an
+// evaluation and leave the rounding to 56 bits.
+constexpr int kChainLevels = 8;
+// The mixed path's prefixes, rounded to df pairs or FP32 afterwards.
+template <int D> constexpr int kPrefixLevels = D >= 16 ? 7 : 8;
 
 // The constant matrices of the generator, A_mk = c sum_j alpha_j K_j with
 // alpha = dt_k {1, scale u_1k, ..., tau_k} and K = {drift_m + off_m O, C_1,
@@ -394,7 +396,7 @@ __device__ __forceinline__ void load_M(const Tm<D, W>& tm, const ProbDev& p, con
 // t = Tr(X K_j), its real (im = 0) or imaginary part, as an integer sum over
 // the team: the lanes' X (56 fractional bits) against the transposed term.
 // |x| < 2^56 and |K| < 2^59 keep the sum of all elements below 2^60 in units
-// of 2^-52; three further bits hold the lanes' rounding near 2^-54.
+// of 2^-52, returned in units of 2^-55.
 template <int D, int W>
 __device__ __forceinline__ long long trace_term(const Terms<D, W>& T, const Tm<D, W>& tm, int j, int im,
                                                 const long long (&x)[Geo<D, W>::NV]) {
@@ -421,10 +423,13 @@ __device__ __forceinline__ long long trace_term(const Terms<D, W>& T, const Tm<D
     mid += (long long)xi1 * q.x;
     mid += (long long)xi0 * q.y;
   }
-  long long t = ((main + (mid >> 32)) << 3) + (long long)((uint32_t)mid >> 29);
+  long long t = main + (mid >> 32);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  return t;
+  // the lanes' low parts added before they are rounded: rounded one by one they
+  // cost gradients much smaller than |X| |K| three bits
+  const uint32_t lo = __reduce_add_sync(0xffffffffu, (uint32_t)mid >> 8);
+  return (t << 3) + ((lo + (1u << 20)) >> 21);
 }
 
 constexpr int kGradBits2 = 2 * 56 + 1;
@@ -487,7 +492,7 @@ __device__ __forceinline__ void times_prefix(const Tm<D, W>& tm, const ProbDev& 
   store_planes<D, W>(tm, pr, x, kSlices);
   store_planes<D, W>(tm, pl, r, kSlices);
   tm.sync();
-  mul_fixed<D, W, kChainLevels<D>>(tm, pl, pr, x);
+  mul_fixed<D, W, kChainLevels>(tm, pl, pr, x);
   const int e = normalize<D, W>(tm, x, E + ER);
   E = max(E, ER) == kNotFinite ? kNotFinite : e;
 }
@@ -828,13 +833,13 @@ template <int D, int W> struct ChainTeam {
            reinterpret_cast<uint32_t*>(smem + 2 * Geo<D, W>::PLANES)},
         pl(smem_u32(smem)), pr(pl + Geo<D, W>::PLANES) {}
   // (r, E) <- left (r, E); an operand that is not finite stays so
-  template <bool R_IS_LEFT>
+  template <bool R_IS_LEFT, int LEVELS = kChainLevels>
   __device__ __forceinline__ void step(long long (&r)[Geo<D, W>::NV], int& E, const long long (&x)[Geo<D, W>::NV], int Ex) {
     tm.sync();  // the last product has read its planes
     store_planes<D, W>(tm, R_IS_LEFT ? pl : pr, r, kSlices);
     store_planes<D, W>(tm, R_IS_LEFT ? pr : pl, x, kSlices);
     tm.sync();
-    mul_fixed<D, W, kChainLevels<D>>(tm, pl, pr, r);
+    mul_fixed<D, W, LEVELS>(tm, pl, pr, r);
     const int e = normalize<D, W>(tm, r, E + Ex);
     E = max(E, Ex) == kNotFinite ? kNotFinite : e;
   }
@@ -956,7 +961,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS, 2) k
       for (int v = 0; v < 2 * H; ++v) r[v] = u[v];
       E = Eu;
     } else {
-      ct.template step<false>(r, E, u, Eu);
+      ct.template step<false, kPrefixLevels<D>>(r, E, u, Eu);
     }
     if (store && k + 1 < k1) {
       const float sc = E == kNotFinite ? __int_as_float(0x7fc00000) : ldexpf(1.f, E - kFrac);
@@ -968,19 +973,19 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS, 2) k
   store_df<D, W>(tm, w.pit_tot + (size_t)item * D * D, r, E == kNotFinite ? 0x7ff : E - kFrac);
 }
 
-// x -> kappa x: each part times a double, in a common frame; returns its
-// exponent (the result is not normalised, but below 2^55).
+// x -> kappa x, normalised: each part times a double, in a common frame;
+// returns its exponent.
 template <int D, int W>
-__device__ __forceinline__ int scale_complex(long long (&x)[Geo<D, W>::NV], int E, double2 kap) {
+__device__ __forceinline__ int scale_complex(const Tm<D, W>& tm, long long (&x)[Geo<D, W>::NV], int E, double2 kap) {
   constexpr int H = Geo<D, W>::NV / 2;
   const int ex = max((int)((uint32_t)__double2hiint(kap.x) >> 20 & 0x7ff), (int)((uint32_t)__double2hiint(kap.y) >> 20 & 0x7ff));
   if (ex == 0x7ff) return kNotFinite;
-  // parts below 2^(ex - 1022) in 60 fractional bits
-  const long long a = from_double(kap.x, ex, 7), b = from_double(kap.y, ex, 7);
+  // parts below 2^(ex - 1022) in 61 fractional bits
+  const long long a = from_double(kap.x, ex, 8), b = from_double(kap.y, ex, 8);
   const int a0 = (int)a, a1 = (int)((a + 0x80000000ll) >> 32), b0 = (int)b, b1 = (int)((b + 0x80000000ll) >> 32);
 #pragma unroll
   for (int v = 0; v < H; ++v) {
-    const long long re = x[v] << 2, im = x[H + v] << 2;
+    const long long re = x[v] << 5, im = x[H + v] << 5;
     const int r0 = (int)re, r1 = (int)((re + 0x80000000ll) >> 32);
     const int i0 = (int)im, i1 = (int)((im + 0x80000000ll) >> 32);
     const long long mr = 0x80000000ll + (long long)r1 * a0 + (long long)r0 * a1 - (long long)i1 * b0 - (long long)i0 * b1;
@@ -988,7 +993,8 @@ __device__ __forceinline__ int scale_complex(long long (&x)[Geo<D, W>::NV], int 
     x[v] = (long long)r1 * a1 - (long long)i1 * b1 + (mr >> 32);
     x[H + v] = (long long)r1 * b1 + (long long)i1 * a1 + (mi >> 32);
   }
-  return E == kNotFinite ? kNotFinite : E + ex - 1022 + 2;
+  const int e = normalize<D, W>(tm, x, E + ex - 1024, 1);
+  return E == kNotFinite ? kNotFinite : e;
 }
 
 template <int D, int W>
@@ -1077,7 +1083,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W) k_fx_combine_df(ProbDev p
       E = Eu;
       tm.sync();  // the maxima are read
     } else {
-      ct.template step<false>(r, E, u, Eu);
+      ct.template step<false, kPrefixLevels<D>>(r, E, u, Eu);
     }
   }
   put_total<D, W>(tm, w, m, r, E);
@@ -1169,7 +1175,7 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
       const int Ex = unpack<D, W>(x);
       ct.template step<false>(r, E, x, Ex);
     }
-    E = scale_complex<D, W>(r, E, kap);
+    E = scale_complex<D, W>(tm, r, E, kap);
     put_packed<D, W>(slot(tm, w.P, base + (size_t)b * len), r, E);
   }
 }
