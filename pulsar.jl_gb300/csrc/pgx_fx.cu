@@ -1202,13 +1202,18 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
 //   Hermitian generators keep the vector's norm, so its exponent never moves:
 //   |x| < 2^58 at the start, so ||x|| < 2^60.5, and G = 60 with ||u|| <= 2^60 in
 //   every row keep each sum inside 63 bits (Cauchy-Schwarz).
-//   Others: |x| < 2^57, renewed every step; |u| < 2^58 below U_k's largest
-//   entry, G = 58.
+//   Others: |x| < 2^57 (2^56 at D = 32), renewed every step; |u| < 2^58 below
+//   U_k's largest entry, G = 58.
+// At D = 32 a lane sums its row in four parts, so the mixed and low sums stay
+// inside 63 bits as at D = 16 (200 slices of 8 members and two pairs at d = 24:
+// 1.01 + 1.12 ms in FP64 on shared memory, 0.55 ms here).
 template <int D> struct StCfg {
   static constexpr int QS = 32 / D < D ? 32 / D : D;  // lanes that share a row
   static constexpr int QN = D / QS;                   // columns of a lane
   static constexpr int ACTIVE = D * QS;               // the other lanes repeat their work
-  static constexpr int CH = D >= 16 ? 2 : D >= 8 ? 8 : 128 / D;  // slices of a chunk
+  static constexpr int CH = D >= 32 ? 1 : D >= 16 ? 2 : D >= 8 ? 8 : 128 / D;  // slices of a chunk
+  static constexpr int QB = QN < 8 ? QN : 8;          // columns summed at a time
+  static constexpr int GUARD = D >= 32 ? 1 : 0;       // one bit less of a vector that may grow (below)
   static constexpr int HELPERS = 8;
   static constexpr int NPT = 2 * CH * D * D / (32 * HELPERS);  // entries of a helper lane and chunk, both directions
   static constexpr int RING = 2 * CH * D * D;         // entries of one chunk
@@ -1226,7 +1231,7 @@ __device__ __forceinline__ long long join2(int lo, int hi) { return ((long long)
 template <int D, bool HERM>
 __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(ProbDev p, WorkDev w, int store) {
   using C = StCfg<D>;
-  constexpr int QN = C::QN, QS = C::QS, CH = C::CH, NPT = C::NPT;
+  constexpr int QN = C::QN, QS = C::QS, QB = C::QB, CH = C::CH, NPT = C::NPT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_f[8];
   __shared__ int s_bad;
@@ -1342,7 +1347,7 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
     const int EX = (int)(__reduce_max_sync(0xffffffffu, max((uint32_t)__double2hiint(v0.x) & 0x7ff00000u,
                                                             (uint32_t)__double2hiint(v0.y) & 0x7ff00000u)) >> 20);
     bad = EX == 0x7ff;
-    const int guard = HERM ? 5 : 4;
+    const int guard = HERM ? 5 : 4 + C::GUARD;
     first = split2(from_double(v0.x, EX, guard), from_double(v0.y, EX, guard));
     E = EX - 1018 - guard;  // x 2^(EX - 1075 - guard)
   }
@@ -1358,41 +1363,49 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
     const int4* U = ring + (size_t)(buf * 2 + dir) * CH * D * D;
     const int4* prev = mine + (buf ? 0 : other) + (CH - 1) * D;
     int4* cur = mine + (buf ? other : 0);
-    int4 u[QN];
+    // U_k's entries of columns q0 + b QB and on (rows in the backward chain)
+    int4 u[QB];
+    auto load = [&](const int4* V, int b) {
 #pragma unroll
-    for (int i = 0; i < QN; ++i) u[i] = fwd ? U[swz(r, q0 + i)] : U[swz(q0 + i, r)];
+      for (int i = 0; i < QB; ++i) {
+        const int q = q0 + b * QB + i;
+        u[i] = V[fwd ? swz(r, q) : swz(q, r)];
+      }
+    };
+    load(U, 0);
 #pragma unroll 1
     for (int sl = 0; sl < n; ++sl) {
-      // re = sum ur xr -+ ui xi, im = sum ur xi +- ui xr (backward: conj(U))
-      // high, mixed and low partial products of the four sums
-      long long pr = 0, pi = 0, nr = 0, ni = 0, mpr = 0, mpi = 0, mnr = 0, mni = 0, lpr = 0, lpi = 0, lnr = 0, lni = 0;
-#pragma unroll
-      for (int i = 0; i < QN; ++i) {
-        const int4 x = prev[q0 + i];
-        pr += (long long)u[i].y * x.y;
-        mpr += (long long)u[i].y * x.x + (long long)u[i].x * x.y;
-        lpr += (long long)u[i].x * x.x;
-        nr += (long long)u[i].w * x.w;
-        mnr += (long long)u[i].w * x.z + (long long)u[i].z * x.w;
-        lnr += (long long)u[i].z * x.z;
-        pi += (long long)u[i].y * x.w;
-        mpi += (long long)u[i].y * x.z + (long long)u[i].x * x.w;
-        lpi += (long long)u[i].x * x.z;
-        ni += (long long)u[i].w * x.y;
-        mni += (long long)u[i].w * x.x + (long long)u[i].z * x.y;
-        lni += (long long)u[i].z * x.x;
-      }
       const int EX = HERM ? 0 : s_eu[(buf * 2 + dir) * CH + sl];
-      if (sl + 1 < n) {
-        const int4* V = U + (sl + 1) * D * D;
+      long long yr = 0, yi = 0;
+#pragma unroll 1
+      for (int b = 0; b < QN / QB; ++b) {
+        // re = sum ur xr -+ ui xi, im = sum ur xi +- ui xr (backward: conj(U))
+        // high, mixed and low partial products of the four sums
+        long long pr = 0, pi = 0, nr = 0, ni = 0, mpr = 0, mpi = 0, mnr = 0, mni = 0, lpr = 0, lpi = 0, lnr = 0, lni = 0;
 #pragma unroll
-        for (int i = 0; i < QN; ++i) u[i] = fwd ? V[swz(r, q0 + i)] : V[swz(q0 + i, r)];
+        for (int i = 0; i < QB; ++i) {
+          const int4 x = prev[q0 + b * QB + i];
+          pr += (long long)u[i].y * x.y;
+          mpr += (long long)u[i].y * x.x + (long long)u[i].x * x.y;
+          lpr += (long long)u[i].x * x.x;
+          nr += (long long)u[i].w * x.w;
+          mnr += (long long)u[i].w * x.z + (long long)u[i].z * x.w;
+          lnr += (long long)u[i].z * x.z;
+          pi += (long long)u[i].y * x.w;
+          mpi += (long long)u[i].y * x.z + (long long)u[i].x * x.w;
+          lpi += (long long)u[i].x * x.z;
+          ni += (long long)u[i].w * x.y;
+          mni += (long long)u[i].w * x.x + (long long)u[i].z * x.y;
+          lni += (long long)u[i].z * x.x;
+        }
+        if (b + 1 < QN / QB) load(U + sl * D * D, b + 1);
+        else if (sl + 1 < n) load(U + (sl + 1) * D * D, 0);
+        constexpr int SH = HERM ? 0 : 2;
+        const long long mr = (fwd ? mpr - mnr : mpr + mnr) + ((fwd ? lpr - lnr : lpr + lnr) >> 30);
+        const long long mi = (fwd ? mpi + mni : mpi - mni) + ((fwd ? lpi + lni : lpi - lni) >> 30);
+        yr += ((fwd ? pr - nr : pr + nr) << SH) + shift_round(mr, 30 - SH);
+        yi += ((fwd ? pi + ni : pi - ni) << SH) + shift_round(mi, 30 - SH);
       }
-      constexpr int SH = HERM ? 0 : 2;
-      const long long mr = (fwd ? mpr - mnr : mpr + mnr) + ((fwd ? lpr - lnr : lpr + lnr) >> 30);
-      const long long mi = (fwd ? mpi + mni : mpi - mni) + ((fwd ? lpi + lni : lpi - lni) >> 30);
-      long long yr = ((fwd ? pr - nr : pr + nr) << SH) + shift_round(mr, 30 - SH);
-      long long yi = ((fwd ? pi + ni : pi - ni) << SH) + shift_round(mi, 30 - SH);
 #pragma unroll
       for (int o = D; o < D * QS; o <<= 1) {
         yr += __shfl_xor_sync(0xffffffffu, yr, o);
@@ -1400,7 +1413,7 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
       }
       if (!HERM) {
         const uint32_t top = __reduce_max_sync(0xffffffffu, max((uint32_t)abs((int)(yr >> 32)), (uint32_t)abs((int)(yi >> 32))));
-        const int sh = __clz(top + 1) - 7;
+        const int sh = __clz(top + 1) - 7 - C::GUARD;
         yr = sh >= 0 ? yr << sh : shift_round(yr, -sh);
         yi = sh >= 0 ? yi << sh : shift_round(yi, -sh);
         E = max(E + EX - 1022 - sh, -(1 << 20));
@@ -1841,6 +1854,7 @@ cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInf
     case 4: return fx::do_states<4>(p, w, li, store);
     case 8: return fx::do_states<8>(p, w, li, store);
     case 16: return fx::do_states<16>(p, w, li, store);
+    case 32: return fx::do_states<32>(p, w, li, store);
     default: return cudaErrorInvalidValue;
   }
 }

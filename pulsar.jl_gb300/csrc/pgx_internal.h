@@ -234,7 +234,7 @@ cudaError_t launch_fx_chain_bwd(const ProbDev& p, const WorkDev& w, const Launch
 cudaError_t launch_fx_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 // FP64 state chains (no tracking) up to Dp = 16, both directions in one launch;
 // lambda is stored without conj(kappa), which the gradient applies.
-__host__ __device__ inline bool lam_unscaled(const ProbDev& p, int Dp) { return p.n_ck == 0 && Dp <= 16; }
+__host__ __device__ inline bool lam_unscaled(const ProbDev& p, int Dp) { return p.n_ck == 0 && Dp <= 32; }
 cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
 // The mixed path's slice propagators and in-block prefixes on the same engine
 // (df pairs in and out), where fx_applies(p) at Dp = 16 and 32.

@@ -765,7 +765,7 @@ static cudaError_t do_chain_fwd(const ProbDev& p, const WorkDev& w, const Launch
   } else if (p.n_ck > 0) {
     ensure_smem(k_track_fwd<D>, smem);
     k_track_fwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
-  } else if constexpr (D > 16) {  // launch_fx_states below
+  } else if constexpr (D > 32) {  // launch_fx_states below
     ensure_smem(k_chain_states_fwd<D>, smem);
     k_chain_states_fwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w, store ? 1 : 0);
   }
@@ -793,7 +793,7 @@ static cudaError_t do_chain_bwd(const ProbDev& p, const WorkDev& w, const Launch
   } else if (p.n_ck > 0) {
     ensure_smem(k_track_bwd<D>, smem);
     k_track_bwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
-  } else if constexpr (D > 16) {
+  } else if constexpr (D > 32) {
     ensure_smem(k_chain_states_bwd<D>, smem);
     k_chain_states_bwd<D><<<grid, G::THREADS, smem, li.stream>>>(p, w);
   }

@@ -167,7 +167,8 @@ def test_gate_chain_blocks(pg, mode, D, n_t, n_m):
 
 @pytest.mark.parametrize("mode", ["exact", "ref_mr", "ref_grape"])
 @pytest.mark.parametrize("D,n_t,n_m,n_p", [(2, 1, 1, 1), (2, 300, 2, 8), (3, 2, 3, 2), (4, 17, 1, 3), (7, 9, 2, 1),
-                                           (8, 40, 2, 8), (13, 3, 1, 5), (16, 21, 2, 8)])
+                                           (8, 40, 2, 8), (13, 3, 1, 5), (16, 21, 2, 8),
+                                           (20, 9, 2, 8), (32, 6, 1, 3)])
 def test_state_chains(pg, mode, D, n_t, n_m, n_p):
     """State chains of one slice to many, one to eight pairs (the fewest slices
     in flight), pairs of very different norms, a dissipative generator.  FP64's
@@ -204,7 +205,8 @@ def test_state_chains(pg, mode, D, n_t, n_m, n_p):
         assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
 
 
-@pytest.mark.parametrize("D,n_t,n_p", [(2, 64, 1), (2, 129, 2), (4, 33, 8), (8, 8, 3), (8, 9, 8), (16, 5, 8), (12, 2, 1)])
+@pytest.mark.parametrize("D,n_t,n_p", [(2, 64, 1), (2, 129, 2), (4, 33, 8), (8, 8, 3), (8, 9, 8), (16, 5, 8), (12, 2, 1),
+                                       (32, 7, 8), (17, 1, 2)])
 def test_state_chains_hermitian(pg, D, n_t, n_p):
     """Unitary state chains at the edges of a chunk of slices (one, exactly
     full, one over), both gradient forms against the oracle."""
