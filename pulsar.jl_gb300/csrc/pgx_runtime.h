@@ -64,6 +64,15 @@ struct pgx_problem {
   // bumped by every setter that changes what run_pipeline enqueues (kernel
   // parameters, team sizes): graphs captured earlier (batches) are stale
   uint64_t generation = 0;
+  // The host evaluation as a graph, without [0] and with [1] the gradient,
+  // captured on a stream of its own (eval_host)
+  struct EvalGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint64_t generation = 0;  // of the evaluations counted, or of the graph
+    int seen = 0;             // evaluations enqueued directly since it changed
+    int64_t launches = 0;
+  } eval_graph[2];
+  cudaStream_t capture = nullptr;
   void refresh_lsym() {
     pd.lsym = pd_grad.lsym = (lsym_fixed && lsym_drift && lsym_ramp) ? 1 : 0;
   }

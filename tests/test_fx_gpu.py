@@ -261,3 +261,34 @@ def test_mixed_series_gradient(pg, target, gen, D, n_t, n_m, n_c, nrm):
     scale = np.abs(Go).max()
     assert F1 == F and abs(F - Fo) <= 1e-8
     assert np.abs(G - Go).max() <= 1e-4 * scale and np.abs(G1 - Go).max() <= 1e-4 * scale
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("target", ["gate", "states"])
+@pytest.mark.parametrize("D,n_t", [(2, 40), (4, 300), (16, 12)])
+def test_repeated_evaluations(pg, precision, target, D, n_t):
+    """Evaluations enqueued directly and replayed as a graph give the same bits,
+    with and without the gradient, and setters take effect in between."""
+    rng = np.random.default_rng(D + n_t)
+    X = rng.normal(size=(4, D, D)) + 1j * rng.normal(size=(4, D, D))
+    X = X + X.conj().transpose(0, 2, 1)
+    Q, _ = np.linalg.qr(rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D)))
+    kw = dict(dt=np.full(n_t, 0.1 / D), target=target, precision=precision, grad_mode="exact", fidelity="square")
+    kw.update(dict(target_op=Q) if target == "gate" else dict(states_init=Q[:1], states_target=Q[1:2]))
+
+    def fresh(drift, u, want_grad):
+        p = pg.Problem(drift[None], X[1:3], **kw)
+        r = p.eval(u, want_grad=want_grad)
+        p.close()
+        return r
+
+    us = rng.normal(size=(7, 2, n_t))
+    p = pg.Problem(X[:1], X[1:3], **kw)
+    for drift in (X[0], X[3]):
+        p.set_drifts(drift[None])
+        for u in us:
+            for want_grad in (True, False):
+                F, G = p.eval(u, want_grad=want_grad)
+                Fo, Go = fresh(drift, u, want_grad)
+                assert F == Fo and (not want_grad or np.array_equal(G, Go))
+    p.close()
