@@ -68,20 +68,15 @@ METRIC = "ensemble-slice grads/s"
 UNIT = "units/s"
 K_EXP = 8  # conventional matrix-product count of one expm in the FLOP model
 
-# DRAM bytes per launch of the dominant kernel from ncu captures of a smaller
-# case (spin-4: 200 of 1000 slices; lindblad3q: 100 of 500), scaled by the
-# units a full launch processes (every unit reads or writes the same bytes).
-TRAFFIC = {("spin4", "fp64", "grad"): 5 * (190.615296e6 + 4.743936e6),
-           # k_expm_mx<16,128,Herm>, 200-slice capture: 0.1 MB read, the df U stack written
-           ("spin4", "mixed", "expm"): 5 * (0.095232e6 + 127.364352e6),
-           ("spin4", "mixed", "grad"): 5 * (94.700544e6 + 2.850816e6),
-           ("spin4", "mixed", "chain_fwd"): 5 * (189.268736e6 + 67.549952e6),
-           # k_expm_oz64 (tensor cores), 100-slice capture: the prologue's planar
-           # generator read once, the df U stack written once
-           ("lindblad3q", "mixed", "expm"): 5 * (210.639104e6 + 194.420224e6)}
-# Tensor-pipe activity of k_expm_oz64 from an ncu capture (lindblad3q, 100 of
-# 500 slices): sm__pipe_tensor_cycles_active, % of peak while active.
-TENSOR_ACTIVE_PCT = {("lindblad3q", "mixed", "expm"): 17.3}
+# DRAM bytes per launch of the dominant kernel from an ncu capture of a smaller
+# case, scaled by the units a full launch processes (every unit reads or writes
+# the same bytes).
+TRAFFIC = {  # k_expm_oz64, 8 of 32 members: the generator read once, the df U stack written once
+           ("lindblad3q", "mixed", "expm"): 4 * 504.4e6}
+# Tensor-pipe activity of the dominant kernel from an ncu capture of a smaller
+# case: sm__pipe_tensor_cycles_active, % of peak while active.
+TENSOR_ACTIVE_PCT = {("lindblad3q", "mixed", "expm"): 19.0, ("spin4", "mixed", "expm"): 28.5,
+                     ("spin4", "fp64", "grad"): 36.2}
 # FP32 operations one df32 complex MAC executes (error-free two_prod / two_sum
 # accumulation) per 8 FLOPs of the FP64 model: the model-FLOP rate a fully
 # busy FP32 pipe could reach on df32 work is the FP32 peak / (DF_OPS / 8).
@@ -862,14 +857,15 @@ def main():
             dom_ms = stages[dom] / max(n_rec, 1)
             achieved = wl.stage_flops(dom) / (dom_ms * 1e-3)
             share = {k: round(v / max(sum(stages.values()), 1e-30), 4) for k, v in stages.items()}
-            # at padded dimension 64 the mixed expm runs on the tensor cores by
-            # default (team 1): the prologue plus the sliced-bf16 kernel
-            tc_expm = pipe == "fp32" and dom == "expm" and wl.p.teams[0] == 1
+            # the mixed expm runs on the tensor cores by default at padded
+            # dimensions 16 to 64 (team 1), the FP64 stages at 8 to 32
+            dp = 1 << (wl.prob.D - 1).bit_length()
+            tc_expm = (pipe == "fp32" and dom == "expm" and wl.p.teams[0] == 1) or (pipe == "fp64" and 8 <= dp <= 32)
             kname = ("k_" + dom) if pipe == "fp64" else {"expm": "k_expm_mx", "chain_fwd": "k_chain_gate_fwd_mx",
                                                          "chain_bwd": "k_chain_gate_bwd_mx",
                                                          "grad": "k_grad_gate_mx", "reduce": "k_reduce"}[dom]
             if tc_expm:
-                kname = "k_expm_prep_oz64 + k_expm_oz64"
+                kname = "k_expm_prep_oz64 + k_expm_oz64" if dp == 64 else "k_fx_" + dom
             roof = {"kernel": kname, "ms_per_launch": dom_ms, "stage_share": share,
                     "traffic": TRAFFIC.get((args.workload, args.precision, dom))}
             pr = wl.prob
@@ -896,11 +892,13 @@ def main():
                      "flop_model": "conventional per-unit W = 8 D^3 (K_exp (1 + 2 n_c) + 3) + 8 n_c D^2 "
                                    "(K_exp = 8) split by stage"})
         if single and tc_expm:
-            roof.update({"pipe": "tensor cores (tcgen05, df products by exact bf16 slicing)",
+            how = ("tcgen05, df products by exact bf16 slicing" if dp == 64 else
+                   "mma.sync FP16 digits, block fixed point, integer joins")
+            roof.update({"pipe": f"tensor cores ({how})",
                          "tensor_pipe_active_pct_ncu": TENSOR_ACTIVE_PCT.get((args.workload, args.precision, dom)),
-                         "tensor_note": "each df product runs 26 bf16 slice-pair products (12 MMAs of N = 128 and "
-                                        "2 of N = 64 per K step group); achieved counts model FLOPs, so frac "
-                                        "is the df-product rate against the bf16 peak"})
+                         "tensor_note": "each product is up to 26 (D = 64) or 34 exact products of 8-bit digits; "
+                                        "achieved counts model FLOPs, so frac is the product rate against the "
+                                        "bf16 peak"})
         elif args.precision == "mixed" and single and dom in ("expm", "chain_fwd"):
             # df32 stages: each model FLOP costs DF_OPS_PER_CMAC / 8 FP32 operations
             eff = pipe_peak / (DF_OPS_PER_CMAC / 8.0)
