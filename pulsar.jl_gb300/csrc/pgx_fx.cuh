@@ -1,5 +1,6 @@
 // Block fixed-point complex matrices on the tensor cores: the products of the
-// FP64 path at D = 8 and 16.
+// FP64 path at D = 8, 16 and 32, and of the mixed path's propagators and
+// prefixes at D = 16 and 32.
 //
 // GB300 issues 1.8 FP64 FMAs per clock and SM (measured), so a 16 x 16 complex
 // FP64 product takes 9,100 SM cycles.  Here a matrix is 64-bit integers with
