@@ -1333,7 +1333,10 @@ int mixed_variants(const ProbDev& p, int kernel, int* out) {
 }
 int mixed_admitted(const ProbDev& p, int kernel, int* out) {
   int n = variants_for(p.Dp, kernel, out);
-  if (tc_eligible(p, kernel)) out[n++] = kTeamTensor;
+  // at D = 16 and 32 the teams of one problem fit every other: where the
+  // tensor-core kernels do not apply (first order, many terms, states) the value
+  // means the default CUDA-core team
+  if (p.Dp == 16 || p.Dp == 32 || tc_eligible(p, kernel)) out[n++] = kTeamTensor;
   return n;
 }
 // Defaults (problems that were never tuned: batches, served jobs) are the

@@ -292,3 +292,25 @@ def test_repeated_evaluations(pg, precision, target, D, n_t):
                 Fo, Go = fresh(drift, u, want_grad)
                 assert F == Fo and (not want_grad or np.array_equal(G, Go))
     p.close()
+
+
+@pytest.mark.parametrize("target", ["gate", "states"])
+@pytest.mark.parametrize("D,n_c", [(16, 2), (16, 26), (32, 9)])
+def test_teams_carry_over(pg, target, D, n_c):
+    """The teams of an exact gate problem are accepted by every problem of its
+    dimension: first order, states, more terms than the tensor cores take."""
+    rng = np.random.default_rng(D + n_c)
+    X = rng.normal(size=(n_c + 1, D, D)) + 1j * rng.normal(size=(n_c + 1, D, D))
+    X = X + X.conj().transpose(0, 2, 1)
+    dt = np.full(3, 0.05 / D)
+    p = pg.Problem(X[:1], X[1:3], dt, target="gate", target_op=np.eye(D), grad_mode="exact", precision="mixed")
+    teams = p.teams
+    p.close()
+    to = dict(target_op=np.eye(D)) if target == "gate" else dict(states_init=np.eye(D)[:1], states_target=np.eye(D)[1:2])
+    u = rng.normal(size=(n_c, 3))
+    p = pg.Problem(X[:1], X[1:], dt, target=target, grad_mode="ref_mr", precision="mixed", **to)
+    F, G = p.eval(u)
+    p.set_teams(*teams)
+    F1, G1 = p.eval(u)
+    p.close()
+    assert F1 == F and np.array_equal(G, G1)
