@@ -884,9 +884,9 @@ def main():
             flops_acct = None
         roof.update({"bound": "tensor", "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
                      "frac": achieved / peak, "peak_source": pk["source"],
-                     "pipe": f"{pipe.upper()} CUDA cores",
+                     "pipe": f"{pipe.upper()} CUDA cores" if single else "tensor cores (d > 8) and CUDA cores",
                      "fp_pipe_peak": pipe_peak / 1e12,
-                     "frac_of_fp_pipe": achieved / pipe_peak if pipe_peak else None,
+                     "frac_of_fp_pipe": achieved / pipe_peak if pipe_peak and single else None,
                      "fp_pipe_peak_source": f"measured in this run: independent-FMA loop kernel on the "
                                             f"{pipe.upper()} pipe",
                      "flop_model": "conventional per-unit W = 8 D^3 (K_exp (1 + 2 n_c) + 3) + 8 n_c D^2 "
