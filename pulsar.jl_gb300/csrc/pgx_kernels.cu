@@ -575,18 +575,42 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_grad(ProbDev p, WorkDev w) 
 // --------------------------------------------------------------------------
 // Stage 5: deterministic ensemble reduction
 // --------------------------------------------------------------------------
-__global__ void k_reduce(ProbDev p, WorkDev w, int want_grad) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = p.n_t * p.n_c;
-  if (want_grad && idx < n) {
-    double s = 0.0;
-    for (int m = 0; m < p.n_members; ++m) s += w.Gm[(size_t)m * n + idx];
-    w.G[idx] = s;
-  }
-  if (idx == 0) {
+// F = sum_m w_m F_m (block 0) and G = sum_m G_m (32 entries a block), the
+// members dealt to the warps and the warps' sums added in order.  Bound: the
+// latency of a thread's loads, one member each, so they are split eight ways
+// (231 members of 2000 entries: 43 us with one thread per entry, 8 here).
+constexpr int kReduceThreads = 256;
+constexpr int kReduceOut = 32;  // gradient entries of a block, one per lane
+
+__global__ void __launch_bounds__(kReduceThreads) k_reduce(ProbDev p, WorkDev w) {
+  constexpr int WARPS = kReduceThreads / 32;
+  __shared__ double part[WARPS][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x == 0) {  // F
     double f = 0.0;
-    for (int m = 0; m < p.n_members; ++m) f += p.m_weight[m] * w.Fm[m];
-    w.F[0] = f;
+    for (int m = threadIdx.x; m < p.n_members; m += kReduceThreads) f += p.m_weight[m] * w.Fm[m];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+    if (lane == 0) part[warp][0] = f;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int i = 1; i < WARPS; ++i) f += part[i][0];
+      w.F[0] = f;
+    }
+    return;
+  }
+  const int n = p.n_t * p.n_c, idx = (blockIdx.x - 1) * kReduceOut + lane;
+  double s = 0.0;
+  if (idx < n) {
+#pragma unroll 4
+    for (int m = warp; m < p.n_members; m += WARPS) s += w.Gm[(size_t)m * n + idx];
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && idx < n) {
+#pragma unroll
+    for (int i = 1; i < WARPS; ++i) s += part[i][lane];
+    w.G[idx] = s;
   }
 }
 
@@ -826,8 +850,8 @@ cudaError_t launch_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li
 
 cudaError_t launch_reduce(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool want_grad) {
   const int n = p.n_t * p.n_c;
-  const int grid = want_grad ? (n + 255) / 256 : 1;
-  k_reduce<<<grid, 256, 0, li.stream>>>(p, w, want_grad ? 1 : 0);
+  const int grid = want_grad ? 1 + (n + kReduceOut - 1) / kReduceOut : 1;
+  k_reduce<<<grid, kReduceThreads, 0, li.stream>>>(p, w);
   ++*li.launches;
   return cudaGetLastError();
 }

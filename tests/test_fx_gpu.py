@@ -314,3 +314,30 @@ def test_teams_carry_over(pg, target, D, n_c):
     F1, G1 = p.eval(u)
     p.close()
     assert F1 == F and np.array_equal(G, G1)
+
+
+@pytest.mark.parametrize("n_m,n_t", [(1, 1), (7, 11), (8, 16), (9, 17), (300, 33)])
+def test_member_sums(pg, n_m, n_t):
+    """F and G of an ensemble against the weighted sums of its members, each
+    evaluated alone: sums of n_m terms, n_m 2^-52 of their absolute sum."""
+    rng = np.random.default_rng(n_m)
+    X = rng.normal(size=(3, 2, 2)) + 1j * rng.normal(size=(3, 2, 2))
+    X = X + X.conj().transpose(0, 2, 1)
+    sc, wt = rng.uniform(0.9, 1.1, n_m), rng.uniform(0.1, 1.0, n_m)
+    wt /= wt.sum()
+    u = rng.normal(size=(2, n_t))
+    kw = dict(dt=np.full(n_t, 0.1), target="gate", target_op=np.eye(2), grad_mode="ref_mr", precision="fp64")
+    p = pg.Problem(X[:1], X[1:], member_scale=sc, member_weight=wt, **kw)
+    F, G = p.eval(u)
+    F1, _ = p.eval(u, want_grad=False)
+    p.close()
+    Fs, Gs = [], []
+    for m in range(n_m):
+        p = pg.Problem(X[:1], X[1:], member_scale=sc[m:m + 1], member_weight=wt[m:m + 1], **kw)
+        f, g = p.eval(u)
+        p.close()
+        Fs.append(f)
+        Gs.append(g)
+    assert F1 == F
+    assert abs(F - sum(Fs)) <= (n_m + 8) * 2.0 ** -52 * np.abs(Fs).sum()
+    assert (np.abs(G - sum(Gs)) <= (n_m + 8) * 2.0 ** -52 * np.abs(Gs).sum(0)).all()
