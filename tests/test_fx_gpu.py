@@ -341,3 +341,29 @@ def test_member_sums(pg, n_m, n_t):
     assert F1 == F
     assert abs(F - sum(Fs)) <= (n_m + 8) * 2.0 ** -52 * np.abs(Fs).sum()
     assert (np.abs(G - sum(Gs)) <= (n_m + 8) * 2.0 ** -52 * np.abs(Gs).sum(0)).all()
+
+
+@pytest.mark.parametrize("mode", ["exact", "ref_grape"])
+@pytest.mark.parametrize("D,n_t,n_m", [(2, 128, 1), (2, 3001, 2), (4, 145, 2), (3, 600, 1), (8, 129, 1), (7, 1000, 3),
+                                       (8, 4000, 1)])
+def test_mixed_many_blocks(pg, mode, D, n_t, n_m):
+    """Mixed gate chains of 16 blocks (the fewest that the eight-warp combine
+    takes) to many, full and short last runs, against the FP64 path.  The mixed
+    path's bars: |dF| 1e-9, gradient 2e-5 of its norm."""
+    rng = np.random.default_rng(n_t)
+    X = rng.normal(size=(3, D, D)) + 1j * rng.normal(size=(3, D, D))
+    X = X + X.conj().transpose(0, 2, 1)
+    Q, _ = np.linalg.qr(rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D)))
+    u = rng.normal(size=(2, n_t))
+    kw = dict(dt=np.full(n_t, 0.5 / D), member_scale=rng.uniform(0.9, 1.1, n_m), target="gate", target_op=Q,
+              fidelity="square", grad_mode=mode)
+    out = []
+    for precision in ("fp64", "mixed"):
+        p = pg.Problem(X[:1], X[1:], precision=precision, **kw)
+        F, G = p.eval(u)
+        F1, _ = p.eval(u, want_grad=False)
+        p.close()
+        assert F1 == F
+        out.append((F, G))
+    assert abs(out[0][0] - out[1][0]) <= 1e-9
+    assert np.linalg.norm(out[0][1] - out[1][1]) <= 2e-5 * np.linalg.norm(out[0][1])
