@@ -557,8 +557,8 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) k_chainf_combine_mx(ProbDev p
 // take a run of the blocks, form their prefixes inside it (kept in shared
 // memory), then the product of the runs before theirs, and multiply it in.
 // B blocks take B / 8 + 7 + B / 8 products of latency where one team takes B:
-// one member of 2000 slices
-// at D = 4, forward and backward chain 55 + 20 us before, 47 + 14 now.
+// one member of 2000 slices at D = 4, forward and backward chain 55 + 20 us
+// before, 47 + 14 now.
 constexpr int kWideTeams = 8;
 constexpr int kWideBlocks = 16;  // fewer blocks: the single team's chain is no longer
 template <int D> size_t wide_fwd_smem(int blocks) {

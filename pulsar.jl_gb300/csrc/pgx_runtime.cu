@@ -363,7 +363,8 @@ static void pit_shape(const pgx_problem_desc* d, int Dp, int num_sms, int* block
   // a member's block products and costates are combined one after another, in
   // both directions: with few members, more than sqrt(2 n_t) blocks lengthen
   // len + 2 blocks (one member, 2000 slices: 250 blocks of 8 took 221 us in
-  // the chains, 63 of 32 take a third)
+  // the chains, 63 of 32 take a third; with the eight-warp combine of D <= 8
+  // 87 blocks are still slower, 90 against 80 us an evaluation)
   while (b > 1 && b * b > 2L * d->n_slices) --b;
   if (b <= 1) return;
   const int L = (int)((d->n_slices + b - 1) / b);
@@ -1044,11 +1045,12 @@ static int enqueue_eval(pgx_problem* p, bool grad, cudaStream_t stream) {
 
 // The evaluation's ten or so enqueues as one graph launch (the gaps between
 // small kernels shrink with it: one qubit, 100 slices 75 -> 67 us, two qubits,
-// 2 x 1000 slices 158 -> 136 us).  A graph is captured at the third evaluation in a row
-// that enqueues the same work (a setter's new generation starts over), so a
-// problem evaluated once or twice does not pay for it, and on a stream of the
-// problem's own, so that nothing another thread enqueues on the context's gets
-// into it.  Returns false when there is none: the caller enqueues directly.
+// one member of 2000 slices 158 -> 136 us).  A graph is captured at the third
+// evaluation in a row that enqueues the same work (a setter's new generation
+// starts over), so a problem evaluated once or twice does not pay for it, and
+// on a stream of the problem's own, so that nothing another thread enqueues on
+// the context's gets into it.  Returns false when there is none: the caller
+// enqueues directly.
 static bool eval_graph_ready(pgx_problem* p, bool grad) {
   constexpr int kDirect = 2;
   pgx_problem::EvalGraph& e = p->eval_graph[grad];
