@@ -21,8 +21,7 @@ constexpr int kNever = 1 << 20;     // an exponent no finite entry reaches
 // slices 2.3 times further off than FP64 products; eight cost 3 % of an
 // evaluation and leave the rounding to 56 bits.
 constexpr int kChainLevels = 8;
-// The mixed path's prefixes, rounded to df pairs or FP32 afterwards.
-template <int D> constexpr int kPrefixLevels = D >= 16 ? 7 : 8;
+constexpr int kPrefixLevels = 7;  // the mixed path's prefixes, rounded to df pairs or FP32 afterwards
 
 // The constant matrices of the generator, A_mk = c sum_j alpha_j K_j with
 // alpha = dt_k {1, scale u_1k, ..., tau_k} and K = {drift_m + off_m O, C_1,
@@ -969,7 +968,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS, 2) k
       for (int v = 0; v < 2 * H; ++v) r[v] = u[v];
       E = Eu;
     } else {
-      ct.template step<false, kPrefixLevels<D>>(r, E, u, Eu);
+      ct.template step<false, kPrefixLevels>(r, E, u, Eu);
     }
     if (store && k + 1 < k1) {
       const float sc = E == kNotFinite ? __int_as_float(0x7fc00000) : ldexpf(1.f, E - kFrac);
@@ -1091,31 +1090,29 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W) k_fx_combine_df(ProbDev p
       E = Eu;
       tm.sync();  // the maxima are read
     } else {
-      ct.template step<false, kPrefixLevels<D>>(r, E, u, Eu);
+      ct.template step<false, kPrefixLevels>(r, E, u, Eu);
     }
   }
   put_total<D, W>(tm, w, m, r, E);
-  if constexpr (D >= 16) {
-    if (p.gen == GEN_HERM && E != kNotFinite) {
-      // one Newton-Schulz step of the polar decomposition, U (3I - U'U) / 2,
-      // before the overlap (k_refine_unitary_mx, which takes 10 us at D = 16
-      // and 76 us at D = 32 on the FP64 pipe)
-      tm.sync();
-      store_planes<D, W>(tm, ct.pl, r, kSlices);
-      tm.sync();
-      long long s[2 * H];
-      mul_fixed<D, W, kMaxLevels, LeftH<D, W>>(tm, ct.pl, ct.pl, s);
-      to_frame<2 * H>(s, 2 * E, 3, kFrac);
+  if (p.gen == GEN_HERM && E != kNotFinite) {
+    // one Newton-Schulz step of the polar decomposition, U (3I - U'U) / 2,
+    // before the overlap (k_refine_unitary_mx, which takes 10 us at D = 16
+    // and 76 us at D = 32 on the FP64 pipe)
+    tm.sync();
+    store_planes<D, W>(tm, ct.pl, r, kSlices);
+    tm.sync();
+    long long s[2 * H];
+    mul_fixed<D, W, kMaxLevels, LeftH<D, W>>(tm, ct.pl, ct.pl, s);
+    to_frame<2 * H>(s, 2 * E, 3, kFrac);
 #pragma unroll
-      for (int v = 0; v < 2 * H; ++v) s[v] = -s[v];
+    for (int v = 0; v < 2 * H; ++v) s[v] = -s[v];
 #pragma unroll
-      for (int i = 0; i < H; ++i)
-        if (at[i] % D == at[i] / D) s[i] += 3ll << (kFrac - 3);
-      store_planes<D, W>(tm, ct.pr, s, kSlices);
-      tm.sync();
-      mul_fixed<D, W, kMaxLevels>(tm, ct.pl, ct.pr, r);
-      E += 2;  // frame 3, halved
-    }
+    for (int i = 0; i < H; ++i)
+      if (at[i] % D == at[i] / D) s[i] += 3ll << (kFrac - 3);
+    store_planes<D, W>(tm, ct.pr, s, kSlices);
+    tm.sync();
+    mul_fixed<D, W, kMaxLevels>(tm, ct.pl, ct.pr, r);
+    E += 2;  // frame 3, halved
   }
   finish_gate<D, W>(tm, p, w, m, r, E, s_red, &s_kap);
 }
@@ -1843,15 +1840,22 @@ bool fx_applies(const ProbDev& p) {
     case 32: { constexpr int D_ = 32; return CALL; }   \
     default: return cudaErrorInvalidValue;             \
   }
+// the mixed path's dimensions
+#define PGX_FX_DISPATCH_DF(CALL)                         \
+  switch (p.Dp) {                                        \
+    case 16: { constexpr int D_ = 16; return CALL; }     \
+    case 32: { constexpr int D_ = 32; return CALL; }     \
+    default: return cudaErrorInvalidValue;               \
+  }
 
 cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
   PGX_FX_DISPATCH((fx::launch_slices<fx::ExpmCfg<D_>, D_>(fx::k_fx_expm<D_, false>, p, w, li)));
 }
 cudaError_t launch_fx_expm_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  PGX_FX_DISPATCH((fx::launch_slices<fx::ExpmCfg<D_>, D_>(fx::k_fx_expm<D_, true>, p, w, li)));
+  PGX_FX_DISPATCH_DF((fx::launch_slices<fx::ExpmCfg<D_>, D_>(fx::k_fx_expm<D_, true>, p, w, li)));
 }
 cudaError_t launch_fx_prefix_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
-  PGX_FX_DISPATCH(fx::do_prefix_df<D_>(p, w, li, store));
+  PGX_FX_DISPATCH_DF(fx::do_prefix_df<D_>(p, w, li, store));
 }
 cudaError_t launch_tf_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
   return p.Dp == 16 ? fx::do_tf_grad<16>(p, w, li) : fx::do_tf_grad<32>(p, w, li);
@@ -1867,11 +1871,10 @@ cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInf
   }
 }
 cudaError_t launch_fx_combine_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
-  PGX_FX_DISPATCH(fx::do_combine_df<D_>(p, w, li, store));
+  PGX_FX_DISPATCH_DF(fx::do_combine_df<D_>(p, w, li, store));
 }
 long fx_prefix_capacity(int Dp) {
   switch (Dp) {
-    case 8: return fx::prefix_capacity<8>();
     case 16: return fx::prefix_capacity<16>();
     // two of 57 KB are resident, but the FP32 suffixes beside them gain from more
     // blocks than the prefixes lose by queueing (64 x 500: 8.67 -> 8.41 ms with 4)
