@@ -967,6 +967,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS, 2) k
 #pragma unroll
       for (int v = 0; v < 2 * H; ++v) r[v] = u[v];
       E = Eu;
+      tm.sync();  // the maxima are read
     } else {
       ct.template step<false, kPrefixLevels>(r, E, u, Eu);
     }

@@ -367,3 +367,35 @@ def test_mixed_many_blocks(pg, mode, D, n_t, n_m):
         out.append((F, G))
     assert abs(out[0][0] - out[1][0]) <= 1e-9
     assert np.linalg.norm(out[0][1] - out[1][1]) <= 2e-5 * np.linalg.norm(out[0][1])
+
+
+@pytest.mark.parametrize("D,n_t,n_m", [(9, 16, 1), (16, 64, 1), (16, 50, 40), (20, 33, 2), (32, 64, 1), (32, 24, 30)])
+def test_mixed_prefixes_of_unequal_slices(pg, D, n_t, n_m):
+    """In-block prefixes of the mixed path whose neighbouring slices differ by
+    2^16 in scale, so a slice read with its neighbour's exponent is off by that
+    factor.  The oracle with the mixed path's bars; the same bits every time."""
+    from oracle import members as mb
+    rng = np.random.default_rng(D * n_t)
+    X = rng.normal(size=(3, D, D)) + 1j * rng.normal(size=(3, D, D))
+    X = (X - np.swapaxes(X.conj(), -1, -2)) / D
+    X[2] = np.eye(D)
+    u = rng.normal(size=(2, n_t))
+    u[1] = 8 * np.log(2.0) * (1 - 2 * (np.arange(n_t) % 2))
+    if n_t % 2:
+        u[1, -1] = 0.0
+    Q, _ = np.linalg.qr(rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D)))
+    kw = dict(drifts=X[:1], controls=X[1:], dt=np.ones(n_t), generator="liouvillian", target="gate", target_op=Q,
+              fidelity="square", offset_op=X[0], member_offset=rng.uniform(-0.1, 0.1, n_m))
+    few = dict(kw, member_offset=kw["member_offset"][:2])
+    p = pg.Problem(grad_mode="exact", precision="mixed", **few)
+    F, G = p.eval(u)
+    p.close()
+    Fo, Go = mb.eval_problem(mb.Problem(n_members=len(few["member_offset"]), **few), u, "exact")
+    assert abs(F - Fo) <= 1e-8
+    assert np.abs(G - Go).max() <= 1e-4 * np.abs(Go).max()
+    p = pg.Problem(grad_mode="exact", precision="mixed", **kw)
+    F, G = p.eval(u)
+    for _ in range(20):
+        F1, G1 = p.eval(u)
+        assert F1 == F and np.array_equal(G1, G)
+    p.close()
