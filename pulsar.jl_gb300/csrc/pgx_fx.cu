@@ -499,7 +499,8 @@ __device__ __forceinline__ void times_prefix(const Tm<D, W>& tm, const ProbDev& 
   E = max(E, ER) == kNotFinite ? kNotFinite : e;
 }
 
-// The gradient of gate targets in any mode, and of exact state targets.  One
+// The gradient of gate targets in any mode, and of exact state targets without
+// tracking (whose co-state lambda_k holds more than U_k' lambda_{k+1}).  One
 // team per slice: g_jk = Re(c dt scale Tr(X C_j)).
 //
 // Exact: X = L_exp(A, M) = sum_n ad_A^n(N) / (n + 1)!, N = M e^A = P_k

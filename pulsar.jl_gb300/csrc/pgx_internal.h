@@ -226,7 +226,7 @@ cudaError_t launch_select_sum(const double* Gm, const int* idx, const double* co
 // and 16 with at most 24 generator terms (drift, controls, ramp).  Slice
 // propagators for every target (gate targets: in the gate chains' own format),
 // the gate chains, and the gradient of gate targets (any mode) and of exact
-// state targets.
+// state targets (launch_grad leaves those with tracking to k_grad).
 bool fx_applies(const ProbDev& p);
 cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 cudaError_t launch_fx_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);

@@ -843,7 +843,11 @@ static cudaError_t do_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo&
   return cudaGetLastError();
 }
 cudaError_t launch_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li) {
-  if ((p.target == TGT_GATE || p.grad_mode == GRAD_EXACT) && fx_applies(p)) return launch_fx_grad(p, w, li);
+  // k_fx_grad pairs psi_k with lambda_k = U_k' lambda_{k+1}; a tracking co-state
+  // lambda_k holds the checkpoint of step k as well, so it takes k_grad, which
+  // pairs psi_k with lambda_{k+1}
+  if ((p.target == TGT_GATE || (p.grad_mode == GRAD_EXACT && p.n_ck == 0)) && fx_applies(p))
+    return launch_fx_grad(p, w, li);
   PGX_DISPATCH(p.Dp, return do_grad<D_>(p, w, li));
   return cudaSuccess;
 }

@@ -155,3 +155,68 @@ def test_phase_kernel_matches_the_oracle(pg):
         pg.grape_phase_kernel(np.zeros((2, 25)), ctrl)
     with pytest.raises(ValueError):
         pg.grape_phase_kernel(phi, ctrl, -amp)
+
+
+def _tracking_restated(kw, u, track, mode):
+    """(F, G) of the checkpoint objective: F = sum w_m w_c Re <psi_s|rho_c psi_s>,
+    the exact gradient from scipy's Frechet derivative, the reference's
+    first-order formula 2 dt Im <chi|C psi> with both taken after the slice."""
+    import scipy.linalg as sla
+    n_c, n_t = u.shape
+    n_m, n_p = len(kw["member_scale"]), len(kw["states_init"])
+    F, G = 0.0, np.zeros((n_c, n_t))
+    for m in range(n_m):
+        sc, w = kw["member_scale"][m], 1.0 / (n_m * n_p)
+        A = [-1j * kw["dt"][k] * (kw["drifts"][0] + sc * np.tensordot(u[:, k], kw["controls"], 1)) for k in range(n_t)]
+        U = [sla.expm(a) for a in A]
+        psi = [kw["states_init"].T]
+        for k in range(n_t):
+            psi.append(U[k] @ psi[-1])
+        chi = np.zeros_like(psi[0])
+        for k in range(n_t, 0, -1):
+            for step, rho, wc in track:
+                if step == k:
+                    F += w * wc * np.vdot(psi[k], rho @ psi[k]).real
+                    chi = chi + 2 * wc * rho @ psi[k]
+            for j in range(n_c):
+                E = -1j * kw["dt"][k - 1] * sc * kw["controls"][j]
+                d = sla.expm_frechet(A[k - 1], E, compute_expm=False) @ psi[k - 1] if mode == "exact" else 2 * E @ psi[k]
+                G[j, k - 1] += w * np.vdot(chi, d).real
+            chi = U[k - 1].conj().T @ chi
+    return F, G
+
+
+@pytest.mark.parametrize("mode", ["exact", "ref_mr"])
+@pytest.mark.parametrize("nrm", [0.1, 4.0])
+@pytest.mark.parametrize("D,n_p", [(2, 1), (4, 3), (5, 2), (8, 1), (9, 8), (16, 2), (20, 3), (32, 1), (33, 2)])
+def test_tracking_gradient_of_every_dimension(pg, D, n_p, nrm, mode):
+    """Checkpoints in the middle of the pulse, two of them on one step, on its
+    first and on its last slice, against the restatement above, at slice norms
+    on either side of the exact gradient's series (FP64's bars); one gradient
+    entry behind a checkpoint also against a finite difference."""
+    rng = np.random.default_rng(17 * D + n_p)
+    n_t = 6
+    X = rng.normal(size=(3, D, D)) + 1j * rng.normal(size=(3, D, D))
+    X = X + np.swapaxes(X.conj(), -1, -2)
+    u = rng.normal(size=(2, n_t))
+    dt = nrm / np.abs(X[0] + np.tensordot(u[:, 0], X[1:], 1)).sum(0).max() * rng.uniform(0.5, 1.0, n_t)
+    V = rng.normal(size=(2, n_p, D)) + 1j * rng.normal(size=(2, n_p, D))
+    V /= np.linalg.norm(V, axis=2, keepdims=True)
+    kw = dict(drifts=X[:1], controls=X[1:], dt=dt, member_scale=np.array([0.9, 1.1]), target="states", states_init=V[0],
+              states_target=V[1])
+    R = rng.normal(size=(5, D, D)) + 1j * rng.normal(size=(5, D, D))
+    R = R @ np.swapaxes(R.conj(), -1, -2) / D
+    track = [(1, R[0], 0.3), (3, R[1], 0.2), (3, R[2], 0.4), (4, R[3], 0.1), (n_t, R[4], 0.5)]
+    Fo, Go = _tracking_restated(kw, u, track, mode)
+    p = pg.Problem(grad_mode=mode, precision="fp64", **kw)
+    p.set_tracking([t[0] for t in track], [t[2] for t in track], np.stack([t[1] for t in track]))
+    F, G = p.eval(u)
+    p.close()
+    assert abs(F - Fo) <= 1e-10
+    assert np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
+    if mode == "exact":
+        du = np.zeros_like(u)
+        du[0, 3] = 1e-5 / max(nrm, 1.0)
+        fd = (_tracking_restated(kw, u + du, track, "ref_mr")[0] -
+              _tracking_restated(kw, u - du, track, "ref_mr")[0]) / (2 * du[0, 3])
+        assert abs(G[0, 3] - fd) <= 1e-6 * np.abs(Go).max()
