@@ -57,10 +57,12 @@ def main(out=sys.stdout):
     vals = ", ".join(f"{theta_for(m, udf):.17g}" for m in range(1, max(DEGREES) + 1))
     print(f"#define PGX_THETADF_ALL_INIT {{{vals}}}  /* index m - 1 */", file=out)
     # block fixed point: log2 of the FP64 and df thresholds of the degrees 4, 6, ..., 20,
-    # and 1/k! = mant 2^(exp - 61)
+    # and 1/k! = mant 2^(exp - 61).  FP64's at 2^-57, the products' own error: with a
+    # degree chosen this closely, 2^-53 left every slice of one pulse the same tail,
+    # which added up along 1500 slices to 1e-14 of F, three times FP64's own rounding
     even = range(4, max(DEGREES) + 1, 2)
     print(f"#define PGX_N_FXDEGREES {len(even)}", file=out)
-    for name, u in (("PGX_LOG2_THETA64_EVEN_INIT", u64), ("PGX_LOG2_THETADF_EVEN_INIT", udf)):
+    for name, u in (("PGX_LOG2_THETA64_EVEN_INIT", 2.0 ** -57), ("PGX_LOG2_THETADF_EVEN_INIT", udf)):
         vals = ", ".join(f"{math.log2(theta_for(m, u)):.9g}f" for m in even)
         print(f"#define {name} {{{vals}}}", file=out)
     coefs = []

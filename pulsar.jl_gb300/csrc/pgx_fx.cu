@@ -268,6 +268,13 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
       const float l1 = log2_norm1<D, W>(tm, r, EA);
       double2* out = w.U + ((size_t)m * p.n_t + k) * D * D;
       const bool packed = !DF && p.target == TGT_GATE;  // the FP64 gate chains' own format
+      // Squares keep an odd number of levels: the first one left out then has no
+      // pair of equal digits, whose squares a (skew-)Hermitian matrix sums into
+      // its diagonal with one sign.  Six levels of df propagators raised a state's
+      // norm by 9e-16 a slice at d = 32 (df products on the FP32 pipe: -5e-16;
+      // seven: 2e-17).  Not for unitary gates of the mixed path, whose U_total is
+      // projected onto the unitary matrices before its overlap: 4 % of this kernel.
+      const int odd = DF && p.target == TGT_GATE && p.gen == GEN_HERM ? 0 : 1;
       int ex;  // U = r 2^ex
       if (EA > kNever / 2 || l1 > 60.f) {
         if constexpr (DF) {
@@ -291,9 +298,9 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
 #pragma unroll 1
       for (int st = 0; st < L + s; ++st) {
         int n;
-        if (st == 0) n = levels(kBits2<DF>, 2 * (EB - (int)fmaxf(l1, 0.f)));
+        if (st == 0) n = min(levels(kBits2<DF>, 2 * (EB - (int)fmaxf(l1, 0.f))) | odd, kMaxLevels);
         else if (st < L) n = levels(kBits2<DF>, EX + EY + (L - 1 - st) * lx);
-        else n = levels(kBits2<DF>, 2 * EY);
+        else n = min(levels(kBits2<DF>, 2 * EY) | odd, kMaxLevels);
         tm.sync();
         if (st == 0) {
           long long x6[NV];

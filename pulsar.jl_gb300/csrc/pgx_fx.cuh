@@ -503,7 +503,9 @@ __device__ __forceinline__ long long from_double(double d, int EX, int guard) {
 __device__ __forceinline__ double to_double(long long r, int k) {
   const unsigned long long u = (unsigned long long)(r < 0 ? -r : r);
   const int lz = __clzll((long long)u);
-  const unsigned long long m = ((u << (lz - 1)) + 0x200) >> 10;  // bit 52 set (or 53 after a carry)
+  // bit 52 set (or 53 after a carry).  Ties to even: r often has a few low zero
+  // bits, and ties away from zero then raised the norm of U by 3e-17 a slice at d = 32
+  const unsigned long long v = u << (lz - 1), m = (v + 0x1ff + (v >> 10 & 1)) >> 10;
   const int be = 63 - lz + k + 1022;                             // biased exponent - 1
   unsigned long long b = m + ((unsigned long long)be << 52);
   if (be > 2045) b = 0x7ff0000000000000ull;
