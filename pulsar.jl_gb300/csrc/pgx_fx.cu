@@ -16,11 +16,6 @@ constexpr int kMaxTerms32 = 7;      // at D = 32: 16 KB of shared memory each be
 // U_total's defect over 1000 slices stayed 2.5 times larger).
 template <bool DF> constexpr int kBits2 = 2 * (DF ? 51 : 57) + 1;
 constexpr int kNever = 1 << 20;     // an exponent no finite entry reaches
-// Levels of a chain product.  Seven leave about 2^-55.5 of the factors' scale,
-// which for matrices near the identity (scale 2 to 4) put U_total after 20
-// slices 2.3 times further off than FP64 products; eight cost 3 % of an
-// evaluation and leave the rounding to 56 bits.
-constexpr int kChainLevels = 8;
 constexpr int kPrefixLevels = 7;  // the mixed path's prefixes, rounded to df pairs or FP32 afterwards
 
 // The constant matrices of the generator, A_mk = c sum_j alpha_j K_j with
@@ -75,9 +70,12 @@ __device__ __forceinline__ void put_member_terms(const Terms<D, W>& T, const Pro
   }
 }
 
-// A = c sum_j alpha_j K_j, 58 fractional bits in the frame returned; a frame
+// A = c sum_j alpha_j K_j, 62 fractional bits in the frame returned; a frame
 // above kNever / 2 means a term is not finite.  |b1| <= 2^27, |a0| <= 2^31 and
-// sum |a1| <= 2^30 keep 24 terms' mixed products inside 63 bits.
+// sum |a1| <= 2^30 keep 24 terms' mixed products inside 63 bits; the products of
+// the low halves are left out (at most 2^-60 of the frame a term).  (The frame
+// holds the sum of the terms' bounds, up to 2^6 times A's largest entry, so
+// 58 bits rounded A more coarsely than doubles do.)
 template <int D, int W>
 __device__ __forceinline__ int assemble(const Terms<D, W>& T, const ProbDev& p, const double* u, int m, int k,
                                         const Tm<D, W>& tm, long long (&A)[Geo<D, W>::NV]) {
@@ -105,7 +103,7 @@ __device__ __forceinline__ int assemble(const Terms<D, W>& T, const ProbDev& p, 
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     main[v] = 0;
-    mid[v] = 0x80000000ll;  // to nearest
+    mid[v] = 1ll << 27;  // to nearest
   }
 #pragma unroll 1
   for (int j = 0; j < T.n; ++j) {
@@ -124,7 +122,7 @@ __device__ __forceinline__ int assemble(const Terms<D, W>& T, const ProbDev& p, 
   }
   // times c: -i for a Hermitian generator, 1 for a Liouvillian
 #pragma unroll
-  for (int v = 0; v < NV; ++v) main[v] += (long long)(int)(mid[v] >> 32);
+  for (int v = 0; v < NV; ++v) main[v] = (main[v] << 4) + (mid[v] >> 28);
 #pragma unroll
   for (int v = 0; v < NV / 2; ++v) {
     A[v] = p.gen == GEN_HERM ? main[NV / 2 + v] : main[v];
@@ -136,7 +134,7 @@ __device__ __forceinline__ int assemble(const Terms<D, W>& T, const ProbDev& p, 
 // log2 of a bound of ||A||_1 (F fractional bits in frame EA): the largest
 // column sum, from D = 32 on over each warp's rows and then added up.
 template <int D, int W> __device__ __forceinline__ float log2_norm1(const Tm<D, W>& tm, const long long (&A)[Geo<D, W>::NV], int EA,
-                                                                                 int F = 58) {
+                                                                                 int F = 62) {
   using G = Geo<D, W>;
   float best = 0.f;
 #pragma unroll
@@ -281,7 +279,7 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
           store_df<D, W>(tm, (float4*)out, r, 0x7ff);
           if (tm.lane == 0 && tm.w == 0) *w.norm_flag = 1;
         } else if (packed) {
-          put_packed<D, W>(tm.mine((longlong2*)out), r, kNotFinite);
+          put_packed<D, W>(tm, tm.mine((longlong2*)out), r, kNotFinite);
         } else {
           store_nan<D, W>(tm, out);
         }
@@ -290,7 +288,7 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
       }
       // B = A and X = B B before the degree is known: scaling by 2^-s only moves
       // exponents
-      int EB = normalize<D, W>(tm, r, EA - 2), EX = 0, EY = EB, F = 60, L = 2, s = 0, g = 1, lx = 0;
+      int EB = normalize<D, W>(tm, r, EA - 6), EX = 0, EY = EB, F = 60, L = 2, s = 0, g = 1, lx = 0;
       uint32_t pa = py;
       // step 0: X = B B; L - 1 Horner steps Y <- X Y + c_{2i+1} B + c_2i I,
       // whose error later meets X^i; s squarings.  One product in the loop
@@ -369,12 +367,13 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
         store_df<D, W>(tm, (float4*)out, r, ex);
         continue;
       }
-      if (packed && s == 0) {
+      if (packed) {  // from 60 fractional bits of frame EY, 56 after squarings
 #pragma unroll
-        for (int v = 0; v < NV; ++v) r[v] = shift_round(r[v], 4);
+        for (int v = 0; v < NV; ++v) r[v] <<= s == 0 ? 3 : 7;
+        put_packed<D, W>(tm, tm.mine((longlong2*)out), r, EY + 1);
+      } else {
+        store_mat<D, W>(tm, out, r, ex);
       }
-      if (packed) put_packed<D, W>(tm.mine((longlong2*)out), r, EY);
-      else store_mat<D, W>(tm, out, r, ex);
     }
   }
 }
@@ -403,13 +402,21 @@ __device__ __forceinline__ void load_M(const Tm<D, W>& tm, const ProbDev& p, con
 }
 
 // t = Tr(X K_j), its real (im = 0) or imaginary part, as an integer sum over
-// the team: the lanes' X (56 fractional bits) against the transposed term.
-// |x| < 2^56 and |K| < 2^59 keep the sum of all elements below 2^60 in units
-// of 2^-52, returned in units of 2^-55.
+// the team: the lanes' X (58 fractional bits) against the transposed term (60).
+// A lane's 2 D D / (32 W) products sum below 2^57 in units of 2^-54; its lowest
+// PS bits join the next 24 in a second word, so the warp's sum stays inside 63
+// bits and no low part is rounded by itself (gradients much smaller than |X|
+// |K| would lose bits).
+struct Trace {
+  long long hi;  // units of 2^(PS - 54)
+  uint32_t lo;   // units of 2^(PS - 78)
+};
+template <int D> constexpr int kTraceShift = D >= 32 ? 4 : 2;
 template <int D, int W>
-__device__ __forceinline__ long long trace_term(const Terms<D, W>& T, const Tm<D, W>& tm, int j, int im,
-                                                const long long (&x)[Geo<D, W>::NV]) {
+__device__ __forceinline__ Trace trace_term(const Terms<D, W>& T, const Tm<D, W>& tm, int j, int im,
+                                            const long long (&x)[Geo<D, W>::NV]) {
   using G = Geo<D, W>;
+  constexpr int PS = kTraceShift<D>;
   const int2* kp = reinterpret_cast<const int2*>(T.k + (size_t)j * W * (G::NV / 2) * 32);
   long long main = 0, mid = 0;
 #pragma unroll
@@ -432,39 +439,48 @@ __device__ __forceinline__ long long trace_term(const Terms<D, W>& T, const Tm<D
     mid += (long long)xi1 * q.x;
     mid += (long long)xi0 * q.y;
   }
-  long long t = main + (mid >> 32);
+  const long long sum = main + (mid >> 32);
+  Trace t;
+  t.hi = sum >> PS;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  // the lanes' low parts added before they are rounded: rounded one by one they
-  // cost gradients much smaller than |X| |K| three bits
-  const uint32_t lo = __reduce_add_sync(0xffffffffu, (uint32_t)mid >> 8);
-  return (t << 3) + ((lo + (1u << 20)) >> 21);
+  for (int o = 16; o > 0; o >>= 1) t.hi += __shfl_xor_sync(0xffffffffu, t.hi, o);
+  t.lo = __reduce_add_sync(0xffffffffu, ((uint32_t)sum & ((1u << PS) - 1)) << (24 - PS) | (uint32_t)mid >> (8 + PS));
+  return t;
 }
 
 constexpr int kGradBits2 = 2 * 56 + 1;
 constexpr unsigned long long kTodo = 0x7ff8dead00000001ull;  // a slice left to k_fx_grad_norm (a NaN no sum produces)
 
 template <int D> constexpr int kTraces = D >= 32 ? kMaxTerms32 + 1 : kMaxTerms;
-template <int D, int PLANE_SETS, int MAX_TEAMS> struct GradCfg {
+// Digits of R_k and V_k in the gradient's product: all, but seven at D = 32,
+// where two teams of eight beside seven terms pass the shared memory.
+template <int D> constexpr int kPrefixDigits = D >= 32 ? kSlices : kFullSlices;
+template <int D, int PLANE_BYTES, int MAX_TEAMS> struct GradCfg {
   static constexpr int W = kWarps<D>;
   static constexpr int TEAMS = MAX_TEAMS;
-  static constexpr int TRACES = W > 1 ? W * kTraces<D> * 8 : 0;  // the warps' traces
-  static constexpr int TEAM_BYTES = PLANE_SETS * Geo<D, W>::PLANES + kRed + TRACES;
+  static constexpr int TRACES = W > 1 ? W * kTraces<D> * 12 : 0;  // the warps' traces, hi and lo
+  static constexpr int TEAM_BYTES = PLANE_BYTES + kRed + TRACES;
+  static_assert(TEAM_BYTES % 16 == 0, "teams' planes are 16-byte aligned");
 };
-template <int D> using SeriesCfg = GradCfg<D, 2, (D >= 32 ? 2 : D >= 16 ? 10 : 12)>;
-template <int D> using NormCfg = GradCfg<D, 4, (D >= 32 ? 1 : D >= 16 ? 7 : 12)>;
+template <int D> constexpr int kPrefixPlane = kPrefixDigits<D> * 2 * Geo<D, kWarps<D>>::PLANE;  // bytes of one factor
+template <int D> using SeriesCfg = GradCfg<D, 2 * kPrefixPlane<D>, (D >= 32 ? 2 : D >= 16 ? 10 : 12)>;
+template <int D> using NormCfg = GradCfg<D, 4 * Geo<D, kWarps<D>>::PLANES, (D >= 32 ? 1 : D >= 16 ? 7 : 12)>;
 
-// g_jk = cds {Re, Im} Tr(X C_j), X 2^(E - 56) the team's: integer traces, lane
+// g_jk = cds {Re, Im} Tr(X C_j), X 2^(E - 58) the team's: integer traces, lane
 // j keeps control j's.  `traces` is free again after the team's next sync.
 template <int D, int W>
 __device__ __forceinline__ void put_traces(const Terms<D, W>& T, const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w,
                                            int m, int k, const long long (&x)[Geo<D, W>::NV], int E, long long* traces) {
-  long long keep = 0;
+  uint32_t* low = reinterpret_cast<uint32_t*>(traces + W * kTraces<D>);
+  Trace keep{0, 0};
 #pragma unroll 1
   for (int j = 0; j < p.n_c; ++j) {
-    const long long t = trace_term<D, W>(T, tm, j + 1, p.gen == GEN_HERM ? 1 : 0, x);
+    const Trace t = trace_term<D, W>(T, tm, j + 1, p.gen == GEN_HERM ? 1 : 0, x);
     if constexpr (W > 1) {
-      if (tm.lane == 0) traces[tm.w * kTraces<D> + j] = t;
+      if (tm.lane == 0) {
+        traces[tm.w * kTraces<D> + j] = t.hi;
+        low[tm.w * kTraces<D> + j] = t.lo;
+      }
     }
     if (tm.lane == j) keep = t;
   }
@@ -472,9 +488,14 @@ __device__ __forceinline__ void put_traces(const Terms<D, W>& T, const Tm<D, W>&
   if (tm.w == 0 && tm.lane < p.n_c) {
     if constexpr (W > 1) {
 #pragma unroll
-      for (int i = 1; i < W; ++i) keep += traces[i * kTraces<D> + tm.lane];
+      for (int i = 1; i < W; ++i) {
+        keep.hi += traces[i * kTraces<D> + tm.lane];
+        keep.lo += low[i * kTraces<D> + tm.lane];
+      }
     }
-    w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] = p.dt[k] * p.m_scale[m] * to_double(keep, E + T.e[tm.lane + 1] - 55);
+    const int e = E + T.e[tm.lane + 1] - 54 + kTraceShift<D>;
+    w.Gm[((size_t)m * p.n_t + k) * p.n_c + tm.lane] =
+        p.dt[k] * p.m_scale[m] * (to_double(keep.hi, e) + to_double(keep.lo, e - 24));
   }
 }
 template <int D, int W>
@@ -488,22 +509,24 @@ template <int D, int W> __device__ __forceinline__ longlong2* slot(const Tm<D, W
   return tm.mine(reinterpret_cast<longlong2*>(stack + i * D * D));
 }
 
-// (x, E) <- R_k x, the product before slice k inside its block (the identity at
-// its start); x's digits go to pr, R_k's to pl.  The result is normalised.
+// (x, E) <- R_k x, full, with the product before slice k inside its block (the
+// identity at its start); x's digits go to pr, R_k's to pl.
 template <int D, int W>
 __device__ __forceinline__ void times_prefix(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m, int k, int len,
                                              uint32_t pl, uint32_t pr, long long (&x)[Geo<D, W>::NV], int& E) {
   if (k % len == 0) return;
+  constexpr int S = kPrefixDigits<D>;
   long long r[Geo<D, W>::NV];
   get_ints<Geo<D, W>::NV>(slot(tm, w.P, (size_t)m * p.n_t + k), r);
-  const int ER = unpack<D, W>(r);
+  const int ER = unpack(r);
   tm.sync();  // the last slice's products have read their planes
-  store_planes<D, W>(tm, pr, x, kSlices);
-  store_planes<D, W>(tm, pl, r, kSlices);
+  store_full<D, W, S>(tm, pr, x);
+  store_full<D, W, S>(tm, pl, r);
   tm.sync();
-  mul_fixed<D, W, kChainLevels>(tm, pl, pr, x);
-  const int e = normalize<D, W>(tm, x, E + ER);
-  E = max(E, ER) == kNotFinite ? kNotFinite : e;
+  const bool bad = max(E, ER) == kNotFinite;
+  E += ER;
+  mul_full<D, W, S>(tm, pl, pr, x, E);
+  if (bad) E = kNotFinite;
 }
 
 // The gradient of gate targets in any mode, and of exact state targets without
@@ -537,10 +560,10 @@ k_fx_grad(ProbDev p, WorkDev w, int run, int len) {
   T.k = reinterpret_cast<int4*>(smem_raw);
   T.e = reinterpret_cast<int*>(smem_raw + (size_t)T.n * G::INTS);
   unsigned char* mine = smem_raw + Terms<D, W>::bytes(T.n) + (size_t)team * C::TEAM_BYTES;
-  const uint32_t pa = smem_u32(mine), pd = pa + G::PLANES;
+  const uint32_t pa = smem_u32(mine), pd = pa + kPrefixPlane<D>;
   const Tm<D, W> tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
-                    reinterpret_cast<uint32_t*>(mine + 2 * G::PLANES)};
-  long long* traces = reinterpret_cast<long long*>(mine + 2 * G::PLANES + kRed);
+                    reinterpret_cast<uint32_t*>(mine + 2 * kPrefixPlane<D>)};
+  long long* traces = reinterpret_cast<long long*>(mine + 2 * kPrefixPlane<D> + kRed);
   for (int j = team; j < p.n_c; j += nt) {
     double x[NV];
     load_mat<D, W>(tm, p.ctrls + (size_t)j * D * D, x);
@@ -560,41 +583,40 @@ k_fx_grad(ProbDev p, WorkDev w, int run, int len) {
 #pragma unroll 1
     for (int k = k0 + team; k < k1; k += nt) {
       long long x[NV];
-      int E;  // N (exact) or M = x 2^(E - 56)
+      int E;  // N (exact) or M = x 2^(E - 64)
       if (p.target == TGT_GATE) {
         // slot k holds V_k U_k = Lambda_{k-1} up to the block's prefix; V_k is
         // the next slice's, or W_b at the end of the block
         if (p.grad_mode != GRAD_REF_MR) get_ints<NV>(slot(tm, w.U, (size_t)m * p.n_t + k), x);
         else if ((k + 1) % len != 0 && k + 1 < p.n_t) get_ints<NV>(slot(tm, w.U, (size_t)m * p.n_t + k + 1), x);
         else get_ints<NV>(slot(tm, w.P, (size_t)m * p.n_t + k / len * len), x);
-        E = unpack<D, W>(x);
+        E = unpack(x);
         times_prefix<D, W>(tm, p, w, m, k, len, pa, pd, x, E);
       } else {
         double d[NV];
         load_M<D, W>(tm, p, w, m, k, k, d);
         const int EXd = max_exponent<D, W>(tm, d);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) x[v] = from_double(d[v], EXd, 2);
+        for (int v = 0; v < NV; ++v) x[v] = from_double(d[v], EXd, 10);
         E = EXd == 0x7ff ? kNotFinite : EXd - 1021;
       }
       tm.sync();
       if (p.grad_mode == GRAD_EXACT && E != kNotFinite) {
-        long long sum[NV], r[NV];
+        long long r[NV];
         const int EA = assemble<D, W>(T, p, w.u, m, k, tm, r);
         const float l2 = log2_norm1<D, W>(tm, r, EA);
         bool todo = l2 > 1.3f;
         if (EA > kNever / 2) E = kNotFinite;
         else if (!todo) {
-          const int EB = normalize<D, W, true>(tm, r, EA - 2);
+          const int EB = normalize<D, W, true>(tm, r, EA - 6);
           store_planes<D, W>(tm, pa, r, kSlices);
-          tm.sync();  // the maxima are read
-          const int EN = normalize<D, W, true>(tm, x, E), fr = EN + 3;
+          const int EN = E;
 #pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            r[v] = x[v];
-            sum[v] = x[v] << 1;  // 60 fractional bits in frame EN + 3
-          }
-          int Er = EN;
+          for (int v = 0; v < NV; ++v) r[v] = shift_round(x[v], 8);  // 56 fractional bits, below 2^55
+          // x becomes the sum, 60 fractional bits in frame EN + h: h = 0 where
+          // the first term is below half of N (so the entries of N keep 2^-60 of
+          // the largest's scale), else 3
+          int Er = EN, h = -4;  // (no term: x as it is)
           float size = 1.f;  // of the terms, in units of N: below 7 the sum stays inside its frame
           todo = true;
 #pragma unroll 1
@@ -610,16 +632,20 @@ k_fx_grad(ProbDev p, WorkDev w, int run, int len) {
             tm.sync();
             commutator<D, W>(tm, pa, pd, min(lev, kMaxLevels), r);
             Er = normalize<D, W, true>(tm, r, EB + Er);
-            size += exp2f((float)(Er + cf.exp - EN));
-            if (size > 7.f) break;
-            const Scaled sc(cf, Er, fr, 60);
+            const int et = Er + cf.exp - EN;  // the term is below 2^(et - 1) N's scale
+            if (n == 1) {
+              h = et <= -1 ? 0 : 3;
 #pragma unroll
-            for (int v = 0; v < NV; ++v) sum[v] = sc(r[v] << 6, sum[v]);
+              for (int v = 0; v < NV; ++v) x[v] = shift_round(x[v], h + 4);
+            }
+            size += exp2f((float)et);
+            if (size > 7.f || et > h) break;
+            const Scaled sc(cf, Er, EN + h, 60);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) x[v] = sc(r[v] << 6, x[v]);
           }
           tm.sync();
-          E = normalize<D, W>(tm, sum, fr - 4);
-#pragma unroll
-          for (int v = 0; v < NV; ++v) x[v] = sum[v];
+          E = normalize_full<D, W>(tm, x, EN + h + 4);
         }
         if (todo && E != kNotFinite) {
           put_grad_value<D, W>(tm, p, w, m, k, kTodo);
@@ -631,6 +657,8 @@ k_fx_grad(ProbDev p, WorkDev w, int run, int len) {
         put_grad_value<D, W>(tm, p, w, m, k, 0x7ff8000000000000ull);
         tm.sync();
       } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) x[v] = shift_round(x[v], 6);
         put_traces<D, W>(T, tm, p, w, m, k, x, E, traces);
         tm.sync();  // the maxima and the traces are read
       }
@@ -688,8 +716,11 @@ k_fx_grad_norm(ProbDev p, WorkDev w, int run, int len) {
       if (p.target == TGT_GATE) {
         if ((k + 1) % len != 0 && k + 1 < p.n_t) get_ints<NV>(slot(tm, w.U, (size_t)m * p.n_t + k + 1), db);
         else get_ints<NV>(slot(tm, w.P, (size_t)m * p.n_t + k / len * len), db);
-        EM = unpack<D, W>(db);
+        EM = unpack(db);
+        // two full factors in the four sets of planes
         times_prefix<D, W>(tm, p, w, m, k, len, px, py, db, EM);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) db[v] = shift_round(db[v], 8);
       } else {
         double x[NV];
         load_M<D, W>(tm, p, w, m, k, k + 1, x);
@@ -712,7 +743,7 @@ k_fx_grad_norm(ProbDev p, WorkDev w, int run, int len) {
       const float nu2 = l2 - (float)s;
       const int lx = min(0, 2 * (int)ceilf(nu2));
       const int g = nu2 <= -1.33f ? 1 : 3;
-      const int EB = normalize<D, W>(tm, b, EA - 2 - s);
+      const int EB = normalize<D, W>(tm, b, EA - 6 - s);
       tm.sync();
       store_planes<D, W>(tm, py, b, kSlices);
       store_planes<D, W>(tm, pdy, db, kSlices);
@@ -809,6 +840,8 @@ k_fx_grad_norm(ProbDev p, WorkDev w, int run, int len) {
           }
         }
       }
+#pragma unroll
+      for (int v = 0; v < NV; ++v) q[v] <<= 2;
       put_traces<D, W>(T, tm, p, w, m, k, q, EdY, traces);
       tm.sync();  // the maxima and the traces are read
     }
@@ -833,87 +866,106 @@ k_fx_grad_norm(ProbDev p, WorkDev w, int run, int len) {
 // 0.82 here; 32 members of 500 slices 2.1 + 4.4 ms, 0.14 + 0.09.
 template <int D> struct ChainCfg {
   static constexpr int W = kWarps<D>;
-  static constexpr int TEAMS = D >= 32 ? 1 : D >= 16 ? 4 : 8;  // (member, block) chains of a CTA
-  static constexpr int COMBINE = D >= 32 ? 2 : TEAMS;          // teams of a member's combine
-  static constexpr int TEAM_BYTES = 2 * Geo<D, W>::PLANES + kRed;
-  // T_b and Lambda_b of a member in shared memory
+  static constexpr int TEAMS = D >= 32 ? 1 : 4;                // (member, block) chains of a CTA, mixed path
+  // of the full chains: one at D = 16, where a CTA of four held 174 registers a
+  // thread and left an SM with four chains (231 members of 1000 slices: forward
+  // and backward 0.98 + 1.14 ms; eight chains, alone or in fours, 0.75 + 0.75
+  // and 0.79 + 0.76)
+  static constexpr int FULL_TEAMS = D >= 16 ? 1 : 8;
+  static constexpr int PER_SM = D >= 32 ? 3 : D >= 16 ? 8 : 24;  // full chains an SM holds
+  static constexpr int MIN_CTAS = D >= 32 ? 2 : D >= 16 ? 8 : 3;
+  static constexpr int COMBINE = D >= 32 ? 2 : D >= 16 ? 4 : 8;  // teams of a member's combine
+  static constexpr int TEAM_BYTES = 2 * Geo<D, W>::PLANES + kRed;            // the mixed path's chains
+  static constexpr int FULL_BYTES = 2 * Geo<D, W>::PLANES_FULL + kRed;
+  // T_b (b > 0) and Lambda_b of a member in shared memory
   static constexpr int MAX_BLOCKS = D >= 32 ? 3 : D >= 16 ? 20 : 96;
 };
 
-template <int D, int W> struct ChainTeam {
+template <int D, int W, int S> struct ChainTeam {
+  static constexpr int SET = S * 2 * Geo<D, W>::PLANE;
   Tm<D, W> tm;
   uint32_t pl, pr;  // planes of the left and the right factor
   __device__ __forceinline__ ChainTeam(unsigned char* smem, int team)
-      : tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team,
-           reinterpret_cast<uint32_t*>(smem + 2 * Geo<D, W>::PLANES)},
-        pl(smem_u32(smem)), pr(pl + Geo<D, W>::PLANES) {}
-  // (r, E) <- left (r, E); an operand that is not finite stays so
-  template <bool R_IS_LEFT, int LEVELS = kChainLevels>
+      : tm{(int)(threadIdx.x & 31), (int)(threadIdx.x >> 5) % W, 1 + team, reinterpret_cast<uint32_t*>(smem + 2 * SET)},
+        pl(smem_u32(smem)), pr(pl + SET) {}
+  // (r, E) <- left (r, E); an operand that is not finite stays so.  Full
+  // matrices with S = 8, else 56 fractional bits and LEVELS levels.
+  template <bool R_IS_LEFT, int LEVELS = kMaxLevels>
   __device__ __forceinline__ void step(long long (&r)[Geo<D, W>::NV], int& E, const long long (&x)[Geo<D, W>::NV], int Ex) {
+    const uint32_t at_r = R_IS_LEFT ? pl : pr, at_x = R_IS_LEFT ? pr : pl;
+    const bool bad = max(E, Ex) == kNotFinite;
     tm.sync();  // the last product has read its planes
-    store_planes<D, W>(tm, R_IS_LEFT ? pl : pr, r, kSlices);
-    store_planes<D, W>(tm, R_IS_LEFT ? pr : pl, x, kSlices);
-    tm.sync();
-    mul_fixed<D, W, LEVELS>(tm, pl, pr, r);
-    const int e = normalize<D, W>(tm, r, E + Ex);
-    E = max(E, Ex) == kNotFinite ? kNotFinite : e;
+    if constexpr (S == kFullSlices) {
+      store_full<D, W, S>(tm, at_r, r);
+      store_full<D, W, S>(tm, at_x, x);
+      tm.sync();
+      E += Ex;
+      mul_full<D, W, S, LEVELS>(tm, pl, pr, r, E);
+    } else {
+      store_planes<D, W>(tm, at_r, r, kSlices);
+      store_planes<D, W>(tm, at_x, x, kSlices);
+      tm.sync();
+      mul_fixed<D, W, LEVELS>(tm, pl, pr, r);
+      E = normalize<D, W>(tm, r, E + Ex);
+    }
+    if (bad) E = kNotFinite;
   }
 };
 
 template <int D>
-__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS)
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::FULL_TEAMS, ChainCfg<D>::MIN_CTAS)
 k_fx_chain_fwd(ProbDev p, WorkDev w, int blocks, int len, int store) {
   using C = ChainCfg<D>;
   constexpr int W = C::W, NV = Geo<D, W>::NV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int team = threadIdx.x / (32 * W);
-  ChainTeam<D, W> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
-  const long item = (long)blockIdx.x * C::TEAMS + team;
+  ChainTeam<D, W, kFullSlices> ct(smem_raw + (size_t)team * C::FULL_BYTES, team);
+  const long item = (long)blockIdx.x * C::FULL_TEAMS + team;
   if (item >= (long)p.n_members * blocks) return;  // whole teams
   const int m = (int)(item / blocks), k0 = (int)(item % blocks) * len, k1 = min(p.n_t, k0 + len);
   const size_t base = (size_t)m * p.n_t;
   long long r[NV], x[NV];
   get_ints<NV>(slot(ct.tm, w.U, base + k0), r);
-  int E = unpack<D, W>(r);
+  int E = unpack(r);
   if (k0 + 1 < k1) get_ints<NV>(slot(ct.tm, w.U, base + k0 + 1), x);
 #pragma unroll 1
   for (int k = k0 + 1; k < k1; ++k) {
     long long u[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) u[v] = x[v];
-    const int Eu = unpack<D, W>(u);
+    const int Eu = unpack(u);
     if (k + 1 < k1) get_ints<NV>(slot(ct.tm, w.U, base + k + 1), x);  // while this product runs
-    if (store) put_packed<D, W>(slot(ct.tm, w.P, base + k), r, E);
+    if (store) put_packed<D, W>(ct.tm, slot(ct.tm, w.P, base + k), r, E);
     ct.template step<false>(r, E, u, Eu);
   }
-  put_packed<D, W>(slot(ct.tm, store ? w.P : w.U, base + k0), r, E);
+  put_packed<D, W>(ct.tm, slot(ct.tm, store ? w.P : w.U, base + k0), r, E);
 }
 
 template <int D>
-__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS)
+__global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::FULL_TEAMS, ChainCfg<D>::MIN_CTAS)
 k_fx_chain_bwd(ProbDev p, WorkDev w, int blocks, int len) {
   using C = ChainCfg<D>;
   constexpr int W = C::W, NV = Geo<D, W>::NV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int team = threadIdx.x / (32 * W);
-  ChainTeam<D, W> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
-  const long item = (long)blockIdx.x * C::TEAMS + team;
+  ChainTeam<D, W, kFullSlices> ct(smem_raw + (size_t)team * C::FULL_BYTES, team);
+  const long item = (long)blockIdx.x * C::FULL_TEAMS + team;
   if (item >= (long)p.n_members * blocks) return;
   const int m = (int)(item / blocks), k0 = (int)(item % blocks) * len, k1 = min(p.n_t, k0 + len);
   const size_t base = (size_t)m * p.n_t;
   long long r[NV], x[NV];
   get_ints<NV>(slot(ct.tm, w.P, base + k0), r);
-  int E = unpack<D, W>(r);
+  int E = unpack(r);
   get_ints<NV>(slot(ct.tm, w.U, base + k1 - 1), x);
 #pragma unroll 1
   for (int k = k1 - 1; k >= k0; --k) {
     long long u[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) u[v] = x[v];
-    const int Eu = unpack<D, W>(u);
+    const int Eu = unpack(u);
     if (k > k0) get_ints<NV>(slot(ct.tm, w.U, base + k - 1), x);
     ct.template step<true>(r, E, u, Eu);
-    put_packed<D, W>(slot(ct.tm, w.U, base + k), r, E);
+    put_packed<D, W>(ct.tm, slot(ct.tm, w.U, base + k), r, E);
   }
 }
 
@@ -945,7 +997,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS, 2) k
   using G = Geo<D, W>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int team = threadIdx.x / (32 * W);
-  ChainTeam<D, W> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
+  ChainTeam<D, W, kSlices> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
   const Tm<D, W>& tm = ct.tm;
   const long item = (long)blockIdx.x * C::TEAMS + team;
   if (item >= (long)p.n_members * w.pit_blocks) return;  // whole teams
@@ -989,39 +1041,40 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W * ChainCfg<D>::TEAMS, 2) k
   store_df<D, W>(tm, w.pit_tot + (size_t)item * D * D, r, E == kNotFinite ? 0x7ff : E - kFrac);
 }
 
-// x -> kappa x, normalised: each part times a double, in a common frame;
-// returns its exponent.
+// x -> kappa x, both full: each part times a double, in a common frame; returns
+// its exponent.
 template <int D, int W>
 __device__ __forceinline__ int scale_complex(const Tm<D, W>& tm, long long (&x)[Geo<D, W>::NV], int E, double2 kap) {
   constexpr int H = Geo<D, W>::NV / 2;
   const int ex = max((int)((uint32_t)__double2hiint(kap.x) >> 20 & 0x7ff), (int)((uint32_t)__double2hiint(kap.y) >> 20 & 0x7ff));
   if (ex == 0x7ff) return kNotFinite;
-  // parts below 2^(ex - 1022) in 61 fractional bits
+  // parts below 2^(ex - 1022) in 61 fractional bits, x in 61
   const long long a = from_double(kap.x, ex, 8), b = from_double(kap.y, ex, 8);
   const int a0 = (int)a, a1 = (int)((a + 0x80000000ll) >> 32), b0 = (int)b, b1 = (int)((b + 0x80000000ll) >> 32);
 #pragma unroll
   for (int v = 0; v < H; ++v) {
-    const long long re = x[v] << 5, im = x[H + v] << 5;
+    const long long re = shift_round(x[v], 3), im = shift_round(x[H + v], 3);
     const int r0 = (int)re, r1 = (int)((re + 0x80000000ll) >> 32);
     const int i0 = (int)im, i1 = (int)((im + 0x80000000ll) >> 32);
-    const long long mr = 0x80000000ll + (long long)r1 * a0 + (long long)r0 * a1 - (long long)i1 * b0 - (long long)i0 * b1;
-    const long long mi = 0x80000000ll + (long long)r1 * b0 + (long long)r0 * b1 + (long long)i1 * a0 + (long long)i0 * a1;
-    x[v] = (long long)r1 * a1 - (long long)i1 * b1 + (mr >> 32);
-    x[H + v] = (long long)r1 * b1 + (long long)i1 * a1 + (mi >> 32);
+    const long long mr = (long long)r1 * a0 + (long long)r0 * a1 - (long long)i1 * b0 - (long long)i0 * b1;
+    const long long mi = (long long)r1 * b0 + (long long)r0 * b1 + (long long)i1 * a0 + (long long)i0 * a1;
+    x[v] = (((long long)r1 * a1 - (long long)i1 * b1) << 3) + shift_round(mr, 29);
+    x[H + v] = (((long long)r1 * b1 + (long long)i1 * a1) << 3) + shift_round(mi, 29);
   }
-  const int e = normalize<D, W>(tm, x, E + ex - 1024, 1);
+  const int e = normalize_full<D, W>(tm, x, E + ex - 1024 + 5, 1);
   return E == kNotFinite ? kNotFinite : e;
 }
 
-template <int D, int W>
+// U_total of a member, r with FRAC fractional bits.
+template <int D, int W, int FRAC>
 __device__ __forceinline__ void put_total(const Tm<D, W>& tm, const WorkDev& w, int m, const long long (&r)[Geo<D, W>::NV], int E) {
   double2* Ut = w.Utot + (size_t)m * D * D;
   if (E == kNotFinite) store_nan<D, W>(tm, Ut);
-  else store_mat<D, W>(tm, Ut, r, E - kFrac);
+  else store_mat<D, W>(tm, Ut, r, E - FRAC);
 }
 // z = Tr(T' U) / D, f and the weighted kappa of a member from U, the team's
-// (r, E); the team is threads 0 .. 32 W - 1 of the block.
-template <int D, int W>
+// (r, E), FRAC fractional bits; the team is threads 0 .. 32 W - 1 of the block.
+template <int D, int W, int FRAC>
 __device__ __forceinline__ void finish_gate(const Tm<D, W>& tm, const ProbDev& p, const WorkDev& w, int m,
                                             const long long (&r)[Geo<D, W>::NV], int E, double2* s_red, double2* s_kap) {
   using G = Geo<D, W>;
@@ -1029,7 +1082,7 @@ __device__ __forceinline__ void finish_gate(const Tm<D, W>& tm, const ProbDev& p
   double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
   for (int b = 0; b < NV / 2; ++b) {
-    double2 v = make_double2(to_double(r[b], E - kFrac), to_double(r[NV / 2 + b], E - kFrac));
+    double2 v = make_double2(to_double(r[b], E - FRAC), to_double(r[NV / 2 + b], E - FRAC));
     if (E == kNotFinite) v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
     acc = cmac_cj(acc, p.target_op[tm.row(b / 2 % G::NI) + D * tm.col(b / 2 / G::NI, b % 2)], v);
   }
@@ -1066,7 +1119,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W) k_fx_combine_df(ProbDev p
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double2 s_red[32 * W];
   __shared__ double2 s_kap;
-  ChainTeam<D, W> ct(smem_raw, 0);
+  ChainTeam<D, W, kSlices> ct(smem_raw, 0);
   const Tm<D, W>& tm = ct.tm;
   const int m = blockIdx.x;
   int at[H];
@@ -1102,7 +1155,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W) k_fx_combine_df(ProbDev p
       ct.template step<false, kPrefixLevels>(r, E, u, Eu);
     }
   }
-  put_total<D, W>(tm, w, m, r, E);
+  put_total<D, W, kFrac>(tm, w, m, r, E);
   if (p.gen == GEN_HERM && E != kNotFinite) {
     // one Newton-Schulz step of the polar decomposition, U (3I - U'U) / 2,
     // before the overlap (k_refine_unitary_mx, which takes 10 us at D = 16
@@ -1123,7 +1176,7 @@ __global__ void __launch_bounds__(32 * ChainCfg<D>::W) k_fx_combine_df(ProbDev p
     mul_fixed<D, W, kMaxLevels>(tm, ct.pl, ct.pr, r);
     E += 2;  // frame 3, halved
   }
-  finish_gate<D, W>(tm, p, w, m, r, E, s_red, &s_kap);
+  finish_gate<D, W, kFrac>(tm, p, w, m, r, E, s_red, &s_kap);
 }
 
 template <int D>
@@ -1137,26 +1190,26 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
   __shared__ double2 s_red[32 * W];
   __shared__ double2 s_kap;
   const int team = threadIdx.x / (32 * W);
-  ChainTeam<D, W> ct(smem_raw + (size_t)team * C::TEAM_BYTES, team);
+  ChainTeam<D, W, kFullSlices> ct(smem_raw + (size_t)team * C::FULL_BYTES, team);
   const Tm<D, W>& tm = ct.tm;
-  longlong2* Ts = reinterpret_cast<longlong2*>(smem_raw + (size_t)TEAMS * C::TEAM_BYTES);
-  longlong2* Ls = Ts + (size_t)blocks * (G::INTS / 16);
+  longlong2* Ls = reinterpret_cast<longlong2*>(smem_raw + (size_t)TEAMS * C::FULL_BYTES);
+  longlong2* Ts = Ls + (size_t)(blocks - 1) * (G::INTS / 16);  // T_b at b, b > 0: after Lambda's last
   const int m = blockIdx.x;
   const size_t base = (size_t)m * p.n_t;
   double2* tot = want_grad ? w.P : w.U;  // where k_fx_chain_fwd left the block products
   long long r[NV], x[NV];
   if (team == 0) {  // T_1 = Tot_0, T_{b+1} = Tot_b T_b
     get_ints<NV>(slot(tm, tot, base), r);
-    int E = unpack<D, W>(r);
+    int E = unpack(r);
 #pragma unroll 1
     for (int b = 1; b < blocks; ++b) {
-      if (want_grad) put_packed<D, W>(tm.mine(Ts + (size_t)b * (G::INTS / 16)), r, E);
+      if (want_grad) put_packed<D, W>(tm, tm.mine(Ts + (size_t)b * (G::INTS / 16)), r, E);
       get_ints<NV>(slot(tm, tot, base + (size_t)b * len), x);
-      const int Ex = unpack<D, W>(x);
+      const int Ex = unpack(x);
       ct.template step<false>(r, E, x, Ex);
     }
-    put_total<D, W>(tm, w, m, r, E);
-    finish_gate<D, W>(tm, p, w, m, r, E, s_red, &s_kap);
+    put_total<D, W, 64>(tm, w, m, r, E);
+    finish_gate<D, W, 64>(tm, p, w, m, r, E, s_red, &s_kap);
   } else if (team == 1 && want_grad) {  // Lambda_B = T', Lambda_{b-1} = Lambda_b Tot_b
     double t[NV];
 #pragma unroll
@@ -1167,14 +1220,14 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
     }
     const int EX = max_exponent<D, W>(tm, t);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) r[v] = from_double(t[v], EX, 2);
-    int E = EX - 1021;
+    for (int v = 0; v < NV; ++v) r[v] = from_double(t[v], EX, 9);
+    int E = EX - 1020;
 #pragma unroll 1
     for (int b = blocks - 1;; --b) {
-      put_packed<D, W>(tm.mine(Ls + (size_t)b * (G::INTS / 16)), r, E);
+      put_packed<D, W>(tm, tm.mine(Ls + (size_t)b * (G::INTS / 16)), r, E);
       if (b == 0) break;
       get_ints<NV>(slot(tm, tot, base + (size_t)b * len), x);
-      const int Ex = unpack<D, W>(x);
+      const int Ex = unpack(x);
       ct.template step<true>(r, E, x, Ex);
     }
   }
@@ -1183,14 +1236,14 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
   const double2 kap = s_kap;
   for (int b = team; b < blocks; b += TEAMS) {  // W_b = kappa T_b Lambda_b
     get_ints<NV>(tm.mine(Ls + (size_t)b * (G::INTS / 16)), r);
-    int E = unpack<D, W>(r);
+    int E = unpack(r);
     if (b > 0) {
       get_ints<NV>(tm.mine(Ts + (size_t)b * (G::INTS / 16)), x);
-      const int Ex = unpack<D, W>(x);
+      const int Ex = unpack(x);
       ct.template step<false>(r, E, x, Ex);
     }
     E = scale_complex<D, W>(tm, r, E, kap);
-    put_packed<D, W>(slot(tm, w.P, base + (size_t)b * len), r, E);
+    put_packed<D, W>(tm, slot(tm, w.P, base + (size_t)b * len), r, E);
   }
 }
 
@@ -1735,10 +1788,10 @@ static cudaError_t launch_slices(void (*kernel)(ProbDev, WorkDev, int, A...), co
 
 // Blocks of the gate chains.  Chains run in two dependent passes of `len`
 // products with one of `blocks` between: more blocks than sqrt(2 n_t) only
-// lengthen the sum, and more (member, block) chains than the SMs hold (about
-// 3 of 57 KB at D = 32, 10 of 14 KB at D = 16, 24 of 4 KB at D = 8) run as a second wave.
+// lengthen the sum, and more (member, block) chains than the SMs hold (3 of 66 KB
+// at D = 32, 8 of 16 KB at D = 16, 24 of 4 KB at D = 8) run as a second wave.
 template <int D> static void chain_shape(const ProbDev& p, int num_sms, int* blocks, int* len) {
-  const long chains = (long)num_sms * (D >= 32 ? 3 : D >= 16 ? 10 : 24);
+  const long chains = (long)num_sms * ChainCfg<D>::PER_SM;
   long b = chains / p.n_members;
   long most = 1;
   while (most < ChainCfg<D>::MAX_BLOCKS && (most + 1) * (most + 1) <= 2L * p.n_t) ++most;
@@ -1752,12 +1805,12 @@ template <int D> static cudaError_t do_chain_fwd(const ProbDev& p, const WorkDev
   using C = ChainCfg<D>;
   int blocks, len;
   chain_shape<D>(p, li.num_sms, &blocks, &len);
-  const size_t smem = (size_t)C::TEAMS * C::TEAM_BYTES;
-  const int threads = 32 * C::W * C::TEAMS;
+  const size_t smem = (size_t)C::FULL_TEAMS * C::FULL_BYTES;
+  const int threads = 32 * C::W * C::FULL_TEAMS;
   set_smem_once((const void*)k_fx_chain_fwd<D>, smem);
   const long items = (long)p.n_members * blocks;
-  k_fx_chain_fwd<D><<<(int)((items + C::TEAMS - 1) / C::TEAMS), threads, smem, li.stream>>>(p, w, blocks, len, store ? 1 : 0);
-  const size_t smem2 = (size_t)C::COMBINE * C::TEAM_BYTES + (store ? (size_t)2 * blocks * Geo<D, C::W>::INTS : 0);
+  k_fx_chain_fwd<D><<<(int)((items + C::FULL_TEAMS - 1) / C::FULL_TEAMS), threads, smem, li.stream>>>(p, w, blocks, len, store ? 1 : 0);
+  const size_t smem2 = (size_t)C::COMBINE * C::FULL_BYTES + (store ? (size_t)(2 * blocks - 1) * Geo<D, C::W>::INTS : 0);
   set_smem_once((const void*)k_fx_chain_combine<D>, smem2);
   k_fx_chain_combine<D><<<p.n_members, 32 * C::W * C::COMBINE, smem2, li.stream>>>(p, w, blocks, len, store ? 1 : 0);
   *li.launches += 2;
@@ -1768,10 +1821,10 @@ template <int D> static cudaError_t do_chain_bwd(const ProbDev& p, const WorkDev
   using C = ChainCfg<D>;
   int blocks, len;
   chain_shape<D>(p, li.num_sms, &blocks, &len);
-  const size_t smem = (size_t)C::TEAMS * C::TEAM_BYTES;
+  const size_t smem = (size_t)C::FULL_TEAMS * C::FULL_BYTES;
   set_smem_once((const void*)k_fx_chain_bwd<D>, smem);
   const long items = (long)p.n_members * blocks;
-  k_fx_chain_bwd<D><<<(int)((items + C::TEAMS - 1) / C::TEAMS), 32 * C::W * C::TEAMS, smem, li.stream>>>(p, w, blocks, len);
+  k_fx_chain_bwd<D><<<(int)((items + C::FULL_TEAMS - 1) / C::FULL_TEAMS), 32 * C::W * C::FULL_TEAMS, smem, li.stream>>>(p, w, blocks, len);
   ++*li.launches;
   return cudaGetLastError();
 }

@@ -33,6 +33,7 @@ namespace fx {
 
 constexpr int kFrac = 56;      // fractional bits of a normalised matrix
 constexpr int kSlices = 7;     // 8-bit digits of a factor
+constexpr int kFullSlices = 8; // digits of a full matrix (below)
 constexpr int kMaxLevels = 8;  // levels 0..7 of digit pairs
 
 // A team of W warps owns one D x D matrix; a warp owns RT-th rows x NTW 8-column
@@ -53,6 +54,7 @@ template <int D, int W> struct Geo {
   static constexpr int KT = RT;                        // 16-deep steps of a product
   static constexpr int PLANE = D * D * 2;              // bytes of one digit plane
   static constexpr int PLANES = kSlices * 2 * PLANE;   // digit planes of a matrix
+  static constexpr int PLANES_FULL = kFullSlices * 2 * PLANE;
   static constexpr int INTS = 2 * D * D * 8;           // 64-bit values of a matrix
   static_assert(NV * 32 * W == 2 * D * D, "a team covers the matrix");
 };
@@ -205,7 +207,7 @@ constexpr uint32_t kPairBias = (0x4B400000u << 8) + 0x4B400000u;  // two magic s
 // left digit, and the right digit of level L + 1 is the one level L uses next.
 // All digit loops are unrolled: as rolled loops the products of the d = 8 and
 // d = 16 chains took 1.5 and 1.25 times as long.
-template <int D, int W, int L, bool TWO, class LeftT = Left<D, W>>
+template <int D, int W, int L, bool TWO, class LeftT = Left<D, W>, int S = kSlices>
 __device__ __forceinline__ void level_pair(uint32_t la, uint32_t rb, uint32_t (&t)[Geo<D, W>::NV]) {
   using G = Geo<D, W>;
   constexpr int NV = G::NV;
@@ -217,14 +219,14 @@ __device__ __forceinline__ void level_pair(uint32_t la, uint32_t rb, uint32_t (&
     for (int v = 0; v < NV; ++v) a0[v] = a1[v] = kMagic;
     const uint32_t pl = la + kt * LeftT::KSTEP, pr = rb + kt * 2 * 128;
     Right<D, W> b[2];
-    if (TWO && L + 1 < kSlices) b[1].load(pr + (L + 1) * kDigit);
+    if (TWO && L + 1 < S) b[1].load(pr + (L + 1) * kDigit);
 #pragma unroll
-    for (int i = 0; i < kSlices; ++i) {
+    for (int i = 0; i < S; ++i) {
       if (i > L + (TWO ? 1 : 0)) break;
       LeftT a;
       a.load(pl + i * kDigit);
       if (i <= L) b[i & 1].load(pr + (L - i) * kDigit);  // b[(i + 1) & 1] holds B_{L + 1 - i}
-      if (TWO && L + 1 - i < kSlices) mma_pair<D, W>(a1, a, b[(i + 1) & 1]);
+      if (TWO && L + 1 - i < S) mma_pair<D, W>(a1, a, b[(i + 1) & 1]);
       if (i <= L) mma_pair<D, W>(a0, a, b[i & 1]);
     }
 #pragma unroll
@@ -265,6 +267,57 @@ __device__ __forceinline__ void mul_fixed(const Tm<D, W>& tm, uint32_t pa, uint3
 #pragma unroll
   for (int v = 0; v < Geo<D, W>::NV; ++v) r[v] = 0;
   mul_levels<D, W, N, LeftT>(LeftT::at(tm, pa), Right<D, W>::at(tm, pb), r);
+}
+
+// A full matrix: value x 2^(E - 64), |x| < 127/128 2^63, its eight digits the
+// bytes of the 64-bit integer (a digit counts 2^(E - 8 (i + 1)) in either
+// format, so full factors and others mix).  The FP64 gate chains use it: their
+// factors are near the identity or the target, and the generator's trace reads
+// the entries far below the largest, which FP64 keeps to their own 53 bits.
+// With 56 bits under one exponent and products rounded at 2^-56 of the factors'
+// scales, the gradients of two-qubit Lindblad pulses below 100 slices were 2.4
+// times further off than FP64's (geometric mean of 40 draws); see k_fx_grad.
+//
+// Largest |high word| -> shift that brings |x| just below 127/128 2^63.
+__device__ __forceinline__ int full_shift(uint32_t M) {
+  const uint32_t m = M + 1;
+  const int lz = __clz(m);
+  return lz - 1 - ((m << lz) >= 0xFE000000u ? 1 : 0);
+}
+template <int D, int W, int N, class LeftT, int S, int L = (N - 1) & ~1>
+__device__ __forceinline__ void mul_low_levels(uint32_t la, uint32_t rb, long long (&r)[Geo<D, W>::NV]) {
+  if constexpr (L > 0) {
+    uint32_t t[Geo<D, W>::NV];
+    level_pair<D, W, L, (L + 1 < N), LeftT, S>(la, rb, t);
+    join_pair<Geo<D, W>::NV>(r, t, L);
+    mul_low_levels<D, W, N, LeftT, S, L - 2>(la, rb, r);
+  }
+}
+// (x, E) <- A B, full and normalised, from S digits of each factor, E the sum
+// of their exponents.  The levels below the leading pair stay 64 bits wide, t
+// 2^48 + r in units of 2^(E - 72), so nothing is rounded before the shift.
+template <int D, int W, int S, int N = kMaxLevels>
+__device__ __forceinline__ void mul_full(const Tm<D, W>& tm, uint32_t pa, uint32_t pb, long long (&x)[Geo<D, W>::NV], int& E) {
+  constexpr int NV = Geo<D, W>::NV;
+  const uint32_t la = Left<D, W>::at(tm, pa), rb = Right<D, W>::at(tm, pb);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) x[v] = 0;
+  mul_low_levels<D, W, N, Left<D, W>, S>(la, rb, x);
+  uint32_t t[NV];
+  level_pair<D, W, 0, (N > 1), Left<D, W>, S>(la, rb, t);
+  uint32_t M = 0;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    t[v] += (uint32_t)((int)(x[v] >> 32) >> 16);
+    M = max(M, (uint32_t)abs((int)t[v]));
+  }
+  const int sh = full_shift(tm.max(M, 0));  // 0 .. 30
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {  // the 96 bits t, x's low 48, 0 moved up, upper 64 kept
+    const uint32_t mid = (uint32_t)(x[v] >> 16), lo = (uint32_t)x[v] << 16;
+    x[v] = (long long)((unsigned long long)__funnelshift_l(mid, t[v], sh) << 32 | __funnelshift_l(lo, mid, sh));
+  }
+  E = max(E + 8 - sh, -(1 << 20));
 }
 
 // Level pair (L, L + 1) with L and `two` chosen by the data: rolled digit loops
@@ -454,6 +507,53 @@ __device__ __forceinline__ void store_planes(const Tm<D, W>& tm, uint32_t base, 
   }
 }
 
+// r 2^(e - 64) -> full, normalised (r != -2^63); returns its exponent.
+template <int D, int W>
+__device__ __forceinline__ int normalize_full(const Tm<D, W>& tm, long long (&r)[Geo<D, W>::NV], int e, int slot = 0) {
+  constexpr int NV = Geo<D, W>::NV;
+  uint32_t M = 0;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) M = max(M, (uint32_t)abs((int)(r[v] >> 32)));
+  const int sh = full_shift(tm.max(M, slot));
+  if (sh >= 0) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] <<= sh;
+  } else {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] = shift_round(r[v], -sh);
+  }
+  return max(e - sh, -(1 << 20));
+}
+// The leading S digit planes of a full matrix into shared memory.
+template <int D, int W, int S>
+__device__ __forceinline__ void store_full(const Tm<D, W>& tm, uint32_t base, const long long (&x)[Geo<D, W>::NV]) {
+  using G = Geo<D, W>;
+  constexpr int NV = G::NV;
+  uint32_t lo[NV], hi[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {  // balanced digits: 128 in every byte
+    const unsigned long long a = (unsigned long long)x[v] + 0x8080808080808080ull;
+    lo[v] = (uint32_t)a;
+    hi[v] = (uint32_t)(a >> 32);
+  }
+  const uint32_t at = base + (tm.nt0() * (D / 8) + 2 * tm.rt()) * 128 + tm.lane * 4;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const int byte = 7 - s;
+#pragma unroll
+    for (int b = 0; b < NV / 2; ++b) {  // columns 2 t, 2 t + 1 of one 8 x 8 block
+      const int part = b / (NV / 4), nt = b % (NV / 4) / G::NI, i = b % G::NI;
+      const uint32_t wa = byte >= 4 ? hi[2 * b] : lo[2 * b], wb = byte >= 4 ? hi[2 * b + 1] : lo[2 * b + 1];
+      const uint32_t t =  // FP16 1024 + byte
+          (__byte_perm(wa, wb, (unsigned)((byte & 3) | (4 + (byte & 3)) << 8)) & 0x00ff00ffu) | 0x64006400u;
+      uint32_t d;
+      asm("sub.f16x2 %0, %1, %2;" : "=r"(d) : "r"(t), "r"(0x64806480u));  // minus 1024 + 128
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + (2 * s + part) * G::PLANE + (nt * (D / 8) + i) * 128), "r"(d)
+                   : "memory");
+    }
+  }
+}
+
 // 64-bit values of a matrix, lane-private (16-byte accesses; s = tm.mine()).
 template <int NV> __device__ __forceinline__ void put_ints(longlong2* s, const long long (&x)[NV]) {
 #pragma unroll
@@ -596,25 +696,22 @@ __device__ __forceinline__ long long from_float(float f, int EX) {
   return ((long long)m ^ s) - s;
 }
 
-// A normalised matrix in global memory, lane-private: x << 7 with its exponent
-// in the low seven bits of each lane's first three values.
+// A full matrix in global memory, lane-private: bit i of its exponent is the
+// lowest bit of lane i's first value (2^-64 of the scale; each warp its own copy).
 constexpr int kExpBias = 1 << 20;
 constexpr int kNotFinite = kExpBias - 1;  // the exponent of a matrix with no finite value
 template <int D, int W>
-__device__ __forceinline__ void put_packed(longlong2* s, const long long (&x)[Geo<D, W>::NV], int E) {
+__device__ __forceinline__ void put_packed(const Tm<D, W>& tm, longlong2* s, const long long (&x)[Geo<D, W>::NV], int E) {
   constexpr int NV = Geo<D, W>::NV;
   const int e = max(min(E, kNotFinite), -kExpBias) + kExpBias;
   long long y[NV];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) y[v] = (x[v] << 7) | (v < 3 ? (e >> (7 * v)) & 127 : 0);
+  for (int v = 0; v < NV; ++v) y[v] = x[v];
+  y[0] = (y[0] & ~1ll) | ((e >> tm.lane) & 1);
   put_ints<NV>(s, y);
 }
-template <int D, int W>
-__device__ __forceinline__ int unpack(long long (&x)[Geo<D, W>::NV]) {
-  const int e = (int)(x[0] & 127) | (int)(x[1] & 127) << 7 | (int)(x[2] & 127) << 14;
-#pragma unroll
-  for (int v = 0; v < Geo<D, W>::NV; ++v) x[v] >>= 7;
-  return e - kExpBias;
+template <int NV> __device__ __forceinline__ int unpack(const long long (&x)[NV]) {  // the whole warp together
+  return (int)__ballot_sync(0xffffffffu, (int)x[0] & 1) - kExpBias;
 }
 
 // U = r 2^ex

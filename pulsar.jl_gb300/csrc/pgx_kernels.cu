@@ -715,7 +715,7 @@ static void ensure_smem(K kernel, size_t bytes) {
 // needs later), and never lowered, so launches already recorded into a CUDA
 // graph stay valid.
 void set_smem_once(const void* fn, size_t bytes) {
-  if (bytes <= 48 * 1024) return;
+  if (bytes <= 40 * 1024) return;  // 48 KB need no attribute, a kernel's static arrays (at most 8 KB) included
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, size_t> limit;
   int dev = 0;

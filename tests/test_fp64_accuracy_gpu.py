@@ -1,9 +1,105 @@
-"""Norms of the FP64 and mixed paths' states along long pulses."""
+"""Rounding of the FP64 path against long double, and norms along long pulses.
+
+The first test holds gate gradients to the error of the same evaluation in
+doubles on the host (scipy's exponential, complex128 products), pooled over a
+few short pulses: there propagators lie near the identity, where doubles keep
+the small entries that the controls read to 53 bits of themselves and a block
+format needs its spare bits.  Pools of three or four pulses scatter, hence half
+as much again.
+"""
 import numpy as np
 import pytest
 import scipy.linalg as sla
 
 pytestmark = pytest.mark.gpu
+
+
+def _dag(x):
+    return np.swapaxes(x.conj(), -1, -2)
+
+
+def _expm_long(A):
+    """exp(A) for norms below 1: the Taylor sum of A / 16, squared four times."""
+    B = A / np.longdouble(16)
+    E = np.eye(len(A), dtype=A.dtype) + B
+    T = B
+    for k in range(2, 20):
+        T = T @ B / np.longdouble(k)
+        E = E + T
+    for _ in range(4):
+        E = E @ E
+    return E
+
+
+def _frechet(A, N, real):
+    """L_exp(A, M) from N = M exp(A): sum of commutators ad_A^n(N) / (n + 1)!."""
+    X, T, f = N, N, real(1)
+    for n in range(1, 26):
+        T = A @ T - T @ A
+        f = f / (n + 1)
+        X = X + f * T
+    return X
+
+
+def _gradient(spec, u, mode, real, cplx):
+    """dF/du of the spec's one member (square fidelity) in the given types, the
+    overlaps times their weight, and sum |dG/d overlap|^2."""
+    c = cplx(-1j) if spec.generator == "hermitian" else cplx(1)
+    ctrls = [np.asarray(x).astype(cplx) for x in spec.controls]
+    di, sc, of, w = spec.members()
+    sc, w = real(sc[0]), real(w[0])
+    H = np.asarray(spec.drifts)[int(di[0])].astype(cplx)
+    if spec.offset_op is not None:
+        H = H + real(of[0]) * np.asarray(spec.offset_op).astype(cplx)
+    A = [c * real(spec.dt[k]) * (H + sum(sc * real(u[j, k]) * ctrls[j] for j in range(len(ctrls)))) for k in range(len(spec.dt))]
+    U = [sla.expm(a) if cplx is np.complex128 else _expm_long(a) for a in A]
+    D = len(A[0])
+    gate = spec.target == "gate"
+    P = [np.eye(D, dtype=cplx) if gate else np.asarray(spec.states_init).astype(cplx).T]
+    for x in U:
+        P.append(x @ P[-1])
+    T = np.asarray(spec.target_op if gate else np.asarray(spec.states_target).T).astype(cplx)
+    z = np.array([np.trace(_dag(T) @ P[-1]) / D]) if gate else (T.conj() * P[-1]).sum(0)
+    G, g = np.zeros(u.shape, real), real(0)
+    for s in range(len(z)):
+        lam = w / D * _dag(T) if gate else w * _dag(T[:, s:s + 1])
+        for k in range(len(U) - 1, -1, -1):
+            X = P[k] if gate else P[k][:, s:s + 1]
+            after, lam = lam, lam @ U[k]
+            X = _frechet(A[k], X @ lam, real) if mode == "exact" else X @ after
+            for j in range(len(ctrls)):
+                d = 2 * c * real(spec.dt[k]) * sc * (X.T * ctrls[j]).sum()
+                G[j, k] += (np.conj(z[s]) * d).real
+                g += abs(d) ** 2
+    return G, z * w, float(g)
+
+
+def _rms(x):
+    return float(np.sqrt((np.abs(x) ** 2).sum()))
+
+
+def _pulses(kind):
+    from pulsar_gb300 import workloads as W
+    if kind == "lindblad":
+        return [W.lindblad_gate(seed=n, n_qubits=2, n_t=n, n_draws=1, duration=2e-6 * n / 500) for n in (21, 33, 45, 60)]
+    if kind == "uneven":
+        return [W.uneven_problem(np.random.default_rng(d), d=d, n_t=30, n_members=1) for d in (5, 8, 20)]
+    return [W.spin4_ensemble(seed=n, n_t=n, n_off=1, n_b1=1) for n in (30, 37, 46, 56)]
+
+
+@pytest.mark.parametrize("mode", ["exact", "ref_mr"])
+@pytest.mark.parametrize("kind", ["lindblad", "uneven", "spin4"])
+def test_gate_gradient_of_short_pulses(pg, kind, mode):
+    device, host = [], []
+    for spec, u in _pulses(kind):
+        G = _gradient(spec, u, mode, np.longdouble, np.clongdouble)[0]
+        p = pg.Problem(**spec.problem_kwargs(mode, "fp64"))
+        _, Gd = p.eval(u)
+        p.close()
+        device.append(_rms(Gd - G) / _rms(G))
+        host.append(_rms(_gradient(spec, u, mode, np.float64, np.complex128)[0] - G) / _rms(G))
+    print(f"{kind} {mode}: device", device, "doubles", host)
+    assert _rms(device) <= 1.5 * _rms(host)
 
 
 @pytest.mark.parametrize("precision,D,n_t", [("fp64", 2, 1500), ("fp64", 6, 1500), ("fp64", 8, 1500), ("fp64", 16, 1500),
