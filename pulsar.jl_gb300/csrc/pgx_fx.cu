@@ -11,10 +11,15 @@ static __constant__ Coef c_coef[PGX_N_INVFACT] = PGX_INVFACT_FX_INIT;
 
 constexpr int kMaxTerms = 24;       // generator terms: drift, controls, ramp
 constexpr int kMaxTerms32 = 7;      // at D = 32: 16 KB of shared memory each beside two teams
-// Absolute error of a slice propagator's products: 2^-57 on the FP64 path;
-// 2^-51 on the mixed path, whose df pairs hold 2^-48 of an element (with 2^-48
-// U_total's defect over 1000 slices stayed 2.5 times larger).
-template <bool DF> constexpr int kBits2 = 2 * (DF ? 51 : 57) + 1;
+// Absolute error of a slice propagator's products: 2^-57 for the FP64 gate
+// chains; 2^-59 for the state chains, whose overlaps can be as small as 1e-4 (at
+// 2^-57 the gradients of four-spin transfers below 100 slices were 0.9, at 2^-59
+// 0.6 of FP64's error, for 3 % of this kernel); 2^-51 on the mixed path, whose df
+// pairs hold 2^-48 of an element (with 2^-48 U_total's defect over 1000 slices
+// stayed 2.5 times larger).
+template <bool DF> __device__ __forceinline__ int bits2_of(const ProbDev& p) {
+  return 2 * (DF ? 51 : p.target == TGT_GATE ? 57 : 59) + 1;
+}
 constexpr int kNever = 1 << 20;     // an exponent no finite entry reaches
 constexpr int kPrefixLevels = 7;  // the mixed path's prefixes, rounded to df pairs or FP32 afterwards
 
@@ -266,6 +271,7 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
       const float l1 = log2_norm1<D, W>(tm, r, EA);
       double2* out = w.U + ((size_t)m * p.n_t + k) * D * D;
       const bool packed = !DF && p.target == TGT_GATE;  // the FP64 gate chains' own format
+      const int bits2 = bits2_of<DF>(p);
       // Squares keep an odd number of levels: the first one left out then has no
       // pair of equal digits, whose squares a (skew-)Hermitian matrix sums into
       // its diagonal with one sign.  Six levels of df propagators raised a state's
@@ -296,9 +302,9 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
 #pragma unroll 1
       for (int st = 0; st < L + s; ++st) {
         int n;
-        if (st == 0) n = min(levels(kBits2<DF>, 2 * (EB - (int)fmaxf(l1, 0.f))) | odd, kMaxLevels);
-        else if (st < L) n = levels(kBits2<DF>, EX + EY + (L - 1 - st) * lx);
-        else n = min(levels(kBits2<DF>, 2 * EY) | odd, kMaxLevels);
+        if (st == 0) n = min(levels(bits2, 2 * (EB - (int)fmaxf(l1, 0.f))) | odd, kMaxLevels);
+        else if (st < L) n = levels(bits2, EX + EY + (L - 1 - st) * lx);
+        else n = min(levels(bits2, 2 * EY) | odd, kMaxLevels);
         tm.sync();
         if (st == 0) {
           long long x6[NV];
@@ -333,7 +339,7 @@ __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_e
         }
         if (st < L) {
           const int i = L - 1 - st;
-          const bool final = packed && i == 0 && s == 0;  // |U| <= e^nu <= 0.75 2^g
+          const bool final = !DF && i == 0 && s == 0;  // |U| <= e^nu <= 0.75 2^g
           const int fr = final ? g : c_coef[2 * i].exp + g;
           F = st > 0 && i == 0 ? 60 : kFrac;
           if (st == 0) {
@@ -1267,8 +1273,10 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
 // a step only rounds its result.  (Without the low one, overlaps of 1e-3 lost
 // five bits against FP64, which keeps small amplitudes to their own scale.)
 //   Hermitian generators keep the vector's norm, so its exponent never moves:
-//   |x| < 2^58 at the start, so ||x|| < 2^60.5, and G = 60 with ||u|| <= 2^60 in
-//   every row keep each sum inside 63 bits (Cauchy-Schwarz).
+//   ||x|| <= 2^60.5 from the start (which leaves a basis state's small
+//   amplitudes 2^-60 of its norm), so a component's high half stays below 2^31,
+//   and G = 60 with ||u|| <= 2^60 in every row: high sums stay below 2^61, the
+//   mixed ones of eight columns below 2^62.3 (Cauchy-Schwarz).
 //   Others: |x| < 2^57 (2^56 at D = 32), renewed every step; |u| < 2^58 below
 //   U_k's largest entry, G = 58.
 // At D = 32 a lane sums its row in four parts, so the mixed and low sums stay
@@ -1414,7 +1422,14 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
     const int EX = (int)(__reduce_max_sync(0xffffffffu, max((uint32_t)__double2hiint(v0.x) & 0x7ff00000u,
                                                             (uint32_t)__double2hiint(v0.y) & 0x7ff00000u)) >> 20);
     bad = EX == 0x7ff;
-    const int guard = HERM ? 5 : 4 + C::GUARD;
+    int guard = 4 + C::GUARD;
+    if (HERM) {  // ||x|| <= 2^60.5, from the norm in units of 2^(EX - 1022)
+      const float re = (float)scalbn(v0.x, 1022 - EX), im = (float)scalbn(v0.y, 1022 - EX);
+      float n2 = fmaf(re, re, im * im);
+#pragma unroll
+      for (int o = 1; o < D; o <<= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+      guard = min(max((int)floorf(7.499f - 0.5f * __log2f(n2)), 0), 8);
+    }
     first = split2(from_double(v0.x, EX, guard), from_double(v0.y, EX, guard));
     E = EX - 1018 - guard;  // x 2^(EX - 1075 - guard)
   }

@@ -102,6 +102,28 @@ def test_gate_gradient_of_short_pulses(pg, kind, mode):
     assert _rms(device) <= 1.5 * _rms(host)
 
 
+@pytest.mark.parametrize("n_t", [30, 56])
+@pytest.mark.parametrize("mode", ["exact", "ref_mr"])
+def test_basis_state_transfer(pg, n_t, mode):
+    """Four-spin transfers between basis states, whose overlaps start at 1e-4.  A
+    step rounds a vector's parts to 2^-60 of its norm and meets propagators
+    rounded to 2^-59, about 2^-61 rms each, independently; four times their sum
+    over 2 n_t steps, through the overlaps (dG / dz) and through the vectors
+    themselves."""
+    from pulsar_gb300 import workloads as W
+    spec, u = W.spin4_state_transfer(seed=n_t, n_t=n_t, n_off=1, n_b1=1)
+    G, zw, g = _gradient(spec, u, mode, np.longdouble, np.clongdouble)
+    p = pg.Problem(**spec.problem_kwargs(mode, "fp64"))
+    _, Gd = p.eval(u)
+    p.close()
+    norms = sum(np.linalg.norm(x, 2) ** 2 for x in np.asarray(spec.controls))
+    reach = np.sqrt((np.asarray(spec.dt) ** 2).sum() * norms) * 2 * _rms(zw)
+    tol = 4 * 2.0 ** -61 * np.sqrt(2 * n_t) * (reach + np.sqrt(g)) + 2.0 ** -52 * _rms(G)
+    err = _rms(Gd - G)
+    print(f"{n_t} slices {mode}: device error {err / _rms(G):.1e} of |G|, bar {tol / _rms(G):.1e}")
+    assert err <= tol
+
+
 @pytest.mark.parametrize("precision,D,n_t", [("fp64", 2, 1500), ("fp64", 6, 1500), ("fp64", 8, 1500), ("fp64", 16, 1500),
                                              ("fp64", 32, 600), ("mixed", 16, 1500), ("mixed", 32, 600)])
 def test_norm_along_long_pulses(pg, precision, D, n_t):
