@@ -1781,7 +1781,15 @@ static cudaError_t launch_slices(void (*kernel)(ProbDev, WorkDev, int, A...), co
   const int n = p.n_c + 1 + (p.n_ramp ? 1 : 0);
   const size_t consts = Terms<D, C::W>::bytes(n);
   const int fit = (int)((kSmemMax - consts) / C::TEAM_BYTES);
-  const int nt = fit < C::TEAMS ? fit : C::TEAMS, threads = 32 * C::W * nt;
+  // fewer teams where every SM still gets its share of the slices: ten slices of
+  // one SM wait for each other, and one or two alone set the generator's terms up
+  // longer (d = 16, one member of 20 slices, F only: mixed states 73 us with ten
+  // teams, 60 with two; df products on the CUDA cores 64.  FP64 72 and 60)
+  constexpr long few = D >= 32 ? 1 : D >= 16 ? 2 : 4;
+  const long share = ((long)p.n_members * p.n_t + li.num_sms - 1) / li.num_sms;
+  int nt = fit < C::TEAMS ? fit : C::TEAMS;
+  if (share < nt) nt = (int)(share > few ? share : few < nt ? few : nt);
+  const int threads = 32 * C::W * nt;
   const size_t smem = consts + (size_t)nt * C::TEAM_BYTES;
   set_smem_once((const void*)kernel, smem);
   int per_sm = 1;
