@@ -1,6 +1,9 @@
-"""Evaluation graphs after every setter."""
+"""Routes of the padded dimensions 8 to 64 that a size alone does not reach: the
+D = 64 mixed kernels through their own evaluation, slices of large norm beside
+small ones, evaluation graphs after every setter, the teams in use."""
 import numpy as np
 import pytest
+import scipy.linalg as sla
 
 pytestmark = pytest.mark.gpu
 
@@ -12,6 +15,119 @@ def _dag(x):
 def _herm(rng, n, D):
     x = rng.normal(size=(n, D, D)) + 1j * rng.normal(size=(n, D, D))
     return x + _dag(x)
+
+
+def _shift(D, k, phase):
+    return phase * np.roll(np.eye(D), k, axis=0)
+
+
+@pytest.mark.parametrize("gen", ["hermitian", "liouvillian"])
+@pytest.mark.parametrize("D", [33, 64])
+@pytest.mark.parametrize("nrm", [0.0, 1e-9, 3e-5, 0.003, 0.03, 0.1, 0.17, 0.4, 0.8, 1.6, 7.0, 60.0])
+def test_mixed_expm_64_through_its_evaluation(pg, gen, D, nrm):
+    """The sliced exponential (block sizes 2 to 4, four to seven levels,
+    squarings) read through F = Re Tr(T'U) / D with shifts T, the mean of D
+    entries of U.  An entry is held to 2^-53 of 1 and stored as a df pair (2^-48
+    of itself), and squarings double the error: a mean of D stays within 4
+    2^-48 2^s.  The CUDA-core team within the same bar."""
+    rng = np.random.default_rng(D + int(1e3 * nrm))
+    H = _herm(rng, 4, D)
+    if gen == "liouvillian":  # dissipative, not normal: the propagator stays bounded
+        H = H * 1j
+        H[0] += -0.2 * np.eye(D) + 0.05 * np.triu(rng.normal(size=(D, D)), 1)
+    u = rng.normal(size=(3, 1))
+    A = H[0] + np.tensordot(u[:, 0], H[1:], 1)
+    dt = nrm / np.abs(A).sum(0).max()
+    E = sla.expm((-1j if gen == "hermitian" else 1.0) * dt * A)
+    s = max(0, int(np.ceil(np.log2(max(nrm, 1e-300) / 0.1))))
+    bar = 4 * 2.0 ** (s - 48) * max(1.0, np.abs(E).max())
+    for k, phase in ((0, 1), (0, 1j), (1, 1), (D // 2, 1j)):
+        T = _shift(D, k, phase)
+        p = pg.Problem(H[:1], H[1:], np.array([dt]), generator=gen, target="gate", target_op=T, fidelity="real",
+                       precision="mixed", grad_mode="exact")
+        assert p.teams[0] == 1
+        F, _ = p.eval(u, want_grad=False)
+        F1, G1 = p.eval(u)
+        p.set_teams(256, 0)
+        Fc, Gc = p.eval(u)
+        p.close()
+        Fo = (np.trace(T.conj().T @ E) / D).real
+        assert F1 == F
+        assert abs(F - Fo) <= bar and abs(Fc - Fo) <= bar
+        # the gradient of the same kernel on either propagators: FP32 class
+        assert np.abs(G1 - Gc).max() <= 1e-5 * max(np.abs(Gc).max(), 1e-30)
+
+
+@pytest.mark.parametrize("n_t", [1, 4, 6, 9])
+def test_mixed_generators_64_of_many_members(pg, n_t):
+    """Members enough for the prologue that assembles four slices of a member at
+    a time, with a short last group: every member's fidelity against its
+    propagators, the bar above for each slice; F-only and CUDA-core teams too."""
+    rng = np.random.default_rng(n_t)
+    n_m, D = 320, 36
+    X = _herm(rng, 4, D)
+    u = rng.normal(size=(2, n_t))
+    sc, of = rng.uniform(0.9, 1.1, n_m), rng.uniform(-0.1, 0.1, n_m)
+    dt = rng.uniform(0.5, 1.0, n_t) * 0.02
+    T = _shift(D, 1, 1j)
+    p = pg.Problem(X[:1], X[1:3], dt, offset_op=X[3], member_scale=sc, member_offset=of, target="gate", target_op=T,
+                   fidelity="real", precision="mixed", grad_mode="exact")
+    F, G = p.eval(u)
+    f = p.member_fidelities()
+    F1, _ = p.eval(u, want_grad=False)
+    p.set_teams(256, 0)
+    Fc, Gc = p.eval(u)
+    p.close()
+    bar = n_t * 4 * 2.0 ** (4 - 48)  # norms up to 1.6
+    assert F1 == F and abs(F - f.mean()) <= 2.0 ** -48 and abs(F - Fc) <= bar
+    assert np.abs(G - Gc).max() <= 1e-5 * np.abs(Gc).max()
+    for m in (0, 1, 151, 152, 303, 304, n_m - 1):
+        E = np.eye(D)
+        for k in range(n_t):
+            E = sla.expm(-1j * dt[k] * (X[0] + of[m] * X[3] + sc[m] * np.tensordot(u[:, k], X[1:3], 1))) @ E
+        assert abs(f[m] - (np.trace(T.conj().T @ E) / D).real) <= bar
+
+
+@pytest.mark.parametrize("target", ["gate", "states"])
+@pytest.mark.parametrize("D,n_t,n_m", [(7, 9, 2), (16, 33, 1), (12, 40, 3), (32, 12, 1), (20, 7, 2)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_one_slice_of_large_norm(pg, precision, target, D, n_t, n_m):
+    """One slice beyond the exact gradient's series among small ones: on the
+    FP64 path that slice alone takes the derivative kernel, on the mixed path the
+    whole evaluation the CUDA-core gradient.  Against the oracle with the paths'
+    bars; where the mixed path falls back, the bits of that team's own run."""
+    from oracle import members as mb
+    rng = np.random.default_rng(D * n_t)
+    X = _herm(rng, 3, D)
+    u = rng.normal(size=(2, n_t))
+    nrm = np.array([np.linalg.norm(X[0] + np.tensordot(u[:, k], X[1:], 1), 2) for k in range(n_t)])
+    Q, _ = np.linalg.qr(rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D)))
+    to = dict(target_op=Q) if target == "gate" else dict(states_init=Q[:2], states_target=Q[2:4])
+    team = 32 if D <= 16 else 128
+    for big in (None, 0, n_t // 2, n_t - 1, "all"):
+        dt = 0.1 / nrm
+        if big == "all":
+            dt = 9.0 / nrm
+        elif big is not None:
+            dt[big] = 9.0 / nrm[big]
+        kw = dict(drifts=X[:1], controls=X[1:], dt=dt, member_scale=rng.uniform(0.95, 1.05, n_m), target=target, **to)
+        Fo, Go = mb.eval_problem(mb.Problem(n_members=n_m, **kw), u, "exact")
+        p = pg.Problem(grad_mode="exact", precision=precision, **kw)
+        F, G = p.eval(u)
+        scale = np.abs(Go).max()
+        if precision == "fp64":
+            assert abs(F - Fo) <= 1e-10 and np.abs(G - Go).max() <= 1e-8 * scale
+        else:
+            assert abs(F - Fo) <= 1e-8 and np.abs(G - Go).max() <= 1e-4 * scale
+            if D > 8:
+                p.set_teams(0, team)
+                F1, G1 = p.eval(u)
+                assert F1 == F
+                if big is None:  # two FP32-class evaluations of 15 products of D terms
+                    assert np.abs(G - G1).max() <= 15 * np.sqrt(D) * 2.0 ** -23 * scale
+                else:
+                    assert np.array_equal(G, G1)
+        p.close()
 
 
 def _setters(pg, precision, target, D, n_t, X, rng):
