@@ -260,12 +260,11 @@ int pgx_penalty_eval(pgx_ctx* ctx, int32_t n_controls, int32_t n_slices, const d
 /* Times every team-size variant (threads per matrix problem, with the
  * matching register blocking) of the problem's slice-parallel mixed-precision
  * kernels at controls u, `reps` launches each, keeps the fastest for this
- * problem and writes a one-line report (nullable).  Variants only re-map work
- * to threads; every dot product is summed in the same order, so results are
- * bit-identical whatever is chosen.  The FP64 path has no variants.  At
- * padded dimension 64 the expm, and the gradient of gate targets with the
- * exact gradient, have one candidate each: the tensor-core engine
- * (PGX_TEAM_TENSOR).                                                        */
+ * problem and writes a one-line report (nullable).  The CUDA-core variants
+ * only re-map work to threads; every dot product is summed in the same order,
+ * so their results are bit-identical.  The FP64 path has no variants.  Where a
+ * tensor-core engine takes the problem (below) it is the only candidate and
+ * nothing is timed.                                                         */
 int pgx_autotune(pgx_problem* prob, const double* u, int32_t reps, char* report, size_t report_len);
 /* Sets the team sizes directly (a plan kept from an earlier pgx_autotune);
  * 0 = the built-in default.  Values the dimension does not admit are refused
@@ -273,13 +272,25 @@ int pgx_autotune(pgx_problem* prob, const double* u, int32_t reps, char* report,
  * Admitted by padded dimension: 32 (<= 8); 32, 64, 128, 256 (16); 128, 256
  * (32); 256 (64), plus 512 for the gradient at 64.  PGX_TEAM_TENSOR (1)
  * selects a tensor-core engine, the default where it exists:
+ *   - the expm at 16 and 32 (every generator and target with at most 24 and 7
+ *     generator terms: drift, controls, ramp), and with it the forward chain of
+ *     gate targets: block fixed-point products, every entry to about 2^-51 of
+ *     the largest (2^-48 of itself in the df pair that leaves), where the
+ *     CUDA-core df products keep about 2^-46 of each entry;
+ *   - the gradient at 16 and 32 with the exact gradient and that expm: a
+ *     commutator series in 3xFP16 (22-bit operands scaled by the matrix's
+ *     largest entry, FP32 sums), FP32-class; an evaluation with a slice whose
+ *     min(||A||_1, ||A^2||_1^(1/2)) passes 1 takes the CUDA-core default team;
  *   - the expm at 64 (every generator and target): df products by exact bf16
  *     slicing (six 8-bit slices per operand, levels 0..6 accumulated exactly
  *     in FP32), df-class like the CUDA-core team 256 but not bit-identical;
  *   - the gradient at 64 of gate targets with the exact gradient: 3xFP16
  *     tcgen05 products, FP32-class like the CUDA-core teams but not
  *     bit-identical to them.
- * The CUDA-core teams stay admitted there for comparisons.                   */
+ * The CUDA-core teams stay admitted there for comparisons.  At 16 and 32 the
+ * value is admitted for every problem of the dimension (the teams of one fit
+ * the others) and means the CUDA-core default where the engine does not take
+ * the problem; pgx_problem_get_team answers the team that runs.              */
 #define PGX_TUNE_EXPM 0
 #define PGX_TUNE_GRAD 1
 #define PGX_TEAM_TENSOR 1
@@ -290,7 +301,8 @@ int pgx_problem_get_team(const pgx_problem* prob, int32_t kernel, int32_t* team)
  * problems created later with the same key -- on any context, a server's
  * private one included -- start from it.  pgx_plan_lookup reports the plan
  * for a descriptor (PGX_ERR_STATE and zeros when none); pgx_plan_clear
- * forgets every plan.  Plans never change results, only time.              */
+ * forgets every plan.  Plans change time, and results only as far as the
+ * engines above differ.                                                     */
 int pgx_plan_lookup(int device, const pgx_problem_desc* desc, int32_t* team_expm, int32_t* team_grad);
 int pgx_plan_clear(void);
 

@@ -178,8 +178,8 @@ void set_smem_once(const void* fn, size_t bytes);
 // default choice.
 // Team values of the tunable mixed kernels: candidates the autotuner times,
 // values pgx_problem_set_team admits, and the default.  kTeamTensor (1)
-// selects the tensor-core engine: of the D = 64 gate-target exact gradient,
-// and of the D = 64 df expm.
+// selects a tensor-core engine: of the D = 64 gate-target exact gradient, of the
+// exact gradient at D = 16 and 32, and of the df expm at 16, 32 and 64.
 constexpr int kTeamTensor = 1;
 bool grad_tc_eligible(const ProbDev& p);
 // Whether an evaluation may run tensor-core kernels (the D = 64 expm, the
@@ -188,9 +188,12 @@ bool tc_kernels_used(const ProbDev& p);
 int mixed_variants(const ProbDev& p, int kernel, int* out);
 int mixed_admitted(const ProbDev& p, int kernel, int* out);
 int mixed_default_team(const ProbDev& p, int kernel);
-// (member, block) prefix chains of the mixed gate chain that the GPU holds at
-// once (the CUDA-core prefix kernel at its occupancy on the current device,
-// times num_sms); 0 when Dp has no such kernel here (Dp > 32).
+// The team `kernel` runs with: li's choice or the default, and the CUDA-core
+// default where kTeamTensor does not apply to the problem as it is now.
+int mixed_running_team(const ProbDev& p, int kernel, const LaunchInfo& li);
+// (member, block) prefix chains of the mixed gate chain that its blocks are cut
+// for: what the GPU holds of the CUDA-core prefix kernel or, at D = 16 and 32,
+// fx_prefix_capacity where that is less; 0 when Dp has no such kernel (Dp > 32).
 long chain_prefix_capacity(int Dp, int num_sms);
 // The df expm over the items of n mixed problems of padded dimension Dp = 2
 // (the only one batches share; device tables ps, ws; problem i's members x

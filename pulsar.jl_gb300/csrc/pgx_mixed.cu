@@ -1482,6 +1482,9 @@ static int grad_team(const ProbDev& p, const LaunchInfo& li) {
   if (t != kTeamTensor || p.Dp == 64) return t;
   return series_eligible(p) && expm_team(p, li) == kTeamTensor ? t : cuda_core_team(p.Dp, kTuneGradMx);
 }
+int mixed_running_team(const ProbDev& p, int kernel, const LaunchInfo& li) {
+  return kernel == kTuneGradMx ? grad_team(p, li) : expm_team(p, li);
+}
 static bool grad_series(const ProbDev& p, const LaunchInfo& li) { return p.Dp < 64 && grad_team(p, li) == kTeamTensor; }
 
 #define PGX_DISPATCH_MX_T(DP, TT, CALL)                                                        \

@@ -480,8 +480,8 @@ static int upload(pgx_problem* p, T** dptr, const std::vector<T>& host) {
 // records its choice under (device, padded dimension, n_controls, generator,
 // target, precision, grad_mode) and every problem created later with the same
 // key -- on any context, the server's private one included -- starts with it.
-// Team sizes never change results (the variants are bit-identical), so a plan
-// only moves time.
+// A plan moves time; the CUDA-core teams are bit-identical, and results differ
+// from theirs only as far as the tensor-core engines' do.
 namespace {
 using PlanKey = std::tuple<int, int, int, int, int, int, int>;
 std::mutex g_plan_mu;
@@ -937,7 +937,7 @@ extern "C" int pgx_problem_set_team(pgx_problem* p, int32_t kernel, int32_t team
 
 extern "C" int pgx_problem_get_team(const pgx_problem* p, int32_t kernel, int32_t* team) {
   if (!p || !team || kernel < 0 || kernel >= pgx::kNumTunable) return PGX_ERR_INVALID;
-  *team = p->team[kernel] ? p->team[kernel] : pgx::mixed_default_team(p->pd, kernel);
+  *team = pgx::mixed_running_team(p->pd, kernel, p->launch_info());
   return PGX_OK;
 }
 

@@ -220,3 +220,40 @@ def test_batch_after_set_drifts(pg):
     for p, q, _ in probs:
         p.close()
         q.close()
+
+
+@pytest.mark.parametrize("D,core", [(16, (128, 32)), (32, (256, 128)), (64, (256, 512))])
+def test_teams_in_use(pg, D, core):
+    """`teams` names the kernels that run: the tensor-core value only where its
+    kernels take the problem, whatever was set, and again once they do."""
+    rng = np.random.default_rng(D)
+    few, many = 2, 30
+    X = _herm(rng, many + 2, D)
+    dt = np.full(3, 0.05 / D)
+    gate = dict(target="gate", target_op=np.eye(D))
+    states = dict(target="states", states_init=np.eye(D)[:1], states_target=np.eye(D)[1:2])
+
+    def teams(n_c, mode, to, teams=None, ramp=False):
+        p = pg.Problem(X[:1], X[1:1 + n_c], dt, precision="mixed", grad_mode=mode, **to)
+        if teams:
+            p.set_teams(*teams)
+        if ramp:
+            p.set_drift_ramp(X[-1:], [0], np.ones(3))
+        t = p.teams
+        p.close()
+        return t
+
+    assert teams(few, "exact", gate) == (1, 1)
+    series = (1, 1) if D < 64 else (1, core[1])
+    assert teams(few, "exact", states) == series
+    assert teams(few, "ref_mr", gate) == (1, core[1])
+    if D < 64:
+        assert teams(many, "exact", gate) == core
+        for to in (gate, states):
+            assert teams(few, "ref_mr", to, (1, 1)) == (1, core[1])
+            assert teams(many, "exact", to, (1, 1)) == core
+        assert teams(few, "exact", gate, (core[0], 0)) == core  # the series needs the tensor-core expm
+        assert teams(few, "exact", gate, (0, core[1])) == (1, core[1])
+        most = 23 if D == 16 else 6  # with a ramp one generator term too many
+        assert teams(most, "exact", gate) == (1, 1)
+        assert teams(most, "exact", gate, ramp=True) == core
