@@ -1958,12 +1958,20 @@ cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInf
 cudaError_t launch_fx_combine_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store) {
   PGX_FX_DISPATCH_DF(fx::do_combine_df<D_>(p, w, li, store));
 }
+// At D = 32 an SM holds two chains of 57 KB, and is given twice as many: the FP32
+// suffixes beside them gain from more blocks than the prefixes lose by queueing,
+// and from 153 to 304 members the chains stay cut at all.  Evaluations of 500
+// slices (60 from 153 members on) in ms with one, two and three times what it
+// holds, in brackets F alone: 16 members 1.57 (0.99), 1.62 (1.08), 1.62 (1.08);
+// 64: 5.42 (3.42), 5.27 (3.33), 5.27 (3.34); 128: 10.85 (6.84), 10.69 (6.81),
+// 10.71 (6.81); 153: 2.61 (1.94), 1.72 (1.16), 1.72 (1.16); 304: 3.71 (2.64),
+// 3.11 (1.99), 3.11 (1.99); 305: 4.46 (3.33) with any.  The same grid on the
+// FP32 pipe's df kernels: never faster.
+constexpr long kPrefixWaves32 = 2;
 long fx_prefix_capacity(int Dp) {
   switch (Dp) {
     case 16: return fx::prefix_capacity<16>();
-    // two of 57 KB are resident, but the FP32 suffixes beside them gain from more
-    // blocks than the prefixes lose by queueing (64 x 500: 8.67 -> 8.41 ms with 4)
-    case 32: return 4;
+    case 32: return kPrefixWaves32 * fx::prefix_capacity<32>();
     default: return 0;
   }
 }

@@ -73,7 +73,9 @@ struct WorkDev {
   double* Gm;       // [n_members][n_t][n_c] per-member weighted gradient
   double2* slab;    // global Taylor workspace for Dp = 64: [slab_teams][10][Dp*Dp]
   int slab_teams;
-  int* norm_flag;   // mixed: raised by a slice of norm > 1 (k_fx_expm), cleared by k_prep_mx
+  // mixed: raised by a slice with min(||A||_1, ||A^2||_1^(1/2)) > 1 (k_fx_expm),
+  // cleared by k_prep_mx
+  int* norm_flag;
   int* expm_plan;   // mixed, Dp = 64: [n_members][n_t] degree choice of each slice's expm
   const double* u;  // [n_t][n_c]  (column-major [n_c x n_t])
   double* G;        // [n_t][n_c]
@@ -226,8 +228,8 @@ cudaError_t launch_residual(const ProbDev& p, const WorkDev& w, int kind, int N,
 cudaError_t launch_select_sum(const double* Gm, const int* idx, const double* coef, int n_sel, int len, double* G,
                               const LaunchInfo& li);
 // The FP64 path on block fixed-point tensor-core products (pgx_fx.cu): Dp = 8
-// and 16 with at most 24 generator terms (drift, controls, ramp).  Slice
-// propagators for every target (gate targets: in the gate chains' own format),
+// and 16 with at most 24 generator terms (drift, controls, ramp), Dp = 32 with
+// at most 7.  Slice propagators for every target (gate targets: in the gate chains' own format),
 // the gate chains, and the gradient of gate targets (any mode) and of exact
 // state targets (launch_grad leaves those with tracking to k_grad).
 bool fx_applies(const ProbDev& p);
@@ -235,7 +237,7 @@ cudaError_t launch_fx_expm(const ProbDev& p, const WorkDev& w, const LaunchInfo&
 cudaError_t launch_fx_chain_fwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
 cudaError_t launch_fx_chain_bwd(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 cudaError_t launch_fx_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
-// FP64 state chains (no tracking) up to Dp = 16, both directions in one launch;
+// FP64 state chains (no tracking) up to Dp = 32, both directions in one launch;
 // lambda is stored without conj(kappa), which the gradient applies.
 __host__ __device__ inline bool lam_unscaled(const ProbDev& p, int Dp) { return p.n_ck == 0 && Dp <= 32; }
 cudaError_t launch_fx_states(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
@@ -247,7 +249,7 @@ cudaError_t launch_fx_prefix_df(const ProbDev& p, const WorkDev& w, const Launch
 // 32; a no-op when w.norm_flag is raised): P holds N_k = P_k Lambda_{k-1}.
 cudaError_t launch_tf_grad(const ProbDev& p, const WorkDev& w, const LaunchInfo& li);
 cudaError_t launch_fx_combine_df(const ProbDev& p, const WorkDev& w, const LaunchInfo& li, bool store);
-long fx_prefix_capacity(int Dp);  // prefix chains one SM holds
+long fx_prefix_capacity(int Dp);  // prefix chains an SM is given: what it holds, twice that at Dp = 32
 // Mixed-precision stages (pgx_mixed.cu), gate targets: df expm and forward
 // chain, FP32 backward chain and gradient.  U stack holds df (float4), the P
 // stack float2.

@@ -149,3 +149,21 @@ def test_norm_along_long_pulses(pg, precision, D, n_t):
         p.close()
         print(f"{precision} d = {D}: {(F - 1) / n_t:.1e} a slice")
         assert abs(F - 1) <= 4 * unit * np.sqrt(n_t) + 2.0 ** -51
+
+
+@pytest.mark.parametrize("D", [8, 16, 32])
+@pytest.mark.parametrize("mode", ["exact", "ref_mr"])
+def test_trace_of_equal_entries(pg, D, mode):
+    """Every product of the trace Tr(X C) at its largest and of one sign (a
+    control of equal entries, states spread evenly, entries just below a power of
+    two): the integer sums hold it.  FP64's bar against the oracle."""
+    from oracle import members as mb
+    psi = np.full((1, D), D ** -0.5, complex)
+    kw = dict(drifts=np.zeros((1, D, D)), controls=np.full((2, D, D), 0.999), dt=np.full(3, 1e-3 / D), target="states",
+              fidelity="real", states_init=psi, states_target=1j * psi, member_weight=np.array([0.74]))
+    u = np.array([[0.3, -0.2, 0.1], [0.1, 0.2, 0.3]])
+    Fo, Go = mb.eval_problem(mb.Problem(n_members=1, **kw), u, mode)
+    p = pg.Problem(grad_mode=mode, precision="fp64", **kw)
+    F, G = p.eval(u)
+    p.close()
+    assert abs(F - Fo) <= 1e-10 and np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
