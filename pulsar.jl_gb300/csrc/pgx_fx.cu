@@ -1422,7 +1422,7 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
     const int EX = (int)(__reduce_max_sync(0xffffffffu, max((uint32_t)__double2hiint(v0.x) & 0x7ff00000u,
                                                             (uint32_t)__double2hiint(v0.y) & 0x7ff00000u)) >> 20);
     bad = EX == 0x7ff;
-    int guard = 4 + C::GUARD;
+    int guard = 4 - C::GUARD;
     if (HERM) {  // ||x|| <= 2^60.5, from the norm in units of 2^(EX - 1022)
       const float re = (float)scalbn(v0.x, 1022 - EX), im = (float)scalbn(v0.y, 1022 - EX);
       float n2 = fmaf(re, re, im * im);

@@ -167,3 +167,23 @@ def test_trace_of_equal_entries(pg, D, mode):
     F, G = p.eval(u)
     p.close()
     assert abs(F - Fo) <= 1e-10 and np.abs(G - Go).max() <= 1e-8 * np.abs(Go).max()
+
+
+@pytest.mark.parametrize("D", [2, 4, 8, 16, 20, 32])
+def test_state_sums_of_equal_entries(pg, D):
+    """A state chain's first step with every product at its largest and of one
+    sign: a propagator I + k (1 - i) J, J all ones, on a vector of equal entries
+    (1 + i) just below a power of two.  Against the closed form; the exponential
+    of norm 9 costs seven squarings, 2^7 (D + 40) 2^-53 relative."""
+    k = 100.0
+    J = np.ones((D, D))
+    a = np.log(1 + D * k * (1 - 1j)) / D
+    v = np.full((1, D), 0.999 * (1 + 1j))
+    kw = dict(drifts=a * J[None], controls=0 * J[None], dt=np.ones(1), generator="liouvillian", target="states",
+              fidelity="square", states_init=v, states_target=v)
+    p = pg.Problem(grad_mode="ref_mr", precision="fp64", **kw)
+    F, G, st = p.eval(np.zeros((1, 1)), stats=True)
+    F1, _ = p.eval(np.zeros((1, 1)), want_grad=False)
+    p.close()
+    z = np.vdot(v, v + k * (1 - 1j) * (J @ v.T).T)
+    assert F1 == F and abs(F / abs(z) ** 2 - 1) <= 2 * 2.0 ** 7 * (D + 40) * 2.0 ** -53
