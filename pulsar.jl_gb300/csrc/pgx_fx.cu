@@ -1277,8 +1277,12 @@ k_fx_chain_combine(ProbDev p, WorkDev w, int blocks, int len, int want_grad) {
 //   amplitudes 2^-60 of its norm), so a component's high half stays below 2^31,
 //   and G = 60 with ||u|| <= 2^60 in every row: high sums stay below 2^61, the
 //   mixed ones of eight columns below 2^62.3 (Cauchy-Schwarz).
-//   Others: |x| < 2^57 (2^56 at D = 32), renewed every step; |u| < 2^58 below
-//   U_k's largest entry, G = 58.
+//   Others: the larger scale of |x| < 2^57 (2^56 at D = 32) and sum |x| < 2^60
+//   over both parts of all components (near a basis state, whose small
+//   components it leaves three more bits), renewed every step; |u| < 2^G of
+//   U_k's largest entry, G = 60 up to D = 8, where a lane has one or two columns,
+//   and 59 above: a row's sum is below 2^62 either way, the mixed sums of eight
+//   columns below 2^62.4.
 // At D = 32 a lane sums its row in four parts, so the mixed and low sums stay
 // inside 63 bits as at D = 16 (200 slices of 8 members and two pairs at d = 24:
 // 1.01 + 1.12 ms in FP64 on shared memory, 0.55 ms here).
@@ -1289,6 +1293,7 @@ template <int D> struct StCfg {
   static constexpr int CH = D >= 32 ? 1 : D >= 16 ? 2 : D >= 8 ? 8 : 128 / D;  // slices of a chunk
   static constexpr int QB = QN < 8 ? QN : 8;          // columns summed at a time
   static constexpr int GUARD = D >= 32 ? 1 : 0;       // one bit less of a vector that may grow (below)
+  __host__ __device__ static constexpr int ubits(bool herm) { return herm || D <= 8 ? 60 : 59; }  // G below
   static constexpr int HELPERS = 8;
   static constexpr int NPT = 2 * CH * D * D / (32 * HELPERS);  // entries of a helper lane and chunk, both directions
   static constexpr int RING = 2 * CH * D * D;         // entries of one chunk
@@ -1366,8 +1371,9 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
       for (int i = 0; i < NPT; ++i) {
         where(c, i, dir, sl, e);
         const int EX = HERM ? 1023 : s_eu[(buf * 2 + dir) * CH + sl];
+        constexpr int guard = C::ubits(HERM) - (HERM ? 52 : 53);
         ring[(size_t)(buf * 2 + dir) * CH * D * D + sl * D * D + swz(e % D, e / D)] =
-            split2(from_double(raw[i].x, EX, HERM ? 8 : 5), from_double(raw[i].y, EX, HERM ? 8 : 5));
+            split2(from_double(raw[i].x, EX, guard), from_double(raw[i].y, EX, guard));
       }
     };
     auto put = [&](int c) {  // the vectors of chunk c
@@ -1422,14 +1428,14 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
     const int EX = (int)(__reduce_max_sync(0xffffffffu, max((uint32_t)__double2hiint(v0.x) & 0x7ff00000u,
                                                             (uint32_t)__double2hiint(v0.y) & 0x7ff00000u)) >> 20);
     bad = EX == 0x7ff;
-    int guard = 4 - C::GUARD;
-    if (HERM) {  // ||x|| <= 2^60.5, from the norm in units of 2^(EX - 1022)
-      const float re = (float)scalbn(v0.x, 1022 - EX), im = (float)scalbn(v0.y, 1022 - EX);
-      float n2 = fmaf(re, re, im * im);
+    // from the norm, ||x|| <= 2^60.5, or the sum of the parts, below 2^60, in
+    // units of 2^(EX - 1022)
+    const float re = (float)scalbn(v0.x, 1022 - EX), im = (float)scalbn(v0.y, 1022 - EX);
+    float sum = HERM ? fmaf(re, re, im * im) : fabsf(re) + fabsf(im);
 #pragma unroll
-      for (int o = 1; o < D; o <<= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-      guard = min(max((int)floorf(7.499f - 0.5f * __log2f(n2)), 0), 8);
-    }
+    for (int o = 1; o < D; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const int guard = HERM ? min(max((int)floorf(7.499f - 0.5f * __log2f(sum)), 0), 8)
+                           : min(max((int)floorf(6.999f - __log2f(sum)), 4 - C::GUARD), 7);
     first = split2(from_double(v0.x, EX, guard), from_double(v0.y, EX, guard));
     E = EX - 1018 - guard;  // x 2^(EX - 1075 - guard)
   }
@@ -1482,7 +1488,7 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
         }
         if (b + 1 < QN / QB) load(U + sl * D * D, b + 1);
         else if (sl + 1 < n) load(U + (sl + 1) * D * D, 0);
-        constexpr int SH = HERM ? 0 : 2;
+        constexpr int SH = 60 - C::ubits(HERM);
         const long long mr = (fwd ? mpr - mnr : mpr + mnr) + ((fwd ? lpr - lnr : lpr + lnr) >> 30);
         const long long mi = (fwd ? mpi + mni : mpi - mni) + ((fwd ? lpi + lni : lpi - lni) >> 30);
         yr += ((fwd ? pr - nr : pr + nr) << SH) + shift_round(mr, 30 - SH);
@@ -1495,7 +1501,9 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
       }
       if (!HERM) {
         const uint32_t top = __reduce_max_sync(0xffffffffu, max((uint32_t)abs((int)(yr >> 32)), (uint32_t)abs((int)(yi >> 32))));
-        const int sh = __clz(top + 1) - 7 - C::GUARD;
+        // the sum of all rows' parts is below part 2^36 (the lanes hold 32 / D copies)
+        const uint32_t part = (__reduce_add_sync(0xffffffffu, ((uint32_t)abs((int)(yr >> 32)) + (uint32_t)abs((int)(yi >> 32))) >> 4) / (32 / D)) + 4 * D;
+        const int sh = max(__clz(top + 1) - 7 - C::GUARD, __clz(part) - 8);
         yr = sh >= 0 ? yr << sh : shift_round(yr, -sh);
         yi = sh >= 0 ? yi << sh : shift_round(yi, -sh);
         E = max(E + EX - 1022 - sh, -(1 << 20));

@@ -41,8 +41,8 @@ def _frechet(A, N, real):
     return X
 
 
-def _gradient(spec, u, mode, real, cplx):
-    """dF/du of the spec's one member (square fidelity) in the given types, the
+def _gradient(spec, u, mode, real, cplx, kappa=None):
+    """dF/du of the spec's one member (square fidelity; kappa = 1: the real part) in the given types, the
     overlaps times their weight, and sum |dG/d overlap|^2."""
     c = cplx(-1j) if spec.generator == "hermitian" else cplx(1)
     ctrls = [np.asarray(x).astype(cplx) for x in spec.controls]
@@ -69,7 +69,7 @@ def _gradient(spec, u, mode, real, cplx):
             X = _frechet(A[k], X @ lam, real) if mode == "exact" else X @ after
             for j in range(len(ctrls)):
                 d = 2 * c * real(spec.dt[k]) * sc * (X.T * ctrls[j]).sum()
-                G[j, k] += (np.conj(z[s]) * d).real
+                G[j, k] += (np.conj(z[s]) * d if kappa is None else kappa * d / 2).real
                 g += abs(d) ** 2
     return G, z * w, float(g)
 
@@ -187,3 +187,28 @@ def test_state_sums_of_equal_entries(pg, D):
     p.close()
     z = np.vdot(v, v + k * (1 - 1j) * (J @ v.T).T)
     assert F1 == F and abs(F / abs(z) ** 2 - 1) <= 2 * 2.0 ** 7 * (D + 40) * 2.0 ** -53
+
+
+@pytest.mark.parametrize("n_qubits,n_t", [(1, 30), (1, 167), (2, 28), (2, 99)])
+def test_dissipative_basis_states(pg, n_qubits, n_t):
+    """First-order gradients of Lindblad pulses between basis states, vectors
+    with one large part, as FP64's small components are: a step rounds each part
+    to about 2^-59 of the vector's sum and the propagators' parts to 2^-59; rms
+    2^-60.5, four times their sum over 2 n_t steps, through the vectors (real
+    overlaps: dG / dz is the gradient itself)."""
+    from pulsar_gb300 import workloads as W
+    spec, u = W.lindblad_gate(seed=n_t, n_qubits=n_qubits, n_t=n_t, n_draws=1, duration=2e-6 * n_t / 500)
+    D, d = 4 ** n_qubits, 2 ** n_qubits
+    e = np.eye(D, dtype=complex)
+    spec.target, spec.target_op, spec.fidelity = "states", None, "real"
+    spec.states_init, spec.states_target = e[:1], e[D - 1:] if n_qubits == 1 else e[d + 1:d + 2]
+    G = _gradient(spec, u, "ref_mr", np.longdouble, np.clongdouble, kappa=1)[0]
+    p = pg.Problem(**spec.problem_kwargs("ref_mr", "fp64"))
+    _, Gd = p.eval(u)
+    p.close()
+    norms = sum(np.linalg.norm(x, 2) ** 2 for x in np.asarray(spec.controls))
+    w = spec.members()[3][0]
+    tol = 4 * 2.0 ** -60.5 * np.sqrt(2 * n_t) * np.sqrt((np.asarray(spec.dt) ** 2).sum() * norms) * w + 2.0 ** -52 * _rms(G)
+    err = _rms(Gd - G)
+    print(f"{n_qubits} qubits, {n_t} slices: device error {err / _rms(G):.1e} of |G|, bar {tol / _rms(G):.1e}")
+    assert err <= tol
