@@ -75,8 +75,8 @@ TRAFFIC = {  # k_expm_oz64, 8 of 32 members: the generator read once, the df U s
            ("lindblad3q", "mixed", "expm"): 4 * 504.4e6}
 # Tensor-pipe activity of the dominant kernel from an ncu capture of a smaller
 # case: sm__pipe_tensor_cycles_active, % of peak while active.
-TENSOR_ACTIVE_PCT = {("lindblad3q", "mixed", "expm"): 19.0, ("spin4", "mixed", "expm"): 28.5,
-                     ("spin4", "fp64", "grad"): 36.2}
+TENSOR_ACTIVE_PCT = {("lindblad3q", "mixed", "expm"): 19.0, ("spin4", "mixed", "expm"): 28.4,
+                     ("spin4", "fp64", "grad"): 36.0}
 # FP32 operations one df32 complex MAC executes (error-free two_prod / two_sum
 # accumulation) per 8 FLOPs of the FP64 model: the model-FLOP rate a fully
 # busy FP32 pipe could reach on df32 work is the FP32 peak / (DF_OPS / 8).

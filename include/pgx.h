@@ -58,9 +58,18 @@ enum { PGX_GRAD_REF_GRAPE = 0,  /* first-order formula of Gradients.jl:254-291,3
        PGX_GRAD_REF_MR = 1,     /* first-order formula of GRAPEState.jl:220-230 /
                                    GRAPELindblad.jl:183-195                            */
        PGX_GRAD_EXACT = 2       /* exact Frechet-derivative gradient                    */ };
-enum { PGX_PREC_FP64 = 0,       /* plain FP64 everywhere                                */
+enum { PGX_PREC_FP64 = 0,       /* FP64 class everywhere (below)                        */
        PGX_PREC_MIXED = 1       /* df32 propagators and forward chain, FP64 overlap and
                                    objective, FP32 backward chain and gradient         */ };
+/* FP64 runs on FP64 arithmetic at padded dimensions 2, 4 and 64, in the chains
+ * and gradients of tracking problems, and beyond 24 generator terms (7 at 32).
+ * Else at 8, 16 and 32 matrices are 64-bit integers under one exponent:
+ * propagators to about 2^-57 (state targets 2^-59) of 1, chains of gates to
+ * 2^-60, gradients' sums to 2^-58 of their largest entry; and state vectors up
+ * to 32 are, to 2^-60 of their norm (2^-59 of their sum for Liouvillians).  F
+ * and G of whole problems are as close to exact as FP64 products make them or
+ * closer; a gradient many orders below |M_k| |C_j| has the absolute error of
+ * the larger, where FP64 products keep small entries to 53 bits of themselves. */
 
 /* A problem is an ensemble of members.  Member m evolves under
  *   G_m(u_k) = drifts[member_drift[m]] + member_offset[m] * offset_op

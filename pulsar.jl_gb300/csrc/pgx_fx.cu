@@ -227,9 +227,9 @@ template <int D> struct ExpmCfg {
 // D = 16).  A slice's planes and integers take 18 KB of shared memory, so an SM
 // holds ten; two warps share one, each with half the columns.
 // DF: the mixed path's propagators, df pairs with 2^-51 products.
-// 231,000 slices at d = 16: 42.5 ms as FP64 FMA products, 3.2 here (issue 60 %,
-// tensor pipe 28 %); as df products on the FP32 pipe 6.4 ms, 2.8 here.  32,000
-// at d = 32 in df: 8.1 and 3.4 ms.
+// 231,000 slices at d = 16: 42.5 ms as FP64 FMA products, 3.4 here (issue 59 %,
+// tensor pipe 33 %); as df products on the FP32 pipe 6.4 ms, 2.8 here (60 and
+// 28 %).  32,000 at d = 32 in df: 8.1 and 3.5 ms.
 template <int D, bool DF>
 __global__ void __launch_bounds__(32 * ExpmCfg<D>::TEAMS * ExpmCfg<D>::W) k_fx_expm(ProbDev p, WorkDev w, int run) {
   using C = ExpmCfg<D>;
@@ -549,9 +549,15 @@ __device__ __forceinline__ void times_prefix(const Tm<D, W>& tm, const ProbDev& 
 // slices are left to k_fx_grad_norm.
 // First order: X = M_k = R_k V_k, or with the costate that includes U_k.
 //
-// Bound: instruction issue (61 %), then the tensor pipe (36 %).  231,000 slices
+// Bound: instruction issue (60 %), then the tensor pipe (36 %).  231,000 slices
 // at d = 16: 109.7 ms as a Frechet form of FP64 FMA products, 11.7 as that form
-// in block fixed point, 9.2 here.
+// in block fixed point, 9.3 here.
+//
+// Accuracy against long double, as a part of the FMA kernels' (whose doubles keep
+// every entry to 53 bits of itself), geometric means over 50 to 200 draws each of
+// 20 to 2000 slices: four-spin gates 0.11, random gates 0.18 to 0.28 (d = 20
+// 0.5), two-qubit Lindblad gates 0.25 (below 100 slices 0.4), four-spin transfers
+// 0.45 (0.6), random transfers 0.25 to 0.5.
 template <int D>
 __global__ void __launch_bounds__(32 * SeriesCfg<D>::TEAMS * SeriesCfg<D>::W)
 k_fx_grad(ProbDev p, WorkDev w, int run, int len) {
@@ -867,9 +873,10 @@ k_fx_grad_norm(ProbDev p, WorkDev w, int run, int len) {
 //                       M_k = P_k Lambda_k = R_k V_k with V_k = V_{k+1} U_{k+1}
 // A block product is a chain of its own, so short pulses of few members fill
 // the chip too; the forward, backward and gradient products are one each.
-// Bound: the latency of a product, a few chains deep per SM.  231 members of
-// 1000 slices at d = 16: 8.1 + 16.6 ms as one FP64 chain per member, 0.90 +
-// 0.82 here; 32 members of 500 slices 2.1 + 4.4 ms, 0.14 + 0.09.
+// Bound: the latency of a product, a few chains deep per SM (issue 42 %, tensor
+// pipe 60 % with eight of them).  231 members of 1000 slices at d = 16: 8.1 + 16.6
+// ms as one FP64 chain per member, 0.75 + 0.75 here; 32 members of 500 slices 2.1
+// + 4.4 ms, 0.12 + 0.08.
 template <int D> struct ChainCfg {
   static constexpr int W = kWarps<D>;
   static constexpr int TEAMS = D >= 32 ? 1 : 4;                // (member, block) chains of a CTA, mixed path
@@ -1558,6 +1565,10 @@ __global__ void __launch_bounds__(32 * (16 + StCfg<D>::HELPERS)) k_fx_states(Pro
 // The series needs ||A|| up to about 1: the propagator kernel raises
 // w.norm_flag for an evaluation that has larger slices, which then runs the
 // CUDA-core gradient (and its chains' pairing M_k instead of N_k).
+//
+// Gradients against long double over the same draws, as a part of the FP32
+// kernels' error: gates 0.4 to 0.6 at d = 9 to 32 (Lindblad 0.37), four-spin
+// transfers 0.45, random transfers 0.99 to 1.00 (their FP32 vectors set it).
 template <int D> struct TfCfg {
   static constexpr int W = kWarps<D>;
   static constexpr int TEAMS = D >= 32 ? 1 : 4;

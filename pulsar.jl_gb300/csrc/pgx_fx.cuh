@@ -4,9 +4,10 @@
 //
 // GB300 issues 1.8 FP64 FMAs per clock and SM (measured), so a 16 x 16 complex
 // FP64 product takes 9,100 SM cycles.  Here a matrix is 64-bit integers with
-// one exponent, value = x 2^(E - 56), |x| < 0.75 2^56, and a product is a sum
-// of exact integer products (the Ozaki scheme): each factor is cut into up to
-// seven balanced 8-bit digits held as FP16, every pair of digit matrices is
+// one exponent, value = x 2^(E - 56), |x| < 0.75 2^56 (the FP64 gate chains: all
+// 64 bits, "full" below), and a product is a sum of exact integer products (the
+// Ozaki scheme): each factor is cut into up to seven (full: eight) balanced 8-bit
+// digits held as FP16, every pair of digit matrices is
 // one real-arithmetic complex product of mma.sync.m16n8k16, and the pairs
 // (i, j) of one level i + j accumulate exactly in FP32.  All seven levels of a
 // 16 x 16 product are 224 MMAs = 448 SM cycles (measured: one m16n8k16 takes 2
@@ -16,14 +17,15 @@
 // products; a warp keeps a whole unit in registers.
 //
 // Exactness.  |digit| <= 128, the leading one <= 192; at K = 32 real terms a
-// level's sum stays within 2^22, so an accumulator started at 1.5 2^23 holds
+// level's sum (eight pairs at most) stays within 2^22, so an accumulator started at 1.5 2^23 holds
 // 2^23 + integer with unit spacing: its bits minus those of 1.5 2^23 are the
 // integer.  Two levels then join in one 32-bit integer, the pairs in one
 // 64-bit integer.  Only the levels left out round: level n's largest
 // neglected sum is about 2^(0.5 - 8 n) of the factors' scale (rms).
 //
-// Every product keeps the levels that hold its absolute error near 2^-57 of
-// the result it enters, so small terms (the inner Horner steps) take few.
+// Every product of an exponential or a series keeps the levels that hold its
+// absolute error near 2^-57 (state targets 2^-59, df 2^-51) of the result it
+// enters, so small terms (the inner Horner steps) take few.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
